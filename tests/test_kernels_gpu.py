@@ -274,6 +274,36 @@ def test_gemm_nt_rows_do_not_depend_on_the_batch(ops):
     assert torch.equal(full[:70], ops.gemm_nt(a[:70].contiguous(), w))
 
 
+# rows on both sides of every border of the few-row and the tile kernels, columns and inner sizes that leave remainders
+@pytest.mark.parametrize("N,K", [(8, 4), (63, 124), (65, 128), (200, 132), (72, 640), (130, 4228), (9, 32772)])
+def test_gemm_nt_kernels_form_the_same_numbers(ops, N, K):
+    """A row's result is the same bits in the few-row kernel, in tiles of 64 and 128 rows and in the general kernel (which
+    serves operands that do not start on 16 bytes), and as exact as sums of K products in float32 can be held to: every
+    partial sum of a segment and of the segments rounds once, so at most (64 + 1 + K / 128) eps of the sum of magnitudes."""
+    M = 1200 if N >= 130 else 300
+    a, w = rnd(M, K, seed=3), rnd(N, K, seed=4)
+    full = ops.gemm_nt(a, w)
+    ref, mag = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    assert bool(((full.double() - ref).abs() <= (65 + K / 128) * 2.0 ** -24 * mag).all())
+    for m in (1, 2, 3, 4, 5, 8, 9, 31, 32, 33, 64, 65, 129):
+        assert torch.equal(full[7:7 + m], ops.gemm_nt(a[7:7 + m].contiguous(), w)), m
+    shifted = torch.empty(M * K + 1, device=DEV)[1:].view(M, K).copy_(a)
+    assert shifted.data_ptr() % 16 and torch.equal(full, ops.gemm_nt(shifted, w))
+
+
+def test_gemm_nt_few_rows_grouped(ops):
+    E, N, K, T = 6, 70, 388, 19
+    w, a = rnd(E, N, K, seed=5), rnd(T, K, seed=6)
+    expert = torch.tensor([0, 1, 1, 4, 5] * 3 + [1] * 4)
+    order = torch.argsort(expert, stable=True)
+    offsets = torch.cat([torch.zeros(1, dtype=torch.long), torch.cumsum(torch.bincount(expert, minlength=E), 0)])
+    rows, out, scale = order.to(torch.int32).to(DEV), rnd(T, N, seed=8), rnd(T, seed=9)
+    ref = out.double() + torch.stack([a[t].double() @ w[int(expert[t])].double().T * scale[t].double() for t in range(T)])
+    ops.gemm_nt(a, w, group_offsets=offsets.to(torch.int32).to(DEV), a_rows=rows, out_rows=rows, rows=T, out=out,
+                accumulate=True, row_scale=scale, scale_rows=rows)
+    assert torch.allclose(out.double(), ref, rtol=1e-5, atol=1e-4)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_gemm_nt_grouped_gather_scatter_accumulate(ops, dtype):
     E, N, K, T = 5, 70, 90, 200
