@@ -11,8 +11,8 @@
 // h reading kv head h / (nq / nkv).  Chunked and windowed visibility are not in the
 // reference; `visible_lo` in common.cuh defines them.
 //
-// The tiles start at the row's lowest visible position, which depends on the row's own
-// position only, so a row's result does not depend on how the step was cut or batched.
+// The tiles start at the row's lowest visible position (in the kernel for float32 rows below: at absolute multiples of 64
+// keys), which depends on the row's own position only, so a row's result does not depend on how the step was cut or batched.
 //
 // Three further rules, each off by default.  `kv_planes` = 1: a page holds keys only and a value is the
 // key row itself (its leading `d` elements): attention whose values are its keys, or keys and values that are
@@ -22,6 +22,7 @@
 // pos - key (distances beyond `far` read row `far`).  `softcap` > 0 bends the scaled score to softcap * tanh(s /
 // softcap) (before any bias); `sinks` [nq] adds exp(sink) of the head to the softmax's denominator.
 #include "common.cuh"
+#include "mma_sync.cuh"
 
 constexpr int ATT_THREADS = 128;
 constexpr int ATT_TILE = 128;
@@ -137,9 +138,272 @@ __global__ void paged_attention_generic_kernel(PagedAttnArgs a) {
     }
 }
 
+// float32 rows of up to 256 elements, a multiple of 4.  One CTA serves up to R query rows that read the same keys: the
+// heads of one key head times the neighbouring tokens of one request (a group: positions of the same multiple of
+// `tokens`; the group's first token leads, the CTAs of the others end at once, so a row of a decode step is a CTA of
+// its own).  Key tiles of 64 at absolute positions come into shared memory by cp.async, the next keys while the values are
+// weighted, the next values while the scores are formed; where a tile's keys lie is looked up a tile ahead, a key a thread.
+// A thread forms R / 8 rows x 4 keys of the scores (two chains over even and odd elements: one paired instruction) and R / 8
+// rows x 4 JJ elements of the sums (neighbouring elements paired).  Every number is formed by the same operations for both
+// R, so a row's bits do not depend on the launch.  Bound by the multiply-adds and the barriers between a tile's parts.
+// 980 rows of 4 requests, 8 heads on 2, head size 128: 556 -> 95 us (before: a block a row and head, one key a thread read
+// element by element); 4 decode rows at 300 keys: 69 -> 48 us.
+constexpr int AR_BK = 64, AR_THREADS = 128, AR_MAX_D = 256;
+
+typedef unsigned long long f32x2;
+__device__ __forceinline__ void fma2(f32x2& d, f32x2 a, f32x2 b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    return (f32x2)__float_as_uint(lo) | ((f32x2)__float_as_uint(hi) << 32);
+}
+__device__ __forceinline__ float lo2(f32x2 v) { return __uint_as_float((unsigned)v); }
+__device__ __forceinline__ float hi2(f32x2 v) { return __uint_as_float((unsigned)(v >> 32)); }
+
+// Floats a row takes in shared memory: an odd number of 16-byte pieces, so that neighbouring rows start in other banks.
+__host__ __device__ __forceinline__ int ar_ld(int d) { return (d / 4) % 2 ? d + 8 : d + 4; }
+
+template <int R, int JJ>
+__global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAttnArgs a, int heads_cta, int tokens) {
+    extern __shared__ __align__(16) float ar_smem[];
+    __shared__ long long off_s[2][AR_BK];                // where the keys of two tiles lie, -1: not there
+    constexpr int RT = R / 8;                            // rows a thread
+    const int d = a.d, ld = ar_ld(d), vec = d / 4;
+    float* q_s = ar_smem;                                // [R][ld]
+    float* k_s = q_s + R * ld;                           // [64][ld]
+    float* v_s = k_s + AR_BK * ld;                       // [64][ld] (keys-only pages: none)
+    float* p_s = v_s + (a.kv_planes == 2 ? AR_BK * ld : 0);   // [R][68]: scores, then probabilities
+    float* corr_s = p_s + R * (AR_BK + 4);               // [R]
+
+    const int t = blockIdx.x, pos0 = a.positions[t], req = a.row_req[t];
+    if (t > 0 && pos0 % tokens != 0 && a.row_req[t - 1] == req && a.positions[t - 1] == pos0 - 1) return;
+    int n_tok = 1;
+    while (n_tok < tokens && t + n_tok < a.T && (pos0 + n_tok) % tokens != 0 && a.row_req[t + n_tok] == req &&
+           a.positions[t + n_tok] == pos0 + n_tok)
+        ++n_tok;
+    const int G = a.nq / a.nkv, chunks = (G + heads_cta - 1) / heads_cta;
+    const int kvh = blockIdx.y / chunks, head0 = kvh * G + (blockIdx.y % chunks) * heads_cta;
+    const int heads_here = min(heads_cta, kvh * G + G - head0);
+    const int n_rows = n_tok * heads_here;               // row r: token r / heads_here, head r % heads_here
+    const int p_last = pos0 + n_tok - 1;
+    const int* table = a.block_table + (size_t)req * a.max_blocks;
+    const size_t plane = (size_t)a.nkv * a.page_size * d;
+    const float* kv = (const float*)a.kv_base;
+
+    const int keep = a.mask_kind == SHARPI_MASK_WINDOW ? a.keep_first : 0;
+    const int b_first = visible_lo(pos0, a.mask_kind, a.mask_span) / AR_BK, b_last = p_last / AR_BK;
+    const int n_keep = min((keep + AR_BK - 1) / AR_BK, b_first);   // tiles with kept positions below the others
+    const int n_iter = n_keep + b_last - b_first + 1;
+    auto key0_of = [&](int it) { return (it < n_keep ? it : b_first + it - n_keep) * AR_BK; };
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, tx = tid & 15, ty = tid >> 4;
+    auto place = [&](int it) -> long long {               // of key tid of a tile
+        const int key = key0_of(it) + tid;
+        const int page = key <= p_last ? table[key / a.page_size] : -1;
+        return page >= 0 ? (long long)page * a.kv_planes * plane + ((long long)kvh * a.page_size + key % a.page_size) * d : -1;
+    };
+    auto load = [&](float* dst, int it, size_t second) {  // a warp copies every fourth row
+#pragma unroll 4
+        for (int r = warp; r < AR_BK; r += AR_THREADS / 32) {
+            const long long off = off_s[it & 1][r];
+            const float* src = kv + (off >= 0 ? off + second : 0);
+            for (int c = lane; c < vec; c += 32) mma16::cp_async_16(dst + r * ld + c * 4, src + (off >= 0 ? c * 4 : 0), off >= 0 ? 16 : 0);
+        }
+        mma16::cp_async_commit();
+    };
+    if (tid < AR_BK) off_s[0][tid] = place(0);
+    __syncthreads();
+    load(k_s, 0, 0);
+    if (a.kv_planes == 2) load(v_s, 0, plane);
+    for (int r = warp; r < R; r += AR_THREADS / 32) {
+        const bool ok = r < n_rows;
+        const float* src = (const float*)a.q + ((size_t)(t + (ok ? r / heads_here : 0)) * a.nq + head0 + (ok ? r % heads_here : 0)) * d;
+        for (int c = lane; c < vec; c += 32)
+            *reinterpret_cast<float4*>(q_s + r * ld + c * 4) = ok ? *reinterpret_cast<const float4*>(src + c * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+
+    f32x2 acc[RT][JJ][2];
+#pragma unroll
+    for (int i = 0; i < RT; ++i)
+#pragma unroll
+        for (int j = 0; j < JJ; ++j) acc[i][j][0] = acc[i][j][1] = 0;
+    float m_run = -INFINITY, l_run = 0.0f;               // of row tid / 4 (four threads a row)
+
+    for (int it = 0; it < n_iter; ++it) {
+        const int key0 = key0_of(it);
+        const long long next = tid < AR_BK && it + 1 < n_iter ? place(it + 1) : -1;      // arrives while the scores are formed
+        if (a.kv_planes == 2) mma16::cp_async_wait<1>(); else mma16::cp_async_wait<0>();
+        __syncthreads();                                 // the keys are here (and the queries); p_s is free
+        {
+            f32x2 s[RT][4];
+#pragma unroll
+            for (int i = 0; i < RT; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) s[i][j] = 0;
+            const float* kr = k_s + tx * ld;
+            const float* qr = q_s + ty * ld;
+#pragma unroll 4
+            for (int c = 0; c < d; c += 4) {
+                ulonglong2 kk[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) kk[j] = *reinterpret_cast<const ulonglong2*>(kr + j * 16 * ld + c);
+#pragma unroll
+                for (int i = 0; i < RT; ++i) {
+                    const ulonglong2 qq = *reinterpret_cast<const ulonglong2*>(qr + i * 8 * ld + c);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) fma2(s[i][j], qq.x, kk[j].x);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) fma2(s[i][j], qq.y, kk[j].y);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < RT; ++i) {
+                const int r = ty + i * 8;
+                const int pos = pos0 + (r < n_rows ? r / heads_here : 0), h = head0 + (r < n_rows ? r % heads_here : 0);
+                const int lo = visible_lo(pos, a.mask_kind, a.mask_span);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int key = key0 + tx + 16 * j;
+                    float v = -INFINITY;
+                    if (key <= pos && (key >= lo || key < keep) && off_s[it & 1][tx + 16 * j] >= 0) {
+                        v = __fmul_rn(__fadd_rn(lo2(s[i][j]), hi2(s[i][j])), a.scale);
+                        if (a.softcap > 0.0f) v = a.softcap * tanhf(v / a.softcap);
+                        if (a.dist_bias) v += a.dist_bias[(size_t)min(pos - key, a.dist_far) * a.nq + h];
+                    }
+                    p_s[r * (AR_BK + 4) + tx + 16 * j] = v;
+                }
+            }
+        }
+        if (tid < AR_BK) off_s[(it + 1) & 1][tid] = next;
+        __syncthreads();                                 // the scores are here; keys are free
+        if (a.kv_planes == 2 && it + 1 < n_iter) load(k_s, it + 1, 0);
+        if (tid < 4 * R) {
+            float* p = p_s + (tid >> 2) * (AR_BK + 4) + (tid & 3) * 4;
+            float m = -INFINITY, l = 0.0f;
+#pragma unroll
+            for (int i = 0; i < AR_BK; i += 16)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) m = fmaxf(m, p[i + c]);
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+            m = fmaxf(m_run, fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2)));
+            const float corr = m_run == -INFINITY ? 0.0f : expf(m_run - m);
+#pragma unroll
+            for (int i = 0; i < AR_BK; i += 16)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const float v = p[i + c], e = v == -INFINITY ? 0.0f : expf(v - m);
+                    p[i + c] = e;
+                    l = __fadd_rn(l, e);
+                }
+            l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 1));
+            l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 2));
+            l_run = __fmaf_rn(l_run, corr, l);
+            m_run = m;
+            if ((tid & 3) == 0) corr_s[tid >> 2] = corr;
+        }
+        if (a.kv_planes == 2) {
+            if (it + 1 < n_iter) mma16::cp_async_wait<1>(); else mma16::cp_async_wait<0>();
+        }
+        __syncthreads();                                 // values, probabilities and corrections are here
+        {
+            f32x2 sum[RT][JJ][2];
+#pragma unroll
+            for (int i = 0; i < RT; ++i)
+#pragma unroll
+                for (int j = 0; j < JJ; ++j) sum[i][j][0] = sum[i][j][1] = 0;
+            const float* vr = (a.kv_planes == 2 ? v_s : k_s) + tx * 4;
+            const float* pr = p_s + ty * (AR_BK + 4);
+#pragma unroll 2
+            for (int k = 0; k < AR_BK; k += 4) {
+                float4 pv[RT];
+#pragma unroll
+                for (int i = 0; i < RT; ++i) pv[i] = *reinterpret_cast<const float4*>(pr + i * 8 * (AR_BK + 4) + k);
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+#pragma unroll
+                    for (int j = 0; j < JJ; ++j) {
+                        // (elements of rows of at most 64 that do not exist: what is read there is not used)
+                        if (JJ > 1 && tx * 4 + 64 * j >= d) continue;
+                        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(vr + (k + c) * ld + 64 * j);
+#pragma unroll
+                        for (int i = 0; i < RT; ++i) {
+                            const float e = c == 0 ? pv[i].x : c == 1 ? pv[i].y : c == 2 ? pv[i].z : pv[i].w;
+                            const f32x2 ee = pack2(e, e);
+                            fma2(sum[i][j][0], ee, v.x);
+                            fma2(sum[i][j][1], ee, v.y);
+                        }
+                    }
+            }
+#pragma unroll
+            for (int i = 0; i < RT; ++i) {
+                const float corr = corr_s[ty + i * 8];
+#pragma unroll
+                for (int j = 0; j < JJ; ++j)
+#pragma unroll
+                    for (int c = 0; c < 2; ++c)
+                        acc[i][j][c] = pack2(__fmaf_rn(lo2(acc[i][j][c]), corr, lo2(sum[i][j][c])),
+                                             __fmaf_rn(hi2(acc[i][j][c]), corr, hi2(sum[i][j][c])));
+            }
+        }
+        if (it + 1 < n_iter) {
+            __syncthreads();                             // the values are free
+            if (a.kv_planes == 2) load(v_s, it + 1, plane); else load(k_s, it + 1, 0);
+        }
+    }
+    __syncthreads();
+    if (tid < 4 * R && (tid & 3) == 0) {
+        float shrink = 1.0f;
+        const int r = tid >> 2, h = head0 + (r < n_rows ? r % heads_here : 0);
+        if (a.sinks) {          // the sink counts once: exp(sink - m) in the denominator, against the larger of the two
+            const float sink = a.sinks[h];
+            if (sink > m_run) {
+                shrink = expf(m_run - sink);
+                l_run = l_run * shrink + 1.0f;
+            } else {
+                l_run += expf(sink - m_run);
+            }
+        }
+        corr_s[r] = shrink / l_run;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < RT; ++i) {
+        const int r = ty + i * 8;
+        if (r >= n_rows) continue;
+        const float f = corr_s[r];
+        float* out = (float*)a.out + ((size_t)(t + r / heads_here) * a.nq + head0 + r % heads_here) * d;
+#pragma unroll
+        for (int j = 0; j < JJ; ++j) {
+            const int c = tx * 4 + 64 * j;
+            if (c < d)
+                *reinterpret_cast<float4*>(out + c) = make_float4(lo2(acc[i][j][0]) * f, hi2(acc[i][j][0]) * f,
+                                                                  lo2(acc[i][j][1]) * f, hi2(acc[i][j][1]) * f);
+        }
+    }
+}
+
+template <int R, int JJ>
+static int launch_rows_f32(const PagedAttnArgs& a, cudaStream_t stream) {
+    const int G = a.nq / a.nkv, heads_cta = G < R ? G : R, tokens = R / heads_cta;
+    const size_t smem = ((size_t)(R + (a.kv_planes == 2 ? 2 : 1) * AR_BK) * ar_ld(a.d) + R * (AR_BK + 4) + R) * sizeof(float);
+    // (the same limit whatever the size: another thread's launch, or a captured one, must not find it lowered)
+    if (cudaFuncSetAttribute(attention_rows_f32_kernel<R, JJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess)
+        return SHARPI_LAUNCH_FAILED;
+    const dim3 grid(a.T, a.nkv * ((G + heads_cta - 1) / heads_cta));
+    attention_rows_f32_kernel<R, JJ><<<grid, AR_THREADS, smem, stream>>>(a, heads_cta, tokens);
+    SHARPI_CHECK_LAUNCH();
+    return SHARPI_OK;
+}
+
+template <int R>
+static int launch_rows_f32(const PagedAttnArgs& a, cudaStream_t stream) {
+    return a.d <= 64 ? launch_rows_f32<R, 1>(a, stream) : a.d <= 128 ? launch_rows_f32<R, 2>(a, stream)
+                                                                       : launch_rows_f32<R, 4>(a, stream);
+}
+
 SHARPI_API int sharpi_paged_attention_generic(const void* q, const void* kv_base, const int* block_table,
                                               const int* row_req, const int* positions, void* out, int dtype,
-                                              int T, int nq, int nkv, int d, int max_blocks, int page_size,
+                                              int T, int B, int nq, int nkv, int d, int max_blocks, int page_size,
                                               int mask_kind, int mask_span, float scale, int kv_planes,
                                               int keep_first, const float* dist_bias, int dist_far,
                                               float softcap, const float* sinks, cudaStream_t stream) {
@@ -155,6 +419,11 @@ SHARPI_API int sharpi_paged_attention_generic(const void* q, const void* kv_base
     a.q = q; a.kv_base = kv_base; a.block_table = block_table; a.row_req = row_req; a.positions = positions;
     a.out = out; a.T = T; a.nq = nq; a.nkv = nkv; a.d = d; a.max_blocks = max_blocks; a.page_size = page_size;
     a.mask_kind = mask_kind; a.mask_span = mask_span; a.scale = scale;
+    // (16 bytes a lane: other row sizes, larger ones and bfloat16 stay with the general kernel)
+    const uintptr_t bases = (uintptr_t)q | (uintptr_t)kv_base | (uintptr_t)out;
+    if (dtype == SHARPI_F32 && d % 4 == 0 && d <= AR_MAX_D && (bases & 15) == 0)
+        // mostly one or two rows a request (decode): a CTA for 8 rows; portions of prompts: for 32
+        return T <= 2 * B ? launch_rows_f32<8>(a, stream) : launch_rows_f32<32>(a, stream);
     dim3 grid(T, nq);
     if (dtype == SHARPI_F32)
         paged_attention_generic_kernel<float><<<grid, ATT_THREADS, 0, stream>>>(a);

@@ -146,9 +146,9 @@ __global__ void __launch_bounds__(256) gemm_nt_kernel(GemmArgs g) {
 
 // float32 operands, rows on 16 bytes.  A thread has rows ty + i BM / 8 and columns tx + 16 j of the tile; a stage is 32 k of
 // the tile's rows as they lie in memory (k in front), 4 floats of padding a row, so that neighbouring rows start in other
-// banks: 12 reads of 16 bytes serve 64 paired multiply-adds.  Bound by those reads (a warp's read of 16 bytes a lane takes
-// four cycles of the SM's shared memory): 980 rows of 8192 x 1024 468 us = 35 TFLOP/s, 694 us = 24 TFLOP/s with 4 x 4 outputs a
-// thread, scalar strided loads and one multiply-add an instruction.
+// banks: 12 reads of 16 bytes serve 64 paired multiply-adds.  Bound by the multiply-adds: 37 TFLOP/s at 2048 rows of 5120 x
+// 5120, and no more with single instead of paired ones, 8 x 8 outputs a thread or another order of lanes.  980 rows of
+// 8192 x 1024: 467 us = 35 TFLOP/s; 694 us with 4 x 4 outputs a thread and scalar strided loads.
 constexpr int GT_N = 64, GT_K = 32, GT_LD = GT_K + 4, GT_STAGES = 3;
 
 template <int BM>
@@ -338,8 +338,8 @@ static int launch_few(const GemmArgs& g, cudaStream_t stream) {
     const int segs = (g.K + GB_SEG - 1) / GB_SEG, groups = (segs + 3) / 4;
     const int warps = groups < GF_MAX_WARPS ? groups : GF_MAX_WARPS, passes = (g.M + MR - 1) / MR;
     const size_t smem = ((size_t)warps * GF_STAGES * (32 + 4 * MR) * GT_LD + (size_t)MR * GF_N * segs) * sizeof(float);
-    if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(gemm_few_kernel<MR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    // (the same limit whatever the size: another thread's launch, or a captured one, must not find it lowered)
+    if (cudaFuncSetAttribute(gemm_few_kernel<MR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess)
         return SHARPI_LAUNCH_FAILED;
     gemm_few_kernel<MR><<<dim3((unsigned)((g.N + GF_N - 1) / GF_N), (unsigned)(passes * g.E)), 32 * warps, smem, stream>>>(g, passes);
     SHARPI_CHECK_LAUNCH();

@@ -34,7 +34,7 @@ SIGNATURES: Dict[str, Tuple[str, list]] = {
     "sharpi_add": ("elementwise", [P, P, P, LL, P]),
     "sharpi_timestamp": ("elementwise", [P, I, P]),
     "sharpi_qkv_post": ("rope_kv", [P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, F, F, I, I, I, P]),
-    "sharpi_paged_attention_generic": ("attention_generic", [P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, I, I, P, I, F, P, P]),
+    "sharpi_paged_attention_generic": ("attention_generic", [P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, F, I, I, P, I, F, P, P]),
     "sharpi_attention_decode": ("attention_decode", [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, F, F, P, P]),
     "sharpi_attention_keys_prefill": ("attention_keys", [P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, P, I, F, P]),
     "sharpi_attention_keys_decode": ("attention_keys", [P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, P, I, I, F, P]),

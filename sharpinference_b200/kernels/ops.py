@@ -242,7 +242,8 @@ def paged_attention_generic(q: torch.Tensor, kv_layer: torch.Tensor, block_table
             raise KernelError(f"dist_bias is {tuple(dist_bias.shape)}, expected [far + 1, {nq}]")
     check(kernel("sharpi_paged_attention_generic")(q.data_ptr(), kv_layer.data_ptr(), block_table.data_ptr(),
                                                    row_req.data_ptr(), positions.data_ptr(), out.data_ptr(),
-                                                   dtype_code(q.dtype), T, nq, nkv, d, block_table.shape[-1],
+                                                   dtype_code(q.dtype), T, block_table.numel() // max(block_table.shape[-1], 1),
+                                                   nq, nkv, d, block_table.shape[-1],
                                                    page_size, mask_kind, mask_span, float(scale),
                                                    int(kv_layer.shape[1]), int(keep_first), _ptr(dist_bias),
                                                    0 if dist_bias is None else dist_bias.shape[0] - 1,

@@ -208,6 +208,34 @@ def test_paged_attention_generic(ops, nq, nkv, d, ps, mask, dtype):
     assert torch.allclose(out.double().cpu(), ref, **tol)
 
 
+# groups of heads that divide the tile's rows and that do not, more heads than rows, row sizes at the borders of the element groups
+@pytest.mark.parametrize("nq,nkv,d", [(4, 1, 4), (10, 2, 64), (3, 3, 68), (40, 1, 128), (12, 2, 132), (8, 4, 256)])
+@pytest.mark.parametrize("mask,keep", [("full", 0), ("chunk", 0), ("window", 0), ("window", 70)])
+def test_paged_attention_float32_rows_alone_and_in_groups(ops, nq, nkv, d, mask, keep):
+    """Two requests' rows served in groups (32 query rows a CTA) are the rows served alone (8 a CTA), bit for bit, whatever
+    starts the group; and both are the statement in 64 bits: a value sum of n keys whose probabilities carry the scores'
+    absolute error (d products in two chains, times the scale) and one exponential each."""
+    lens, span, ps = [333, 97], 131, 16
+    kv, table, ks, vs = paged_setup(lens, nkv, d, ps, torch.float32, seed=d)
+    rows = [(0, p) for p in range(201, 333)] + [(1, p) for p in list(range(40, 60)) + [96]]
+    pos = torch.tensor([p for _, p in rows], dtype=torch.int32, device=DEV)
+    req = torch.tensor([b for b, _ in rows], dtype=torch.int32, device=DEV)
+    q = rnd(len(rows), nq, d, seed=11)
+    code = {"full": ops.MASK_FULL, "chunk": ops.MASK_CHUNK, "window": ops.MASK_WINDOW}[mask]
+    kw = dict(nq=nq, nkv=nkv, d=d, page_size=ps, mask_kind=code, mask_span=span, scale=d ** -0.5, keep_first=keep)
+    out = ops.paged_attention_generic(q, kv, table, req, pos, **kw)
+    for at in (0, 1, 31, 130, 132, 140, len(rows) - 1):
+        one = ops.paged_attention_generic(q[at:at + 1], kv, table, req[at:at + 1], pos[at:at + 1], **kw)
+        assert torch.equal(out[at:at + 1], one), at
+        b, p = rows[at]
+        lo = {"full": 0, "chunk": p // span * span, "window": max(0, p - span + 1)}[mask]
+        see = sorted(set(range(min(keep, lo))) | set(range(lo, p + 1)))
+        for h in range(nq):
+            k, v = ks[b][see, h // (nq // nkv)], vs[b][see, h // (nq // nkv)]
+            ref = torch.softmax((k @ q[at, h].double().cpu()) * d ** -0.5, dim=0) @ v
+            assert torch.allclose(one.view(nq, d)[h].double().cpu(), ref, rtol=1e-5, atol=1e-5), (at, h)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_attention_finds_one_far_key_among_hundreds(ops, dtype):
     """One key far back is made to match the query; its value must dominate the output.  A kernel
