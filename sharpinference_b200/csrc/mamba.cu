@@ -11,8 +11,9 @@
 //                            S[c][n] <- exp(dt[c] A[c][n]) S[c][n] + dt[c] x[c] B[n],  A = -exp(A_log)
 //                            y[c] = sum_n S[c][n] C[n] + D[c] x[c],  out = y g[c]
 //                        with dt the step sizes (after their softplus) and g the gate (after its silu),
-//                        all in float32 (exp(dt A) as exp2 of dt A log2(e)).  A group of lanes owns one channel,
-//                        each lane eight states in registers; the sum over the states is a fixed tree of exchanges,
+//                        all in float32 (exp(dt A) as exp2 of dt A log2(e)); or with dt before bias and softplus and z
+//                        before its silu, which the walk's warps then apply to every element once.  A group of lanes owns
+//                        one channel, a lane two states in registers; the sum over the states is a fixed tree of exchanges,
 //                        and the walk over a request's rows is sequential, so a row's result does not depend on how
 //                        the prompt was cut or batched.
 #include "common.cuh"
@@ -117,12 +118,13 @@ SHARPI_API int sharpi_slice_cols(const float* src, int ld, int col0, int ncols, 
 
 struct ScanArgs {
     const float* x;          // [T, C] after convolution and silu
-    const float* dtraw;      // [T, C]: the step sizes (after bias and softplus)
+    const float* dtraw;      // [T, C]: the step sizes (with dt_bias: before bias and softplus)
+    const float* dt_bias;    // [C], or null: dtraw and z are the step sizes and gates themselves
     const float* bc;         // [T, ld_bc]: B at col_b, C at col_c, N columns each
     int ld_bc, col_b, col_c;
     const float* a_log;      // [C, N]
     const float* dskip;      // [C]
-    const float* z;          // [T, ld_z]: the gate (after its silu)
+    const float* z;          // [T, ld_z]: the gate (with dt_bias: before its silu)
     int ld_z;
     const int* row_offsets;
     const int* state_slots;
@@ -132,11 +134,12 @@ struct ScanArgs {
     int C, N;
     int vec_ch, vec_bc;      // whether the channel arrays / B and C may be fetched 16 bytes at a time
     int ch;                  // rows a chunk (at most SCAN_CH; fewer when no request brings that many)
+    int alone;               // a long walk: the next kernel's blocks stay off the SMs until it ends
 };
 
-constexpr int SCAN_NPT = 8;      // states a lane keeps
 constexpr int SCAN_CH = 16;      // rows a chunk at most
-constexpr int SCAN_STAGES = 3;   // chunks in shared memory: one being walked, two on their way
+constexpr int SCAN_HELPERS = 1;  // warps that prepare for one that walks
+constexpr int SCAN_RB = 8;       // rows whose exponentials and sums are formed side by side
 
 __device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem));
@@ -149,18 +152,35 @@ template <int N> __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// A block of W warps (four, or one when that is what it takes to give every SM a block) serves CPB = W * 32 / G
-// channels of one request.  The rows' inputs arrive in shared memory
-// by cp.async, two chunks of SCAN_CH rows on their way while a third is walked: per row the block's channels of dtraw, x and z and the row's B
-// and C.  What does not depend on the state (the softplus of the step sizes, the silu of the gate) was formed over
-// all rows at once by the kernels before this one.
-template <typename TO, int G>    // G lanes a channel (a power of two): N <= 8 G
-__global__ void __launch_bounds__(128) selective_scan_kernel(ScanArgs a) {
+// A block serves CPB = warps * 32 / G channels of one request: G lanes a channel, NPT states a lane.  The rows' inputs arrive
+// in shared memory by cp.async, two chunks of SCAN_CH rows on their way while a third is walked: per row the block's
+// channels of dtraw, x and z and the row's B and C.  A warp then forms (dt, dt x) and the gate of its own channels, each
+// once.  Rows are taken SCAN_RB at a time: the states' chain is one multiply-add a row, everything else of the eight rows is
+// independent of it, and the eight rows' sums over the lanes are formed by halving exchanges (7 for 8 rows on 8 lanes), after
+// which a lane holds and stores 8 / G of them.
+//   The sum over the states: pairs of neighbouring states, then a tree over the pairs that halves their number from the
+// top (pair l with pair l + P / 2, and so on).  Lane g holds the pairs g, g + G, ...: the tree's first levels are in its
+// registers, the others exchanges, and the additions are the same for every NPT and G.
+//   Few states a lane where a prompt is alone (its rows can only be walked, and nothing hides a row's latency but other
+// warps: 4096 channels of 16 states are 1024 warps with two states a lane, 256 with eight); eight where there are warps
+// enough, because a lane's share of a row (its inputs from shared memory, the exchanges) is the same for two states.
+//   SPLIT (few states a lane): half of the block's warps walk, the others fetch and prepare the next chunk meanwhile;
+// otherwise a warp prepares its chunk before it walks it.
+// One prompt of 2048 rows of 4096 channels x 16 states, softplus, silu and all: 354 + 36 us with eight states a lane, row by row,
+// and softplus in a kernel of its own; 230 two states a lane; 177 with walkers and helpers; 152 with the fetching
+// in the helpers too (157 with two helpers a walker).  What bounds it is the chain of a chunk (reads, exponentials, sums, barrier)
+// at three to four warps a scheduler: 62 % of the issue slots.
+template <typename TO, int NPT, int G, bool SPLIT>
+__global__ void __launch_bounds__(SPLIT ? 64 * (1 + SCAN_HELPERS) : 128) selective_scan_kernel(ScanArgs a) {
+    constexpr int SCAN_STAGES = SPLIT ? 4 : 3;         // chunks in shared memory: walked, (prepared,) two on their way
     extern __shared__ __align__(16) float sm[];
-    pdl_wait();
-    constexpr int CPW = 32 / G;
-    const int CPB = (blockDim.x >> 5) * CPW;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (a.alone) pdl_wait_only(); else pdl_wait();
+    constexpr int CPW = 32 / G, NP = G * NPT;
+    const int warps = (blockDim.x >> 5) / (SPLIT ? 1 + SCAN_HELPERS : 1), CPB = warps * CPW;
+    const int lane = threadIdx.x & 31;
+    const bool helper = SPLIT && (int)(threadIdx.x >> 5) >= warps;
+    const int warp = (int)(threadIdx.x >> 5) % warps;          // a helper prepares rows of the same channels as this walker
+    const int part = helper ? (int)(threadIdx.x >> 5) / warps - 1 : 0, parts = helper ? SCAN_HELPERS : 1;
     const int sub = lane % G;
     const int cl = warp * CPW + lane / G;              // channel within the block
     const int c0 = blockIdx.x * CPB;
@@ -168,70 +188,71 @@ __global__ void __launch_bounds__(128) selective_scan_kernel(ScanArgs a) {
     const int c = live ? c0 + cl : a.C - 1;
     const int b = blockIdx.y;
     const int first = a.row_offsets[b], end = a.row_offsets[b + 1];
-    const int N = a.N, n0 = sub * SCAN_NPT, NP = G * SCAN_NPT;
-    // one buffer: [CH][4][CPB] (dt | dt x | D x | gate) then [CH][2][NP] (B | C)
-    const int CH = a.ch;
-    const int buf_floats = CH * (4 * CPB + 2 * NP);
+    const int N = a.N;
+    auto n_of = [&](int i) { return 2 * (sub + (i >> 1) * G) + (i & 1); };      // the state behind register i
+    // one buffer: [CH] rows of dt | x | gate [CPB each], (dt, dt x) [CPB pairs], B | C [NP each]
+    const int CH = a.ch, stride = 5 * CPB + 2 * NP, buf_floats = CH * stride;
+    const bool raw = a.dt_bias != nullptr;
     float* S_g = a.state + (size_t)a.state_slots[b] * a.state_stride + (size_t)c * N;
-    float S[SCAN_NPT], A[SCAN_NPT];
-    const bool vec = (N % 4 == 0) && ((reinterpret_cast<uintptr_t>(S_g) & 15) == 0);
+    float S[NPT], A[NPT];
+    const bool vec = NPT % 2 == 0 && N % 2 == 0 && (reinterpret_cast<uintptr_t>(S_g) & 7) == 0;
     if (vec) {
 #pragma unroll
-        for (int i = 0; i < SCAN_NPT; i += 4) {
-            float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (n0 + i < N) v = *reinterpret_cast<const float4*>(S_g + n0 + i);
-            S[i] = v.x; S[i + 1] = v.y; S[i + 2] = v.z; S[i + 3] = v.w;
+        for (int i = 0; i < NPT; i += 2) {
+            float2 v = make_float2(0.0f, 0.0f);
+            if (n_of(i) < N) v = *reinterpret_cast<const float2*>(S_g + n_of(i));
+            S[i] = v.x; S[i + 1] = v.y;
         }
     } else {
 #pragma unroll
-        for (int i = 0; i < SCAN_NPT; ++i) S[i] = n0 + i < N ? S_g[n0 + i] : 0.0f;
+        for (int i = 0; i < NPT; ++i) S[i] = n_of(i) < N ? S_g[n_of(i)] : 0.0f;
     }
 #pragma unroll
-    for (int i = 0; i < SCAN_NPT; ++i)
-        A[i] = n0 + i < N ? -expf(a.a_log[(size_t)c * N + n0 + i]) * 1.4426950408889634f : 0.0f;
-    // states beyond N stay zero in both buffers' B and C
+    for (int i = 0; i < NPT; ++i)
+        A[i] = n_of(i) < N ? -expf(a.a_log[(size_t)c * N + n_of(i)]) * 1.4426950408889634f : 0.0f;
+    // states beyond N stay zero in every buffer's B and C
     if (NP != N) for (int i = threadIdx.x; i < SCAN_STAGES * buf_floats; i += blockDim.x) {
-        const int within = i % buf_floats, row_part = within % (4 * CPB + 2 * NP);
-        if (row_part >= 4 * CPB && (row_part - 4 * CPB) % NP >= N) sm[i] = 0.0f;
+        const int part = i % buf_floats % stride;
+        if (part >= 5 * CPB && (part - 5 * CPB) % NP >= N) sm[i] = 0.0f;
     }
     const int live_ch = min(CPB, a.C - c0);
+    const int fetcher = threadIdx.x - (SPLIT ? warps * 32 : 0), fetchers = blockDim.x - (SPLIT ? warps * 32 : 0);
     auto fetch = [&](int t0, int buf) {
         const int rows = max(0, min(CH, end - t0));           // none: an empty group keeps the count of groups even
         float* base = sm + buf * buf_floats;
-        const int stride = 4 * CPB + 2 * NP;
         if (a.vec_ch) {
             const int q = live_ch >> 2;
-            for (int i = threadIdx.x; i < rows * q; i += blockDim.x) {
+            for (int i = fetcher; i < rows * q; i += fetchers) {
                 const int tt = i / q, ch = (i % q) * 4;
                 float* row = base + tt * stride;
                 const size_t t = (size_t)(t0 + tt);
                 cp_async16(row + ch, a.dtraw + t * a.C + c0 + ch);
                 cp_async16(row + CPB + ch, a.x + t * a.C + c0 + ch);
-                cp_async16(row + 3 * CPB + ch, a.z + t * a.ld_z + c0 + ch);
+                cp_async16(row + 2 * CPB + ch, a.z + t * a.ld_z + c0 + ch);
             }
         } else {
-            for (int i = threadIdx.x; i < rows * live_ch; i += blockDim.x) {
+            for (int i = fetcher; i < rows * live_ch; i += fetchers) {
                 const int tt = i / live_ch, ch = i % live_ch;
                 float* row = base + tt * stride;
                 const size_t t = (size_t)(t0 + tt);
                 cp_async4(row + ch, a.dtraw + t * a.C + c0 + ch);
                 cp_async4(row + CPB + ch, a.x + t * a.C + c0 + ch);
-                cp_async4(row + 3 * CPB + ch, a.z + t * a.ld_z + c0 + ch);
+                cp_async4(row + 2 * CPB + ch, a.z + t * a.ld_z + c0 + ch);
             }
         }
         if (a.vec_bc) {
             const int q = N >> 2;
-            for (int i = threadIdx.x; i < rows * q; i += blockDim.x) {
+            for (int i = fetcher; i < rows * q; i += fetchers) {
                 const int tt = i / q, n = (i % q) * 4;
-                float* row = base + tt * stride + 4 * CPB;
+                float* row = base + tt * stride + 5 * CPB;
                 const float* src = a.bc + (size_t)(t0 + tt) * a.ld_bc;
                 cp_async16(row + n, src + a.col_b + n);
                 cp_async16(row + NP + n, src + a.col_c + n);
             }
         } else {
-            for (int i = threadIdx.x; i < rows * N; i += blockDim.x) {
+            for (int i = fetcher; i < rows * N; i += fetchers) {
                 const int tt = i / N, n = i % N;
-                float* row = base + tt * stride + 4 * CPB;
+                float* row = base + tt * stride + 5 * CPB;
                 const float* src = a.bc + (size_t)(t0 + tt) * a.ld_bc;
                 cp_async4(row + n, src + a.col_b + n);
                 cp_async4(row + NP + n, src + a.col_c + n);
@@ -239,83 +260,178 @@ __global__ void __launch_bounds__(128) selective_scan_kernel(ScanArgs a) {
         }
         cp_async_commit();
     };
-    fetch(first, 0);
-    fetch(first + CH, 1);
+    const float dsk = a.dskip[c];
+    const int pc = warp * CPW + lane % CPW, ptt = lane / CPW;              // channel and row this lane prepares
+    const float bias = raw && c0 + pc < a.C ? a.dt_bias[c0 + pc] : 0.0f;
+    auto prepare = [&](int t0, int buf) {                     // the warp's channels of a chunk, an element a lane
+        const int rows = min(CH, end - t0);
+        float* base = sm + buf * buf_floats;
+        for (int tt = ptt + part * G; tt < rows; tt += parts * G) {
+            float* row = base + tt * stride;
+            float dt = row[pc];
+            if (raw) {
+                const float v = dt + bias;
+                dt = v > 20.0f ? v : log1pf(expf(v));
+                row[2 * CPB + pc] = silu_f(row[2 * CPB + pc]);
+            }
+            *reinterpret_cast<float2*>(row + 3 * CPB + 2 * pc) = make_float2(dt, dt * row[CPB + pc]);
+        }
+    };
+#pragma unroll
+    for (int i = 0; i < SCAN_STAGES - 1; ++i)
+        if (!SPLIT || helper) fetch(first + i * CH, i);
+    if (SPLIT) {
+        cp_async_wait<SCAN_STAGES - 2>();
+        __syncthreads();
+        if (helper) prepare(first, 0);
+    }
     int buf = 0;
     for (int t0 = first; t0 < end; t0 += CH, buf = (buf + 1) % SCAN_STAGES) {
         const int rows = min(CH, end - t0);
-        cp_async_wait<1>();       // all but the newest group: this chunk is here
-        __syncthreads();          // ... for everyone, and everyone has left the chunk before
-        fetch(t0 + 2 * CH, (buf + 2) % SCAN_STAGES);         // two chunks ahead, into the buffer of the chunk before
-        const float* base = sm + buf * buf_floats;
-        const float dsk = a.dskip[c];
-#pragma unroll 1
-        for (int tt = 0; tt < rows; ++tt) {
-            const float* row = base + tt * (4 * CPB + 2 * NP);
-            const float dt = row[cl], xv = row[CPB + cl], dtx = dt * xv;
-            const float4* B4 = reinterpret_cast<const float4*>(row + 4 * CPB + n0);
-            const float4* C4 = reinterpret_cast<const float4*>(row + 4 * CPB + NP + n0);
-            float acc = 0.0f;
-#pragma unroll
-            for (int i = 0; i < SCAN_NPT / 4; ++i) {
-                const float4 Bv = B4[i], Cv = C4[i];
-                S[4 * i] = fmaf(ex2_approx(dt * A[4 * i]), S[4 * i], dtx * Bv.x);             acc = fmaf(S[4 * i], Cv.x, acc);
-                S[4 * i + 1] = fmaf(ex2_approx(dt * A[4 * i + 1]), S[4 * i + 1], dtx * Bv.y); acc = fmaf(S[4 * i + 1], Cv.y, acc);
-                S[4 * i + 2] = fmaf(ex2_approx(dt * A[4 * i + 2]), S[4 * i + 2], dtx * Bv.z); acc = fmaf(S[4 * i + 2], Cv.z, acc);
-                S[4 * i + 3] = fmaf(ex2_approx(dt * A[4 * i + 3]), S[4 * i + 3], dtx * Bv.w); acc = fmaf(S[4 * i + 3], Cv.w, acc);
+        cp_async_wait<1>();       // all but the newest group: this chunk (SPLIT: and the next one) is here
+        __syncthreads();          // ... for everyone, prepared, and everyone has left the chunk before
+        if (!SPLIT || helper)         // into the buffer of the chunk before
+            fetch(t0 + (SCAN_STAGES - 1) * CH, (buf + SCAN_STAGES - 1) % SCAN_STAGES);
+        if (SPLIT) {
+            if (helper) {
+                prepare(t0 + CH, (buf + 1) % SCAN_STAGES);
+                continue;
             }
+        } else {
+            prepare(t0, buf);
+            __syncwarp();
+        }
+        const float* base = sm + buf * buf_floats;
+        // RB rows: everything that does not hang on the states first, then their chain; acc: the lane's parts of the sums
+        auto walk = [&](const float* row, auto& acc) {
+            constexpr int RB = sizeof(acc) / sizeof(float);
+            float2 d[RB], B[RB][NPT / 2], Cn[RB][NPT / 2];
 #pragma unroll
-            for (int o = G >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-            if (live && sub == 0)
-                ((TO*)a.out)[(size_t)(t0 + tt) * a.C + c] = from_float<TO>(fmaf(dsk, xv, acc) * row[3 * CPB + cl]);
+            for (int r = 0; r < RB; ++r) {
+                d[r] = *reinterpret_cast<const float2*>(row + r * stride + 3 * CPB + 2 * cl);
+                const float* Br = row + r * stride + 5 * CPB + 2 * sub;
+#pragma unroll
+                for (int i = 0; i < NPT / 2; ++i) {
+                    B[r][i] = *reinterpret_cast<const float2*>(Br + 2 * i * G);
+                    Cn[r][i] = *reinterpret_cast<const float2*>(Br + NP + 2 * i * G);
+                }
+            }
+            float e[RB][NPT];
+#pragma unroll
+            for (int r = 0; r < RB; ++r)
+#pragma unroll
+                for (int i = 0; i < NPT; ++i) e[r][i] = ex2_approx(d[r].x * A[i]);
+#pragma unroll
+            for (int r = 0; r < RB; ++r) {
+                float p[NPT / 2];
+#pragma unroll
+                for (int i = 0; i < NPT / 2; ++i) {
+                    S[2 * i] = fmaf(e[r][2 * i], S[2 * i], d[r].y * B[r][i].x);
+                    S[2 * i + 1] = fmaf(e[r][2 * i + 1], S[2 * i + 1], d[r].y * B[r][i].y);
+                    p[i] = fmaf(S[2 * i + 1], Cn[r][i].y, __fmul_rn(S[2 * i], Cn[r][i].x));
+                }
+#pragma unroll
+                for (int o = NPT / 4; o > 0; o >>= 1)
+#pragma unroll
+                    for (int i = 0; i < o; ++i) p[i] += p[i + o];
+                acc[r] = p[0];
+            }
+        };
+        auto store = [&](int tt, float sum) {
+            const float* row = base + tt * stride;
+            ((TO*)a.out)[(size_t)(t0 + tt) * a.C + c] = from_float<TO>(fmaf(dsk, row[CPB + cl], sum) * row[2 * CPB + cl]);
+        };
+        int tt = 0;
+        if (G <= SCAN_RB) {
+            for (; tt + SCAN_RB <= rows; tt += SCAN_RB) {
+                float acc[SCAN_RB];
+                constexpr int RB = NPT <= 4 ? SCAN_RB : 2;      // (what the registers hold)
+#pragma unroll
+                for (int r = 0; r < SCAN_RB; r += RB) walk(base + (tt + r) * stride, *reinterpret_cast<float(*)[RB]>(acc + r));
+                int held = 0;                                  // the first row this lane still holds
+#pragma unroll
+                for (int o = G / 2, n = SCAN_RB / 2; o > 0; o >>= 1, n >>= 1) {
+                    const bool upper = sub & o;
+                    held += upper ? n : 0;
+#pragma unroll
+                    for (int j = 0; j < n; ++j) {
+                        const float send = upper ? acc[j] : acc[j + n], keep = upper ? acc[j + n] : acc[j];
+                        acc[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                    }
+                }
+                if (live)
+#pragma unroll
+                    for (int j = 0; j < (G <= SCAN_RB ? SCAN_RB / G : 1); ++j) store(tt + held + j, acc[j]);
+            }
+        }
+        for (; tt < rows; ++tt) {
+            float acc[1];
+            walk(base + tt * stride, acc);
+#pragma unroll
+            for (int o = G >> 1; o > 0; o >>= 1) acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+            if (live && sub == 0) store(tt, acc[0]);
         }
     }
-    if (live) {
+    if (live && !helper) {
         if (vec) {
 #pragma unroll
-            for (int i = 0; i < SCAN_NPT; i += 4)
-                if (n0 + i < N) *reinterpret_cast<float4*>(S_g + n0 + i) = make_float4(S[i], S[i + 1], S[i + 2], S[i + 3]);
+            for (int i = 0; i < NPT; i += 2)
+                if (n_of(i) < N) *reinterpret_cast<float2*>(S_g + n_of(i)) = make_float2(S[i], S[i + 1]);
         } else {
 #pragma unroll
-            for (int i = 0; i < SCAN_NPT; ++i)
-                if (n0 + i < N) S_g[n0 + i] = S[i];
+            for (int i = 0; i < NPT; ++i)
+                if (n_of(i) < N) S_g[n_of(i)] = S[i];
         }
     }
 }
 
-template <typename TO>
+template <typename TO, int NPT, int G, bool SPLIT = false>
 static int launch_scan(ScanArgs a, int B, int T, cudaStream_t stream) {
-    int G = 1;
-    while (G * SCAN_NPT < a.N) G <<= 1;
-    if (G > 32) return SHARPI_BAD_ARGUMENT;
-    int warps = 4;
-    if ((long long)((a.C + 4 * (32 / G) - 1) / (4 * (32 / G))) * B < 296) warps = 1;     // too few blocks for 148 SMs
+    // two walking warps a block spread a single prompt's channels evenly over the SMs; otherwise four
+    const int warps = SPLIT ? 2 : 4;
     const int cpb = warps * (32 / G);
     const dim3 grid((a.C + cpb - 1) / cpb, B);
-    a.ch = T - B + 1 < SCAN_CH ? (T - B + 1 < 1 ? 1 : T - B + 1) : SCAN_CH;    // no request brings more rows than T - B + 1
-    const size_t smem = (size_t)SCAN_STAGES * a.ch * (4 * cpb + 2 * G * SCAN_NPT) * sizeof(float);
+    const int most = T - B + 1 < 1 ? 1 : T - B + 1;                  // no request brings more rows
+    a.ch = most < SCAN_CH ? most : SCAN_CH;
+    a.alone = most > SCAN_CH;
+    const size_t smem = (size_t)(SPLIT ? 4 : 3) * a.ch * (5 * cpb + 2 * G * NPT) * sizeof(float);
     const uintptr_t chp = reinterpret_cast<uintptr_t>(a.dtraw) | reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.z);
     a.vec_ch = (a.C % 4 == 0 && cpb % 4 == 0 && a.ld_z % 4 == 0 && (chp & 15) == 0) ? 1 : 0;
-    a.vec_bc = (a.N % 4 == 0 && a.col_b % 4 == 0 && a.col_c % 4 == 0 && a.ld_bc % 4 == 0 &&
+    a.vec_bc = (a.N % 4 == 0 && cpb % 4 == 0 && a.col_b % 4 == 0 && a.col_c % 4 == 0 && a.ld_bc % 4 == 0 &&
                 (reinterpret_cast<uintptr_t>(a.bc) & 15) == 0) ? 1 : 0;
-#define SCAN_CASE(GG)                                                                                          \
-    case GG: {                                                                                                 \
-        auto kern = selective_scan_kernel<TO, GG>;                                                             \
-        if (smem > 48 * 1024 &&                                                                                \
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) \
-            return SHARPI_LAUNCH_FAILED;                                                                       \
-        SHARPI_LAUNCH_PDL(kern, grid, warps * 32, smem, stream, a);                                            \
-        break;                                                                                                 \
+    auto kern = selective_scan_kernel<TO, NPT, G, SPLIT>;
+    // (the same limit whatever the size: another thread's launch must not find it lowered)
+    if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess)
+        return SHARPI_LAUNCH_FAILED;
+    if (a.alone) {
+        kern<<<grid, warps * (SPLIT ? 32 * (1 + SCAN_HELPERS) : 32), smem, stream>>>(a);
+        SHARPI_CHECK_LAUNCH();
+    } else {
+        SHARPI_LAUNCH_PDL(kern, grid, warps * (SPLIT ? 32 * (1 + SCAN_HELPERS) : 32), smem, stream, a);
     }
-    switch (G) {
-        SCAN_CASE(1) SCAN_CASE(2) SCAN_CASE(4) SCAN_CASE(8) SCAN_CASE(16) SCAN_CASE(32)
-        default: return SHARPI_BAD_ARGUMENT;
-    }
-#undef SCAN_CASE
     return SHARPI_OK;
 }
 
-SHARPI_API int sharpi_selective_scan(const float* x, const float* dtraw, const float* bc,
+template <typename TO>
+static int launch_scan(const ScanArgs& a, int B, int T, cudaStream_t stream) {
+    const int NP = a.N <= 4 ? 4 : a.N <= 8 ? 8 : a.N <= 16 ? 16 : a.N <= 32 ? 32 : a.N <= 64 ? 64 : a.N <= 128 ? 128 : 256;
+    // Rows to walk and fewer warps (of eight states a lane) than schedulers: two states a lane.  us, two split / four / eight
+    // states a lane, 4096 channels of 16 states: one prompt of 2048 rows 152 / 296 / 455; two of 1024 133 / 165 / 230; three of
+    // 683 140 / 126 / 173; eight of 2048 909 / 765 / 1015.  Single rows (the state streams through): 200 requests 240 / 63 / 45.
+    const bool walk = T - B + 1 > SCAN_CH;
+    const bool few = walk && (long long)a.C * B * NP / (8 * 32) < 4 * 148;
+    switch (NP) {
+        case 4: return few ? launch_scan<TO, 2, 2, true>(a, B, T, stream) : launch_scan<TO, 4, 1>(a, B, T, stream);
+        case 8: return few ? launch_scan<TO, 2, 4, true>(a, B, T, stream) : launch_scan<TO, 8, 1>(a, B, T, stream);
+        case 16: return few ? launch_scan<TO, 2, 8, true>(a, B, T, stream) : walk ? launch_scan<TO, 4, 4>(a, B, T, stream) : launch_scan<TO, 8, 2>(a, B, T, stream);
+        case 32: return few ? launch_scan<TO, 2, 16, true>(a, B, T, stream) : launch_scan<TO, 8, 4>(a, B, T, stream);
+        case 64: return few ? launch_scan<TO, 2, 32, true>(a, B, T, stream) : launch_scan<TO, 8, 8>(a, B, T, stream);
+        case 128: return few ? launch_scan<TO, 4, 32, true>(a, B, T, stream) : launch_scan<TO, 8, 16>(a, B, T, stream);
+        default: return launch_scan<TO, 8, 32>(a, B, T, stream);
+    }
+}
+
+SHARPI_API int sharpi_selective_scan(const float* x, const float* dtraw, const float* dt_bias, const float* bc,
                                      int ld_bc, int col_b, int col_c, const float* a_log, const float* dskip,
                                      const float* z, int ld_z, const int* row_offsets, const int* state_slots,
                                      float* state, long long state_stride, void* out, int out_dtype, int T, int B,
@@ -323,7 +439,7 @@ SHARPI_API int sharpi_selective_scan(const float* x, const float* dtraw, const f
     if (B <= 0) return SHARPI_OK;
     if (C <= 0 || N <= 0 || N > 256) return SHARPI_BAD_ARGUMENT;
     ScanArgs a;
-    a.x = x; a.dtraw = dtraw; a.bc = bc; a.ld_bc = ld_bc; a.col_b = col_b; a.col_c = col_c;
+    a.x = x; a.dtraw = dtraw; a.dt_bias = dt_bias; a.bc = bc; a.ld_bc = ld_bc; a.col_b = col_b; a.col_c = col_c;
     a.a_log = a_log; a.dskip = dskip; a.z = z; a.ld_z = ld_z; a.row_offsets = row_offsets; a.state_slots = state_slots;
     a.state = state; a.state_stride = state_stride; a.out = out; a.C = C; a.N = N;
     if (out_dtype == SHARPI_F32) return launch_scan<float>(a, B, T, stream);

@@ -1174,10 +1174,15 @@ def slice_cols(src: torch.Tensor, col0: int, ncols: int, out_dtype: torch.dtype)
 def selective_scan(x: torch.Tensor, dt: torch.Tensor, bc: torch.Tensor, col_b: int,
                    col_c: int, a_log: torch.Tensor, dskip: torch.Tensor, xz: torch.Tensor, col_z: int, *,
                    row_offsets: torch.Tensor, state_slots: torch.Tensor, state: torch.Tensor,
-                   out_dtype: torch.dtype) -> torch.Tensor:
+                   out_dtype: torch.dtype, dt_bias: Optional[torch.Tensor] = None) -> torch.Tensor:
     """The selective scan over the rows of every request from and into ``state [slots, channels * states]``:
     ``(S C + D x) * g`` in ``out_dtype``, with ``dt`` the step sizes themselves (after their softplus) and ``g`` the
-    gate (already ``silu(z)``) in the columns of ``xz`` from ``col_z``."""
+    gate (already ``silu(z)``) in the columns of ``xz`` from ``col_z``.  With ``dt_bias [channels]`` both come raw: the
+    step sizes are ``softplus(dt + dt_bias)`` and the gate ``silu`` of those columns."""
+    if dt_bias is not None:
+        _need(dt_bias, "dt_bias", torch.float32)
+        if dt_bias.numel() != x.shape[1]:
+            raise KernelError(f"dt_bias has {dt_bias.numel()} entries for {x.shape[1]} channels")
     for name, t in (("x", x), ("dt", dt), ("bc", bc), ("a_log", a_log), ("dskip", dskip),
                     ("xz", xz), ("state", state)):
         _need(t, name, torch.float32)
@@ -1189,7 +1194,7 @@ def selective_scan(x: torch.Tensor, dt: torch.Tensor, bc: torch.Tensor, col_b: i
         raise KernelError("the gate's columns lie outside the fused projection")
     out = torch.empty((T, C), dtype=out_dtype, device=x.device)
     z = xz[:, col_z:]
-    check(kernel("sharpi_selective_scan")(x.data_ptr(), dt.data_ptr(), bc.data_ptr(),
+    check(kernel("sharpi_selective_scan")(x.data_ptr(), dt.data_ptr(), _ptr(dt_bias), bc.data_ptr(),
                                           bc.shape[1], col_b, col_c, a_log.data_ptr(), dskip.data_ptr(), z.data_ptr(),
                                           xz.shape[1], row_offsets.data_ptr(), state_slots.data_ptr(), state.data_ptr(),
                                           state.stride(0), out.data_ptr(), dtype_code(out_dtype), T, state_slots.numel(),

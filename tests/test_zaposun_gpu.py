@@ -286,6 +286,33 @@ def test_convolution_and_selective_scan_kernels(C, N, R, taps):
         assert float((scan_state[slot].double().cpu().view(C, N) - want[b][2]).abs().max()) < 3e-5 * max(1.0, float(want[b][2].abs().max()))
 
 
+@pytest.mark.parametrize("C,N", [(12, 16), (40, 9), (37, 16), (6, 3), (9, 48), (5, 100), (3, 250)])
+def test_selective_scan_raw_inputs_and_cuts(C, N):
+    """Raw step sizes and gates give what the kernels for softplus and silu before the walk give (the same functions of the
+    same numbers: the same bits), and a prompt in one step the bits of the same prompt in portions (groups of eight rows,
+    rows that are left, chunks of sixteen)."""
+    from sharpinference_b200.kernels import ops
+    g = torch.Generator().manual_seed(C + N)
+    T, R = 53, 4
+    f = lambda *s: torch.randn(*s, generator=g).to(DEV)
+    x, dt, bc, z, bias, dsk = f(T, C), f(T, C), f(T, R + 2 * N), f(T, C), f(C), f(C)
+    a_log = (-2.0 + 2.0 * torch.rand(C, N, generator=g)).to(DEV)
+    run = lambda rows, state, **kw: ops.selective_scan(x[rows].contiguous(), kw.pop("dt", dt)[rows].contiguous(), bc[rows].contiguous(),
+                                                       R, R + N, a_log, dsk, kw.pop("z", z)[rows].contiguous(), 0,
+                                                       row_offsets=_step_meta([rows.stop - rows.start], [0])[1],
+                                                       state_slots=_step_meta([1], [0])[2], state=state, out_dtype=torch.float32, **kw)
+    s_whole, s_cut, s_given = (torch.zeros(1, C * N, device=DEV) for _ in range(3))
+    whole = run(slice(0, T), s_whole, dt_bias=bias)
+    at, parts = 0, []
+    for n in (1, 8, 3, 17, 24):
+        parts.append(run(slice(at, at + n), s_cut, dt_bias=bias))
+        at += n
+    assert at == T and torch.equal(torch.cat(parts), whole) and torch.equal(s_cut, s_whole)
+    given = run(slice(0, T), s_given, dt=ops.bias_act(dt, bias, ops.ACT_SOFTPLUS, torch.float32),
+                z=ops.bias_act(z, None, ops.ACT_SILU, torch.float32))
+    assert torch.equal(given, whole) and torch.equal(s_given, s_whole)
+
+
 @pytest.mark.parametrize("layout", ["halves", "interleaved"])
 @pytest.mark.parametrize("nq,nkv,dk,dv,rot", [(4, 2, 16, 32, 8), (2, 1, 64, 64, 64), (3, 3, 24, 10, 0), (1, 1, 2, 2, 2)])
 def test_rotation_with_norm_first_and_rotated_values(layout, nq, nkv, dk, dv, rot):
