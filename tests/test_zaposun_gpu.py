@@ -286,6 +286,27 @@ def test_convolution_and_selective_scan_kernels(C, N, R, taps):
         assert float((scan_state[slot].double().cpu().view(C, N) - want[b][2]).abs().max()) < 3e-5 * max(1.0, float(want[b][2].abs().max()))
 
 
+@pytest.mark.parametrize("taps", [1, 2, 3, 4])
+@pytest.mark.parametrize("C,dtype", [(6000, torch.bfloat16), (5620, torch.float32), (5120, torch.bfloat16)])
+def test_causal_convolution_rows_at_a_time(taps, C, dtype):
+    """Portions shorter than the window and longer, that start anywhere in a group of eight rows: outputs, state and gate are
+    the bits that the kernel for a channel a thread forms (which an odd leading size selects)."""
+    from sharpinference_b200.kernels import ops
+    g = torch.Generator().manual_seed(C + taps)
+    lens = [1, 2, 3, 9, 40, 1, 16, 7, 70] if C > 5120 else [3, 140, 1, 33]
+    T, B = sum(lens), len(lens)
+    rr, off, sl = _step_meta(lens, list(range(B))[::-1])
+    w, b = (torch.randn(C, taps, generator=g) * 0.5).to(DEV), torch.randn(C, generator=g).to(DEV)
+    xz = torch.randn(T, 2 * C, generator=g).to(DEV)
+    state = torch.randn(B, max(taps - 1, 1) * C, generator=g).to(DEV)
+    odd = torch.cat([xz, xz[:, :1]], dim=1)
+    s_a, s_b = state.clone(), state.clone()
+    kw = dict(row_request=rr, row_offsets=off, state_slots=sl, act_dtype=dtype, gate_col=C)
+    x_a, act_a = ops.causal_conv(xz, C, w, b, s_a, **kw)
+    x_b, act_b = ops.causal_conv(odd, C, w, b, s_b, **kw)
+    assert torch.equal(x_a, x_b) and torch.equal(act_a, act_b) and torch.equal(s_a, s_b) and torch.equal(xz, odd[:, :-1])
+
+
 @pytest.mark.parametrize("C,N", [(12, 16), (40, 9), (37, 16), (6, 3), (9, 48), (5, 100), (3, 250)])
 def test_selective_scan_raw_inputs_and_cuts(C, N):
     """Raw step sizes and gates give what the kernels for softplus and silu before the walk give (the same functions of the
