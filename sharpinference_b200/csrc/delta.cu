@@ -411,23 +411,6 @@ __device__ __forceinline__ float transpose_sum32(float (&acc)[32], int lane) {
     return acc[0];
 }
 
-// Two neighbouring elements in three bfloat16 pieces each (24 bits together), packed as an operand register.
-struct Pieces {
-    uint32_t v[3];
-};
-__device__ __forceinline__ Pieces split3(float x, float y) {
-    Pieces r;
-#pragma unroll
-    for (int p = 0; p < 3; ++p) {
-        r.v[p] = mma16::pack_bf16(x, y);
-        if (p < 2) {
-            x -= __uint_as_float(r.v[p] << 16);
-            y -= __uint_as_float(r.v[p] & 0xffff0000u);
-        }
-    }
-    return r;
-}
-
 // The operands of the tensor-core walk in the order in which its lanes (g = lane / 4, t = lane % 4) take them, 16 bytes each.
 // Of the 32 rows -W | D q - B W, per 16 key channels, piece and pair of row tiles: words (tile 0: channels 2t, 2t + 1 of
 // row g | the same 8 further | tile 1 likewise); of the decayed keys, per 16 key channels and piece: (channel g: rows 2t,
@@ -556,7 +539,7 @@ __global__ void __launch_bounds__(DC_THREADS, SPLIT ? 3 : 2) delta_chunk_kernel(
         if (SPLIT) {
 #pragma unroll
             for (int t = 0; t < DC_ROWS; ++t) {                // the two rows of a pair go to different tiles
-                const Pieces x = split3(w[t], b[t]);
+                const mma16::Pieces x = mma16::split3(w[t], b[t]);
 #pragma unroll
                 for (int p = 0; p < 3; ++p) {
                     half[cm_m_half(p, t, j)] = (uint16_t)x.v[p];
@@ -579,7 +562,7 @@ __global__ void __launch_bounds__(DC_THREADS, SPLIT ? 3 : 2) delta_chunk_kernel(
         if (SPLIT) {
 #pragma unroll
             for (int t = 0; t < DC_ROWS / 2; ++t) {
-                const Pieces x = split3(w[2 * t], w[2 * t + 1]);
+                const mma16::Pieces x = mma16::split3(w[2 * t], w[2 * t + 1]);
 #pragma unroll
                 for (int p = 0; p < 3; ++p) ops_s[cm_k_word(dp, p, t, j)] = x.v[p];
             }
@@ -862,7 +845,7 @@ __global__ void __launch_bounds__(WARPS * 32) delta_carry_mma_kernel(DeltaArgs a
 #pragma unroll
             for (int r = 0; r < 4; ++r) {                      // (g, 2t..), (g + 8, 2t..), (g, 2t + 8..), (g + 8, 2t + 8..)
                 const float* s = S[2 * kb + (r >> 1)] + 2 * (r & 1);
-                const Pieces v = split3(s[0], s[1]);
+                const mma16::Pieces v = mma16::split3(s[0], s[1]);
                 x[0][r] = v.v[0]; x[1][r] = v.v[1]; x[2][r] = v.v[2];
             }
             mma_split<4>(P, x, b);
@@ -889,7 +872,7 @@ __global__ void __launch_bounds__(WARPS * 32) delta_carry_mma_kernel(DeltaArgs a
                 sum.y += v[w].y + v[w + 1].y;
             }
             if (n < 2) {
-                const Pieces x = split3(sum.x, sum.y);
+                const mma16::Pieces x = mma16::split3(sum.x, sum.y);
 #pragma unroll
                 for (int p = 0; p < 3; ++p) u_s[(p * 32 + lane) * 4 + 2 * n + half] = x.v[p];
             } else if (from[k]) {

@@ -19,6 +19,7 @@
 //                       consecutive parts, each with its own mean (float32; output in the activation dtype).
 #include "common.cuh"
 #include "mma_sync.cuh"
+#include "chunk_mma.cuh"
 
 constexpr int SSD_THREADS = 256;
 constexpr int SSD_LANES = 8;                         // lanes that share one value column
@@ -41,6 +42,7 @@ struct SsdArgs {
     long long state_stride;
     float* y;                // [T, heads * P]
     int heads, groups, N, P;
+    int skip;                // requests of this many rows or more are not walked (the chunk kernels serve them)
     int walk;                // some request brings more than one row: launched the plain way, onto an empty GPU
 };
 
@@ -60,7 +62,7 @@ __global__ void __launch_bounds__(SSD_THREADS) ssd_scan_kernel(SsdArgs a) {
     const int req = blockIdx.z, h = blockIdx.y;
     const int g = h / (a.heads / a.groups);
     const int first = a.row_offsets[req], rows = a.row_offsets[req + 1] - first;
-    if (rows <= 0) return;
+    if (rows <= 0 || rows >= a.skip) return;
     const int lane = threadIdx.x % SSD_LANES;
     const int col = threadIdx.x / SSD_LANES;
     const int v = blockIdx.x * SSD_COLS + col;
@@ -180,10 +182,33 @@ static int ssd_launch(const SsdArgs& a, dim3 grid, cudaStream_t stream) {
     return SHARPI_OK;
 }
 
+// The recurrence in chunks (chunk_mma.cuh): B are the keys, C the queries, dt scales what enters.
+struct SsdChunks {
+    static constexpr bool NORM = false;
+    SsdArgs s;
+    __device__ __forceinline__ void decay(int t, int h, float& a, float& b) const {
+        b = softplus_f(s.dt[(size_t)t * s.ld_dt + s.col_dt + h] + s.dt_bias[h]);
+        a = expf(-expf(s.a_log[h]) * b);
+    }
+    __device__ __forceinline__ float* state(int slot, int h, int row, int col) const {
+        return s.state + (size_t)slot * s.state_stride + ((size_t)h * s.N + row) * s.P + col;
+    }
+    __device__ __forceinline__ float* norm(int, int, int) const { return nullptr; }
+    __device__ __forceinline__ void store_norm(int, int, float) const {}
+    __device__ __forceinline__ float2 finish(int t, int h, int c, float2 o) const {
+        const float2 x = *reinterpret_cast<const float2*>(s.xbc + (size_t)t * s.ld_x + s.col_x + h * s.P + c);
+        const float d = s.dskip[h];
+        return make_float2(o.x + d * x.x, o.y + d * x.y);
+    }
+};
+
+// `sums` (nullable; `chunks` * (heads * N * P + heads) floats): requests of at least `least` rows run in chunks, `chunks` of
+// them at most, on the tensor cores; the others, and without it all, are walked.
 SHARPI_API int sharpi_ssd_scan(const float* xbc, int ld_x, int col_x, int col_b, int col_c, const float* dt, int ld_dt,
                                int col_dt, const float* dt_bias, const float* a_log, const float* dskip,
                                const int* row_offsets, const int* state_slots, float* state, long long state_stride,
-                               float* y, int T, int B, int heads, int groups, int N, int P, cudaStream_t stream) {
+                               float* y, int T, int B, int heads, int groups, int N, int P, float* sums, int chunks,
+                               int least, cudaStream_t stream) {
     if (T <= 0 || B <= 0) return SHARPI_OK;
     if (heads <= 0 || groups <= 0 || heads % groups != 0 || N <= 0 || N > SSD_MAX_STATES || P <= 0 || heads > 65535 ||
         B > 65535 || col_x + heads * P > ld_x || col_b + groups * N > ld_x || col_c + groups * N > ld_x ||
@@ -193,7 +218,21 @@ SHARPI_API int sharpi_ssd_scan(const float* xbc, int ld_x, int col_x, int col_b,
     a.xbc = xbc; a.ld_x = ld_x; a.col_x = col_x; a.col_b = col_b; a.col_c = col_c; a.dt = dt; a.ld_dt = ld_dt;
     a.col_dt = col_dt; a.dt_bias = dt_bias; a.a_log = a_log; a.dskip = dskip; a.row_offsets = row_offsets;
     a.state_slots = state_slots; a.state = state; a.state_stride = state_stride; a.y = y; a.heads = heads;
-    a.groups = groups; a.N = N; a.P = P; a.walk = T > B;
+    a.groups = groups; a.N = N; a.P = P; a.walk = T > B; a.skip = 0x7fffffff;
+    if (sums) {
+        if (least < 1) return SHARPI_BAD_ARGUMENT;
+        chunked::Args c;
+        c.q = xbc + col_c; c.k = xbc + col_b; c.v = xbc + col_x; c.ld_q = c.ld_k = c.ld_v = ld_x;
+        c.d = N; c.dv = P; c.heads = heads; c.key_heads = groups; c.group = 1;
+        c.row_offsets = row_offsets; c.state_slots = state_slots; c.B = B; c.least = least;
+        c.sums = sums; c.norms = (long long)chunks * heads * N * P; c.total = sums + c.norms; c.out = y;
+        if ((reinterpret_cast<uintptr_t>(state) & 15) != 0 || state_stride % 4 != 0) return SHARPI_BAD_ARGUMENT;
+        SsdChunks f;
+        f.s = a;
+        const int rc = chunked::launch(c, f, chunks, stream);
+        if (rc != SHARPI_OK || (B == 1 && T >= least)) return rc;
+        a.skip = least;
+    }
     const dim3 grid((P + SSD_COLS - 1) / SSD_COLS, heads, B);
     const int per_lane = (N + SSD_LANES - 1) / SSD_LANES;
     if (per_lane <= 4) return ssd_launch<4>(a, grid, stream);

@@ -33,6 +33,7 @@
 //
 // State of one request and layer, per head: for every slice of 32 value columns [d][32] floats of S (columns beyond
 // dv are zeros), then n [d], then m and three unused floats.  `head_stride` floats per head.
+#include "chunk_mma.cuh"
 #include "common.cuh"
 
 constexpr int MLSTM_CHUNK = 8;       // rows staged in shared memory at a time (half as many at the largest key size)
@@ -54,6 +55,7 @@ struct MlstmArgs {
     float* coef;             // [T, heads, 4]: log a, log b, m, unused
     float* o_raw;            // [T, heads * dv]: S^T q, not yet divided
     float* nq;               // [T, heads]: n . q
+    int skip;                // requests of this many rows or more are not walked (the chunk kernels serve them)
 };
 
 __device__ __forceinline__ float log_sigmoid(float x) {
@@ -167,7 +169,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) mlstm_scan_kernel(MlstmArgs a, i
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int wg = warp * 4 + (lane >> 3), c4 = (lane & 7) * CPT;
     const int r0 = a.row_offsets[b], r1 = a.row_offsets[b + 1];
-    if (r1 <= r0) return;
+    if (r1 <= r0 || r1 - r0 >= a.skip) return;
     const int d = a.d, dv = a.dv;
     const bool norm_slice = (int)blockIdx.z == col_blocks;      // the CTA that carries n in its first column
     const int col0 = blockIdx.z * CW;                   // first value column of this CTA
@@ -314,13 +316,36 @@ static int launch_scan(const MlstmArgs& a, int B, cudaStream_t stream) {
     return SHARPI_OK;
 }
 
+// The recurrence in chunks (chunk_mma.cuh), from the coefficients that the gates kernel left.
+struct MlstmChunks {
+    static constexpr bool NORM = true;
+    MlstmArgs m;
+    __device__ __forceinline__ void decay(int t, int h, float& a, float& b) const {
+        const float* c = m.coef + ((size_t)t * m.heads + h) * 4;
+        a = expf(c[0]);
+        b = expf(c[1]);
+    }
+    __device__ __forceinline__ float* head(int slot, int h) const {
+        return m.state + (size_t)slot * m.state_stride + (size_t)h * m.head_stride;
+    }
+    __device__ __forceinline__ float* state(int slot, int h, int row, int col) const {
+        return head(slot, h) + ((size_t)(col >> 5) * m.d + row) * 32 + (col & 31);
+    }
+    __device__ __forceinline__ float* norm(int slot, int h, int i) const { return head(slot, h) + (size_t)m.slices * m.d * 32 + i; }
+    __device__ __forceinline__ void store_norm(int t, int h, float s) const { m.nq[(size_t)t * m.heads + h] = s * m.q_scale; }
+    __device__ __forceinline__ float2 finish(int, int, int, float2 o) const { return make_float2(o.x * m.q_scale, o.y * m.q_scale); }
+};
+
+// `sums` (nullable; `chunks` * heads * (d * dv + d + 1) floats): requests of at least `least` rows run in chunks, `chunks` of
+// them at most, on the tensor cores; the others, and without it all, are walked.
 // The recurrence over the step's rows: leaves the numerators o_raw [T, heads * dv], n . q in nq [T, heads], the
 // running maximum of every row in coef[.., 2] (coef: T * heads * 4 floats) and the new state.
 SHARPI_API int sharpi_mlstm_recurrence(const float* proj, int ld, int col_q, int col_k, int col_v, int col_i, int col_f,
                                        const float* bias_i, const float* bias_f, const int* row_offsets,
                                        const int* state_slots, float* state, long long state_stride, int head_stride,
                                        int B, int T, int heads, int d, int dv, float cap, float q_scale, float* coef,
-                                       float* o_raw, float* nq, cudaStream_t stream) {
+                                       float* o_raw, float* nq, float* sums, int chunks, int least,
+                                       cudaStream_t stream) {
     if (B <= 0 || T <= 0) return SHARPI_OK;
     if (heads <= 0 || d <= 0 || dv <= 0 || d > MLSTM_MAX_D || !(cap > 0.0f)) return SHARPI_BAD_ARGUMENT;
     if (heads > 65535 || (dv + 31) / 32 + 1 > 65535) return SHARPI_BAD_ARGUMENT;
@@ -328,7 +353,7 @@ SHARPI_API int sharpi_mlstm_recurrence(const float* proj, int ld, int col_q, int
     a.proj = proj; a.ld = ld; a.col_q = col_q; a.col_k = col_k; a.col_v = col_v; a.col_i = col_i;
     a.col_f = col_f; a.bias_i = bias_i; a.bias_f = bias_f; a.row_offsets = row_offsets; a.state_slots = state_slots;
     a.state = state; a.state_stride = state_stride; a.head_stride = head_stride; a.heads = heads; a.d = d; a.dv = dv;
-    a.slices = (dv + 31) / 32; a.cap = cap; a.q_scale = q_scale; a.coef = coef; a.o_raw = o_raw; a.nq = nq;
+    a.slices = (dv + 31) / 32; a.cap = cap; a.q_scale = q_scale; a.coef = coef; a.o_raw = o_raw; a.nq = nq; a.skip = 0x7fffffff;
     if ((long long)head_stride < (long long)a.slices * d * 32 + d + 1) return SHARPI_BAD_ARGUMENT;
     if (T > 256) {                   // many rows: the gates' tanh and logsigmoid for all rows at once, ahead of the walk
         const long long items = (long long)T * heads;
@@ -339,6 +364,21 @@ SHARPI_API int sharpi_mlstm_recurrence(const float* proj, int ld, int col_q, int
         mlstm_gates_kernel<false><<<dim3(B, heads), 32, 0, stream>>>(a);
     }
     SHARPI_CHECK_LAUNCH();
+    if (sums) {
+        if (least < 1 || (reinterpret_cast<uintptr_t>(state) & 15) != 0 || state_stride % 4 != 0 || head_stride % 4 != 0)
+            return SHARPI_BAD_ARGUMENT;
+        chunked::Args c;
+        c.q = proj + col_q; c.k = proj + col_k; c.v = proj + col_v; c.ld_q = c.ld_k = c.ld_v = ld;
+        c.d = d; c.dv = dv; c.heads = c.key_heads = heads; c.group = 1;
+        c.row_offsets = row_offsets; c.state_slots = state_slots; c.B = B; c.least = least;
+        c.sums = sums; c.norms = (long long)chunks * heads * d * dv; c.total = sums + c.norms + (long long)chunks * heads * d;
+        c.out = o_raw;
+        MlstmChunks f;
+        f.m = a;
+        const int rc = chunked::launch(c, f, chunks, stream);
+        if (rc != SHARPI_OK || (B == 1 && T >= least)) return rc;
+        a.skip = least;
+    }
     if (d <= 16) return launch_scan<1>(a, B, stream);
     if (d <= 32) return launch_scan<2>(a, B, stream);
     if (d <= 64) return launch_scan<4>(a, B, stream);

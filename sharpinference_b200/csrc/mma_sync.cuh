@@ -63,4 +63,21 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// Two neighbouring elements in three bfloat16 pieces each (24 bits together), packed as an operand register.
+struct Pieces {
+    uint32_t v[3];
+};
+__device__ __forceinline__ Pieces split3(float x, float y) {
+    Pieces r;
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+        r.v[p] = pack_bf16(x, y);
+        if (p < 2) {
+            x -= __uint_as_float(r.v[p] << 16);
+            y -= __uint_as_float(r.v[p] & 0xffff0000u);
+        }
+    }
+    return r;
+}
+
 }  // namespace mma16

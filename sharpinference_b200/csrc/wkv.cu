@@ -16,6 +16,8 @@
 // other and a column's parts are added in a fixed order, so a row's result is the same sequence of operations
 // whether it came in a prompt portion or alone.  Heads of more than 128 elements take the form in which
 // a column's key channels are dealt over several threads (wkv_recurrence_kernel).
+// Requests of many rows may run in chunks of 64 rows that work side by side, on the tensor cores (below).
+#include "chunk_mma.cuh"
 #include "common.cuh"
 
 struct WkvArgs {
@@ -136,6 +138,7 @@ struct WkvScanArgs {
     float* o;
     int heads, d, aligned;
     int ch;                // rows a chunk (at most WKV_CH; fewer when no request brings that many)
+    int skip;              // requests of this many rows or more are not walked (the chunk kernels serve them)
 };
 
 constexpr int WKV_CH = 16;     // rows a chunk at most
@@ -160,6 +163,7 @@ __global__ void __launch_bounds__(MAXT) wkv_scan_kernel(WkvScanArgs a) {
     float* part = v_s + WKV_STAGES * CH * DVP;                // [CH][KG][DVP]
     float* bon = part + CH * KG * DVP;                        // [STAGES][CH]
     const int first = a.row_offsets[b], end = a.row_offsets[b + 1];
+    if (end - first >= a.skip) return;
     const size_t hd = (size_t)a.heads * d, col = (size_t)head * d;
     float* S_g = a.state + (size_t)a.state_slots[b] * a.state_stride + (size_t)head * d * d;
     float S[KT][CPT];
@@ -303,12 +307,366 @@ static int launch_wkv_scan(WkvScanArgs a, int B, int T, cudaStream_t stream) {
     return SHARPI_OK;
 }
 
+// -------------------------------------------------------------------------------------------------------------
+// Chunks of 64 rows for heads of up to 64 elements.  With W_(s,t] the product of the decays of rows s + 1 .. t, per channel:
+//   (1) wkv_sums_kernel    U = sum_s (W_(s,last] k_s) v_s^T and the chunk's decay per channel; wraw <- the decays
+//   (2) wkv_carry_kernel   the state before each chunk in U's place
+//   (3) wkv_outs_kernel    o_t = (W_(first-1,t-1] r_t)^T S + sum_(s<t) A_ts v_s + (r_t . u k_t) v_t,
+//                          A_ts = sum_i r_t[i] W_(s,t-1][i] k_s[i]
+// A decay per channel cannot be taken out of A as a factor of its row (1 / W overflows).  The chunk is four blocks of sixteen
+// rows, a warp's each: between blocks A is a product of r times the decays since its block began (and of the whole
+// blocks between) with k times the decays up to its block's end, every factor at most 1; inside a block lanes walk their two
+// channels.  All other products run on the tensor cores in bfloat16 pieces of 24 bits (chunk_mma.cuh).
+// -------------------------------------------------------------------------------------------------------------
+constexpr int WC_D = 64, WC_LD = WC_D + 8, WC_PLANE = chunked::ROWS * WC_LD, WC_THREADS = chunked::THREADS, WC_R = WC_D + 4;
+
+struct WkvChunkArgs {
+    const float *r, *k, *v, *w0, *u;
+    float* w;              // [T, heads * d]: raw, then the decay
+    const int* row_offsets;
+    const int* state_slots;
+    int B, least;
+    float* state;
+    long long state_stride;
+    float* o;
+    int heads, d;
+    float* sums;           // [chunks][heads][d][d]
+    float* total;          // [chunks][heads][64]
+};
+
+__device__ __forceinline__ void store_pieces(bf16* planes, int at, float x) {
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+        const bf16 b = __float2bfloat16_rn(x);
+        planes[p * WC_PLANE + at] = b;
+        x -= __bfloat162float(b);
+    }
+}
+
+__global__ void __launch_bounds__(WC_THREADS, 3) wkv_sums_kernel(WkvChunkArgs a) {
+    extern __shared__ __align__(16) uint8_t wkv_smem[];
+    bf16* k_s = reinterpret_cast<bf16*>(wkv_smem);            // three planes [64 rows][64 channels]
+    bf16* v_s = k_s + 3 * WC_PLANE;
+    __shared__ float half_s[WC_D];
+    chunked::Place p;
+    if (!chunked::find_chunk(a.row_offsets, a.B, a.least, blockIdx.y, p)) return;
+    const int head = blockIdx.x, d = a.d, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const size_t hd = (size_t)a.heads * d, at0 = (size_t)p.row0 * hd + (size_t)head * d;
+    chunked::load_split<chunked::ROWS, WC_D>(v_s, a.v + at0, hd, p.rows, d, nullptr);
+    {
+        constexpr int HALF = chunked::ROWS / 2;
+        const int c = threadIdx.x % WC_D, half = threadIdx.x / WC_D;
+        float w[HALF], k[HALF];
+        const float w0 = c < d ? a.w0[(size_t)head * d + c] : 0.0f;
+#pragma unroll
+        for (int r = 0; r < HALF; ++r) {
+            const int row = half * HALF + r;
+            const bool ok = row < p.rows && c < d;
+            w[r] = ok ? a.w[at0 + (size_t)row * hd + c] : 0.0f;
+            k[r] = ok ? a.k[at0 + (size_t)row * hd + c] : 0.0f;
+        }
+        float tail = 1.0f;                                   // the decays behind a row, inside its half
+#pragma unroll
+        for (int r = HALF - 1; r >= 0; --r) {
+            const int row = half * HALF + r;
+            const bool ok = row < p.rows && c < d;
+            const float x = ok ? expf(-expf(w[r] + w0)) : 1.0f;
+            if (ok) a.w[at0 + (size_t)row * hd + c] = x;
+            k[r] *= tail;
+            tail *= x;
+        }
+        if (half == 1) half_s[c] = tail;
+        __syncthreads();
+        const float after = half == 0 ? half_s[c] : 1.0f;
+        if (half == 0) a.total[((size_t)blockIdx.y * a.heads + head) * WC_D + c] = tail * after;
+#pragma unroll
+        for (int r = 0; r < HALF; ++r) store_pieces(k_s, (half * HALF + r) * WC_LD + c, k[r] * after);
+    }
+    __syncthreads();
+    float acc[8][4], small[8][4];
+    chunked::clear(acc);
+    chunked::clear(small);
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+        uint32_t x[3][4];
+#pragma unroll
+        for (int q = 0; q < 3; ++q)                          // stored [row][channel], taken transposed
+            mma16::ldmatrix_x4_trans(x[q], k_s + q * WC_PLANE + (kk * 16 + (lane / 16) * 8 + lane % 8) * WC_LD + warp * 16 + ((lane / 8) % 2) * 8);
+#pragma unroll
+        for (int n = 0; n < 8; n += 4) {
+            uint32_t b[3][4][2];
+            chunked::right_operand<WC_LD, WC_PLANE>(b, v_s, kk * 16, n * 8, lane);
+            chunked::mma_pieces(acc + n, small + n, x, b);
+        }
+    }
+    chunked::add_small(acc, small);
+    float* out = a.sums + ((size_t)blockIdx.y * a.heads + head) * d * d;
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const int row = warp * 16 + lane / 4 + 8 * e;
+        if (row >= d) continue;
+#pragma unroll
+        for (int n = 0; n < 8; ++n) {
+            const int c = n * 8 + (lane % 4) * 2;
+            if (c < d) *reinterpret_cast<float2*>(out + (size_t)row * d + c) = make_float2(acc[n][2 * e], acc[n][2 * e + 1]);
+        }
+    }
+}
+
+__global__ void __launch_bounds__(chunked::CARRY_THREADS) wkv_carry_kernel(WkvChunkArgs a) {
+    const int b = blockIdx.z, head = blockIdx.y, d = a.d, rows = a.row_offsets[b + 1] - a.row_offsets[b];
+    if (rows < a.least) return;
+    const int base = chunked::chunks_before(a.row_offsets, b, a.least);
+    const int i = (blockIdx.x * chunked::CARRY_THREADS + threadIdx.x) * 4;
+    if (i >= d * d) return;
+    const int n = (rows + chunked::ROWS - 1) / chunked::ROWS;
+    const float* total = a.total + ((size_t)base * a.heads + head) * WC_D + i / d;
+    float4* s = reinterpret_cast<float4*>(a.state + (size_t)a.state_slots[b] * a.state_stride + (size_t)head * d * d + i);
+    const size_t step = (size_t)a.heads * d * d;
+    float* u = a.sums + ((size_t)base * a.heads + head) * d * d + i;
+    constexpr int AHEAD = 8;
+    float4 S = *s, next[AHEAD];
+    float decay[AHEAD];
+#pragma unroll
+    for (int k = 0; k < AHEAD; ++k)
+        if (k < n) {
+            next[k] = *reinterpret_cast<const float4*>(u + k * step);
+            decay[k] = total[(size_t)k * a.heads * WC_D];
+        }
+    for (int c = 0; c < n; c += AHEAD) {
+#pragma unroll
+        for (int k = 0; k < AHEAD; ++k) {
+            if (c + k >= n) break;
+            const float4 own = next[k];
+            const float A = decay[k];
+            if (c + k + AHEAD < n) {
+                next[k] = *reinterpret_cast<const float4*>(u + (size_t)(c + k + AHEAD) * step);
+                decay[k] = total[(size_t)(c + k + AHEAD) * a.heads * WC_D];
+            }
+            *reinterpret_cast<float4*>(u + (size_t)(c + k) * step) = S;
+            S = make_float4(fmaf(A, S.x, own.x), fmaf(A, S.y, own.y), fmaf(A, S.z, own.z), fmaf(A, S.w, own.w));
+        }
+    }
+    *s = S;
+}
+
+constexpr size_t WC_OUTS_SMEM = (size_t)6 * WC_PLANE * sizeof(bf16) + (size_t)(chunked::ROWS * WC_R + 4 * 16 * 17 + 4 * WC_D) * sizeof(float);
+
+__global__ void __launch_bounds__(WC_THREADS, 2) wkv_outs_kernel(WkvChunkArgs a) {
+    extern __shared__ __align__(16) uint8_t wkv_smem[];
+    bf16* k_s = reinterpret_cast<bf16*>(wkv_smem);            // k times the decays up to its block's end; then the state
+    bf16* v_s = k_s + 3 * WC_PLANE;
+    float* r_s = reinterpret_cast<float*>(v_s + 3 * WC_PLANE);  // [64][WC_R]: r times the decays since its block began
+    float* A_s = r_s + chunked::ROWS * WC_R;                   // [warp][16][17]: A inside a block
+    float* W_s = A_s + 4 * 16 * 17;                            // [block][64]: a block's decay
+    chunked::Place p;
+    if (!chunked::find_chunk(a.row_offsets, a.B, a.least, blockIdx.y, p)) return;
+    const int head = blockIdx.x, d = a.d, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane / 4, t = lane % 4;
+    const size_t hd = (size_t)a.heads * d, at0 = (size_t)p.row0 * hd + (size_t)head * d;
+    {
+        float r[16][2], k[16][2], w[16][2], u[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) u[e] = lane + 32 * e < d ? a.u[(size_t)head * d + lane + 32 * e] : 0.0f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int row = warp * 16 + i, c = lane + 32 * e;
+                const bool ok = row < p.rows && c < d;
+                const size_t at = at0 + (size_t)row * hd + c;
+                r[i][e] = ok ? a.r[at] : 0.0f;
+                k[i][e] = ok ? a.k[at] : 0.0f;
+                w[i][e] = ok ? a.w[at] : 1.0f;
+            }
+        chunked::load_split<chunked::ROWS, WC_D>(v_s, a.v + at0, hd, p.rows, d, nullptr);
+        // columns s and s + 1 of the block's A: a lane's channels down the rows, then lane 16 e + t has A of row t, column s + e
+#pragma unroll
+        for (int s = 0; s < 16; s += 2) {
+            float acc[32];
+#pragma unroll
+            for (int i = 0; i < 32; ++i) acc[i] = 0.0f;
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int col = s + e;
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    acc[16 * e + col] = fmaf(r[col][c] * u[c], k[col][c], acc[16 * e + col]);
+                    float x = k[col][c];
+#pragma unroll
+                    for (int i = col + 1; i < 16; ++i) {
+                        acc[16 * e + i] = fmaf(r[i][c], x, acc[16 * e + i]);
+                        x *= w[i][c];
+                    }
+                }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int i = 0; i < o; ++i) {
+                    const bool up = lane & o;
+                    const float give = up ? acc[i] : acc[i + o], keep = up ? acc[i + o] : acc[i];
+                    acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                }
+            A_s[(warp * 16 + lane % 16) * 17 + s + lane / 16] = acc[0];
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int c = lane + 32 * e;
+            float x = 1.0f;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                r_s[(warp * 16 + i) * WC_R + c] = r[i][e] * x;
+                x *= w[i][e];
+            }
+            W_s[warp * WC_D + c] = x;
+            x = 1.0f;
+#pragma unroll
+            for (int i = 15; i >= 0; --i) {
+                store_pieces(k_s, (warp * 16 + i) * WC_LD + c, k[i][e] * x);
+                x *= w[i][e];
+            }
+        }
+    }
+    __syncthreads();
+    // the left operand of this warp's rows: r_s times the decays of the whole blocks `from` .. warp - 1, sixteen channels
+    auto left = [&](uint32_t (&x)[3][4], int kk, int from) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int c = kk * 16 + 2 * t + 8 * h;
+            float m0 = 1.0f, m1 = 1.0f;
+            for (int b = from; b < warp; ++b) {
+                const float2 f = *reinterpret_cast<const float2*>(W_s + b * WC_D + c);
+                m0 *= f.x; m1 *= f.y;
+            }
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const float2 v = *reinterpret_cast<const float2*>(r_s + (warp * 16 + g + 8 * e) * WC_R + c);
+                const mma16::Pieces s = mma16::split3(v.x * m0, v.y * m1);
+#pragma unroll
+                for (int q = 0; q < 3; ++q) x[q][2 * h + e] = s.v[q];
+            }
+        }
+    };
+    float score[3][2][4];
+#pragma unroll
+    for (int J = 0; J < 3; ++J) {
+        chunked::clear(score[J]);
+        if (J >= warp) continue;
+        float few[2][4];
+        chunked::clear(few);
+#pragma unroll
+        for (int k2 = 0; k2 < 2; ++k2) {
+            uint32_t b[2][3][2][2];
+#pragma unroll
+            for (int q = 0; q < 3; ++q)
+#pragma unroll
+                for (int n = 0; n < 2; ++n) {
+                    uint32_t m[4];
+                    mma16::ldmatrix_x4(m, k_s + q * WC_PLANE + (J * 16 + n * 8 + lane % 8) * WC_LD + k2 * 32 + (lane / 8) * 8);
+                    b[0][q][n][0] = m[0]; b[0][q][n][1] = m[1]; b[1][q][n][0] = m[2]; b[1][q][n][1] = m[3];
+                }
+#pragma unroll
+            for (int k1 = 0; k1 < 2; ++k1) {
+                uint32_t x[3][4];
+                left(x, 2 * k2 + k1, J + 1);
+                chunked::mma_pieces(score[J], few, x, b[k1]);
+            }
+        }
+        chunked::add_small(score[J], few);
+    }
+    __syncthreads();                                           // the keys are free
+    chunked::load_split<WC_D, WC_D>(k_s, a.sums + ((size_t)blockIdx.y * a.heads + head) * d * d, d, d, d, nullptr);
+    __syncthreads();
+    float acc[8][4], small[8][4];
+    chunked::clear(acc);
+    chunked::clear(small);
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+        uint32_t x[3][4];
+        left(x, kk, 0);
+#pragma unroll
+        for (int n = 0; n < 8; n += 4) {
+            uint32_t b[3][4][2];
+            chunked::right_operand<WC_LD, WC_PLANE>(b, k_s, kk * 16, n * 8, lane);
+            chunked::mma_pieces(acc + n, small + n, x, b);
+        }
+    }
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+        if (kk > warp) continue;
+        uint32_t x[3][4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int n = e >> 1, row = g + 8 * (e & 1);
+            float u0 = 0.0f, u1 = 0.0f;
+            if (kk == warp) {
+                u0 = A_s[(warp * 16 + row) * 17 + n * 8 + 2 * t];
+                u1 = A_s[(warp * 16 + row) * 17 + n * 8 + 2 * t + 1];
+            } else if (kk < 3) {
+                u0 = score[kk < 3 ? kk : 0][n][2 * (e & 1)];
+                u1 = score[kk < 3 ? kk : 0][n][2 * (e & 1) + 1];
+            }
+            const mma16::Pieces s = mma16::split3(u0, u1);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) x[q][e] = s.v[q];
+        }
+#pragma unroll
+        for (int n = 0; n < 8; n += 4) {
+            uint32_t b[3][4][2];
+            chunked::right_operand<WC_LD, WC_PLANE>(b, v_s, kk * 16, n * 8, lane);
+            chunked::mma_pieces(acc + n, small + n, x, b);
+        }
+    }
+    chunked::add_small(acc, small);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const int row = warp * 16 + g + 8 * e;
+        if (row >= p.rows) continue;
+#pragma unroll
+        for (int n = 0; n < 8; ++n) {
+            const int c = n * 8 + 2 * t;
+            if (c < d) *reinterpret_cast<float2*>(a.o + at0 + (size_t)row * hd + c) = make_float2(acc[n][2 * e], acc[n][2 * e + 1]);
+        }
+    }
+}
+
+static int launch_wkv_chunks(const WkvChunkArgs& a, int chunks, cudaStream_t stream) {
+    constexpr size_t smem_sums = (size_t)6 * WC_PLANE * sizeof(bf16);
+    if (cudaFuncSetAttribute(wkv_sums_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_sums) != cudaSuccess ||
+        cudaFuncSetAttribute(wkv_outs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WC_OUTS_SMEM) != cudaSuccess)
+        return SHARPI_LAUNCH_FAILED;
+    const dim3 grid(a.heads, chunks);
+    wkv_sums_kernel<<<grid, WC_THREADS, smem_sums, stream>>>(a);
+    SHARPI_CHECK_LAUNCH();
+    wkv_carry_kernel<<<dim3((a.d * a.d / 4 + chunked::CARRY_THREADS - 1) / chunked::CARRY_THREADS, a.heads, a.B), chunked::CARRY_THREADS, 0, stream>>>(a);
+    SHARPI_CHECK_LAUNCH();
+    wkv_outs_kernel<<<grid, WC_THREADS, WC_OUTS_SMEM, stream>>>(a);
+    SHARPI_CHECK_LAUNCH();
+    return SHARPI_OK;
+}
+
+// `sums` (nullable; `chunks` * heads * (d * d + 64) floats): requests of at least `least` rows run in chunks, `chunks` of them
+// at most, on the tensor cores (d <= 64); the others, and without it all, are walked.
 SHARPI_API int sharpi_wkv_recurrence(const float* r, const float* k, const float* v, float* wraw,
                                      const float* w0, const float* u, const int* row_offsets, const int* state_slots,
                                      float* state, long long state_stride, float* o, float* bonus, int T, int B,
-                                     int heads, int d, cudaStream_t stream) {
+                                     int heads, int d, float* sums, int chunks, int least, cudaStream_t stream) {
     if (B <= 0) return SHARPI_OK;
     if (heads <= 0 || d <= 0 || d > 256 || T <= 0) return SHARPI_BAD_ARGUMENT;
+    int skip = 0x7fffffff;
+    if (sums) {
+        const uintptr_t bases = (uintptr_t)v | (uintptr_t)sums | (uintptr_t)state | (uintptr_t)o;
+        if (d > WC_D || d % 4 != 0 || (bases & 15) != 0 || state_stride % 4 != 0 || chunks < 1 || chunks > 65535 || B > 65535 ||
+            heads > 65535 || least < 1)
+            return SHARPI_BAD_ARGUMENT;
+        WkvChunkArgs c;
+        c.r = r; c.k = k; c.v = v; c.w = wraw; c.w0 = w0; c.u = u; c.row_offsets = row_offsets; c.state_slots = state_slots;
+        c.B = B; c.least = least; c.state = state; c.state_stride = state_stride; c.o = o; c.heads = heads; c.d = d;
+        c.sums = sums; c.total = sums + (size_t)chunks * heads * d * d;
+        const int rc = launch_wkv_chunks(c, chunks, stream);
+        if (rc != SHARPI_OK || (B == 1 && T >= least)) return rc;
+        skip = least;
+    }
     if (d <= 128) {
         // the decay and the bonus' scalar for all rows at once, then the walk
         const long long work = (long long)T * heads;
@@ -316,7 +674,7 @@ SHARPI_API int sharpi_wkv_recurrence(const float* r, const float* k, const float
                           heads, d);
         WkvScanArgs s;
         s.r = r; s.k = k; s.v = v; s.w = wraw; s.bonus = bonus; s.row_offsets = row_offsets; s.state_slots = state_slots;
-        s.state = state; s.state_stride = state_stride; s.o = o; s.heads = heads; s.d = d;
+        s.state = state; s.state_stride = state_stride; s.o = o; s.heads = heads; s.d = d; s.skip = skip;
         const uintptr_t ptrs = reinterpret_cast<uintptr_t>(r) | reinterpret_cast<uintptr_t>(k) |
                                reinterpret_cast<uintptr_t>(wraw) | reinterpret_cast<uintptr_t>(v);
         s.aligned = (d % 4 == 0 && (ptrs & 15) == 0) ? 1 : 0;

@@ -854,14 +854,42 @@ def mlstm_state_floats(heads: int, d: int, dv: int):
     return per_head, heads * per_head
 
 
+# Requests of this many rows or more of a step run in chunks of 64 rows on the tensor cores where a caller allows it and the
+# step as a whole is faster so
+CHUNKED_LEAST = 128
+# What a step's recurrence takes, us: walked, w * max(rows of the longest request, rows of the step * heads / s) (a request's rows
+# are a chain; s (request, head) pairs keep the GPU busy); in chunks, 27 + c * rows * heads.  (w, s, c), walked -> in chunks at one
+# request of 128, 512 and 2048 rows, eight of 128 and four of 2048: mlstm (8 heads) 25 -> 30, 85 -> 46, 321 -> 126, 68 -> 70,
+# 589 -> 448; ssd (64 heads) 44 -> 30, 164 -> 58, 646 -> 212, 188 -> 147, 1740 -> 809; wkv (32 heads) 34 -> 28, 120 -> 33, 423 -> 121,
+# 41 -> 75, 543 -> 485.
+_WALK_OR_CHUNKS = {"mlstm": (0.16, 20, 0.0065), "ssd": (0.32, 100, 0.0016), "wkv": (0.21, 200, 0.0018)}
+
+
+def _chunks(kind: str, T: int, B: int, max_rows: Optional[int], heads: int, d: int, dv: int, *aligned: int) -> int:
+    """How many chunks the requests of a step that run in chunks can have together (each ends in one that may be short);
+    0: none has the rows, walking is faster, or the sizes are not the chunk kernels'.  ``max_rows``: rows of the longest
+    request (None or 0: at most ``T - B + 1``); ``aligned``: column numbers, strides and addresses in floats, which the chunk
+    kernels want on 16 bytes."""
+    longest = max_rows or T - B + 1
+    if longest < CHUNKED_LEAST or d > 128 or d % 4 or dv % 4 or any(x % 4 for x in aligned):
+        return 0
+    w, s, c = _WALK_OR_CHUNKS[kind]
+    if w * max(longest, T * heads / s) < 27 + c * T * heads:
+        return 0
+    return (T + 63) // 64 if B == 1 else T // 64 + min(B, T // CHUNKED_LEAST)
+
+
 def mlstm_recurrence(proj: torch.Tensor, *, col_q: int, col_k: int, col_v: int, col_i: int, col_f: int,
                      bias_i: torch.Tensor, bias_f: torch.Tensor, row_offsets: torch.Tensor, state_slots: torch.Tensor,
-                     state: torch.Tensor, heads: int, d: int, dv: int, cap: float, q_scale: float):
+                     state: torch.Tensor, heads: int, d: int, dv: int, cap: float, q_scale: float, split: bool = False,
+                     max_rows: Optional[int] = None):
     """The matrix-memory recurrence over the step's rows (``mlstm.cu``): reads q, k, v and the raw gates from the
     fused float32 projection ``proj [T, ld]`` at the given first columns and advances ``state [slots, floats]`` of
     the step's requests (``state_slots [B]``, rows ``row_offsets [B + 1]``).  Returns ``(num, nq, coef)``: the
     numerators ``S^T q`` float32 ``[T, heads * dv]``, ``n . q`` ``[T, heads]`` and per row and head ``(log a, log b,
-    m, -)``, which :func:`mlstm_out` turns into the mixer's output."""
+    m, -)``, which :func:`mlstm_out` turns into the mixer's output.  ``split``: requests of many rows may run in chunks
+    whose products are formed on the tensor cores, every float32 operand in bfloat16 pieces of 24 bits together;
+    ``max_rows``: the rows of the longest request, if known (a choice of kernels, no result depends on it but by rounding)."""
     _need(proj, "proj", torch.float32)
     _need(bias_i, "bias_i", torch.float32)
     _need(bias_f, "bias_f", torch.float32)
@@ -880,11 +908,14 @@ def mlstm_recurrence(proj: torch.Tensor, *, col_q: int, col_k: int, col_v: int, 
     coef = torch.empty((T, heads, 4), dtype=torch.float32, device=proj.device)
     o_raw = torch.empty((T, heads * dv), dtype=torch.float32, device=proj.device)
     nq = torch.empty((T, heads), dtype=torch.float32, device=proj.device)
+    chunks = _chunks("mlstm", T, B, max_rows, heads, d, dv, ld, col_q, col_k, col_v, per_head, state.stride(0),
+                     proj.data_ptr() // 4, state.data_ptr() // 4) if split else 0
+    sums = torch.empty(chunks * heads * (d * dv + d + 1), dtype=torch.float32, device=proj.device) if chunks else None
     check(kernel("sharpi_mlstm_recurrence")(proj.data_ptr(), ld, col_q, col_k, col_v, col_i, col_f, bias_i.data_ptr(),
                                             bias_f.data_ptr(), row_offsets.data_ptr(), state_slots.data_ptr(),
                                             state.data_ptr(), state.stride(0), per_head, B, T, heads, d, dv,
                                             float(cap), float(q_scale), coef.data_ptr(), o_raw.data_ptr(), nq.data_ptr(),
-                                            _stream()),
+                                            _ptr(sums), chunks, CHUNKED_LEAST, _stream()),
           "sharpi_mlstm_recurrence")
     return o_raw, nq, coef
 
@@ -1098,10 +1129,10 @@ WKV_MAX_HEAD_SIZE = 256
 
 def wkv_recurrence(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, wraw: torch.Tensor, w0: torch.Tensor,
                    u: torch.Tensor, *, row_offsets: torch.Tensor, state_slots: torch.Tensor, state: torch.Tensor,
-                   heads: int, d: int) -> torch.Tensor:
+                   heads: int, d: int, split: bool = False, max_rows: Optional[int] = None) -> torch.Tensor:
     """``o_t = (S + diag(u) k_t v_t^T)^T r_t``, ``S <- diag(exp(-exp(wraw_t + w0))) S + k_t v_t^T`` per head over
     the rows of every request, from and into ``state [slots, heads * d * d]``; float32 ``[T, heads * d]``.
-    ``wraw`` is overwritten (with the decay, for heads of up to 128 elements)."""
+    ``wraw`` is overwritten.  ``split``, ``max_rows``: as in :func:`mlstm_recurrence` (heads of up to 64 elements)."""
     for name, t in (("r", r), ("k", k), ("v", v), ("wraw", wraw), ("w0", w0), ("u", u), ("state", state)):
         _need(t, name, torch.float32)
     T = r.shape[0]
@@ -1111,10 +1142,15 @@ def wkv_recurrence(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, wraw: torc
         raise KernelError(f"state is {tuple(state.shape)}, expected [slots, {heads * d * d}]")
     o = torch.empty((T, heads * d), dtype=torch.float32, device=r.device)
     bonus = torch.empty((T, heads), dtype=torch.float32, device=r.device)
+    B = state_slots.numel()
+    chunks = _chunks("wkv", T, B, max_rows, heads, d, d, state.stride(0), v.data_ptr() // 4,
+                     state.data_ptr() // 4) if split and d <= 64 else 0
+    sums = torch.empty(chunks * heads * (d * d + 64), dtype=torch.float32, device=r.device) if chunks else None
     check(kernel("sharpi_wkv_recurrence")(r.data_ptr(), k.data_ptr(), v.data_ptr(), wraw.data_ptr(), w0.data_ptr(),
                                           u.data_ptr(), row_offsets.data_ptr(), state_slots.data_ptr(),
                                           state.data_ptr(), state.stride(0), o.data_ptr(), bonus.data_ptr(), T,
-                                          state_slots.numel(), heads, d, _stream()), "sharpi_wkv_recurrence")
+                                          B, heads, d, _ptr(sums), chunks, CHUNKED_LEAST, _stream()),
+          "sharpi_wkv_recurrence")
     return o
 
 
@@ -1394,20 +1430,27 @@ SSD_MAX_STATES = 256
 
 def ssd_scan(xbc: torch.Tensor, proj: torch.Tensor, *, col_x: int, col_b: int, col_c: int, col_dt: int,
              dt_bias: torch.Tensor, a_log: torch.Tensor, dskip: torch.Tensor, row_offsets: torch.Tensor,
-             state_slots: torch.Tensor, state: torch.Tensor, heads: int, groups: int, states: int, vdim: int) -> torch.Tensor:
+             state_slots: torch.Tensor, state: torch.Tensor, heads: int, groups: int, states: int, vdim: int,
+             split: bool = False, max_rows: Optional[int] = None) -> torch.Tensor:
     """The state-space-duality recurrence over the rows of every request, from and into ``state [slots, heads *
     states * vdim]``: ``y`` float32 ``[T, heads * vdim]``.  ``xbc`` float32 holds x, B and C at the given columns,
-    ``proj`` float32 the raw step sizes at ``col_dt``; ``dt = softplus(raw + dt_bias)``, decay ``exp(-exp(A_log) dt)``."""
+    ``proj`` float32 the raw step sizes at ``col_dt``; ``dt = softplus(raw + dt_bias)``, decay ``exp(-exp(A_log) dt)``.
+    ``split``, ``max_rows``: as in :func:`mlstm_recurrence`."""
     for name, t in (("xbc", xbc), ("proj", proj), ("dt_bias", dt_bias), ("a_log", a_log), ("dskip", dskip), ("state", state)):
         _need(t, name, torch.float32)
     T = xbc.shape[0]
     if state.shape[-1] != heads * states * vdim or min(dt_bias.numel(), a_log.numel(), dskip.numel()) < heads:
         raise KernelError("scan inputs disagree on heads, states or the value size")
     y = torch.empty((T, heads * vdim), dtype=torch.float32, device=xbc.device)
+    B = state_slots.numel()
+    chunks = _chunks("ssd", T, B, max_rows, heads, states, vdim, xbc.shape[1], col_x, col_b, col_c, state.stride(0),
+                     xbc.data_ptr() // 4, state.data_ptr() // 4) if split else 0
+    sums = torch.empty(chunks * heads * (states * vdim + 1), dtype=torch.float32, device=xbc.device) if chunks else None
     check(kernel("sharpi_ssd_scan")(xbc.data_ptr(), xbc.shape[1], col_x, col_b, col_c, proj.data_ptr(), proj.shape[1], col_dt,
                                     dt_bias.data_ptr(), a_log.data_ptr(), dskip.data_ptr(), row_offsets.data_ptr(),
                                     state_slots.data_ptr(), state.data_ptr(), state.stride(0), y.data_ptr(), T,
-                                    state_slots.numel(), heads, groups, states, vdim, _stream()), "sharpi_ssd_scan")
+                                    B, heads, groups, states, vdim, _ptr(sums), chunks, CHUNKED_LEAST, _stream()),
+          "sharpi_ssd_scan")
     return y
 
 

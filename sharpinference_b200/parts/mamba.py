@@ -116,7 +116,8 @@ class StateSpaceDualityMixer(Mixer):
         y = ops.ssd_scan(xbc, proj, col_x=0, col_b=self.inner, col_c=self.inner + self.groups * self.states,
                          col_dt=self.channels + self.inner, dt_bias=self.dt_bias, a_log=self.a_log, dskip=self.d_skip,
                          row_offsets=ctx.row_offsets, state_slots=ctx.state_slots, state=slot.states["S"],
-                         heads=self.heads, groups=self.groups, states=self.states, vdim=self.value_dim)
+                         heads=self.heads, groups=self.groups, states=self.states, vdim=self.value_dim,
+                         split=self.act_dtype == torch.bfloat16, max_rows=ctx.max_rows_per_request)
         u = ops.gated_group_norm(y, proj, self.channels, self.norm_weight, self.eps, self.norm_groups, self.act_dtype)
         return self.out(u)
 

@@ -16,8 +16,9 @@ multiplied by a weight and by ``sigmoid(Wg h_t)``, and projected by ``Wo``.  ``c
 The projections q, k, v, g and the two gate rows are one fused product whose result stays float32; from there on
 everything is float32: gates, exponentials, the state ``(S, n, m)`` and the products of the recurrence.  The state
 lives in the cache manager's per-request slots (zeroed when a request is admitted) and is carried from step to
-step, so a prompt may arrive in portions of any size and a decoded token is a portion of one row: a row's result
-is the same sequence of operations either way.
+step, so a prompt may arrive in portions of any size and a decoded token is a portion of one row.  Portions are walked
+row by row, the same operations for a row however a prompt is cut; in bfloat16 models long portions run in chunks of 64
+rows on the tensor cores with operands of 24 bits, whose sums are rounded in another order (``csrc/chunk_mma.cuh``).
 
 The reference keeps per-sequence state of fixed size for another recurrent layer
 (src/SharpInference.Engine/GdnStateCache.cs); the recurrence here is ``csrc/mlstm.cu``.
@@ -80,7 +81,7 @@ class MLSTMMixer(Mixer):
             p, col_q=self.col_q, col_k=self.col_k, col_v=self.col_v, col_i=self.col_i, col_f=self.col_f,
             bias_i=self.bias_i, bias_f=self.bias_f, row_offsets=ctx.row_offsets, state_slots=ctx.state_slots,
             state=slot.state, heads=self.heads, d=self.key_dim, dv=self.value_dim, cap=self.gate_cap,
-            q_scale=self.q_scale)
+            q_scale=self.q_scale, split=self.act_dtype == torch.bfloat16, max_rows=ctx.max_rows_per_request)
         o = ops.mlstm_out(num, nq, coef, p, self.col_g, self.head_norm_weight, self.eps, self.heads, self.value_dim,
                           self.act_dtype)
         return self.out(o)

@@ -14,9 +14,10 @@ by the gate, and projected by ``W_o``.
 The mixes, the decay with its two exponentials, the state and every product of the recurrence are float32; the
 projections round their inputs to the activation dtype.  Two things are per-request state: the previous input
 ``h'`` (``state_specs["prev"]``) and ``S`` (``state_specs["S"]``, ``[heads, d, d]``, key channel first), both zero
-at a sequence's start; a prompt may therefore arrive in portions of any size, and a row's result is the same
-sequence of operations either way (``csrc/wkv.cu``).  The reference keeps per-sequence state of fixed size for
-another recurrent layer (src/SharpInference.Engine/GdnStateCache.cs).
+at a sequence's start; a prompt may therefore arrive in portions of any size.  Portions are walked row by row, the same
+operations for a row however a prompt is cut; in bfloat16 models long portions run in chunks of 64 rows on the tensor
+cores with operands of 24 bits, whose sums are rounded in another order (``csrc/wkv.cu``).  The reference keeps
+per-sequence state of fixed size for another recurrent layer (src/SharpInference.Engine/GdnStateCache.cs).
 """
 from __future__ import annotations
 
@@ -87,5 +88,6 @@ class WKVMixer(Mixer):
             r, k, v, g = self.r(mixes[0]), self.k(mixes[1]), self.v(mixes[2]), self.g(mixes[3])
         wraw = self.w2(ops.tanh(self.w1(mixes[4]), self.act_dtype))
         o = ops.wkv_recurrence(r, k, v, wraw, self.w0, self.u, row_offsets=ctx.row_offsets,
-                               state_slots=ctx.state_slots, state=slot.states["S"], heads=self.heads, d=self.head_dim)
+                               state_slots=ctx.state_slots, state=slot.states["S"], heads=self.heads, d=self.head_dim,
+                               split=self.act_dtype == torch.bfloat16, max_rows=ctx.max_rows_per_request)
         return self.out(ops.wkv_out(o, g, self.head_norm_weight, self.eps, self.heads, self.head_dim, self.act_dtype))

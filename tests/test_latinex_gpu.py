@@ -188,6 +188,41 @@ def test_state_space_duality_scan(heads, groups, N, P):
     assert float(state[4].min()) == 7.0 and float(state[1].abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("heads,groups,N,P", [(4, 2, 16, 8), (6, 1, 128, 64), (3, 3, 64, 100), (10, 2, 68, 36), (1, 1, 4, 4)])
+def test_state_space_duality_in_chunks(monkeypatch, heads, groups, N, P):
+    """Requests on both sides of the border between walk and chunks in one step and a step that goes on from their state,
+    against the plain walk in 64 bits, at the tolerance that the float32 walk is held to above."""
+    from sharpinference_b200.kernels import ops
+    monkeypatch.setattr(ops, "_WALK_OR_CHUNKS", dict.fromkeys(ops._WALK_OR_CHUNKS, (1e9, 1, 0.0)))       # in chunks whatever is faster
+    g = torch.Generator().manual_seed(heads * 1000 + N + P)
+    inner, bc = heads * P, groups * N
+    cuts = ([ops.CHUNKED_LEAST, 1, 300, ops.CHUNKED_LEAST - 1], [129, 40, 200, 3])
+    lens = [sum(c[b] for c in cuts) for b in range(4)]
+    seqs = [0.7 * torch.randn(n, inner + 2 * bc, generator=g, dtype=F64) for n in lens]
+    dts = [torch.randn(n, heads, generator=g, dtype=F64) for n in lens]
+    dt_bias, a_log = -2.0 + 2.0 * torch.rand(heads, generator=g, dtype=F64), -3.0 + 5.0 * torch.rand(heads, generator=g, dtype=F64)
+    dskip = torch.randn(heads, generator=g, dtype=F64)
+    want = [_plain_ssd(s[:, :inner].reshape(-1, heads, P), s[:, inner:inner + bc].reshape(-1, groups, N),
+                       s[:, inner + bc:].reshape(-1, groups, N), d, dt_bias, a_log, dskip, heads, groups) for s, d in zip(seqs, dts)]
+    states = [torch.zeros(5, heads * N * P, device=DEV) for _ in range(2)]
+    got, at = [[] for _ in seqs], [0] * 4
+    for cut in cuts:
+        _, off, sl = _step_meta(cut, [4, 0, 2, 3])
+        xbc = torch.cat([seqs[b][at[b]:at[b] + cut[b]] for b in range(4)])
+        dt = torch.cat([dts[b][at[b]:at[b] + cut[b]] for b in range(4)])
+        y = [ops.ssd_scan(f32(xbc), f32(dt), col_x=0, col_b=inner, col_c=inner + bc, col_dt=0, dt_bias=f32(dt_bias),
+                          a_log=f32(a_log), dskip=f32(dskip), row_offsets=off, state_slots=sl, state=st, heads=heads,
+                          groups=groups, states=N, vdim=P, split=split) for st, split in zip(states, (True, False))]
+        r = 0
+        for b in range(4):
+            got[b].append(y[0][r:r + cut[b]].double().cpu())
+            r += cut[b]
+            at[b] += cut[b]
+        assert float((states[0] - states[1]).abs().max()) <= 1e-5 * max(1.0, float(states[1].abs().max()))
+    for b in range(4):
+        assert float((torch.cat(got[b]) - want[b]).abs().max()) < 2e-5 * max(float(want[b].abs().max()), 1.0)
+
+
 @pytest.mark.parametrize("N,P", [(48, 24), (64, 32), (128, 64)])
 def test_scan_rows_do_not_depend_on_the_cut(N, P):
     """The walk adds a row's parts in one fixed order: a prompt in one step and the same prompt in portions of 1, 2

@@ -290,6 +290,37 @@ def test_mlstm_recurrence_kernel(heads, d, dv):
         assert torch.allclose(nq_got, nq_want, atol=3e-5 * max(1.0, float(nq_want.abs().max()))), b
 
 
+@pytest.mark.parametrize("heads,d,dv", [(2, 24, 40), (3, 64, 64), (1, 128, 256), (2, 68, 132), (1, 4, 4)])
+def test_mlstm_recurrence_in_chunks(monkeypatch, heads, d, dv):
+    """Requests on both sides of the border between walk and chunks in one step, then a step that goes on from the state they
+    left: numerators, n . q, running maximum and state as the walk leaves them, up to float32 rounding of sums of up to 300
+    terms (both forms are held to 2e-5 of the largest value against the plain recurrence elsewhere; here to 1e-5 of each
+    other), from gates over their whole range."""
+    from sharpinference_b200.kernels import ops
+    monkeypatch.setattr(ops, "_WALK_OR_CHUNKS", dict.fromkeys(ops._WALK_OR_CHUNKS, (1e9, 1, 0.0)))       # in chunks whatever is faster
+    from sharpinference_b200.parts.mlstm import fused_mlstm_columns
+    g = torch.Generator().manual_seed(heads * 1000 + d)
+    cq, ck, cv, cg, ci, cf, width = fused_mlstm_columns(heads, d, dv)
+    per_request = ops.mlstm_state_floats(heads, d, dv)[1]
+    bias = torch.randn(2, heads, generator=g).to(DEV)
+    states = [torch.zeros(6, per_request, device=DEV) for _ in range(2)]
+    for lens in ([ops.CHUNKED_LEAST, 1, 300, ops.CHUNKED_LEAST - 1], [129, 40, 193, 2], [257]):
+        T = sum(lens)
+        proj = torch.randn(T, width, generator=g)
+        proj[:, ci:ci + heads] *= 4.0
+        proj[:, cf:cf + heads] = proj[:, cf:cf + heads] * 4.0 + 2.0
+        offs = torch.tensor([sum(lens[:i]) for i in range(len(lens) + 1)], dtype=torch.int32, device=DEV)
+        slots = torch.tensor([4, 0, 2, 5][:len(lens)], dtype=torch.int32, device=DEV)
+        out = [ops.mlstm_recurrence(proj.to(DEV), col_q=cq, col_k=ck, col_v=cv, col_i=ci, col_f=cf, bias_i=bias[0], bias_f=bias[1],
+                                    row_offsets=offs, state_slots=slots, state=st, heads=heads, d=d, dv=dv, cap=9.0,
+                                    q_scale=d ** -0.5, split=split) for st, split in zip(states, (False, True))]
+        assert torch.equal(out[0][2][..., :3], out[1][2][..., :3])
+        for a, b in [(out[0][0], out[1][0]), (out[0][1], out[1][1]), tuple(states)]:
+            assert float((a - b).abs().max()) <= 1e-5 * max(1.0, float(a.abs().max()))
+        short = [r for i, n in enumerate(lens) if n < ops.CHUNKED_LEAST for r in range(int(offs[i]), int(offs[i + 1]))]
+        assert torch.equal(out[0][0][short], out[1][0][short])
+
+
 def test_mlstm_out_kernel():
     from sharpinference_b200.kernels import ops
     g = torch.Generator().manual_seed(9)

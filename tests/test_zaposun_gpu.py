@@ -286,6 +286,29 @@ def test_convolution_and_selective_scan_kernels(C, N, R, taps):
         assert float((scan_state[slot].double().cpu().view(C, N) - want[b][2]).abs().max()) < 3e-5 * max(1.0, float(want[b][2].abs().max()))
 
 
+@pytest.mark.parametrize("heads,d", [(2, 64), (3, 20), (1, 4), (5, 48)])
+def test_wkv_recurrence_in_chunks(monkeypatch, heads, d):
+    """Requests on both sides of the border between walk and chunks in one step, then a step that goes on from their state:
+    outputs and state as the float32 walk leaves them, from decays next to one down to decays that vanish within a row
+    (both forms are sums of at most 300 products a value, rounded in another order: 1e-5 of the largest)."""
+    from sharpinference_b200.kernels import ops
+    monkeypatch.setattr(ops, "_WALK_OR_CHUNKS", dict.fromkeys(ops._WALK_OR_CHUNKS, (1e9, 1, 0.0)))       # in chunks whatever is faster
+    g = torch.Generator().manual_seed(heads * 100 + d)
+    hd = heads * d
+    u, w0 = torch.randn(hd, generator=g).to(DEV), torch.linspace(-8.0, 2.5, hd).to(DEV)
+    states = [torch.zeros(6, heads * d * d, device=DEV) for _ in range(2)]
+    for lens in ([ops.CHUNKED_LEAST, 1, 300, ops.CHUNKED_LEAST - 1], [129, 40, 193, 2], [257]):
+        T = sum(lens)
+        _, off, sl = _step_meta(lens, [4, 0, 2, 5][:len(lens)])
+        r, k, v, w = (torch.randn(T, hd, generator=g).to(DEV) for _ in range(4))
+        out = [ops.wkv_recurrence(r, k, v, w.clone(), w0, u, row_offsets=off, state_slots=sl, state=st, heads=heads, d=d, split=split)
+               for st, split in zip(states, (False, True))]
+        for a, b in (tuple(out), tuple(states)):
+            assert float((a - b).abs().max()) <= 1e-5 * max(1.0, float(a.abs().max()))
+        short = [x for i, n in enumerate(lens) if n < ops.CHUNKED_LEAST for x in range(sum(lens[:i]), sum(lens[:i + 1]))]
+        assert torch.equal(out[0][short], out[1][short])
+
+
 @pytest.mark.parametrize("taps", [1, 2, 3, 4])
 @pytest.mark.parametrize("C,dtype", [(6000, torch.bfloat16), (5620, torch.float32), (5120, torch.bfloat16)])
 def test_causal_convolution_rows_at_a_time(taps, C, dtype):
