@@ -27,6 +27,13 @@
 // Two optional rules: a score cap (the CAP kernels: softcap * tanh(s / softcap) on the scaled score, formed from the
 // raw score with one ex2 and one division), and a sink per head whose exponential joins the row's denominator.
 //
+// KEYS: pages that hold keys only, a value being the leading DV elements of its key row (attention whose values are its keys,
+// latent attention).  A key block is loaded once and is the right operand of both products, K-major for the scores and
+// MN-major for the sums: the same bytes in shared memory.  The tile list cuts 64 rows there, so a CTA serves two query heads of
+// one key head, rows 0-63 and 64-127 of the MMA.  One CTA an SM at the larger sizes (the queries alone take 80 KB at 320
+// elements), three key blocks in flight.  16 heads on one row of 320 with sums of 256, a prompt of 2048 rows: 54 us, 269 us
+// with m16n8k16 (attention_keys.cu, which keeps the sizes, masks and biases that this form does not take).
+//
 // Sizes: head size 64 or 128, pages of a multiple of 64 positions, bf16.  Everything else takes the
 // warp-level kernel (attention_prefill.cu) or the generic one.  The reference's counterparts are the
 // f16 mma.sync prefill kernels (src/SharpInference.Cuda/CudaTextKernels.cs:7657, :8086-8110).
@@ -42,7 +49,6 @@ constexpr int TQ = 128;        // query rows per CTA (MMA M)
 constexpr int TK = 64;         // keys per block
 constexpr int SOFTMAX_WARPS = 8;
 constexpr int TC_ATT_THREADS = (SOFTMAX_WARPS + 2) * 32;
-constexpr int KV_STAGES = 2;
 
 struct PrefillTcArgs {
     const int* block_table;   // [B, max_blocks]
@@ -89,26 +95,30 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
 
 enum { ERR_Q = 11, ERR_K = 12, ERR_V = 13, ERR_S = 14, ERR_P = 15, ERR_O = 16, ERR_EMPTY = 17, ERR_ALIGN = 18 };
 
-template <int D>
+template <int D, int DV = D, bool KEYS = false>
 struct AttCfg {
     static constexpr int HALVES = D / 64;
+    static constexpr int KV_STAGES = KEYS && D <= 320 ? 3 : 2;
     static constexpr int Q_BYTES = TQ * D * 2;
     static constexpr int KV_BYTES = TK * D * 2;           // one K or V block
     static constexpr int P_BYTES = TQ * TK * 2;
     static constexpr int BAR_BYTES = 256;
     // the dynamic shared memory window has to start on a 1024-byte boundary (the kernel checks): there
     // is no room for padding when two CTAs of head size 128 share an SM
-    static constexpr int SMEM = Q_BYTES + 2 * KV_STAGES * KV_BYTES + P_BYTES + BAR_BYTES;
+    static constexpr int SMEM = Q_BYTES + (KEYS ? 1 : 2) * KV_STAGES * KV_BYTES + P_BYTES + BAR_BYTES;
     static constexpr int S_COL = 0;                        // S[2]: 64 columns each
-    static constexpr int O_COL = 2 * TK;                   // O: D columns
-    static constexpr int TMEM_COLS = 256;                  // 128 + D <= 256
+    static constexpr int O_COL = 2 * TK;                   // O: DV columns
+    static constexpr int TMEM_COLS = DV <= 128 ? 256 : 512;  // 128 + DV
+    static constexpr int CTAS = TMEM_COLS == 256 && SMEM <= 113 * 1024 ? 2 : 1;      // an SM
 };
 
-template <int D, bool CAP>
-__global__ void __launch_bounds__(TC_ATT_THREADS, 2)
+template <int D, int DV, bool CAP, bool KEYS>
+__global__ void __launch_bounds__(TC_ATT_THREADS, (AttCfg<D, DV, KEYS>::CTAS))
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap kv_map,
                        const PrefillTcArgs a) {
-    using Cfg = AttCfg<D>;
+    using Cfg = AttCfg<D, DV, KEYS>;
+    constexpr int KV_STAGES = Cfg::KV_STAGES;
+    constexpr int HEADS = KEYS ? 2 : 1, TILE = TQ / HEADS;      // query heads of a CTA, rows of each
     extern __shared__ __align__(1024) uint8_t smem[];
     if (smem_u32(smem) & 1023u) {                  // the swizzled tiles need it; nothing has been set up yet
         if (threadIdx.x == 0) atomicExch(a.status, ERR_ALIGN);
@@ -116,7 +126,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
     }
     uint8_t* q_s = smem;
     uint8_t* k_s = q_s + Cfg::Q_BYTES;                          // [stages][halves][64 keys][64]
-    uint8_t* v_s = k_s + KV_STAGES * Cfg::KV_BYTES;
+    uint8_t* v_s = KEYS ? k_s : k_s + KV_STAGES * Cfg::KV_BYTES;
     uint8_t* p_s = v_s + KV_STAGES * Cfg::KV_BYTES;             // [128 rows][64 keys]
     uint64_t* bars = reinterpret_cast<uint64_t*>(p_s + Cfg::P_BYTES);
     uint64_t* q_full = bars;
@@ -136,7 +146,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
     const int* tile = a.tiles + (size_t)(gridDim.y - 1 - blockIdx.y) * 4;
     const int row0 = tile[0], n_rows = tile[1], p0 = tile[2];
     const int* table = a.block_table + (size_t)tile[3] * a.max_blocks;
-    const int head = blockIdx.x;
+    const int head = blockIdx.x * HEADS;
     const int kvh = head / (a.nq / a.nkv);
     const int p_last = p0 + n_rows - 1;
     const int key_lo = visible_lo(p0, a.mask_kind, a.mask_span);
@@ -170,7 +180,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             mbar_arrive_expect_tx(q_full, Cfg::Q_BYTES);
 #pragma unroll
             for (int hf = 0; hf < Cfg::HALVES; ++hf)
-                tma_load_2d(q_s + hf * TQ * 128, &q_map, q_full, head * D + hf * 64, row0);
+#pragma unroll
+                for (int e = 0; e < HEADS; ++e)
+                    tma_load_2d(q_s + hf * TQ * 128 + e * TILE * 128, &q_map, q_full, (head + e) * D + hf * 64, row0);
             bool ok = true;
             for (int j = 0; j < n_blocks && ok; ++j) {
                 const int st = j % KV_STAGES, use = j / KV_STAGES;
@@ -178,14 +190,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 const int blk = key0 >> a.page_shift;
                 const int page = table[blk];
                 const int off = key0 - (blk << a.page_shift);
-                const int row_k = ((page * 2 + 0) * a.nkv + kvh) * a.page_size + off;
-                const int row_v = ((page * 2 + 1) * a.nkv + kvh) * a.page_size + off;
+                const int row_k = (page * (KEYS ? 1 : 2) * a.nkv + kvh) * a.page_size + off;
                 if (use > 0) ok = mbar_wait(&k_empty[st], (use - 1) & 1);
                 if (!ok) { atomicExch(a.status, ERR_EMPTY); break; }
                 mbar_arrive_expect_tx(&k_full[st], Cfg::KV_BYTES);
 #pragma unroll
                 for (int hf = 0; hf < Cfg::HALVES; ++hf)
                     tma_load_2d(k_s + st * Cfg::KV_BYTES + hf * TK * 128, &kv_map, &k_full[st], hf * 64, row_k);
+                if (KEYS) continue;
+                const int row_v = row_k + a.nkv * a.page_size;
                 if (use > 0) ok = mbar_wait(&v_empty[st], (use - 1) & 1);
                 if (!ok) { atomicExch(a.status, ERR_EMPTY); break; }
                 mbar_arrive_expect_tx(&v_full[st], Cfg::KV_BYTES);
@@ -198,13 +211,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         // ---- MMA issuer ------------------------------------------------------------------------
         if (lane == 0) {
             const uint32_t idesc_qk = instr_desc_bf16(TQ, TK);
-            const uint32_t idesc_pv = instr_desc_bf16(TQ, D, true);
+            const uint32_t idesc_pv = instr_desc_bf16(TQ, DV, true);
             bool ok = mbar_wait(q_full, 0);
             if (!ok) atomicExch(a.status, ERR_Q);
             auto pv = [&](int i) -> bool {
                 const int st = i % KV_STAGES;
                 if (!mbar_wait(p_full, i & 1)) { atomicExch(a.status, ERR_P); return false; }
-                if (!mbar_wait(&v_full[st], (i / KV_STAGES) & 1)) { atomicExch(a.status, ERR_V); return false; }
+                if (!KEYS && !mbar_wait(&v_full[st], (i / KV_STAGES) & 1)) { atomicExch(a.status, ERR_V); return false; }
                 tcgen05_fence_after();
                 const uint8_t* pt = p_s;
                 const uint8_t* vt = v_s + st * Cfg::KV_BYTES;
@@ -212,7 +225,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 for (int ks = 0; ks < TK / 16; ++ks)
                     mma_bf16_ss(tmem_base + Cfg::O_COL, smem_desc_k_sw128(pt, ks * 32),
                                 smem_desc_mn_sw128(vt, TK * 128, ks * 2048), idesc_pv, (i | ks) != 0);
-                mma_commit(&v_empty[st]);
+                mma_commit(KEYS ? &k_empty[st] : &v_empty[st]);
                 mma_commit(pv_done);
                 return true;
             };
@@ -227,7 +240,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                     mma_bf16_ss(tmem_base + Cfg::S_COL + (j & 1) * TK,
                                 smem_desc_k_sw128(q_s + (ks / 4) * TQ * 128, (ks % 4) * 32),
                                 smem_desc_k_sw128(kt + (ks / 4) * TK * 128, (ks % 4) * 32), idesc_qk, ks != 0);
-                mma_commit(&k_empty[st]);
+                if (!KEYS) mma_commit(&k_empty[st]);
                 mma_commit(&s_full[j & 1]);
                 if (j >= 1) ok = pv(j - 1);
             }
@@ -238,7 +251,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         constexpr int HALF = TK / 2;                         // keys of a block per thread
         const int quarter = warp & 3, half = warp >> 2;
         const int r = quarter * 32 + lane;
-        const int pos_r = p0 + r;
+        const int pos_r = p0 + r % TILE;
         const int lo_r = visible_lo(pos_r, a.mask_kind, a.mask_span);
         const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
         constexpr float RAISE = 8.0f;       // in log2 units: the reference maximum lags by at most this much
@@ -297,7 +310,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
             // share the decision to touch O (and the row's two warps decide alike), each row uses its own factor
             const bool raise = m_blk > m_ref + RAISE;               // also true for the row's first visible block
             if (__any_sync(0xffffffffu, raise)) {
-                const float m_new = fmaxf(m_ref, m_blk);
+                // KEYS: a row whose own maximum need not rise keeps it (factor 1): its numbers do not depend on its neighbours
+                const float m_new = KEYS && !raise ? m_ref : fmaxf(m_ref, m_blk);
                 const float factor = (m_ref == -INFINITY) ? 0.0f : exp2f(m_ref - m_new);   // nothing of value in O yet
                 if (j > 0) {
                     // O holds the sums of blocks 0 .. j-1 once the PV of block j-1 is complete; this thread
@@ -305,7 +319,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                     if (!mbar_wait(pv_done, (j - 1) & 1)) { atomicExch(a.status, ERR_O); ok = false; break; }
                     tcgen05_fence_after();
 #pragma unroll
-                    for (int c0 = half * (D / 2); c0 < (half + 1) * (D / 2); c0 += 32) {
+                    for (int c0 = half * (DV / 2); c0 < (half + 1) * (DV / 2); c0 += 32) {
                         uint32_t v[32];
                         tmem_ld_32_nowait(lane_addr + Cfg::O_COL + c0, v);
                         tmem_ld_wait();
@@ -362,7 +376,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         float l_row = l_s[r] + l_s[TQ + r];                // the same order in both threads
         float shrink = 1.0f;
         if (a.sinks && m_ref != -INFINITY) {               // the sink against the row's reference (log2 units), whichever is larger
-            const float sink = a.sinks[head] * 1.4426950408889634f;
+            const float sink = a.sinks[head + r / TILE] * 1.4426950408889634f;
             if (sink > m_ref) {
                 shrink = exp2f(m_ref - sink);
                 l_row = l_row * shrink + 1.0f;
@@ -373,13 +387,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
         if (ok) {
             tcgen05_fence_after();
             const float inv = shrink / l_row;
-            bf16* dst = a.out + ((size_t)(row0 + r) * a.nq + head) * D;
+            bf16* dst = a.out + ((size_t)(row0 + r % TILE) * a.nq + head + r / TILE) * DV;
 #pragma unroll
-            for (int c0 = half * (D / 2); c0 < (half + 1) * (D / 2); c0 += 32) {
+            for (int c0 = half * (DV / 2); c0 < (half + 1) * (DV / 2); c0 += 32) {
                 uint32_t v[32];
                 tmem_ld_32_nowait(lane_addr + Cfg::O_COL + c0, v);      // whole-warp operation: all rows take part
                 tmem_ld_wait();
-                if (r < n_rows) {
+                if (r % TILE < n_rows) {
 #pragma unroll
                     for (int c = 0; c < 32; c += 8) {
                         uint4 w;
@@ -403,17 +417,17 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
     }
 }
 
-template <int D, bool CAP>
+template <int D, bool CAP, int DV = D, bool KEYS = false>
 static int launch_tc(const CUtensorMap& qm, const CUtensorMap& kvm, const PrefillTcArgs& a, int n_tiles, cudaStream_t stream) {
-    using Cfg = AttCfg<D>;
+    using Cfg = AttCfg<D, DV, KEYS>;
     static bool configured = false;
     if (!configured) {
-        if (cudaFuncSetAttribute(attn_prefill_tc_kernel<D, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM) !=
+        if (cudaFuncSetAttribute(attn_prefill_tc_kernel<D, DV, CAP, KEYS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM) !=
             cudaSuccess)
             return SHARPI_LAUNCH_FAILED;
         configured = true;
     }
-    attn_prefill_tc_kernel<D, CAP><<<dim3(a.nq, n_tiles), TC_ATT_THREADS, Cfg::SMEM, stream>>>(qm, kvm, a);
+    attn_prefill_tc_kernel<D, DV, CAP, KEYS><<<dim3(KEYS ? a.nq / 2 : a.nq, n_tiles), TC_ATT_THREADS, Cfg::SMEM, stream>>>(qm, kvm, a);
     SHARPI_CHECK_LAUNCH();
     return SHARPI_OK;
 }
@@ -452,4 +466,51 @@ SHARPI_API int sharpi_attention_prefill_tc(const void* q, const void* kv, const 
     }
     if (d == 64) return launch_tc<64, false>(qm, kvm, a, n_tiles, stream);
     return launch_tc<128, false>(qm, kvm, a, n_tiles, stream);
+}
+
+// Keys-only pages: q [T, nq, D], kv [num_pages, 1, nkv, page_size, D] bf16, the value of a key the first dv elements of its row;
+// tiles of up to 64 rows; an even number of query heads a key head; full or window mask without kept positions.
+template <int D>
+static int launch_keys(int dv, const CUtensorMap& qm, const CUtensorMap& kvm, const PrefillTcArgs& a, int n_tiles, cudaStream_t stream) {
+    if (dv == 64) return launch_tc<D, false, 64, true>(qm, kvm, a, n_tiles, stream);
+    if constexpr (D >= 128)
+        if (dv == 128) return launch_tc<D, false, 128, true>(qm, kvm, a, n_tiles, stream);
+    if constexpr (D >= 192)
+        if (dv == 192) return launch_tc<D, false, 192, true>(qm, kvm, a, n_tiles, stream);
+    if constexpr (D >= 256)
+        if (dv == 256) return launch_tc<D, false, 256, true>(qm, kvm, a, n_tiles, stream);
+    return SHARPI_BAD_ARGUMENT;
+}
+
+SHARPI_API int sharpi_attention_keys_prefill_tc(const void* q, const void* kv, const int* block_table, const int* tiles,
+                                                void* out, int* status, int T, int num_pages, int n_tiles, int nq, int nkv,
+                                                int D, int dv, int max_blocks, int page_size, int mask_kind, int mask_span,
+                                                float scale, cudaStream_t stream) {
+    if (n_tiles <= 0) return SHARPI_OK;
+    if (n_tiles > 65535 || nq <= 0 || nkv <= 0 || nq % nkv != 0 || (nq / nkv) % 2 != 0 || max_blocks <= 0 || !status)
+        return SHARPI_BAD_ARGUMENT;
+    if (!(scale > 0.0f) || page_size < 64 || (page_size & (page_size - 1)) != 0) return SHARPI_BAD_ARGUMENT;
+    if (mask_kind != SHARPI_MASK_FULL && mask_span <= 0) return SHARPI_BAD_ARGUMENT;
+    if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(kv) | reinterpret_cast<uintptr_t>(out)) & 15)
+        return SHARPI_UNALIGNED;
+    CUtensorMap qm, kvm;
+    if (!tmap::make_bf16_map(&qm, q, (uint64_t)nq * D, (uint64_t)T, 0, 64, TQ / 2)) return SHARPI_LAUNCH_FAILED;
+    if (!tmap::make_bf16_map(&kvm, kv, (uint64_t)D, (uint64_t)num_pages * nkv * page_size, 0, 64, TK)) return SHARPI_LAUNCH_FAILED;
+    PrefillTcArgs a;
+    a.block_table = block_table; a.tiles = tiles; a.out = (bf16*)out; a.status = status;
+    a.nq = nq; a.nkv = nkv; a.max_blocks = max_blocks; a.page_size = page_size; a.mask_kind = mask_kind;
+    a.mask_span = mask_span; a.scale_log2 = scale * 1.4426950408889634f;
+    a.page_shift = 0;
+    while ((1 << a.page_shift) < page_size) ++a.page_shift;
+    a.sinks = nullptr;
+    a.cap_in = a.cap_out = 0.0f;
+    switch (D) {
+        case 64: return launch_keys<64>(dv, qm, kvm, a, n_tiles, stream);
+        case 128: return launch_keys<128>(dv, qm, kvm, a, n_tiles, stream);
+        case 192: return launch_keys<192>(dv, qm, kvm, a, n_tiles, stream);
+        case 256: return launch_keys<256>(dv, qm, kvm, a, n_tiles, stream);
+        case 320: return launch_keys<320>(dv, qm, kvm, a, n_tiles, stream);
+        case 384: return launch_keys<384>(dv, qm, kvm, a, n_tiles, stream);
+    }
+    return SHARPI_BAD_ARGUMENT;
 }

@@ -326,6 +326,15 @@ def keys_attention_supported(dtype: torch.dtype, d: int, dv: int) -> bool:
     return dtype == torch.bfloat16 and d % 16 == 0 and dv % 16 == 0 and 0 < dv <= d <= 512
 
 
+def keys_prefill_tc_supported(nq: int, nkv: int, d: int, dv: int, page_size: int, keep_first: int, biased: bool,
+                              scale: float) -> bool:
+    """Whether the tcgen05 kernel takes a prompt tile over keys-only pages: rows of 64 to 384 elements and values of 64 to 256,
+    multiples of 64 (what tensor memory and shared memory hold beside the scores and two heads' queries), an even number of
+    query heads a key head, pages of 64 * 2^k positions, no distance bias and no kept positions."""
+    return (d % 64 == 0 and d <= 384 and dv % 64 == 0 and dv <= 256 and (nq // nkv) % 2 == 0 and page_size >= 64
+            and page_size & (page_size - 1) == 0 and not keep_first and not biased and scale > 0)
+
+
 def attention_keys_prefill(q: torch.Tensor, kv_layer: torch.Tensor, block_table: torch.Tensor, tiles: torch.Tensor,
                            out: torch.Tensor, *, nq: int, nkv: int, d: int, dv: int, page_size: int, mask_kind: int,
                            mask_span: int, scale: float, keep_first: int = 0,
@@ -344,6 +353,13 @@ def attention_keys_prefill(q: torch.Tensor, kv_layer: torch.Tensor, block_table:
         _need(dist_bias, "dist_bias", torch.float32)
         if dist_bias.dim() != 2 or dist_bias.shape[1] != nq:
             raise KernelError(f"dist_bias is {tuple(dist_bias.shape)}, expected [far + 1, {nq}]")
+    if keys_prefill_tc_supported(nq, nkv, d, dv, page_size, keep_first, dist_bias is not None, scale):
+        check(kernel("sharpi_attention_keys_prefill_tc")(q.data_ptr(), kv_layer.data_ptr(), block_table.data_ptr(),
+                                                         tiles.data_ptr(), out.data_ptr(), status_word(q.device).data_ptr(),
+                                                         q.numel() // (nq * d), kv_layer.shape[0], tiles.shape[0], nq, nkv, d, dv,
+                                                         block_table.shape[-1], page_size, mask_kind, mask_span, float(scale),
+                                                         _stream()), "sharpi_attention_keys_prefill_tc")
+        return
     check(kernel("sharpi_attention_keys_prefill")(q.data_ptr(), kv_layer.data_ptr(), block_table.data_ptr(), tiles.data_ptr(),
                                                   out.data_ptr(), tiles.shape[0], nq, nkv, d, dv, block_table.shape[-1],
                                                   page_size, mask_kind, mask_span, int(keep_first), _ptr(dist_bias),

@@ -394,6 +394,35 @@ def test_tensor_core_attention_over_keys_only_pages(nq, nkv, d, dv, page):
     assert torch.equal(other[:233], out[:233])
 
 
+@pytest.mark.parametrize("nq,nkv,d,dv", [(16, 1, 320, 256), (4, 2, 128, 128), (2, 1, 64, 64), (4, 1, 384, 192), (6, 1, 256, 64), (2, 1, 192, 128)])
+@pytest.mark.parametrize("window", [0, 100, 64])
+def test_tcgen05_attention_over_keys_only_pages(nq, nkv, d, dv, window):
+    """Two heads a CTA, one key block as both operands: tiles of every length and start, whole blocks behind the window, key
+    blocks that wrap around the ring, against softmax in 64 bits; a row's bits do not depend on the tile it is cut into.
+    bfloat16 probabilities and output: the tolerance of the test above."""
+    from sharpinference_b200.kernels import ops
+    g = torch.Generator().manual_seed(d + dv + window)
+    n, page = 400, 128
+    assert ops.keys_prefill_tc_supported(nq, nkv, d, dv, page, 0, False, 0.1)
+    keys, q = torch.randn(n, nkv, d, generator=g).to(torch.bfloat16), torch.randn(n, nq, d, generator=g).to(torch.bfloat16)
+    scale = d ** -0.5
+    vis = plain.window_with_first(n, window, 0) if window else plain.causal(n)
+    want = torch.stack([plain.softmax_rows(q[:, h].double() @ keys[:, h // (nq // nkv)].double().T * scale, vis)
+                        @ keys[:, h // (nq // nkv), :dv].double() for h in range(nq)], dim=1)
+    kv, bt = _paged_keys(keys.float(), page, seed=d)
+    kv, bt = kv.to(torch.bfloat16).to(DEV), bt.to(DEV)
+    outs = []
+    for cut in ([64, 64, 1, 63, 64, 64, 64, 16], [5, 64, 64, 64, 33, 64, 64, 42]):
+        starts = [sum(cut[:i]) for i in range(len(cut))]
+        tiles = torch.tensor([[s, c, s, 0] for s, c in zip(starts, cut)], dtype=torch.int32, device=DEV)
+        outs.append(torch.zeros(n, nq * dv, dtype=torch.bfloat16, device=DEV))
+        ops.attention_keys_prefill(q.to(DEV).view(n, nq * d), kv, bt, tiles, outs[-1], nq=nq, nkv=nkv, d=d, dv=dv, page_size=page,
+                                   mask_kind=ops.MASK_WINDOW if window else ops.MASK_FULL, mask_span=max(window, 1), scale=scale)
+        ops.check_status(DEV)
+        assert float((outs[-1].double().cpu().view(n, nq, dv) - want).abs().max()) < 3e-2
+    assert torch.equal(outs[0], outs[1])
+
+
 @pytest.mark.parametrize("d,dv,window,keep", [(80, 80, 100, 3), (320, 256, 300, 70), (128, 128, 256, 0), (16, 16, 7, 257)])
 def test_single_rows_with_whole_splits_behind_the_window(d, dv, window, keep):
     """Single rows deep in a sequence of 1200 positions: between the kept first positions and the window lie whole
