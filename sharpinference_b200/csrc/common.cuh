@@ -76,6 +76,13 @@ template <typename T> __device__ __forceinline__ T from_float(float v);
 template <> __device__ __forceinline__ float from_float<float>(float v) { return v; }
 template <> __device__ __forceinline__ bf16 from_float<bf16>(float v) { return __float2bfloat16_rn(v); }
 
+// Four neighbouring elements at once (16 or 8 bytes)
+__device__ __forceinline__ void store_four(float* p, const float (&v)[4]) { *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]); }
+__device__ __forceinline__ void store_four(bf16* p, const float (&v)[4]) {
+    const bf16 b[4] = {from_float<bf16>(v[0]), from_float<bf16>(v[1]), from_float<bf16>(v[2]), from_float<bf16>(v[3])};
+    *reinterpret_cast<uint2*>(p) = *reinterpret_cast<const uint2*>(b);
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -267,11 +267,57 @@ gated_group_norm_kernel(const float* y, const float* z, int ld_z, const float* _
     }
 }
 
+// The same for parts of at most 4096 elements, a multiple of four, on 16 bytes: the part in registers, read once and all at once.
+// 1777 rows of 4096: 36 us with two passes of scalar loads, 18 us so.
+template <typename TO>
+__global__ void __launch_bounds__(256)
+gated_group_norm_vec_kernel(const float* y, const float* z, int ld_z, const float* __restrict__ w, float eps, int width, int parts, TO* out) {
+    __shared__ float scratch[32];
+    pdl_wait();
+    const int t = blockIdx.x, part = blockIdx.y, n = width / parts;
+    const float* yr = y + (size_t)t * width + (size_t)part * n;
+    const float* zr = z + (size_t)t * ld_z + (size_t)part * n;
+    float4 u[4], g[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int i = (q * 256 + threadIdx.x) * 4;
+        u[q] = i < n ? *reinterpret_cast<const float4*>(yr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        g[q] = i < n ? *reinterpret_cast<const float4*>(zr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float ss = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        u[q].x *= g[q].x / (1.0f + expf(-g[q].x)); u[q].y *= g[q].y / (1.0f + expf(-g[q].y));
+        u[q].z *= g[q].z / (1.0f + expf(-g[q].z)); u[q].w *= g[q].w / (1.0f + expf(-g[q].w));
+        ss += u[q].x * u[q].x + u[q].y * u[q].y + (u[q].z * u[q].z + u[q].w * u[q].w);
+    }
+    ss = block_sum(ss, scratch);
+    const float scale = 1.0f / sqrtf(ss / (float)n + eps);
+    TO* orow = out + (size_t)t * width + (size_t)part * n;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int i = (q * 256 + threadIdx.x) * 4;
+        if (i >= n) continue;
+        const float4 v = *reinterpret_cast<const float4*>(w + (size_t)part * n + i);
+        const float r[4] = {u[q].x * scale * v.x, u[q].y * scale * v.y, u[q].z * scale * v.z, u[q].w * scale * v.w};
+        store_four(orow + i, r);
+    }
+}
+
 SHARPI_API int sharpi_gated_group_norm(const float* y, const float* z, int ld_z, const float* w, float eps, int T,
                                        int width, int parts, void* out, int out_dtype, cudaStream_t stream) {
     if (T <= 0) return SHARPI_OK;
     if (width <= 0 || parts <= 0 || width % parts != 0 || parts > 65535 || ld_z < width) return SHARPI_BAD_ARGUMENT;
     const dim3 grid(T, parts);
+    const int n = width / parts;
+    const uintptr_t bases = (uintptr_t)y | (uintptr_t)z | (uintptr_t)w | (uintptr_t)out;
+    if (n % 4 == 0 && n <= 4096 && ld_z % 4 == 0 && (bases & 15) == 0 && (out_dtype == SHARPI_F32 || out_dtype == SHARPI_BF16)) {
+        if (out_dtype == SHARPI_F32)
+            SHARPI_LAUNCH_PDL(gated_group_norm_vec_kernel<float>, grid, 256, 0, stream, y, z, ld_z, w, eps, width, parts, (float*)out);
+        else
+            SHARPI_LAUNCH_PDL(gated_group_norm_vec_kernel<bf16>, grid, 256, 0, stream, y, z, ld_z, w, eps, width, parts, (bf16*)out);
+        return SHARPI_OK;
+    }
     if (out_dtype == SHARPI_F32)
         SHARPI_LAUNCH_PDL(gated_group_norm_kernel<float>, grid, 256, 0, stream, y, z, ld_z, w, eps, width, parts, (float*)out);
     else if (out_dtype == SHARPI_BF16)

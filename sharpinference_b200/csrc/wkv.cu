@@ -716,12 +716,44 @@ wkv_out_kernel(const float* o, const float* gate, const float* __restrict__ weig
     }
 }
 
+// The same for heads of 4 LANES elements on 16 bytes: LANES lanes a (row, head), four elements each, loads all under way at once.
+// 2048 rows of 32 heads of 64: 25 us with a warp a (row, head), 11 us so.
+template <typename TO, int LANES>
+__global__ void __launch_bounds__(256)
+wkv_out_vec_kernel(const float* o, const float* gate, const float* __restrict__ weight, TO* out, long long work, int heads, float eps) {
+    pdl_wait();
+    constexpr int d = 4 * LANES;
+    const long long item = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / LANES;
+    const int e = threadIdx.x % LANES * 4;
+    const bool ok = item < work;
+    const size_t at = (size_t)(ok ? item : 0) * d + e;
+    const float4 v = *reinterpret_cast<const float4*>(o + at), g = *reinterpret_cast<const float4*>(gate + at);
+    const float4 w = *reinterpret_cast<const float4*>(weight + (size_t)((ok ? item : 0) % heads) * d + e);
+    float ss = v.x * v.x + v.y * v.y + (v.z * v.z + v.w * v.w);
+#pragma unroll
+    for (int x = LANES / 2; x > 0; x >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, x);
+    const float scale = 1.0f / sqrtf(ss / (float)d + eps);
+    const float y[4] = {v.x * scale * w.x * (g.x / (1.0f + expf(-g.x))), v.y * scale * w.y * (g.y / (1.0f + expf(-g.y))),
+                        v.z * scale * w.z * (g.z / (1.0f + expf(-g.z))), v.w * scale * w.w * (g.w / (1.0f + expf(-g.w)))};
+    if (!ok) return;
+    store_four(out + at, y);
+}
+
 SHARPI_API int sharpi_wkv_out(const float* o, const float* gate, const float* weight, void* out, int out_dtype, int T,
                               int heads, int d, float eps, cudaStream_t stream) {
     if (T <= 0) return SHARPI_OK;
     if (heads <= 0 || d <= 0) return SHARPI_BAD_ARGUMENT;
     const long long work = (long long)T * heads;
     const unsigned blocks = (unsigned)((work + 7) / 8);
+    const uintptr_t bases = (uintptr_t)o | (uintptr_t)gate | (uintptr_t)weight | (uintptr_t)out;
+    if ((d == 64 || d == 128) && (bases & 15) == 0 && (out_dtype == SHARPI_F32 || out_dtype == SHARPI_BF16)) {
+        const unsigned n = (unsigned)((work * (d / 4) + 255) / 256);
+        if (d == 64 && out_dtype == SHARPI_F32) SHARPI_LAUNCH_PDL((wkv_out_vec_kernel<float, 16>), n, 256, 0, stream, o, gate, weight, (float*)out, work, heads, eps);
+        else if (d == 64) SHARPI_LAUNCH_PDL((wkv_out_vec_kernel<bf16, 16>), n, 256, 0, stream, o, gate, weight, (bf16*)out, work, heads, eps);
+        else if (out_dtype == SHARPI_F32) SHARPI_LAUNCH_PDL((wkv_out_vec_kernel<float, 32>), n, 256, 0, stream, o, gate, weight, (float*)out, work, heads, eps);
+        else SHARPI_LAUNCH_PDL((wkv_out_vec_kernel<bf16, 32>), n, 256, 0, stream, o, gate, weight, (bf16*)out, work, heads, eps);
+        return SHARPI_OK;
+    }
     if (out_dtype == SHARPI_F32)
         SHARPI_LAUNCH_PDL(wkv_out_kernel<float>, blocks, 256, 0, stream, o, gate, weight, (float*)out, work, heads, d, eps);
     else if (out_dtype == SHARPI_BF16)

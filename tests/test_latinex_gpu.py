@@ -264,6 +264,23 @@ def test_gate_then_norm_in_parts(width, parts):
     assert not torch.allclose(want, other, atol=1e-2)
 
 
+@pytest.mark.parametrize("width,parts,dtype", [(4, 1, torch.float32), (1028, 1, torch.bfloat16), (4096, 1, torch.float32),
+                                               (4096, 4, torch.bfloat16), (4100, 1, torch.float32)])
+def test_gate_then_norm_sixteen_bytes_a_lane(width, parts, dtype):
+    """Rows on 16 bytes with parts of up to 4096 elements, and just beyond: the same numbers (a few roundings of float32, of
+    a result of up to about 5, and bfloat16's where it is written so)."""
+    from sharpinference_b200.kernels import ops
+    g = torch.Generator().manual_seed(width + parts)
+    T, col = 3, 8
+    y = 2 * torch.randn(T, width, generator=g, dtype=F64)
+    proj = torch.randn(T, col + width, generator=g, dtype=F64)
+    w = torch.randn(width, generator=g, dtype=F64)
+    u = y.float().double() * plain.silu(proj[:, col:col + width].float().double())
+    want = plain.rms(u.view(T, parts, width // parts), 1e-3).reshape(T, width) * w.float().double()
+    got = ops.gated_group_norm(f32(y), f32(proj), col, f32(w), 1e-3, parts, dtype).double().cpu()
+    assert float(((got - want).abs() - (2.0 ** -8 if dtype == torch.bfloat16 else 0.0) * want.abs()).max()) < 2e-5
+
+
 def _paged_keys(keys, page_size, seed):
     """Keys [T, nkv, d] written into shuffled pages of a pool that also holds garbage: (kv_layer, block_table)."""
     T, nkv, d = keys.shape

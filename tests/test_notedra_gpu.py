@@ -339,6 +339,55 @@ def test_mlstm_out_kernel():
     assert torch.allclose(got.double().cpu(), want, atol=1e-5)
 
 
+@pytest.mark.parametrize("heads,dv,dtype", [(3, 4, torch.float32), (2, 128, torch.bfloat16), (1, 132, torch.float32),
+                                            (2, 256, torch.float32), (1, 260, torch.float32)])
+def test_mlstm_out_sixteen_bytes_a_lane(heads, dv, dtype):
+    """Gate columns on 16 bytes: value sizes of up to 256 in registers, and just beyond; the tolerance of the test above."""
+    from sharpinference_b200.kernels import ops
+    g = torch.Generator().manual_seed(heads + dv)
+    T, col_g, ld = 9, 12, 12 + heads * dv
+    num, nq, coef = torch.randn(T, heads * dv, generator=g) * 4, torch.randn(T, heads, generator=g) * 2, torch.randn(T, heads, 4, generator=g)
+    proj, w = torch.randn(T, ld, generator=g), torch.randn(heads * dv, generator=g)
+    got = ops.mlstm_out(num.to(DEV), nq.to(DEV), coef.to(DEV), proj.to(DEV), col_g, w.to(DEV), 1e-4, heads, dv, dtype).double().cpu()
+    den = torch.maximum(nq.double().abs(), torch.exp(-coef.double()[:, :, 2])) + 1e-6
+    o = num.double().view(T, heads, dv) / den[:, :, None]
+    want = plain.unit_rms(o, 1e-4).reshape(T, -1) * w.double() * torch.sigmoid(proj.double()[:, col_g:])
+    assert float(((got - want).abs() - (2.0 ** -8 if dtype == torch.bfloat16 else 0.0) * want.abs()).max()) < 1e-5
+
+
+@pytest.mark.parametrize("lens", [[1, 31, 32, 33], [257], [64, 3, 300]])
+def test_mlstm_gates_are_the_serial_chain(lens):
+    """Log coefficients and running maximum at block borders of 32 rows, from a maximum of -1 in the slots: m = max(f + m, i)
+    in float32, one row after the other, with the gates themselves to a few roundings (values of up to 10, 300 of them)."""
+    from sharpinference_b200.kernels import ops
+    from sharpinference_b200.parts.mlstm import fused_mlstm_columns
+    heads, d, dv, cap = 2, 4, 4, 9.0
+    g = torch.Generator().manual_seed(sum(lens))
+    cq, ck, cv, cg, ci, cf, width = fused_mlstm_columns(heads, d, dv)
+    per_head, per_request = ops.mlstm_state_floats(heads, d, dv)
+    T = sum(lens)
+    proj, bias = 3 * torch.randn(T, width, generator=g), torch.randn(2, heads, generator=g)
+    state = torch.zeros(5, per_request)
+    at = (dv + 31) // 32 * d * 32 + d                        # the running maximum's place behind the memory and the normaliser
+    state.view(5, heads, per_head)[:, :, at] = -1.0
+    offs = torch.tensor([sum(lens[:i]) for i in range(len(lens) + 1)], dtype=torch.int32, device=DEV)
+    slots = torch.tensor([3, 1, 0, 4][:len(lens)], dtype=torch.int32, device=DEV)
+    st = state.to(DEV)
+    coef = ops.mlstm_recurrence(proj.to(DEV), col_q=cq, col_k=ck, col_v=cv, col_i=ci, col_f=cf, bias_i=bias[0].to(DEV),
+                                bias_f=bias[1].to(DEV), row_offsets=offs, state_slots=slots, state=st, heads=heads, d=d, dv=dv,
+                                cap=cap, q_scale=0.5)[2].double().cpu()
+    i = cap * torch.tanh((proj[:, ci:ci + heads].double() + bias[0].double()) / cap)
+    f = torch.nn.functional.logsigmoid(cap * torch.tanh((proj[:, cf:cf + heads].double() + bias[1].double()) / cap))
+    for b, n in enumerate(lens):
+        m, r0 = torch.full((heads,), -1.0, dtype=torch.float64), int(offs[b])
+        for r in range(r0, r0 + n):
+            new = torch.maximum(f[r] + m, i[r])
+            want = torch.stack([f[r] + m - new, i[r] - new, new], dim=-1)
+            assert float((coef[r, :, :3] - want).abs().max()) < 2e-4
+            m = new
+        assert float((st.view(5, heads, per_head)[int(slots[b]), :, at].double().cpu() - m).abs().max()) < 2e-4
+
+
 # ------------------------------------------------------------------------------------------
 # whole models through the engine
 # ------------------------------------------------------------------------------------------

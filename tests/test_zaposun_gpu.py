@@ -160,6 +160,43 @@ def test_small_and_large_steps_give_the_same_bits():
     assert torch.equal(st_a[0], h[-1]) and torch.equal(st_b[0], h[19])
 
 
+@pytest.mark.parametrize("T,heads,d", [(1, 1, 64), (37, 3, 64), (5, 2, 128), (600, 1, 64), (5, 2, 60)])
+def test_wkv_out_sixteen_bytes_a_lane(T, heads, d):
+    """Heads of 64 and 128 elements have a kernel of their own, whose last block may be part empty; 60 keeps the general one."""
+    from sharpinference_b200.kernels import ops
+    g = torch.Generator().manual_seed(T * heads + d)
+    o, gate, w = (torch.randn(n, heads * d, generator=g) for n in (T, T, 1))
+    x = o.double().view(T, heads, d)
+    want = (x * torch.rsqrt(x.square().mean(-1, keepdim=True) + 1e-5)).reshape(T, -1) * w.double() * torch.nn.functional.silu(gate.double())
+    for dtype, rel in ((torch.float32, 0.0), (torch.bfloat16, 2.0 ** -8)):
+        got = ops.wkv_out(o.to(DEV), gate.to(DEV), w[0].to(DEV), 1e-5, heads, d, dtype).double().cpu()
+        assert float(((got - want).abs() - rel * want.abs()).max()) < 2e-5
+
+
+@pytest.mark.parametrize("T,H,dtype", [(511, 64, torch.float32), (512, 4, torch.float32), (513, 1028, torch.bfloat16),
+                                       (600, 1026, torch.float32)])
+def test_token_shift_of_long_steps(T, H, dtype):
+    """Several requests in a step of many rows, widths on 16 bytes and not: the first row of each reads its slot, the last
+    one is left there, and each mix is h + (h' - h) mu."""
+    from sharpinference_b200.kernels import ops
+    g = torch.Generator().manual_seed(T + H)
+    h, mu, state = torch.randn(T, H, generator=g), torch.rand(3, H, generator=g), torch.randn(4, H, generator=g)
+    lens, slots = [1, 200, T - 201], [2, 0, 3]
+    first = [sum(lens[:i]) for i in range(3)]
+    before = torch.cat([torch.zeros(1, H), h[:-1]])
+    for f, sl in zip(first, slots):
+        before[f] = state[sl]
+    want = h.double() + (before - h).double()[None] * mu.double()[:, None]
+    left = state.clone()
+    for f, n, sl in zip(first, lens, slots):
+        left[sl] = h[f + n - 1]
+    rr, off, sl = _step_meta(lens, slots)
+    st = state.to(DEV)
+    got = ops.token_shift(h.to(DEV), mu.to(DEV), st, row_request=rr, row_offsets=off, state_slots=sl, out_dtype=dtype)
+    assert float(((got.double().cpu() - want).abs() - (2.0 ** -8 if dtype == torch.bfloat16 else 0.0) * want.abs()).max()) < 2e-6
+    assert torch.equal(st.cpu(), left)
+
+
 def test_pair_embedding_uses_the_previous_token_of_the_request():
     from sharpinference_b200.kernels import ops
     g = torch.Generator().manual_seed(6)
