@@ -17,7 +17,7 @@
 //    the same products as with the standard fragment order;
 //  * the first weight loads are issued before the kernel waits for the kernel before it: weights are written by
 //    nobody, so where the kernel is started early (programmatic dependent launch) the stream begins during the
-//    predecessor's tail (the host launches it the plain way, see launch_variant);
+//    predecessor's tail (only where the caller allows it, see launch_variant);
 //  * the warps' partial sums meet in shared memory and are added in warp order; the epilogue stores (with an
 //    optional bias), adds into the output with reductions (one addend per element from this launch), or applies
 //    SwiGLU (a tile of gate rows and the tile of their up rows side by side) and writes bfloat16.
@@ -72,12 +72,14 @@ struct DenseRowsParams {
     const float* bias;      // [N] or null (DR_STORE)
     void* out;              // fp32 [M, N], or bf16 [M, N / 2] with DR_SWIGLU
     int M, N, K;
+    bool early;             // may start before the kernel in front of it has ended
 };
 
 // WIDE: more than eight activation rows.  DR_TILES: tiles of eight weight rows per group (with SwiGLU half of them
 // gate rows, half their up rows); DR_U: adjacent 32-element pieces of K per step of a warp, so a lane's loads of
 // a step cover DR_U * 64 bytes of its row in a run.  DR_TILES * DR_U 16-byte loads per lane are in flight.
-template <int MODE, bool WIDE, int DR_TILES, int DR_U>
+// AHEAD: the next step's weights are asked for before the products of this one (few tiles leave the registers for it).
+template <int MODE, bool WIDE, int DR_TILES, int DR_U, bool AHEAD>
 __global__ void __launch_bounds__(DR_THREADS, DR_CTAS_PER_SM)
 dense_rows_kernel(const DenseRowsParams p) {
     static_assert(MODE != DR_SWIGLU || DR_TILES % 2 == 0, "gate and up tiles come in pairs");
@@ -116,14 +118,31 @@ dense_rows_kernel(const DenseRowsParams p) {
 #pragma unroll
             for (int j = 0; j < 4; ++j) c[i][j] = 0.0f;
 
-        for (int s = warp; s < steps; s += DR_WARPS) {
-            uint4 wv[DR_TILES][DR_U], av[WIDE ? 2 : 1][DR_U];
+        auto load_weights = [&](uint4 (&wv)[DR_TILES][DR_U], int s) {
 #pragma unroll
             for (int u = 0; u < DR_U; ++u) {
                 const int piece = (s * DR_U + u) * 4 + t;
 #pragma unroll
                 for (int i = 0; i < DR_TILES; ++i)
                     wv[i][u] = (piece < pieces && row_ok[i]) ? load_stream(wrow[i] + piece) : zero;
+            }
+        };
+        uint4 next[DR_TILES][AHEAD ? DR_U : 1];
+        // step j of this warp: a warp has runs of RUN steps, so that the shapes for up to 8 and up to 16 rows deal K to the warps
+        // alike and a row's sum is the same in both
+        constexpr int RUN = WIDE && DR_TILES == 1 ? 2 : 1;
+        auto step = [&](int j) { return (j / RUN * DR_WARPS + warp) * RUN + j % RUN; };
+        if constexpr (AHEAD) load_weights(next, step(0));
+        for (int j = 0, s = step(0); s < steps; s = step(++j)) {
+            uint4 wv[DR_TILES][DR_U], av[WIDE ? 2 : 1][DR_U];
+            if constexpr (AHEAD) {
+#pragma unroll
+                for (int u = 0; u < DR_U; ++u)
+#pragma unroll
+                    for (int i = 0; i < DR_TILES; ++i) wv[i][u] = next[i][u];
+                load_weights(next, step(j + 1));         // (zeros behind the last piece)
+            } else {
+                load_weights(wv, s);
             }
             if (!waited) {                               // the weights are nobody's output: they are on their way
                 pdl_wait();                              // before the kernel that writes the activations has ended
@@ -182,24 +201,29 @@ dense_rows_kernel(const DenseRowsParams p) {
     if (!waited) pdl_wait();
 }
 
-template <int MODE, bool WIDE, int TILES, int U>
+template <int MODE, bool WIDE, int TILES, int U, bool AHEAD = false>
 int launch_variant(const DenseRowsParams& p, int sms, cudaStream_t stream) {
     // CTAs that are resident at once: the rows are dealt over exactly that many, so there is one wave
     static int resident = 0;
     if (resident == 0) {
         int per_sm = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dense_rows_kernel<MODE, WIDE, TILES, U>, DR_THREADS,
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dense_rows_kernel<MODE, WIDE, TILES, U, AHEAD>, DR_THREADS,
                                                           0) != cudaSuccess || per_sm <= 0)
             return SHARPI_LAUNCH_FAILED;
         resident = sms * (per_sm < DR_CTAS_PER_SM ? per_sm : DR_CTAS_PER_SM);
     }
     const int n_out = MODE == DR_SWIGLU ? p.N / 2 : p.N;
     const int grid = resident < n_out ? resident : n_out;
-    // Launched the plain way: started early (programmatic dependent launch), its CTAs sit on every SM with all
-    // the registers while the kernel before it is still at work, and a decode step came out slower (Scout sizes,
-    // 8 layers, batch 1, qkv and o on this kernel: 568 against 617 tok/s), although between two small kernels
-    // the early start saves 1.5 us.  The kernel after this one may still start early (pdl_wait signals it).
-    dense_rows_kernel<MODE, WIDE, TILES, U><<<grid, DR_THREADS, 0, stream>>>(p);
+    // Launched the plain way unless the caller says otherwise: started early (programmatic dependent launch), its CTAs
+    // sit on every SM with all the registers while the kernel before it is still at work, and a decode step of large
+    // products came out slower (Scout sizes, 8 layers, batch 1, qkv and o on this kernel: 568 against 617 tok/s).
+    // Between small kernels the early start pays (a step of 4 layers of width 1024: 144 -> 129 us).  The kernel after this one may still start early
+    // (pdl_wait signals it).
+    if (p.early) {
+        SHARPI_LAUNCH_PDL((dense_rows_kernel<MODE, WIDE, TILES, U, AHEAD>), grid, DR_THREADS, 0, stream, p);
+        return SHARPI_OK;
+    }
+    dense_rows_kernel<MODE, WIDE, TILES, U, AHEAD><<<grid, DR_THREADS, 0, stream>>>(p);
     SHARPI_CHECK_LAUNCH();
     return SHARPI_OK;
 }
@@ -207,7 +231,9 @@ int launch_variant(const DenseRowsParams& p, int sms, cudaStream_t stream) {
 // Which shape of the kernel: a CTA should take its rows in one pass (a second, nearly empty group costs a whole
 // walk over K), with runs of 256 bytes per row where three tiles are enough for that and 192 bytes with four
 // (measured on B200 at 5120 x 5120, 5120 x 8192 and 7168 x 5120: 9.9 / 14.8 / 15.6 us with three tiles of
-// four pieces, 10.7 / 16.5 / 12.8 us with four tiles of three; the last has 25 rows per CTA).
+// four pieces, 10.7 / 16.5 / 12.8 us with four tiles of three; the last has 25 rows per CTA).  Narrow weights give a CTA one
+// or two tiles; the loads that the others would have had in flight are longer runs and the next step's there: 2048 x 8192
+// 12.9 -> 10.2 us, 1024 x 4096 7.5 -> 5.9 us, 2048 x 4096 8.3 -> 6.7 us at one row, between two other kernels.
 template <int MODE, bool WIDE>
 int launch_dense_rows(const DenseRowsParams& p, cudaStream_t stream) {
     static int sms = 0;
@@ -217,9 +243,14 @@ int launch_dense_rows(const DenseRowsParams& p, cudaStream_t stream) {
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
             return SHARPI_LAUNCH_FAILED;
     }
-    if (MODE != DR_SWIGLU) {
-        const int slots = sms * DR_CTAS_PER_SM;
-        if ((p.N + slots - 1) / slots <= 3 * DR_TILE) return launch_variant<MODE == DR_SWIGLU ? DR_STORE : MODE, WIDE, 3, 4>(p, sms, stream);
+    const int slots = sms * DR_CTAS_PER_SM;
+    if constexpr (MODE == DR_SWIGLU) {
+        if ((p.N / 2 + slots - 1) / slots <= DR_TILE) return launch_variant<MODE, WIDE, 2, 4, true>(p, sms, stream);
+    } else {
+        const int rows = (p.N + slots - 1) / slots;
+        if (rows <= DR_TILE) return launch_variant<MODE, WIDE, 1, WIDE ? 4 : 8, true>(p, sms, stream);
+        if (rows <= 2 * DR_TILE) return launch_variant<MODE, WIDE, 2, 4, true>(p, sms, stream);
+        if (rows <= 3 * DR_TILE) return launch_variant<MODE, WIDE, 3, 4>(p, sms, stream);
     }
     return launch_variant<MODE, WIDE, 4, 3>(p, sms, stream);
 }
@@ -228,9 +259,10 @@ int launch_dense_rows(const DenseRowsParams& p, cudaStream_t stream) {
 
 // A [M, K] bf16 (1 <= M <= 16), W [N, K] bf16, K a multiple of 8, both 16-byte aligned.
 // mode 0: out fp32 [M, N] = A W^T (+ bias); 1: out += A W^T with reductions; 2: N = 2 I, out bf16 [M, I] =
-// silu(A Wg^T) * (A Wu^T) with Wg the first I rows of W and Wu the rest.
+// silu(A Wg^T) * (A Wu^T) with Wg the first I rows of W and Wu the rest.  `early`: W and the bias were not written by the
+// kernel right before this one in the stream, so that they may be read while that one still runs.
 SHARPI_API int sharpi_dense_rows(const void* A, const void* W, const float* bias, void* out, int M, int N, int K,
-                                 int mode, cudaStream_t stream) {
+                                 int mode, int early, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return SHARPI_OK;
     if (M > 16 || K <= 0 || K % 8 != 0) return SHARPI_BAD_ARGUMENT;
     if (mode == DR_SWIGLU && N % 2 != 0) return SHARPI_BAD_ARGUMENT;
@@ -238,7 +270,7 @@ SHARPI_API int sharpi_dense_rows(const void* A, const void* W, const float* bias
     if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) return SHARPI_UNALIGNED;
     DenseRowsParams p;
     p.A = reinterpret_cast<const bf16*>(A); p.W = reinterpret_cast<const bf16*>(W); p.bias = bias; p.out = out;
-    p.M = M; p.N = N; p.K = K;
+    p.M = M; p.N = N; p.K = K; p.early = early != 0;
     const bool wide = M > 8;
     switch (mode) {
         case DR_STORE: return wide ? launch_dense_rows<DR_STORE, true>(p, stream) : launch_dense_rows<DR_STORE, false>(p, stream);

@@ -46,10 +46,11 @@ class EngineOptions:
     cuda_graphs: bool = True            # capture decode-only steps as CUDA graphs (when the model's parts allow)
     # Dense bfloat16 products of steps of up to this many rows (at most 16) run on the engine's own
     # weight-streaming kernel instead of the vendor library (which the reference also uses only for batched
-    # projections, its single-token products being kernels of its own).  0: the library everywhere, which is
-    # the faster step on B200 (Scout sizes, 8 layers, batch 1: 614 against 593 tok/s) although the own kernel
-    # is the faster product alone (parts/linear.py has the figures).  The LM head keeps the library either way
-    # (2 GB of weights: 322 against 299 us).  The results differ by rounding only.
+    # projections, its single-token products being kernels of its own).  0: small products only
+    # (parts/linear.py, SMALL_PRODUCTS), the library for the others, which is the faster step on B200 (Scout sizes, 8
+    # layers, batch 1: 614 against 593 tok/s) although the own kernel is the faster product alone (parts/linear.py has
+    # the figures).  The LM head keeps the library either way (2 GB of weights: 322 against 299 us) unless it is small.
+    # The results differ by rounding only.
     own_dense_rows: int = 0
     # Launch kernels with programmatic stream serialization: a kernel's set-up overlaps the tail of the one
     # before it.  False launches every kernel the plain way.  One switch for the process (the kernel libraries
@@ -102,10 +103,10 @@ class Engine:
         self.model = load_model(model, self.dtype, self.device) if isinstance(model, str) else model
         o = self.options
         library.set_programmatic_launch(o.programmatic_launch)
-        if o.own_dense_rows > 0:
-            for lin in _linears(self.model):
-                if lin is not getattr(self.model, "head", None):      # the LM head streams 2 GB: the library's job
-                    lin.stream_rows = o.own_dense_rows
+        for lin in _linears(self.model):
+            lin.stream_small = True
+            if o.own_dense_rows > 0 and lin is not getattr(self.model, "head", None):      # the LM head streams 2 GB: the library's job
+                lin.stream_rows = o.own_dense_rows
         num_pages = self._size_cache()
         self.cache = CacheManager(self.model.schedule, self.model.blocks, page_size=o.page_size,
                                   num_pages=num_pages, max_requests=o.max_batch, dtype=self.model.act_dtype,

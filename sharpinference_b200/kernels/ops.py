@@ -707,10 +707,12 @@ DENSE_ROWS_MAX = 16           # rows the weight-streaming dense kernel takes
 
 
 def dense_rows(a: torch.Tensor, w: torch.Tensor, *, swiglu: bool = False, out: Optional[torch.Tensor] = None,
-               accumulate: bool = False, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
+               accumulate: bool = False, bias: Optional[torch.Tensor] = None, early: bool = False) -> torch.Tensor:
     """``a . w^T`` for up to 16 bfloat16 rows against a bfloat16 weight ``[N, K]`` that streams in once
     (``dense_rows.cu``): float32 ``[M, N]`` (plus ``bias``), added into ``out`` with reductions when
-    ``accumulate``, or with ``swiglu`` (``w`` = gate rows then up rows) ``silu(g) * u`` in bfloat16 ``[M, N / 2]``."""
+    ``accumulate``, or with ``swiglu`` (``w`` = gate rows then up rows) ``silu(g) * u`` in bfloat16 ``[M, N / 2]``.
+    ``early``: weight and bias were there before the kernel in front of this one, whose end the product need not await to
+    read them."""
     _need(a, "a", torch.bfloat16)
     _need(w, "w", torch.bfloat16)
     M, K = a.shape
@@ -734,7 +736,7 @@ def dense_rows(a: torch.Tensor, w: torch.Tensor, *, swiglu: bool = False, out: O
             raise KernelError(f"out is {tuple(out.shape)} for a product of {M} rows and a weight of {N} rows")
     mode = 2 if swiglu else 1 if accumulate else 0
     check(kernel("sharpi_dense_rows")(a.data_ptr(), w.data_ptr(), _ptr(bias), out.data_ptr(), M, N, K, mode,
-                                      _stream()), "sharpi_dense_rows")
+                                      int(early), _stream()), "sharpi_dense_rows")
     return out
 
 

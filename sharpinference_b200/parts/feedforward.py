@@ -81,8 +81,8 @@ class DenseSwiGLU(FeedForward):
             self.inner(ctx, h, act)
         elif self.activation != "silu":
             act = ops.gated_act(self.gate_up(h), ops.ACTIVATIONS[self.activation], self.act_dtype)
-        elif self.act_dtype == torch.bfloat16 and self.gate_up.streams(h):
-            act = ops.dense_rows(h, self.gate_up.weight, swiglu=True)     # SwiGLU in the product's epilogue
+        elif self.act_dtype == torch.bfloat16 and self.gate_up.streams(h, fused=True):
+            act = ops.dense_rows(h, self.gate_up.weight, swiglu=True, early=self.gate_up.small(h.shape[0], True))   # SwiGLU in its epilogue
         else:
             act = ops.swiglu(self.gate_up(h), self.act_dtype)
         return self.down(act, out=out, accumulate=accumulate)

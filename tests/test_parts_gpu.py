@@ -217,6 +217,29 @@ def test_linear_adds_into_its_output():
     assert torch.allclose(added, base + alone, rtol=1e-6, atol=1e-6)
 
 
+@pytest.mark.parametrize("rows,N,K,own", [(1, 8, 8, True), (8, 40, 72, True), (16, 300, 264, True), (17, 40, 72, False),
+                                          (8, 4096, 4096, True), (9, 4096, 4096, False), (8, 4104, 4096, False)])
+def test_small_products_of_an_engines_weights(rows, N, K, own):
+    """Up to which sizes a product runs on the weight-streaming kernel where the weights are known to be there already, and
+    its result behind a kernel that has just written the activations (float32 sums of up to 4096 products of bfloat16
+    numbers: 1e-5 of the largest sum of magnitudes)."""
+    from sharpinference_b200.kernels import ops
+    from sharpinference_b200.parts import Linear
+    w, x = rnd(N, K, scale=0.1, seed=1).to(torch.bfloat16).to(DEV), rnd(rows, 2 * K, seed=2).to(DEV)
+    bias = rnd(N, seed=3).to(DEV)
+    lin = Linear(w, bias=bias)
+    act = ops.swiglu(x, torch.bfloat16)
+    assert not lin.streams(act)
+    lin.stream_small = True
+    assert lin.streams(act) == own and not lin.adds_with_reductions(act)
+    for _ in range(3):
+        act = ops.swiglu(x, torch.bfloat16)
+        got = lin(act)
+        a, b = act.double(), w.double()
+        assert float((got.double() - (a @ b.T + bias.double())).abs().max()) <= 1e-5 * float((a.abs() @ b.abs().T).max())
+        x = x + 0.5
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_linear_with_a_bias(dtype):
     from sharpinference_b200.parts import Linear
