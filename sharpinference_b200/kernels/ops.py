@@ -927,7 +927,7 @@ def mlstm_recurrence(proj: torch.Tensor, *, col_q: int, col_k: int, col_v: int, 
     o_raw = torch.empty((T, heads * dv), dtype=torch.float32, device=proj.device)
     nq = torch.empty((T, heads), dtype=torch.float32, device=proj.device)
     chunks = _chunks("mlstm", T, B, max_rows, heads, d, dv, ld, col_q, col_k, col_v, per_head, state.stride(0),
-                     proj.data_ptr() // 4, state.data_ptr() // 4) if split else 0
+                     proj.data_ptr() // 4, state.data_ptr() // 4) if split and T - B + 1 >= CHUNKED_LEAST else 0
     sums = torch.empty(chunks * heads * (d * dv + d + 1), dtype=torch.float32, device=proj.device) if chunks else None
     check(kernel("sharpi_mlstm_recurrence")(proj.data_ptr(), ld, col_q, col_k, col_v, col_i, col_f, bias_i.data_ptr(),
                                             bias_f.data_ptr(), row_offsets.data_ptr(), state_slots.data_ptr(),
@@ -1162,7 +1162,7 @@ def wkv_recurrence(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, wraw: torc
     bonus = torch.empty((T, heads), dtype=torch.float32, device=r.device)
     B = state_slots.numel()
     chunks = _chunks("wkv", T, B, max_rows, heads, d, d, state.stride(0), v.data_ptr() // 4,
-                     state.data_ptr() // 4) if split and d <= 64 else 0
+                     state.data_ptr() // 4) if split and d <= 64 and T - B + 1 >= CHUNKED_LEAST else 0
     sums = torch.empty(chunks * heads * (d * d + 64), dtype=torch.float32, device=r.device) if chunks else None
     check(kernel("sharpi_wkv_recurrence")(r.data_ptr(), k.data_ptr(), v.data_ptr(), wraw.data_ptr(), w0.data_ptr(),
                                           u.data_ptr(), row_offsets.data_ptr(), state_slots.data_ptr(),
@@ -1462,7 +1462,7 @@ def ssd_scan(xbc: torch.Tensor, proj: torch.Tensor, *, col_x: int, col_b: int, c
     y = torch.empty((T, heads * vdim), dtype=torch.float32, device=xbc.device)
     B = state_slots.numel()
     chunks = _chunks("ssd", T, B, max_rows, heads, states, vdim, xbc.shape[1], col_x, col_b, col_c, state.stride(0),
-                     xbc.data_ptr() // 4, state.data_ptr() // 4) if split else 0
+                     xbc.data_ptr() // 4, state.data_ptr() // 4) if split and T - B + 1 >= CHUNKED_LEAST else 0
     sums = torch.empty(chunks * heads * (states * vdim + 1), dtype=torch.float32, device=xbc.device) if chunks else None
     check(kernel("sharpi_ssd_scan")(xbc.data_ptr(), xbc.shape[1], col_x, col_b, col_c, proj.data_ptr(), proj.shape[1], col_dt,
                                     dt_bias.data_ptr(), a_log.data_ptr(), dskip.data_ptr(), row_offsets.data_ptr(),
