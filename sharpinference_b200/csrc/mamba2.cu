@@ -1,5 +1,5 @@
-// The state-space-duality recurrence (Mamba-2) from per-request state, walked row by row, and the gated norm in
-// groups behind it.
+// The state-space-duality recurrence (Mamba-2) from per-request state, walked row by row (long portions in chunks where
+// the caller allows it), and the gated norm in groups behind it.
 //
 //   sharpi_ssd_scan     per head h (its group g = h / (heads / groups)), for the rows of a request in order:
 //                         dt = softplus(dt_raw[h] + dt_bias[h]);  a = exp(-exp(A_log[h]) * dt)
