@@ -440,6 +440,37 @@ def test_tcgen05_attention_over_keys_only_pages(nq, nkv, d, dv, window):
     assert torch.equal(outs[0], outs[1])
 
 
+def test_tcgen05_attention_keeps_the_largest_probability_exact():
+    """Rows whose largest score, 2 to 7 (log2) above the one before it, comes two blocks later: taken against the row's maximum its
+    probability is exactly one in bfloat16.  What is left is the rounding of the smaller probability (2^-9 of at most a fifth of the
+    result) and of the output (at most 2^-9), independent of each other: sqrt(1 + 1/25) = 1.02 times the error of rounding the
+    exact output at most, in the root mean square.  With the largest probability rounded as well it is 1.26 times it."""
+    from sharpinference_b200.kernels import ops
+    g = torch.Generator().manual_seed(3)
+    n, nq, d, page = 192, 2, 128, 64
+    keys = torch.randn(n, 1, d, generator=g)
+    keys[:, :, :3] = torch.tensor([0.0, 0.0, -4.0])                    # the third column keeps all others far below
+    keys[5, 0, :3], keys[130, 0, :3] = torch.tensor([4.0, 0.0, 0.0]), torch.tensor([0.0, 4.0, 0.0])
+    keys = keys.to(torch.bfloat16)
+    q = torch.zeros(n, nq, d)
+    q[..., 0], q[..., 2] = 2.0, 8.0
+    q[..., 1] = 2.0 + (2.0 + 5.0 * torch.rand(n, nq, generator=g)) * math.log(2.0) / 4.0
+    q = q.to(torch.bfloat16)
+    scale = 1.0
+    k64 = keys[:, 0].double()
+    want = torch.stack([plain.softmax_rows(q[:, h].double() @ k64.T * scale, plain.causal(n)) @ k64 for h in range(nq)], dim=1)
+    kv, bt = _paged_keys(keys.float(), page, seed=1)
+    tiles = torch.tensor([[t, 64, t, 0] for t in range(0, n, 64)], dtype=torch.int32, device=DEV)
+    out = torch.zeros(n, nq * d, dtype=torch.bfloat16, device=DEV)
+    assert ops.keys_prefill_tc_supported(nq, 1, d, d, page, 0, False, scale)
+    ops.attention_keys_prefill(q.to(DEV).view(n, nq * d), kv.to(torch.bfloat16).to(DEV), bt.to(DEV), tiles, out, nq=nq, nkv=1, d=d, dv=d,
+                               page_size=page, mask_kind=ops.MASK_FULL, mask_span=1, scale=scale)
+    ops.check_status(DEV)
+    got, late = out.double().cpu().view(n, nq, d)[130:, :, 3:], want[130:, :, 3:]
+    rounding = (late.to(torch.bfloat16).double() - late).square().mean().sqrt()
+    assert float((got - late).square().mean().sqrt()) <= 1.1 * float(rounding)
+
+
 @pytest.mark.parametrize("d,dv,window,keep", [(80, 80, 100, 3), (320, 256, 300, 70), (128, 128, 256, 0), (16, 16, 7, 257)])
 def test_single_rows_with_whole_splits_behind_the_window(d, dv, window, keep):
     """Single rows deep in a sequence of 1200 positions: between the kept first positions and the window lie whole
