@@ -151,6 +151,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
     const int p_last = p0 + n_rows - 1;
     const int key_lo = visible_lo(p0, a.mask_kind, a.mask_span);
     const int kb_first = key_lo / TK, n_blocks = p_last / TK - kb_first + 1;
+    const int behind = TK - 1 - p_last % TK;       // positions of the last block that lie behind the tile's last row
 
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
@@ -174,6 +175,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
 
     if (warp == SOFTMAX_WARPS) {
         // ---- TMA producer ----------------------------------------------------------------------
+        bool ok = true;
         if (lane == 0) {
             prefetch_tensormap(&q_map);
             prefetch_tensormap(&kv_map);
@@ -183,7 +185,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
 #pragma unroll
                 for (int e = 0; e < HEADS; ++e)
                     tma_load_2d(q_s + hf * TQ * 128 + e * TILE * 128, &q_map, q_full, (head + e) * D + hf * 64, row0);
-            bool ok = true;
             for (int j = 0; j < n_blocks && ok; ++j) {
                 const int st = j % KV_STAGES, use = j / KV_STAGES;
                 const int key0 = (kb_first + j) * TK;
@@ -191,12 +192,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 const int page = table[blk];
                 const int off = key0 - (blk << a.page_shift);
                 const int row_k = (page * (KEYS ? 1 : 2) * a.nkv + kvh) * a.page_size + off;
+                uint64_t* arrival = KEYS && behind > 0 && j == n_blocks - 1 ? &v_full[0] : &k_full[st];
                 if (use > 0) ok = mbar_wait(&k_empty[st], (use - 1) & 1);
                 if (!ok) { atomicExch(a.status, ERR_EMPTY); break; }
-                mbar_arrive_expect_tx(&k_full[st], Cfg::KV_BYTES);
+                mbar_arrive_expect_tx(arrival, Cfg::KV_BYTES);
 #pragma unroll
                 for (int hf = 0; hf < Cfg::HALVES; ++hf)
-                    tma_load_2d(k_s + st * Cfg::KV_BYTES + hf * TK * 128, &kv_map, &k_full[st], hf * 64, row_k);
+                    tma_load_2d(k_s + st * Cfg::KV_BYTES + hf * TK * 128, &kv_map, arrival, hf * 64, row_k);
                 if (KEYS) continue;
                 const int row_v = row_k + a.nkv * a.page_size;
                 if (use > 0) ok = mbar_wait(&v_empty[st], (use - 1) & 1);
@@ -206,6 +208,20 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_c
                 for (int hf = 0; hf < Cfg::HALVES; ++hf)
                     tma_load_2d(v_s + st * Cfg::KV_BYTES + hf * TK * 128, &kv_map, &v_full[st], hf * 64, row_v);
             }
+        }
+        if (KEYS && behind > 0) {
+            // What the page holds behind the last row is whatever its last owner left there.  Its weight is zero, but zero times a
+            // NaN is NaN: those rows become zeros.  The last block arrives at a barrier of its own (values have none here), and
+            // is passed on when they are cleared.
+            const int st = (n_blocks - 1) % KV_STAGES;
+            ok = __shfl_sync(0xffffffffu, (int)ok, 0);
+            if (ok && !mbar_wait(&v_full[0], 0)) { atomicExch(a.status, ERR_K); ok = false; }
+            uint8_t* rows = k_s + st * Cfg::KV_BYTES + (TK - behind) * 128;     // (the swizzle stays inside a row's 128 bytes)
+            if (ok)
+                for (int i = lane; i < Cfg::HALVES * behind * 8; i += 32)
+                    *reinterpret_cast<uint4*>(rows + i / (behind * 8) * (TK * 128) + i % (behind * 8) * 16) = make_uint4(0u, 0u, 0u, 0u);
+            fence_proxy_async();
+            if (__all_sync(0xffffffffu, ok) && lane == 0) mbar_arrive(&k_full[st]);
         }
     } else if (warp == SOFTMAX_WARPS + 1) {
         // ---- MMA issuer ------------------------------------------------------------------------

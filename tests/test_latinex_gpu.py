@@ -440,6 +440,30 @@ def test_tcgen05_attention_over_keys_only_pages(nq, nkv, d, dv, window):
     assert torch.equal(outs[0], outs[1])
 
 
+@pytest.mark.parametrize("bad", [math.nan, math.inf])
+@pytest.mark.parametrize("nq,d,dv,page", [(2, 64, 64, 64), (16, 320, 256, 64), (4, 384, 192, 128), (2, 192, 128, 256)])
+def test_tcgen05_attention_ignores_what_a_page_held_before(nq, d, dv, page, bad):
+    """Positions behind a prompt's last row are whatever the page's last owner left there: not finite in all of them, they
+    change no bit, for last blocks of 1 to 64 rows at every place in a page and in the ring of key blocks."""
+    from sharpinference_b200.kernels import ops
+    g = torch.Generator().manual_seed(d + page)
+    for n in (1, 36, 63, 64, 65, 127, 129, 190, 257, 300):
+        q = torch.randn(n, nq * d, generator=g).to(torch.bfloat16).to(DEV)
+        pages = (n + page - 1) // page
+        kv = torch.randn(pages, 1, 1, page, d, generator=g).to(torch.bfloat16).to(DEV)
+        bt = torch.arange(pages, dtype=torch.int32, device=DEV).view(1, -1)
+        tiles = torch.tensor([[t, min(64, n - t), t, 0] for t in range(0, n, 64)], dtype=torch.int32, device=DEV)
+        outs = []
+        for behind in (0.0, bad):
+            kv.view(-1, d)[n:] = behind
+            outs.append(torch.zeros(n, nq * dv, dtype=torch.bfloat16, device=DEV))
+            assert ops.keys_prefill_tc_supported(nq, 1, d, dv, page, 0, False, 0.1)
+            ops.attention_keys_prefill(q, kv, bt, tiles, outs[-1], nq=nq, nkv=1, d=d, dv=dv, page_size=page, mask_kind=ops.MASK_FULL,
+                                       mask_span=1, scale=0.1)
+            ops.check_status(DEV)
+        assert bool(torch.isfinite(outs[0]).all()) and torch.equal(outs[0], outs[1]), n
+
+
 def test_tcgen05_attention_keeps_the_largest_probability_exact():
     """Rows whose largest score, 2 to 7 (log2) above the one before it, comes two blocks later: taken against the row's maximum its
     probability is exactly one in bfloat16.  What is left is the rounding of the smaller probability (2^-9 of at most a fifth of the
