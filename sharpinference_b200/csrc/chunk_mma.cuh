@@ -95,9 +95,9 @@ __device__ __forceinline__ int chunks_before(const int* row_offsets, int b, int 
 
 // R x C floats (C a power of two; those with r < rows and c < cols, zeros elsewhere) as three planes of bfloat16 pieces,
 // rows C + 8 apart (neighbouring rows start in other banks); row r times f[r] where `f` is given.  All of a thread's loads
-// are under way before the first is split.
+// are under way before the first is split.  Returns whether all that this thread loaded is finite.
 template <int R, int C>
-__device__ __forceinline__ void load_split(bf16* dst, const float* src, size_t ld, int rows, int cols, const float* f) {
+__device__ __forceinline__ bool load_split(bf16* dst, const float* src, size_t ld, int rows, int cols, const float* f) {
     constexpr int LD = C + 8, PLANE = R * LD, N = R * C / 4 / THREADS;
     float4 x[N];
 #pragma unroll
@@ -105,9 +105,11 @@ __device__ __forceinline__ void load_split(bf16* dst, const float* src, size_t l
         const int i = threadIdx.x + p * THREADS, r = i / (C / 4), e = (i % (C / 4)) * 4;
         x[p] = r < rows && e < cols ? *reinterpret_cast<const float4*>(src + (size_t)r * ld + e) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
+    float zero = 0.0f;                                         // a NaN as soon as one of them is not
 #pragma unroll
     for (int p = 0; p < N; ++p) {
         const int i = threadIdx.x + p * THREADS, r = i / (C / 4), e = (i % (C / 4)) * 4;
+        zero = fmaf(x[p].x, 0.0f, fmaf(x[p].y, 0.0f, fmaf(x[p].z, 0.0f, fmaf(x[p].w, 0.0f, zero))));
         if (f) {
             const float s = f[r];
             x[p].x *= s; x[p].y *= s; x[p].z *= s; x[p].w *= s;
@@ -116,6 +118,7 @@ __device__ __forceinline__ void load_split(bf16* dst, const float* src, size_t l
 #pragma unroll
         for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(dst + q * PLANE + r * LD + e) = make_uint2(lo.v[q], hi.v[q]);
     }
+    return zero == 0.0f;
 }
 
 // x b[n] for N neighbouring n-tiles, all pieces, a tile after the other for each.  The tensor core's own additions cut off what
@@ -167,6 +170,27 @@ __device__ __forceinline__ void right_operand(uint32_t (&b)[3][4][2], const bf16
             mma16::ldmatrix_x4_trans(r, planes + p * PLANE + (k0 + (lane % 8) + ((lane / 8) % 2) * 8) * LD + n0 + n * 8 + (lane / 16) * 8);
             b[p][n][0] = r[0]; b[p][n][1] = r[1]; b[p][n + 1][0] = r[2]; b[p][n + 1][1] = r[3];
         }
+}
+
+// A warp's own sixteen rows among themselves where a value is not finite: the tensor core multiplies what a row must not see by
+// zero, and zero times a NaN is NaN.  acc += u v over the rows up to each one: u as the left operand's elements lie in the
+// lanes (rows lane / 4 and + 8), v the sixteen rows' values from column `c` on (two a lane and n-tile), cols of them, rows rows.
+__device__ __forceinline__ void own_rows_exact(float (&acc)[8][4], const float (&u)[4][2], const float* v, size_t ld, int rows, int cols, int lane) {
+    const int g = lane / 4, t = lane % 4;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+        const int e = 2 * (j / 8), src = g * 4 + (j % 8) / 2;
+        const float w0 = __shfl_sync(0xffffffffu, u[e][j % 2], src), w1 = __shfl_sync(0xffffffffu, u[e + 1][j % 2], src);
+        if (j >= rows) continue;
+#pragma unroll
+        for (int n = 0; n < 8; ++n) {
+            const int c = n * 8 + 2 * t;
+            if (c >= cols) continue;
+            const float2 x = *reinterpret_cast<const float2*>(v + (size_t)j * ld + c);
+            if (j <= g) { acc[n][0] = fmaf(w0, x.x, acc[n][0]); acc[n][1] = fmaf(w0, x.y, acc[n][1]); }
+            if (j <= g + 8) { acc[n][2] = fmaf(w1, x.x, acc[n][2]); acc[n][3] = fmaf(w1, x.y, acc[n][3]); }
+        }
+    }
 }
 
 // a_t and b_t of the chunk's rows for head h into shared memory (1 and 0 behind the last row)
@@ -398,8 +422,8 @@ __global__ void __launch_bounds__(THREADS, 2) outs_kernel(Args a, F f) {
             have = h;
         }
         load_split<DP, COLS>(k_s, a.sums + head * a.d * a.dv + c0, a.dv, a.d, a.dv - c0, nullptr);
-        load_split<ROWS, COLS>(v_s, a.v + (size_t)p.row0 * a.ld_v + (size_t)h * a.dv + c0, a.ld_v, p.rows, a.dv - c0, nullptr);
-        __syncthreads();
+        const float* values = a.v + (size_t)p.row0 * a.ld_v + (size_t)h * a.dv + c0;
+        const bool odd = __syncthreads_or(!load_split<ROWS, COLS>(v_s, values, a.ld_v, p.rows, a.dv - c0, nullptr));
         float acc[8][4];
         clear(acc);
 #pragma unroll
@@ -425,16 +449,23 @@ __global__ void __launch_bounds__(THREADS, 2) outs_kernel(Args a, F f) {
         for (int kk = 0; kk < 4; ++kk) {
             if (kk > warp) continue;
             uint32_t w[3][4];
+            float u[4][2];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int r = e & 1 ? i1 : i0, n = 2 * kk + (e >> 1), c = n * 8 + 2 * t;
-                // (selected, not multiplied by zero: what a later row brings must not reach this one through a NaN)
+                // (selected, not multiplied by zero: what a later row's key brings must not reach this one through a NaN; for its
+                // values see own_rows_exact)
                 const float u0 = c <= r ? score[n][2 * (e & 1)] * D_s[r * LD_D + c] : 0.0f;
                 const float u1 = c + 1 <= r ? score[n][2 * (e & 1) + 1] * D_s[r * LD_D + c + 1] : 0.0f;
                 if (F::NORM) (e & 1 ? row1 : row0) += u0 + u1;
+                u[e][0] = u0; u[e][1] = u1;
                 const mma16::Pieces s = mma16::split3(u0, u1);
 #pragma unroll
                 for (int q = 0; q < 3; ++q) w[q][e] = s.v[q];
+            }
+            if (odd && kk == warp) {
+                own_rows_exact(acc, u, values + (size_t)(warp * 16) * a.ld_v, a.ld_v, p.rows - warp * 16, a.dv - c0, lane);
+                continue;
             }
 #pragma unroll
             for (int n = 0; n < 8; n += 4) {

@@ -223,6 +223,34 @@ def test_state_space_duality_in_chunks(monkeypatch, heads, groups, N, P):
         assert float((torch.cat(got[b]) - want[b]).abs().max()) < 2e-5 * max(float(want[b].abs().max()), 1.0)
 
 
+@pytest.mark.parametrize("bad", [math.nan, math.inf])
+@pytest.mark.parametrize("heads,groups,N,P", [(4, 2, 64, 8), (3, 1, 128, 100)])
+def test_state_space_duality_in_chunks_keeps_later_values_out(monkeypatch, heads, groups, N, P, bad):
+    """One value of one row that is not finite, at the first, a middle and the last row of a block of sixteen: the rows before it and
+    all other columns are what they are without it (float32 sums of up to 200 products, 1e-5 of the largest), and from its
+    row on its column is not finite, as in the walk."""
+    from sharpinference_b200.kernels import ops
+    monkeypatch.setattr(ops, "_WALK_OR_CHUNKS", dict.fromkeys(ops._WALK_OR_CHUNKS, (1e9, 1, 0.0)))       # in chunks whatever is faster
+    g = torch.Generator().manual_seed(N + P)
+    T, inner, bc, col = 200, heads * P, groups * N, P + 3
+    xbc, dt, params = torch.randn(T, inner + 2 * bc, generator=g), torch.randn(T, heads, generator=g), torch.randn(3, heads, generator=g)
+    _, off, sl = _step_meta([T], [0])
+
+    def run(x, split):
+        return ops.ssd_scan(x.to(DEV), dt.to(DEV), col_x=0, col_b=inner, col_c=inner + bc, col_dt=0, dt_bias=f32(params[0]),
+                            a_log=f32(params[1]), dskip=f32(params[2]), row_offsets=off, state_slots=sl,
+                            state=torch.zeros(1, heads * N * P, device=DEV), heads=heads, groups=groups, states=N, vdim=P, split=split).cpu()
+    want = run(xbc, True)
+    for row in (0, 15, 64, 73, 127, 195):
+        other = xbc.clone()
+        other[row, col] = bad
+        got, walked = run(other, True), run(other, False)
+        rest = torch.ones(T, inner, dtype=torch.bool)
+        rest[row:, col] = False
+        assert float((got - want)[rest].abs().max()) <= 1e-5 * float(want.abs().max()), row
+        assert not bool(torch.isfinite(got[row:, col]).any()) and not bool(torch.isfinite(walked[row:, col]).any())
+
+
 @pytest.mark.parametrize("N,P", [(48, 24), (64, 32), (128, 64)])
 def test_scan_rows_do_not_depend_on_the_cut(N, P):
     """The walk adds a row's parts in one fixed order: a prompt in one step and the same prompt in portions of 1, 2

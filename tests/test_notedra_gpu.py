@@ -321,6 +321,36 @@ def test_mlstm_recurrence_in_chunks(monkeypatch, heads, d, dv):
         assert torch.equal(out[0][0][short], out[1][0][short])
 
 
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("heads,d,dv", [(2, 24, 40), (1, 128, 132)])
+def test_mlstm_recurrence_in_chunks_keeps_later_values_out(monkeypatch, heads, d, dv, bad):
+    """One value of one row that is not finite, at the first, a middle and the last row of a block of sixteen: the rows before it and
+    all other columns are what they are without it (1e-5 of the largest), and from its row on its column is not finite."""
+    from sharpinference_b200.kernels import ops
+    monkeypatch.setattr(ops, "_WALK_OR_CHUNKS", dict.fromkeys(ops._WALK_OR_CHUNKS, (1e9, 1, 0.0)))       # in chunks whatever is faster
+    from sharpinference_b200.parts.mlstm import fused_mlstm_columns
+    g = torch.Generator().manual_seed(d + dv)
+    cq, ck, cv, cg, ci, cf, width = fused_mlstm_columns(heads, d, dv)
+    T, col = 200, dv - 3
+    proj, bias = torch.randn(T, width, generator=g), torch.randn(2, heads, generator=g).to(DEV)
+    offs, slots = torch.tensor([0, T], dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+
+    def run(x):
+        state = torch.zeros(1, ops.mlstm_state_floats(heads, d, dv)[1], device=DEV)
+        return ops.mlstm_recurrence(x.to(DEV), col_q=cq, col_k=ck, col_v=cv, col_i=ci, col_f=cf, bias_i=bias[0], bias_f=bias[1] + 3,
+                                    row_offsets=offs, state_slots=slots, state=state, heads=heads, d=d, dv=dv, cap=9.0, q_scale=d ** -0.5,
+                                    split=True)[:2]
+    want, want_n = run(proj)
+    for row in (0, 15, 64, 73, 127, 195):
+        other = proj.clone()
+        other[row, cv + col] = bad
+        got, got_n = run(other)
+        rest = torch.ones(T, heads * dv, dtype=torch.bool, device=DEV)
+        rest[row:, col] = False
+        assert float((got - want)[rest].abs().max()) <= 1e-5 * float(want.abs().max()), row
+        assert not bool(torch.isfinite(got[row:, col]).any()) and torch.equal(got_n, want_n)
+
+
 def test_mlstm_out_kernel():
     from sharpinference_b200.kernels import ops
     g = torch.Generator().manual_seed(9)
