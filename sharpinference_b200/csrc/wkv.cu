@@ -463,6 +463,7 @@ __global__ void __launch_bounds__(WC_THREADS, 2) wkv_outs_kernel(WkvChunkArgs a)
     if (!chunked::find_chunk(a.row_offsets, a.B, a.least, blockIdx.y, p)) return;
     const int head = blockIdx.x, d = a.d, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane / 4, t = lane % 4;
     const size_t hd = (size_t)a.heads * d, at0 = (size_t)p.row0 * hd + (size_t)head * d;
+    bool finite;                                               // whether the values that this thread loaded are
     {
         float r[16][2], k[16][2], w[16][2], u[2];
 #pragma unroll
@@ -478,7 +479,7 @@ __global__ void __launch_bounds__(WC_THREADS, 2) wkv_outs_kernel(WkvChunkArgs a)
                 k[i][e] = ok ? a.k[at] : 0.0f;
                 w[i][e] = ok ? a.w[at] : 1.0f;
             }
-        chunked::load_split<chunked::ROWS, WC_D>(v_s, a.v + at0, hd, p.rows, d, nullptr);
+        finite = chunked::load_split<chunked::ROWS, WC_D>(v_s, a.v + at0, hd, p.rows, d, nullptr);
         // columns s and s + 1 of the block's A: a lane's channels down the rows, then lane 16 e + t has A of row t, column s + e
 #pragma unroll
         for (int s = 0; s < 16; s += 2) {
@@ -527,7 +528,7 @@ __global__ void __launch_bounds__(WC_THREADS, 2) wkv_outs_kernel(WkvChunkArgs a)
             }
         }
     }
-    __syncthreads();
+    const bool odd = __syncthreads_or(!finite);
     // the left operand of this warp's rows: r_s times the decays of the whole blocks `from` .. warp - 1, sixteen channels
     auto left = [&](uint32_t (&x)[3][4], int kk, int from) {
 #pragma unroll
@@ -593,7 +594,7 @@ __global__ void __launch_bounds__(WC_THREADS, 2) wkv_outs_kernel(WkvChunkArgs a)
     }
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk) {
-        if (kk > warp) continue;
+        if (kk > warp || (odd && kk == warp)) continue;
         uint32_t x[3][4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -618,6 +619,14 @@ __global__ void __launch_bounds__(WC_THREADS, 2) wkv_outs_kernel(WkvChunkArgs a)
         }
     }
     chunked::add_small(acc, small);
+    if (odd) {                                                 // this warp's own rows, left out above
+        float own[4][2];
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) own[e][i] = A_s[(warp * 16 + g + 8 * (e & 1)) * 17 + (e >> 1) * 8 + 2 * t + i];
+        chunked::own_rows_exact(acc, own, a.v + at0 + (size_t)(warp * 16) * hd, hd, p.rows - warp * 16, d, lane);
+    }
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
         const int row = warp * 16 + g + 8 * e;

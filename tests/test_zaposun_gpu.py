@@ -346,6 +346,31 @@ def test_wkv_recurrence_in_chunks(monkeypatch, heads, d):
         assert torch.equal(out[0][short], out[1][short])
 
 
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("heads,d", [(2, 64), (3, 20)])
+def test_wkv_recurrence_in_chunks_keeps_later_values_out(monkeypatch, heads, d, bad):
+    """One value of one row that is not finite, at the first, a middle and the last row of a block of sixteen: the rows before it and
+    all other columns are what they are without it (1e-5 of the largest), and from its row on its column is not finite."""
+    from sharpinference_b200.kernels import ops
+    monkeypatch.setattr(ops, "_WALK_OR_CHUNKS", dict.fromkeys(ops._WALK_OR_CHUNKS, (1e9, 1, 0.0)))       # in chunks whatever is faster
+    g = torch.Generator().manual_seed(heads + d)
+    T, hd, col = 200, heads * d, d + 5
+    _, off, sl = _step_meta([T], [0])
+    r, k, v, w = (torch.randn(T, hd, generator=g).to(DEV) for _ in range(4))
+    u, w0 = torch.randn(hd, generator=g).to(DEV), torch.linspace(-6.0, 0.0, hd).to(DEV)
+    run = lambda x: ops.wkv_recurrence(r, k, x, w.clone(), w0, u, row_offsets=off, state_slots=sl, state=torch.zeros(1, heads * d * d, device=DEV),
+                                       heads=heads, d=d, split=True)
+    want = run(v)
+    for row in (0, 15, 64, 73, 127, 195):
+        other = v.clone()
+        other[row, col] = bad
+        got = run(other)
+        rest = torch.ones(T, hd, dtype=torch.bool, device=DEV)
+        rest[row:, col] = False
+        assert float((got - want)[rest].abs().max()) <= 1e-5 * float(want.abs().max()), row
+        assert not bool(torch.isfinite(got[row:, col]).any())
+
+
 @pytest.mark.parametrize("taps", [1, 2, 3, 4])
 @pytest.mark.parametrize("C,dtype", [(6000, torch.bfloat16), (5620, torch.float32), (5120, torch.bfloat16)])
 def test_causal_convolution_rows_at_a_time(taps, C, dtype):
