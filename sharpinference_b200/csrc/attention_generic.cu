@@ -24,6 +24,8 @@
 #include "common.cuh"
 #include "mma_sync.cuh"
 
+#include <type_traits>
+
 constexpr int ATT_THREADS = 128;
 constexpr int ATT_TILE = 128;
 constexpr int ATT_MAX_D = 1024;
@@ -145,7 +147,10 @@ __global__ void paged_attention_generic_kernel(PagedAttnArgs a) {
 // weighted, the next values while the scores are formed; where a tile's keys lie is looked up a tile ahead, a key a thread.
 // A thread forms R / 8 rows x 4 keys of the scores (two chains over even and odd elements: one paired instruction) and R / 8
 // rows x 4 JJ elements of the sums (neighbouring elements paired).  Every number is formed by the same operations for both
-// R, so a row's bits do not depend on the launch.  Bound by the multiply-adds and the barriers between a tile's parts.
+// R, so a row's bits do not depend on the launch.  What a row must not see does not reach it, finite or not: keys that no row
+// of the group sees are not loaded (zeros in their place), and in tiles that some of its rows see and others do not a
+// hidden value is left out of the sum (zero times a NaN would be NaN); a hidden probability is minus zero there, which no
+// exponential is.  Bound by the multiply-adds and the barriers between a tile's parts.
 // 980 rows of 4 requests, 8 heads on 2, head size 128: 556 -> 95 us (before: a block a row and head, one key a thread read
 // element by element); 4 decode rows at 300 keys: 69 -> 48 us.
 constexpr int AR_BK = 64, AR_THREADS = 128, AR_MAX_D = 256;
@@ -159,6 +164,9 @@ __device__ __forceinline__ f32x2 pack2(float lo, float hi) {
 }
 __device__ __forceinline__ float lo2(f32x2 v) { return __uint_as_float((unsigned)v); }
 __device__ __forceinline__ float hi2(f32x2 v) { return __uint_as_float((unsigned)(v >> 32)); }
+
+// In place of a hidden score: a NaN that no operation makes, so that a score of minus infinity remains one.
+constexpr unsigned AR_HIDDEN = 0x7fa51dedu;
 
 // Floats a row takes in shared memory: an odd number of 16-byte pieces, so that neighbouring rows start in other banks.
 __host__ __device__ __forceinline__ int ar_ld(int d) { return (d / 4) % 2 ? d + 8 : d + 4; }
@@ -191,7 +199,8 @@ __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAtt
     const float* kv = (const float*)a.kv_base;
 
     const int keep = a.mask_kind == SHARPI_MASK_WINDOW ? a.keep_first : 0;
-    const int b_first = visible_lo(pos0, a.mask_kind, a.mask_span) / AR_BK, b_last = p_last / AR_BK;
+    const int lo_first = visible_lo(pos0, a.mask_kind, a.mask_span), lo_last = visible_lo(p_last, a.mask_kind, a.mask_span);
+    const int b_first = lo_first / AR_BK, b_last = p_last / AR_BK;
     const int n_keep = min((keep + AR_BK - 1) / AR_BK, b_first);   // tiles with kept positions below the others
     const int n_iter = n_keep + b_last - b_first + 1;
     auto key0_of = [&](int it) { return (it < n_keep ? it : b_first + it - n_keep) * AR_BK; };
@@ -199,7 +208,7 @@ __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAtt
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, tx = tid & 15, ty = tid >> 4;
     auto place = [&](int it) -> long long {               // of key tid of a tile
         const int key = key0_of(it) + tid;
-        const int page = key <= p_last ? table[key / a.page_size] : -1;
+        const int page = key <= p_last && (key >= lo_first || key < keep) ? table[key / a.page_size] : -1;
         return page >= 0 ? (long long)page * a.kv_planes * plane + ((long long)kvh * a.page_size + key % a.page_size) * d : -1;
     };
     auto load = [&](float* dst, int it, size_t second) {  // a warp copies every fourth row
@@ -264,7 +273,7 @@ __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAtt
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const int key = key0 + tx + 16 * j;
-                    float v = -INFINITY;
+                    float v = __uint_as_float(AR_HIDDEN);
                     if (key <= pos && (key >= lo || key < keep) && off_s[it & 1][tx + 16 * j] >= 0) {
                         v = __fmul_rn(__fadd_rn(lo2(s[i][j]), hi2(s[i][j])), a.scale);
                         if (a.softcap > 0.0f) v = a.softcap * tanhf(v / a.softcap);
@@ -291,7 +300,7 @@ __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAtt
             for (int i = 0; i < AR_BK; i += 16)
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
-                    const float v = p[i + c], e = v == -INFINITY ? 0.0f : expf(v - m);
+                    const float v = p[i + c], e = __float_as_uint(v) == AR_HIDDEN ? -0.0f : v == -INFINITY ? 0.0f : expf(v - m);
                     p[i + c] = e;
                     l = __fadd_rn(l, e);
                 }
@@ -313,27 +322,37 @@ __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAtt
                 for (int j = 0; j < JJ; ++j) sum[i][j][0] = sum[i][j][1] = 0;
             const float* vr = (a.kv_planes == 2 ? v_s : k_s) + tx * 4;
             const float* pr = p_s + ty * (AR_BK + 4);
+            // some row of the group sees a key of this tile that another one does not
+            const bool mixed = n_tok > 1 && (key0 + AR_BK - 1 > pos0 || (key0 < lo_last && key0 + AR_BK > keep));
+            auto weigh = [&](auto guarded) {
 #pragma unroll 2
-            for (int k = 0; k < AR_BK; k += 4) {
-                float4 pv[RT];
+                for (int k = 0; k < AR_BK; k += 4) {
+                    float4 pv[RT];
 #pragma unroll
-                for (int i = 0; i < RT; ++i) pv[i] = *reinterpret_cast<const float4*>(pr + i * 8 * (AR_BK + 4) + k);
+                    for (int i = 0; i < RT; ++i) pv[i] = *reinterpret_cast<const float4*>(pr + i * 8 * (AR_BK + 4) + k);
 #pragma unroll
-                for (int c = 0; c < 4; ++c)
+                    for (int c = 0; c < 4; ++c)
 #pragma unroll
-                    for (int j = 0; j < JJ; ++j) {
-                        // (elements of rows of at most 64 that do not exist: what is read there is not used)
-                        if (JJ > 1 && tx * 4 + 64 * j >= d) continue;
-                        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(vr + (k + c) * ld + 64 * j);
+                        for (int j = 0; j < JJ; ++j) {
+                            // (elements of rows of at most 64 that do not exist: what is read there is not used)
+                            if (JJ > 1 && tx * 4 + 64 * j >= d) continue;
+                            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(vr + (k + c) * ld + 64 * j);
 #pragma unroll
-                        for (int i = 0; i < RT; ++i) {
-                            const float e = c == 0 ? pv[i].x : c == 1 ? pv[i].y : c == 2 ? pv[i].z : pv[i].w;
-                            const f32x2 ee = pack2(e, e);
-                            fma2(sum[i][j][0], ee, v.x);
-                            fma2(sum[i][j][1], ee, v.y);
+                            for (int i = 0; i < RT; ++i) {
+                                const float e = c == 0 ? pv[i].x : c == 1 ? pv[i].y : c == 2 ? pv[i].z : pv[i].w;
+                                if (guarded && __float_as_uint(e) == 0x80000000u) continue;
+                                const f32x2 ee = pack2(e, e);
+                                fma2(sum[i][j][0], ee, v.x);
+                                fma2(sum[i][j][1], ee, v.y);
+                            }
                         }
-                    }
-            }
+                }
+            };
+            // (for 32 rows a loop without the question where it need not be asked: 60 rows behind 340 119 -> 110 us; 8 rows lose by a
+            // second loop, 64 -> 70 us)
+            if constexpr (R == 8) weigh(mixed);
+            else if (mixed) weigh(std::true_type{});
+            else weigh(std::false_type{});
 #pragma unroll
             for (int i = 0; i < RT; ++i) {
                 const float corr = corr_s[ty + i * 8];

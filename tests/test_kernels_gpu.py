@@ -236,6 +236,31 @@ def test_paged_attention_float32_rows_alone_and_in_groups(ops, nq, nkv, d, mask,
             assert torch.allclose(one.view(nq, d)[h].double().cpu(), ref, rtol=1e-5, atol=1e-5), (at, h)
 
 
+@pytest.mark.parametrize("nq,nkv,d,planes", [(4, 1, 64, 2), (3, 3, 68, 2), (2, 1, 256, 1)])
+@pytest.mark.parametrize("mask,keep", [("full", 0), ("chunk", 0), ("window", 0), ("window", 70)])
+def test_paged_attention_float32_rows_read_visible_keys_only(ops, nq, nkv, d, planes, mask, keep):
+    """Every position that a row must not see is made a NaN, or an infinity, in the pages: the row keeps its bits, alone and in a
+    group with rows that do see those positions (later tokens, or tokens whose window or chunk begins earlier)."""
+    n, span, ps, first = 200, 45, 16, 120
+    kv = rnd(13, planes, nkv, ps, d, seed=d)
+    table = torch.arange(13, dtype=torch.int32, device=DEV).view(1, -1)
+    pos = torch.arange(first, n, dtype=torch.int32, device=DEV)
+    req, q = torch.zeros_like(pos), rnd(n - first, nq, d, seed=12)
+    code = {"full": ops.MASK_FULL, "chunk": ops.MASK_CHUNK, "window": ops.MASK_WINDOW}[mask]
+    kw = dict(nq=nq, nkv=nkv, d=d, page_size=ps, mask_kind=code, mask_span=span, scale=d ** -0.5, keep_first=keep)
+    want = ops.paged_attention_generic(q, kv, table, req, pos, **kw)
+    assert bool(torch.isfinite(want).all())
+    for row in (0, 5, 8, 14, 15, 31, 63, 78, 79):
+        p = first + row
+        lo = {"full": 0, "chunk": p // span * span, "window": max(0, p - span + 1)}[mask]
+        hidden = torch.tensor([k for k in range(13 * ps) if not (lo <= k <= p or k < min(keep, lo))], device=DEV)
+        for bad in (float("nan"), float("inf"), -float("inf")):
+            other = kv.clone()
+            other[hidden // ps, :, :, hidden % ps] = bad
+            assert torch.equal(ops.paged_attention_generic(q, other, table, req, pos, **kw)[row], want[row]), (row, bad)
+            assert torch.equal(ops.paged_attention_generic(q[row:row + 1], other, table, req[:1], pos[row:row + 1], **kw)[0], want[row])
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_attention_finds_one_far_key_among_hundreds(ops, dtype):
     """One key far back is made to match the query; its value must dominate the output.  A kernel
