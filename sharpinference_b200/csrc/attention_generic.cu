@@ -420,6 +420,21 @@ static int launch_rows_f32(const PagedAttnArgs& a, cudaStream_t stream) {
                                                                        : launch_rows_f32<R, 4>(a, stream);
 }
 
+// Whether CTAs take 32 rows instead of 8.  A CTA of 8 walks its keys in two thirds of the time and three to six of them share an
+// SM (of 32 rows: one to three), so 32 only where CTAs of 8 do not fit the SMs at once and 32 rows a CTA leave well fewer of them
+// (single rows beside a portion stay a CTA each).  us, 8 / 32 rows a CTA, head size 128, 400 positions: 8 heads on 2: 60 rows
+// 66 / 109, 300 rows 80 / 111, 60 rows and 63 single ones 75 / 118, four portions of 250 181 / 128; 32 heads on 8, 2500 positions:
+// 100 rows 475 / 645, 150 rows 900 / 647, 16 portions of 16 1372 / 1278, 64 of 3 1386 / 1294, 300 rows and 63 single ones 1840 / 1917.
+static bool rows_f32_wide(const PagedAttnArgs& a, int B) {
+    const int G = a.nq / a.nkv, first = a.T < B ? a.T : B;       // rows that open a request's portion, at most
+    auto ctas = [&](int R) {
+        const int heads_cta = G < R ? G : R, tokens = R / heads_cta;
+        return (long long)((a.T - first) / tokens + first) * a.nkv * ((G + heads_cta - 1) / heads_cta);
+    };
+    const int per_sm = a.d <= 64 ? 6 : a.d <= 128 ? 3 : 1;
+    return ctas(8) > 148 * per_sm && 2 * ctas(8) > 5 * ctas(32);
+}
+
 SHARPI_API int sharpi_paged_attention_generic(const void* q, const void* kv_base, const int* block_table,
                                               const int* row_req, const int* positions, void* out, int dtype,
                                               int T, int B, int nq, int nkv, int d, int max_blocks, int page_size,
@@ -441,8 +456,7 @@ SHARPI_API int sharpi_paged_attention_generic(const void* q, const void* kv_base
     // (16 bytes a lane: other row sizes, larger ones and bfloat16 stay with the general kernel)
     const uintptr_t bases = (uintptr_t)q | (uintptr_t)kv_base | (uintptr_t)out;
     if (dtype == SHARPI_F32 && d % 4 == 0 && d <= AR_MAX_D && (bases & 15) == 0)
-        // mostly one or two rows a request (decode): a CTA for 8 rows; portions of prompts: for 32
-        return T <= 2 * B ? launch_rows_f32<8>(a, stream) : launch_rows_f32<32>(a, stream);
+        return rows_f32_wide(a, B) ? launch_rows_f32<32>(a, stream) : launch_rows_f32<8>(a, stream);
     dim3 grid(T, nq);
     if (dtype == SHARPI_F32)
         paged_attention_generic_kernel<float><<<grid, ATT_THREADS, 0, stream>>>(a);

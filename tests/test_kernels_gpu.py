@@ -236,14 +236,16 @@ def test_paged_attention_float32_rows_alone_and_in_groups(ops, nq, nkv, d, mask,
             assert torch.allclose(one.view(nq, d)[h].double().cpu(), ref, rtol=1e-5, atol=1e-5), (at, h)
 
 
-@pytest.mark.parametrize("nq,nkv,d,planes", [(4, 1, 64, 2), (3, 3, 68, 2), (2, 1, 256, 1)])
+# (200 positions: CTAs of 8 rows; 1000: of 32 for the group, of 8 for a row alone)
+@pytest.mark.parametrize("nq,nkv,d,planes,n", [(4, 1, 64, 2, 200), (3, 3, 68, 2, 200), (2, 1, 256, 1, 200), (8, 8, 128, 2, 1000),
+                                               (24, 2, 64, 1, 1000), (6, 3, 252, 2, 1000)])
 @pytest.mark.parametrize("mask,keep", [("full", 0), ("chunk", 0), ("window", 0), ("window", 70)])
-def test_paged_attention_float32_rows_read_visible_keys_only(ops, nq, nkv, d, planes, mask, keep):
+def test_paged_attention_float32_rows_read_visible_keys_only(ops, nq, nkv, d, planes, n, mask, keep):
     """Every position that a row must not see is made a NaN, or an infinity, in the pages: the row keeps its bits, alone and in a
     group with rows that do see those positions (later tokens, or tokens whose window or chunk begins earlier)."""
-    n, span, ps, first = 200, 45, 16, 120
-    kv = rnd(13, planes, nkv, ps, d, seed=d)
-    table = torch.arange(13, dtype=torch.int32, device=DEV).view(1, -1)
+    span, ps, first, pages = 45, 16, 120, n // 16 + 1
+    kv = rnd(pages, planes, nkv, ps, d, seed=d)
+    table = torch.arange(pages, dtype=torch.int32, device=DEV).view(1, -1)
     pos = torch.arange(first, n, dtype=torch.int32, device=DEV)
     req, q = torch.zeros_like(pos), rnd(n - first, nq, d, seed=12)
     code = {"full": ops.MASK_FULL, "chunk": ops.MASK_CHUNK, "window": ops.MASK_WINDOW}[mask]
@@ -253,7 +255,7 @@ def test_paged_attention_float32_rows_read_visible_keys_only(ops, nq, nkv, d, pl
     for row in (0, 5, 8, 14, 15, 31, 63, 78, 79):
         p = first + row
         lo = {"full": 0, "chunk": p // span * span, "window": max(0, p - span + 1)}[mask]
-        hidden = torch.tensor([k for k in range(13 * ps) if not (lo <= k <= p or k < min(keep, lo))], device=DEV)
+        hidden = torch.tensor([k for k in range(pages * ps) if not (lo <= k <= p or k < min(keep, lo))], device=DEV)
         for bad in (float("nan"), float("inf"), -float("inf")):
             other = kv.clone()
             other[hidden // ps, :, :, hidden % ps] = bad
