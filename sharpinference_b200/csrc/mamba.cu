@@ -494,14 +494,16 @@ static int launch_scan(const ScanArgs& a, int B, int T, cudaStream_t stream) {
     // states a lane, 4096 channels of 16 states: one prompt of 2048 rows 152 / 296 / 455; two of 1024 133 / 165 / 230; three of
     // 683 140 / 126 / 173; eight of 2048 909 / 765 / 1015.  Single rows (the state streams through): 200 requests 240 / 63 / 45.
     const bool walk = T - B + 1 > SCAN_CH;
-    const bool few = walk && (long long)a.C * B * NP / (8 * 32) < 4 * 148;
+    // More than 16 states are more than 8 lanes of two, whose rows are walked and summed one by one: one prompt of 2048 rows, two /
+    // eight states a lane, 2048 channels of 64 states 915 / 357, 1024 of 128 948 / 510, 4096 of 32 490 / 405.
+    const bool few = walk && NP <= 16 && (long long)a.C * B * NP / (8 * 32) < 4 * 148;
     switch (NP) {
         case 4: return few ? launch_scan<TO, 2, 2, true>(a, B, T, stream) : launch_scan<TO, 4, 1>(a, B, T, stream);
         case 8: return few ? launch_scan<TO, 2, 4, true>(a, B, T, stream) : launch_scan<TO, 8, 1>(a, B, T, stream);
         case 16: return few ? launch_scan<TO, 2, 8, true>(a, B, T, stream) : walk ? launch_scan<TO, 4, 4>(a, B, T, stream) : launch_scan<TO, 8, 2>(a, B, T, stream);
-        case 32: return few ? launch_scan<TO, 2, 16, true>(a, B, T, stream) : launch_scan<TO, 8, 4>(a, B, T, stream);
-        case 64: return few ? launch_scan<TO, 2, 32, true>(a, B, T, stream) : launch_scan<TO, 8, 8>(a, B, T, stream);
-        case 128: return few ? launch_scan<TO, 4, 32, true>(a, B, T, stream) : launch_scan<TO, 8, 16>(a, B, T, stream);
+        case 32: return launch_scan<TO, 8, 4>(a, B, T, stream);
+        case 64: return launch_scan<TO, 8, 8>(a, B, T, stream);
+        case 128: return launch_scan<TO, 8, 16>(a, B, T, stream);
         default: return launch_scan<TO, 8, 32>(a, B, T, stream);
     }
 }
