@@ -488,15 +488,21 @@ static int launch_scan(ScanArgs a, int B, int T, cudaStream_t stream) {
 }
 
 template <typename TO>
-static int launch_scan(const ScanArgs& a, int B, int T, cudaStream_t stream) {
+static int launch_scan(const ScanArgs& a, int B, int T, int longest, cudaStream_t stream) {
     const int NP = a.N <= 4 ? 4 : a.N <= 8 ? 8 : a.N <= 16 ? 16 : a.N <= 32 ? 32 : a.N <= 64 ? 64 : a.N <= 128 ? 128 : 256;
     // Rows to walk and fewer warps (of eight states a lane) than schedulers: two states a lane.  us, two split / four / eight
     // states a lane, 4096 channels of 16 states: one prompt of 2048 rows 152 / 296 / 455; two of 1024 133 / 165 / 230; three of
     // 683 140 / 126 / 173; eight of 2048 909 / 765 / 1015.  Single rows (the state streams through): 200 requests 240 / 63 / 45.
-    const bool walk = T - B + 1 > SCAN_CH;
     // More than 16 states are more than 8 lanes of two, whose rows are walked and summed one by one: one prompt of 2048 rows, two /
     // eight states a lane, 2048 channels of 64 states 915 / 357, 1024 of 128 948 / 510, 4096 of 32 490 / 405.
-    const bool few = walk && NP <= 16 && (long long)a.C * B * NP / (8 * 32) < 4 * 148;
+    // Requests count as walks by their rows over those of the longest.  Every request, a single row too, costs a set of blocks
+    // with their set-up, 1.2 us with two states a lane and 0.25 with four at 4096 channels, and a row of the longest 0.08 us less
+    // with two: hence the last condition.  One prompt beside 63 single rows, two / four states a lane: 1985 rows 174 / 332,
+    // 300 rows 94 / 56, 60 rows 83 / 27; 1800 rows beside 200 337 / 311; of 2048 channels 1985 rows 137 / 300, 300 rows 48 / 50.
+    const bool walk = (longest ? longest : T - B + 1) > SCAN_CH;
+    const double walks = longest ? (double)T / longest : B;
+    const bool few = walk && NP <= 16 && walks * a.C * NP / (8 * 32) < 4 * 148 &&
+                     (long long)(longest ? longest : T - B + 1) * 340 > (long long)a.C * B;
     switch (NP) {
         case 4: return few ? launch_scan<TO, 2, 2, true>(a, B, T, stream) : launch_scan<TO, 4, 1>(a, B, T, stream);
         case 8: return few ? launch_scan<TO, 2, 4, true>(a, B, T, stream) : launch_scan<TO, 8, 1>(a, B, T, stream);
@@ -508,18 +514,19 @@ static int launch_scan(const ScanArgs& a, int B, int T, cudaStream_t stream) {
     }
 }
 
+// `longest`: the rows of the longest request, 0 where it is not known (a choice of kernels, no result depends on it).
 SHARPI_API int sharpi_selective_scan(const float* x, const float* dtraw, const float* dt_bias, const float* bc,
                                      int ld_bc, int col_b, int col_c, const float* a_log, const float* dskip,
                                      const float* z, int ld_z, const int* row_offsets, const int* state_slots,
                                      float* state, long long state_stride, void* out, int out_dtype, int T, int B,
-                                     int C, int N, cudaStream_t stream) {
+                                     int C, int N, int longest, cudaStream_t stream) {
     if (B <= 0) return SHARPI_OK;
     if (C <= 0 || N <= 0 || N > 256) return SHARPI_BAD_ARGUMENT;
     ScanArgs a;
     a.x = x; a.dtraw = dtraw; a.dt_bias = dt_bias; a.bc = bc; a.ld_bc = ld_bc; a.col_b = col_b; a.col_c = col_c;
     a.a_log = a_log; a.dskip = dskip; a.z = z; a.ld_z = ld_z; a.row_offsets = row_offsets; a.state_slots = state_slots;
     a.state = state; a.state_stride = state_stride; a.out = out; a.C = C; a.N = N;
-    if (out_dtype == SHARPI_F32) return launch_scan<float>(a, B, T, stream);
-    if (out_dtype == SHARPI_BF16) return launch_scan<bf16>(a, B, T, stream);
+    if (out_dtype == SHARPI_F32) return launch_scan<float>(a, B, T, longest, stream);
+    if (out_dtype == SHARPI_BF16) return launch_scan<bf16>(a, B, T, longest, stream);
     return SHARPI_BAD_ARGUMENT;
 }

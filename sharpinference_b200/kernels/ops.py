@@ -1228,11 +1228,13 @@ def slice_cols(src: torch.Tensor, col0: int, ncols: int, out_dtype: torch.dtype)
 def selective_scan(x: torch.Tensor, dt: torch.Tensor, bc: torch.Tensor, col_b: int,
                    col_c: int, a_log: torch.Tensor, dskip: torch.Tensor, xz: torch.Tensor, col_z: int, *,
                    row_offsets: torch.Tensor, state_slots: torch.Tensor, state: torch.Tensor,
-                   out_dtype: torch.dtype, dt_bias: Optional[torch.Tensor] = None) -> torch.Tensor:
+                   out_dtype: torch.dtype, dt_bias: Optional[torch.Tensor] = None,
+                   max_rows: Optional[int] = None) -> torch.Tensor:
     """The selective scan over the rows of every request from and into ``state [slots, channels * states]``:
     ``(S C + D x) * g`` in ``out_dtype``, with ``dt`` the step sizes themselves (after their softplus) and ``g`` the
     gate (already ``silu(z)``) in the columns of ``xz`` from ``col_z``.  With ``dt_bias [channels]`` both come raw: the
-    step sizes are ``softplus(dt + dt_bias)`` and the gate ``silu`` of those columns."""
+    step sizes are ``softplus(dt + dt_bias)`` and the gate ``silu`` of those columns.  ``max_rows``: the rows of the longest
+    request, if known (a choice of kernels, no result depends on it)."""
     if dt_bias is not None:
         _need(dt_bias, "dt_bias", torch.float32)
         if dt_bias.numel() != x.shape[1]:
@@ -1252,7 +1254,7 @@ def selective_scan(x: torch.Tensor, dt: torch.Tensor, bc: torch.Tensor, col_b: i
                                           bc.shape[1], col_b, col_c, a_log.data_ptr(), dskip.data_ptr(), z.data_ptr(),
                                           xz.shape[1], row_offsets.data_ptr(), state_slots.data_ptr(), state.data_ptr(),
                                           state.stride(0), out.data_ptr(), dtype_code(out_dtype), T, state_slots.numel(),
-                                          C, N, _stream()), "sharpi_selective_scan")
+                                          C, N, int(max_rows or 0), _stream()), "sharpi_selective_scan")
     return out
 
 

@@ -71,7 +71,8 @@ class SelectiveScanMixer(Mixer):
         dt = self.dt_proj(ops.slice_cols(dbc, 0, self.dt_rank, self.act_dtype))
         y = ops.selective_scan(x32, dt, dbc, self.dt_rank, self.dt_rank + self.states, self.a_log,
                                self.d_skip, xz, self.inner, row_offsets=ctx.row_offsets, state_slots=ctx.state_slots,
-                               state=slot.states["S"], out_dtype=self.act_dtype, dt_bias=self.dt_bias)
+                               state=slot.states["S"], out_dtype=self.act_dtype, dt_bias=self.dt_bias,
+                               max_rows=ctx.max_rows_per_request)
         return self.out(y)
 
 
