@@ -6,6 +6,7 @@ is no CPU path: a tensor that is not on a CUDA device is an error.
 """
 from __future__ import annotations
 
+import math
 from typing import Optional
 
 import torch
@@ -872,29 +873,38 @@ def mlstm_state_floats(heads: int, d: int, dv: int):
     return per_head, heads * per_head
 
 
-# Requests of this many rows or more of a step run in chunks of 64 rows on the tensor cores where a caller allows it and the
-# step as a whole is faster so
+# Requests of fewer rows are always walked
 CHUNKED_LEAST = 128
-# What a step's recurrence takes, us: walked, w * max(rows of the longest request, rows of the step * heads / s) (a request's rows
-# are a chain; s (request, head) pairs keep the GPU busy); in chunks, 27 + c * rows * heads.  (w, s, c), walked -> in chunks at one
-# request of 128, 512 and 2048 rows, eight of 128 and four of 2048: mlstm (8 heads) 25 -> 30, 85 -> 46, 321 -> 126, 68 -> 70,
-# 589 -> 448; ssd (64 heads) 44 -> 30, 164 -> 58, 646 -> 212, 188 -> 147, 1740 -> 809; wkv (32 heads) 34 -> 28, 120 -> 33, 423 -> 121,
-# 41 -> 75, 543 -> 485.
-_WALK_OR_CHUNKS = {"mlstm": (0.16, 20, 0.0065), "ssd": (0.32, 100, 0.0016), "wkv": (0.21, 200, 0.0018)}
+# Of that many or more, a request runs in chunks of 64 rows on the tensor cores, where a caller allows it, from the row count on at
+# which its walk alone, w us a row, takes s + c * heads us: (w, s, c).  s is about what the three chunk kernels take however short
+# the request is.  c is for WKV: its chunks cost 1.5 times its walk where a step has several requests to walk side by side, so with
+# more heads a request has to bring more rows.  The choice looks at the request's own rows and the model's sizes, never at the
+# rest of the step, so a request's numbers do not depend on who shares its steps.
+# us, walked / in chunks: one request of 128, 256, 2048 rows; eight of 128, eight of 256, four of 512 in a step:
+#   mlstm  8 heads 128 x 256    25 / 30, 45 / 34, 321 / 122;  67 / 71, 127 / 103, 150 / 104
+#         16 heads 64 x 64      20 / 23, 35 / 26, 243 / 82;   39 / 33, 71 / 54, 110 / 56
+#   ssd   64 heads 128 x 64     44 / 31, 84 / 38, 647 / 214;  189 / 133, 366 / 218, 442 / 213   (a key head each: the same to 3 %)
+#         24 heads 16 x 64      26 / 18, 48 / 20, 357 / 62;   38 / 40, 71 / 54, 111 / 56
+#   wkv   32 heads of 64        33 / 27, 63 / 28, 390 / 120;  40 / 70, 77 / 138, 134 / 135
+#         16 heads of 64        33 / 27, 61 / 27, 367 / 62;   36 / 39, 68 / 68, 124 / 67
+#         64 heads of 64        35 / 28, 64 / 31, 488 / 209;  80 / 144, 163 / 257, 160 / 252
+_WALK_OR_CHUNKS = {"mlstm": (0.16, 30, 0.0), "ssd": (0.32, 30, 0.0), "wkv": (0.21, 15, 0.8)}
+
+
+def chunked_least(kind: str, heads: int) -> int:
+    """The rows from which on a request's recurrence (``mlstm``, ``ssd``, ``wkv``) runs in chunks where a caller allows it."""
+    w, s, c = _WALK_OR_CHUNKS[kind]
+    return max(CHUNKED_LEAST, math.ceil((s + c * heads) / w))
 
 
 def _chunks(kind: str, T: int, B: int, max_rows: Optional[int], heads: int, d: int, dv: int, *aligned: int) -> int:
     """How many chunks the requests of a step that run in chunks can have together (each ends in one that may be short);
-    0: none has the rows, walking is faster, or the sizes are not the chunk kernels'.  ``max_rows``: rows of the longest
-    request (None or 0: at most ``T - B + 1``); ``aligned``: column numbers, strides and addresses in floats, which the chunk
-    kernels want on 16 bytes."""
-    longest = max_rows or T - B + 1
-    if longest < CHUNKED_LEAST or d > 128 or d % 4 or dv % 4 or any(x % 4 for x in aligned):
+    0: none has the rows, or the sizes are not the chunk kernels'.  ``max_rows``: rows of the longest request (None or 0: at
+    most ``T - B + 1``); ``aligned``: column numbers, strides and addresses in floats, which the chunk kernels want on 16 bytes."""
+    least = chunked_least(kind, heads)
+    if (max_rows or T - B + 1) < least or d > 128 or d % 4 or dv % 4 or any(x % 4 for x in aligned):
         return 0
-    w, s, c = _WALK_OR_CHUNKS[kind]
-    if w * max(longest, T * heads / s) < 27 + c * T * heads:
-        return 0
-    return (T + 63) // 64 if B == 1 else T // 64 + min(B, T // CHUNKED_LEAST)
+    return (T + 63) // 64 if B == 1 else T // 64 + min(B, T // least)
 
 
 def mlstm_recurrence(proj: torch.Tensor, *, col_q: int, col_k: int, col_v: int, col_i: int, col_f: int,
@@ -907,7 +917,7 @@ def mlstm_recurrence(proj: torch.Tensor, *, col_q: int, col_k: int, col_v: int, 
     numerators ``S^T q`` float32 ``[T, heads * dv]``, ``n . q`` ``[T, heads]`` and per row and head ``(log a, log b,
     m, -)``, which :func:`mlstm_out` turns into the mixer's output.  ``split``: requests of many rows may run in chunks
     whose products are formed on the tensor cores, every float32 operand in bfloat16 pieces of 24 bits together;
-    ``max_rows``: the rows of the longest request, if known (a choice of kernels, no result depends on it but by rounding)."""
+    ``max_rows``: the rows of the longest request, if known (no result depends on it)."""
     _need(proj, "proj", torch.float32)
     _need(bias_i, "bias_i", torch.float32)
     _need(bias_f, "bias_f", torch.float32)
@@ -933,7 +943,7 @@ def mlstm_recurrence(proj: torch.Tensor, *, col_q: int, col_k: int, col_v: int, 
                                             bias_f.data_ptr(), row_offsets.data_ptr(), state_slots.data_ptr(),
                                             state.data_ptr(), state.stride(0), per_head, B, T, heads, d, dv,
                                             float(cap), float(q_scale), coef.data_ptr(), o_raw.data_ptr(), nq.data_ptr(),
-                                            _ptr(sums), chunks, CHUNKED_LEAST, _stream()),
+                                            _ptr(sums), chunks, chunked_least("mlstm", heads), _stream()),
           "sharpi_mlstm_recurrence")
     return o_raw, nq, coef
 
@@ -1167,7 +1177,7 @@ def wkv_recurrence(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, wraw: torc
     check(kernel("sharpi_wkv_recurrence")(r.data_ptr(), k.data_ptr(), v.data_ptr(), wraw.data_ptr(), w0.data_ptr(),
                                           u.data_ptr(), row_offsets.data_ptr(), state_slots.data_ptr(),
                                           state.data_ptr(), state.stride(0), o.data_ptr(), bonus.data_ptr(), T,
-                                          B, heads, d, _ptr(sums), chunks, CHUNKED_LEAST, _stream()),
+                                          B, heads, d, _ptr(sums), chunks, chunked_least("wkv", heads), _stream()),
           "sharpi_wkv_recurrence")
     return o
 
@@ -1469,7 +1479,7 @@ def ssd_scan(xbc: torch.Tensor, proj: torch.Tensor, *, col_x: int, col_b: int, c
     check(kernel("sharpi_ssd_scan")(xbc.data_ptr(), xbc.shape[1], col_x, col_b, col_c, proj.data_ptr(), proj.shape[1], col_dt,
                                     dt_bias.data_ptr(), a_log.data_ptr(), dskip.data_ptr(), row_offsets.data_ptr(),
                                     state_slots.data_ptr(), state.data_ptr(), state.stride(0), y.data_ptr(), T,
-                                    B, heads, groups, states, vdim, _ptr(sums), chunks, CHUNKED_LEAST, _stream()),
+                                    B, heads, groups, states, vdim, _ptr(sums), chunks, chunked_least("ssd", heads), _stream()),
           "sharpi_ssd_scan")
     return y
 

@@ -1001,3 +1001,40 @@ def test_a_wait_that_runs_out_is_reported_and_the_kernel_returns(ops):
     ref = torch.stack([a[t].double() @ w[int(expert[t])].double().cpu().T for t in order.tolist()])
     assert torch.allclose(out.double().cpu(), ref, rtol=1e-4, atol=1e-3)
 
+
+
+# sizes whose chunks were once chosen, or not, by all rows of the step: each request's alone and beside the others
+@pytest.mark.parametrize("kind,heads,d,dv,lens", [("wkv", 32, 64, 64, [300] * 9 + [100]), ("mlstm", 8, 32, 32, [200, 2000, 60]),
+                                                  ("ssd", 64, 16, 8, [130] + [1] * 60 + [127]), ("wkv", 4, 20, 20, [700, 131, 5])])
+def test_recurrences_of_a_request_do_not_depend_on_its_company(ops, kind, heads, d, dv, lens):
+    """Outputs and state of every request of a step, walked or in chunks as its own rows say, are the bits of the request served alone."""
+    from sharpinference_b200.parts.mlstm import fused_mlstm_columns
+    assert min(lens) < ops.chunked_least(kind, heads) <= max(lens)
+    T, hd = sum(lens), heads * d
+    ins, vec = [rnd(T, hd, seed=i) for i in range(4)], [rnd(hd, scale=0.3, seed=9 + i) for i in range(3)]
+    xbc, dt = rnd(T, heads * dv + 2 * d, scale=0.5, seed=7), rnd(T, heads, seed=8)
+    cols = fused_mlstm_columns(heads, d, dv)
+    proj = rnd(T, cols[-1], seed=6)
+    floats = heads * d * dv if kind != "mlstm" else ops.mlstm_state_floats(heads, d, dv)[1]
+
+    def run(at, n, known):
+        rows = slice(sum(lens[:at]), sum(lens[:at + n]))
+        part = lens[at:at + n]
+        state = torch.zeros(n, floats, device=DEV)
+        kw = dict(row_offsets=torch.tensor([sum(part[:i]) for i in range(n + 1)], dtype=torch.int32, device=DEV), state=state,
+                  state_slots=torch.arange(n, dtype=torch.int32, device=DEV), heads=heads, split=True, max_rows=max(part) if known else None)
+        if kind == "wkv":
+            r, k, v, w = (x[rows].clone() for x in ins)
+            out = ops.wkv_recurrence(r, k, v, w, vec[0], vec[1], d=d, **kw)
+        elif kind == "ssd":
+            out = ops.ssd_scan(xbc[rows].clone(), dt[rows].clone(), col_x=0, col_b=heads * dv, col_c=heads * dv + d, col_dt=0,
+                               dt_bias=vec[0], a_log=vec[1], dskip=vec[2], groups=1, states=d, vdim=dv, **kw)
+        else:
+            out = ops.mlstm_recurrence(proj[rows].clone(), col_q=cols[0], col_k=cols[1], col_v=cols[2], col_i=cols[4], col_f=cols[5],
+                                       bias_i=vec[0], bias_f=vec[1], d=d, dv=dv, cap=15.0, q_scale=d ** -0.5, **kw)[0]
+        return out, state
+    for known in (True, False):
+        whole, states = run(0, len(lens), known)
+        for b in sorted({0, 1, len(lens) - 2, len(lens) - 1}):
+            out, state = run(b, 1, known)
+            assert torch.equal(out, whole[sum(lens[:b]):sum(lens[:b + 1])]) and torch.equal(state[0], states[b]), (b, known)

@@ -75,3 +75,19 @@ def test_keys_bucket_of_a_captured_decode_step():
         changes = sum(a != b for a, b in zip(buckets, buckets[1:]))
         assert changes <= 4096 // 256 + 1, (rows, changes)
     assert len({StepRunner.keys_bucket(8 * (8192 - 57 + i), 8) for i in range(58)}) == 1
+
+
+def test_chunk_bounds_hold_for_drawn_steps():
+    """Chunks of the requests of a step that run in chunks: the bound that sizes scratch and grids, from the step's totals alone,
+    and no scratch where the longest request has too few rows."""
+    r = random.Random(1)
+    for _ in range(3000):
+        kind, heads = r.choice(["mlstm", "ssd", "wkv"]), r.choice([1, 4, 8, 32, 64, 200])
+        least = ops.chunked_least(kind, heads)
+        assert least >= ops.CHUNKED_LEAST
+        lens = [r.choice([1, 1, r.randint(1, 300), least - 1, least, least + 1, r.randint(1, 3000)]) for _ in range(r.randint(1, 12))]
+        need = sum((n + 63) // 64 for n in lens if n >= least)
+        for known in (None, max(lens)):
+            got = ops._chunks(kind, sum(lens), len(lens), known, heads, 64, 64)
+            assert got >= need, (kind, heads, lens)
+            assert known is None or (got > 0) == (max(lens) >= least)
