@@ -203,12 +203,12 @@ struct SsdChunks {
 };
 
 // `sums` (nullable; `chunks` * (heads * N * P + heads) floats): requests of at least `least` rows run in chunks, `chunks` of
-// them at most, on the tensor cores; the others, and without it all, are walked.
+// them at most, on the tensor cores; the others, and without it all, are walked (`walk` = 0: there are no others).
 SHARPI_API int sharpi_ssd_scan(const float* xbc, int ld_x, int col_x, int col_b, int col_c, const float* dt, int ld_dt,
                                int col_dt, const float* dt_bias, const float* a_log, const float* dskip,
                                const int* row_offsets, const int* state_slots, float* state, long long state_stride,
                                float* y, int T, int B, int heads, int groups, int N, int P, float* sums, int chunks,
-                               int least, cudaStream_t stream) {
+                               int least, int walk, cudaStream_t stream) {
     if (T <= 0 || B <= 0) return SHARPI_OK;
     if (heads <= 0 || groups <= 0 || heads % groups != 0 || N <= 0 || N > SSD_MAX_STATES || P <= 0 || heads > 65535 ||
         B > 65535 || col_x + heads * P > ld_x || col_b + groups * N > ld_x || col_c + groups * N > ld_x ||
@@ -230,7 +230,7 @@ SHARPI_API int sharpi_ssd_scan(const float* xbc, int ld_x, int col_x, int col_b,
         SsdChunks f;
         f.s = a;
         const int rc = chunked::launch(c, f, chunks, stream);
-        if (rc != SHARPI_OK || (B == 1 && T >= least)) return rc;
+        if (rc != SHARPI_OK || !walk) return rc;
         a.skip = least;
     }
     const dim3 grid((P + SSD_COLS - 1) / SSD_COLS, heads, B);

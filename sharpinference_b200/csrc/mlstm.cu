@@ -356,7 +356,7 @@ struct MlstmChunks {
 };
 
 // `sums` (nullable; `chunks` * heads * (d * dv + d + 1) floats): requests of at least `least` rows run in chunks, `chunks` of
-// them at most, on the tensor cores; the others, and without it all, are walked.
+// them at most, on the tensor cores; the others, and without it all, are walked (`walk` = 0: there are no others).
 // The recurrence over the step's rows: leaves the numerators o_raw [T, heads * dv], n . q in nq [T, heads], the
 // running maximum of every row in coef[.., 2] (coef: T * heads * 4 floats) and the new state.
 SHARPI_API int sharpi_mlstm_recurrence(const float* proj, int ld, int col_q, int col_k, int col_v, int col_i, int col_f,
@@ -364,7 +364,7 @@ SHARPI_API int sharpi_mlstm_recurrence(const float* proj, int ld, int col_q, int
                                        const int* state_slots, float* state, long long state_stride, int head_stride,
                                        int B, int T, int heads, int d, int dv, float cap, float q_scale, float* coef,
                                        float* o_raw, float* nq, float* sums, int chunks, int least,
-                                       cudaStream_t stream) {
+                                       int walk, cudaStream_t stream) {
     if (B <= 0 || T <= 0) return SHARPI_OK;
     if (heads <= 0 || d <= 0 || dv <= 0 || d > MLSTM_MAX_D || !(cap > 0.0f)) return SHARPI_BAD_ARGUMENT;
     if (heads > 65535 || (dv + 31) / 32 + 1 > 65535) return SHARPI_BAD_ARGUMENT;
@@ -395,7 +395,7 @@ SHARPI_API int sharpi_mlstm_recurrence(const float* proj, int ld, int col_q, int
         MlstmChunks f;
         f.m = a;
         const int rc = chunked::launch(c, f, chunks, stream);
-        if (rc != SHARPI_OK || (B == 1 && T >= least)) return rc;
+        if (rc != SHARPI_OK || !walk) return rc;
         a.skip = least;
     }
     if (d <= 16) return launch_scan<1>(a, B, stream);

@@ -655,11 +655,12 @@ static int launch_wkv_chunks(const WkvChunkArgs& a, int chunks, cudaStream_t str
 }
 
 // `sums` (nullable; `chunks` * heads * (d * d + 64) floats): requests of at least `least` rows run in chunks, `chunks` of them
-// at most, on the tensor cores (d <= 64); the others, and without it all, are walked.
+// at most, on the tensor cores (d <= 64); the others, and without it all, are walked (`walk` = 0: there are no others).
 SHARPI_API int sharpi_wkv_recurrence(const float* r, const float* k, const float* v, float* wraw,
                                      const float* w0, const float* u, const int* row_offsets, const int* state_slots,
                                      float* state, long long state_stride, float* o, float* bonus, int T, int B,
-                                     int heads, int d, float* sums, int chunks, int least, cudaStream_t stream) {
+                                     int heads, int d, float* sums, int chunks, int least, int walk,
+                                     cudaStream_t stream) {
     if (B <= 0) return SHARPI_OK;
     if (heads <= 0 || d <= 0 || d > 256 || T <= 0) return SHARPI_BAD_ARGUMENT;
     int skip = 0x7fffffff;
@@ -673,7 +674,7 @@ SHARPI_API int sharpi_wkv_recurrence(const float* r, const float* k, const float
         c.B = B; c.least = least; c.state = state; c.state_stride = state_stride; c.o = o; c.heads = heads; c.d = d;
         c.sums = sums; c.total = sums + (size_t)chunks * heads * d * d;
         const int rc = launch_wkv_chunks(c, chunks, stream);
-        if (rc != SHARPI_OK || (B == 1 && T >= least)) return rc;
+        if (rc != SHARPI_OK || !walk) return rc;
         skip = least;
     }
     if (d <= 128) {

@@ -60,13 +60,13 @@ SIGNATURES: Dict[str, Tuple[str, list]] = {
     "sharpi_router_topk": ("moe_topk", [P, P, P, I, I, I, I, F, I, P, P, P, P, I, P]),
     "sharpi_moe_pair_tokens": ("moe_topk", [P, I, I, P, P]),
     "sharpi_moe_combine": ("moe_topk", [P, P, P, I, I, I, P]),
-    "sharpi_mlstm_recurrence": ("mlstm", [P, I, I, I, I, I, I, P, P, P, P, P, LL, I, I, I, I, I, I, F, F, P, P, P, P, I, I, P]),
+    "sharpi_mlstm_recurrence": ("mlstm", [P, I, I, I, I, I, I, P, P, P, P, P, LL, I, I, I, I, I, I, F, F, P, P, P, P, I, I, I, P]),
     "sharpi_mlstm_out": ("mlstm", [P, P, P, P, I, P, F, I, I, I, P, I, P]),
     "sharpi_embed_pair": ("hyper", [P, P, P, I, P, P, P, P, P, I, I, I, I, I, I, I, P]),
     "sharpi_hc_mix_norm": ("hyper", [P, P, P, P, P, P, P, P, I, I, I, I, I, F, P]),
     "sharpi_token_shift": ("hyper", [P, P, P, LL, P, P, P, P, I, I, I, I, P]),
     "sharpi_norm_mean2": ("hyper", [P, P, P, P, P, I, I, F, F, P]),
-    "sharpi_wkv_recurrence": ("wkv", [P, P, P, P, P, P, P, P, P, LL, P, P, I, I, I, I, P, I, I, P]),
+    "sharpi_wkv_recurrence": ("wkv", [P, P, P, P, P, P, P, P, P, LL, P, P, I, I, I, I, P, I, I, I, P]),
     "sharpi_wkv_out": ("wkv", [P, P, P, P, I, I, I, I, F, P]),
     "sharpi_causal_conv": ("mamba", [P, I, P, P, P, LL, P, P, P, P, P, I, I, I, I, I, I, P]),
     "sharpi_slice_cols": ("mamba", [P, I, I, I, P, I, I, P]),
@@ -82,7 +82,7 @@ SIGNATURES: Dict[str, Tuple[str, list]] = {
     "sharpi_head_major": ("latent", [P, I, I, I, I, I, I, P, I, I, P]),
     "sharpi_head_minor": ("latent", [P, I, I, I, I, I, P, I, P, I, I, P]),
     "sharpi_latent_q_join": ("latent", [P, P, P, P, I, I, I, I, I, I, I, P, I, I, F, P]),
-    "sharpi_ssd_scan": ("mamba2", [P, I, I, I, I, P, I, I, P, P, P, P, P, P, LL, P, I, I, I, I, I, I, P, I, I, P]),
+    "sharpi_ssd_scan": ("mamba2", [P, I, I, I, I, P, I, I, P, P, P, P, P, P, LL, P, I, I, I, I, I, I, P, I, I, I, P]),
     "sharpi_add_layernorm": ("elementwise", [P, P, P, P, F, P, I, I, P, I, P, P]),
     "sharpi_qkv_post_wide": ("rope_kv", [P, I, P, P, P, P, P, F, I, I, P, P, I, I, I, I, I, I, I, F, F, I, I, P]),
     "sharpi_add_rmsnorm_pair": ("elementwise", [P, P, P, P, F, I, I, P, P, I, P, P]),

@@ -907,6 +907,12 @@ def _chunks(kind: str, T: int, B: int, max_rows: Optional[int], heads: int, d: i
     return (T + 63) // 64 if B == 1 else T // 64 + min(B, T // least)
 
 
+def _others_walk(T: int, B: int, max_rows: Optional[int]) -> int:
+    """Whether requests beside those in chunks may have rows to walk: not where the one request is known to have all of the step's
+    rows (the row count alone does not say so: the rows may lie behind the last request's)."""
+    return int(not (B == 1 and max_rows == T))
+
+
 def mlstm_recurrence(proj: torch.Tensor, *, col_q: int, col_k: int, col_v: int, col_i: int, col_f: int,
                      bias_i: torch.Tensor, bias_f: torch.Tensor, row_offsets: torch.Tensor, state_slots: torch.Tensor,
                      state: torch.Tensor, heads: int, d: int, dv: int, cap: float, q_scale: float, split: bool = False,
@@ -943,7 +949,8 @@ def mlstm_recurrence(proj: torch.Tensor, *, col_q: int, col_k: int, col_v: int, 
                                             bias_f.data_ptr(), row_offsets.data_ptr(), state_slots.data_ptr(),
                                             state.data_ptr(), state.stride(0), per_head, B, T, heads, d, dv,
                                             float(cap), float(q_scale), coef.data_ptr(), o_raw.data_ptr(), nq.data_ptr(),
-                                            _ptr(sums), chunks, chunked_least("mlstm", heads), _stream()),
+                                            _ptr(sums), chunks, chunked_least("mlstm", heads),
+                                            _others_walk(T, B, max_rows), _stream()),
           "sharpi_mlstm_recurrence")
     return o_raw, nq, coef
 
@@ -1177,7 +1184,8 @@ def wkv_recurrence(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, wraw: torc
     check(kernel("sharpi_wkv_recurrence")(r.data_ptr(), k.data_ptr(), v.data_ptr(), wraw.data_ptr(), w0.data_ptr(),
                                           u.data_ptr(), row_offsets.data_ptr(), state_slots.data_ptr(),
                                           state.data_ptr(), state.stride(0), o.data_ptr(), bonus.data_ptr(), T,
-                                          B, heads, d, _ptr(sums), chunks, chunked_least("wkv", heads), _stream()),
+                                          B, heads, d, _ptr(sums), chunks, chunked_least("wkv", heads),
+                                          _others_walk(T, B, max_rows), _stream()),
           "sharpi_wkv_recurrence")
     return o
 
@@ -1479,7 +1487,8 @@ def ssd_scan(xbc: torch.Tensor, proj: torch.Tensor, *, col_x: int, col_b: int, c
     check(kernel("sharpi_ssd_scan")(xbc.data_ptr(), xbc.shape[1], col_x, col_b, col_c, proj.data_ptr(), proj.shape[1], col_dt,
                                     dt_bias.data_ptr(), a_log.data_ptr(), dskip.data_ptr(), row_offsets.data_ptr(),
                                     state_slots.data_ptr(), state.data_ptr(), state.stride(0), y.data_ptr(), T,
-                                    B, heads, groups, states, vdim, _ptr(sums), chunks, chunked_least("ssd", heads), _stream()),
+                                    B, heads, groups, states, vdim, _ptr(sums), chunks,
+                                    chunked_least("ssd", heads), _others_walk(T, B, max_rows), _stream()),
           "sharpi_ssd_scan")
     return y
 

@@ -1038,3 +1038,31 @@ def test_recurrences_of_a_request_do_not_depend_on_its_company(ops, kind, heads,
         for b in sorted({0, 1, len(lens) - 2, len(lens) - 1}):
             out, state = run(b, 1, known)
             assert torch.equal(out, whole[sum(lens[:b]):sum(lens[:b + 1])]) and torch.equal(state[0], states[b]), (b, known)
+
+
+@pytest.mark.parametrize("kind", ["wkv", "mlstm", "ssd"])
+def test_recurrences_of_a_few_rows_in_a_longer_buffer(ops, kind):
+    """One request of 50 rows whose step's buffers hold 300: its rows are walked, whatever the buffers' length suggests, and the
+    rest has no part in it."""
+    from sharpinference_b200.parts.mlstm import fused_mlstm_columns
+    n, heads, d = 50, 2, 32
+    cols = fused_mlstm_columns(heads, d, d)
+    ins, vec = [rnd(300, heads * d, seed=i) for i in range(4)], [rnd(heads * d, scale=0.3, seed=9 + i) for i in range(3)]
+    xbc, dt, proj = rnd(300, heads * d + 2 * d, scale=0.5, seed=7), rnd(300, heads, seed=8), rnd(300, cols[-1], seed=6)
+
+    def run(T, split):
+        state = torch.zeros(1, heads * d * d if kind != "mlstm" else ops.mlstm_state_floats(heads, d, d)[1], device=DEV)
+        kw = dict(row_offsets=torch.tensor([0, n], dtype=torch.int32, device=DEV), state_slots=torch.zeros(1, dtype=torch.int32, device=DEV),
+                  state=state, heads=heads, split=split)
+        if kind == "wkv":
+            out = ops.wkv_recurrence(*(x[:T].clone() for x in ins), vec[0], vec[1], d=d, **kw)
+        elif kind == "ssd":
+            out = ops.ssd_scan(xbc[:T], dt[:T], col_x=0, col_b=heads * d, col_c=heads * d + d, col_dt=0, dt_bias=vec[0], a_log=vec[1],
+                               dskip=vec[2], groups=1, states=d, vdim=d, **kw)
+        else:
+            out = ops.mlstm_recurrence(proj[:T], col_q=cols[0], col_k=cols[1], col_v=cols[2], col_i=cols[4], col_f=cols[5], bias_i=vec[0],
+                                       bias_f=vec[1], d=d, dv=d, cap=15.0, q_scale=0.2, **kw)[0]
+        return out[:n], state
+    want, left = run(n, False)
+    got, state = run(300, True)
+    assert bool(left.any()) and torch.equal(got, want) and torch.equal(state, left)
