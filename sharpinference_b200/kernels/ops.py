@@ -904,7 +904,9 @@ def _chunks(kind: str, T: int, B: int, max_rows: Optional[int], heads: int, d: i
     least = chunked_least(kind, heads)
     if (max_rows or T - B + 1) < least or d > 128 or d % 4 or dv % 4 or any(x % 4 for x in aligned):
         return 0
-    return (T + 63) // 64 if B == 1 else T // 64 + min(B, T // least)
+    chunks = (T + 63) // 64 if B == 1 else T // 64 + min(B, T // least)
+    # what the chunk kernels' grids and offsets hold (the walks take more)
+    return chunks if max(chunks, B, heads) <= 65535 and d * dv <= 1 << 24 else 0
 
 
 def _others_walk(T: int, B: int, max_rows: Optional[int]) -> int:

@@ -91,3 +91,12 @@ def test_chunk_bounds_hold_for_drawn_steps():
             got = ops._chunks(kind, sum(lens), len(lens), known, heads, 64, 64)
             assert got >= need, (kind, heads, lens)
             assert known is None or (got > 0) == (max(lens) >= least)
+
+
+def test_chunk_kernels_are_left_alone_beyond_their_sizes():
+    """Steps and sizes that the walks take and the chunk kernels refuse are walked: more chunks than a grid's third extent, values whose
+    memory has more than 2^24 elements a head, odd sizes and addresses."""
+    assert ops._chunks("ssd", 1 << 22, 1, None, 8, 64, 64) == 0 and ops._chunks("ssd", 65535 * 64, 1, None, 8, 64, 64) == 65535
+    assert ops._chunks("mlstm", 4096, 1, None, 1, 128, 1 << 17) > 0 and ops._chunks("mlstm", 4096, 1, None, 1, 128, (1 << 17) + 4) == 0
+    assert ops._chunks("mlstm", 4096, 1, None, 8, 130, 64) == 0 and ops._chunks("mlstm", 4096, 1, None, 8, 128, 66) == 0
+    assert ops._chunks("ssd", 4096, 1, None, 8, 64, 64, 4, 1) == 0
