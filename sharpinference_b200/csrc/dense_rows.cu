@@ -72,7 +72,7 @@ struct DenseRowsParams {
     const float* bias;      // [N] or null (DR_STORE)
     void* out;              // fp32 [M, N], or bf16 [M, N / 2] with DR_SWIGLU
     int M, N, K;
-    bool early;             // may start before the kernel in front of it has ended
+    bool early;             // may start before the kernels in front of it have ended
 };
 
 // WIDE: more than eight activation rows.  DR_TILES: tiles of eight weight rows per group (with SwiGLU half of them
@@ -259,8 +259,10 @@ int launch_dense_rows(const DenseRowsParams& p, cudaStream_t stream) {
 
 // A [M, K] bf16 (1 <= M <= 16), W [N, K] bf16, K a multiple of 8, both 16-byte aligned.
 // mode 0: out fp32 [M, N] = A W^T (+ bias); 1: out += A W^T with reductions; 2: N = 2 I, out bf16 [M, I] =
-// silu(A Wg^T) * (A Wu^T) with Wg the first I rows of W and Wu the rest.  `early`: W and the bias were not written by the
-// kernel right before this one in the stream, so that they may be read while that one still runs.
+// silu(A Wg^T) * (A Wu^T) with Wg the first I rows of W and Wu the rest.  `early`: the kernel may start
+// before the ones in front of it have ended (several of them: each of those may have started so too), and reads W and the bias at
+// once: they were there before the last operation in the stream that waited for all before it, a copy, a graph's launch or a
+// kernel launched the plain way.
 SHARPI_API int sharpi_dense_rows(const void* A, const void* W, const float* bias, void* out, int M, int N, int K,
                                  int mode, int early, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return SHARPI_OK;

@@ -91,6 +91,9 @@ def _linears(root, depth: int = 4, seen=None):
 
 
 class Engine:
+    """Serves a model: a folder, or one that the program built.  The engine reads the model's weights where they are; a program
+    that writes into them does so between steps, on the stream that the steps run on."""
+
     def __init__(self, model: Union[str, object], *, dtype="bfloat16", device="cuda:0",
                  options: Optional[EngineOptions] = None):
         self.device = torch.device(device)
@@ -103,16 +106,17 @@ class Engine:
         self.model = load_model(model, self.dtype, self.device) if isinstance(model, str) else model
         o = self.options
         library.set_programmatic_launch(o.programmatic_launch)
-        for lin in _linears(self.model):
-            lin.stream_small = True
-            if o.own_dense_rows > 0 and lin is not getattr(self.model, "head", None):      # the LM head streams 2 GB: the library's job
-                lin.stream_rows = o.own_dense_rows
+        if o.own_dense_rows > 0:
+            for lin in _linears(self.model):
+                if lin is not getattr(self.model, "head", None):      # the LM head streams 2 GB: the library's job
+                    lin.stream_rows = o.own_dense_rows
         num_pages = self._size_cache()
         self.cache = CacheManager(self.model.schedule, self.model.blocks, page_size=o.page_size,
                                   num_pages=num_pages, max_requests=o.max_batch, dtype=self.model.act_dtype,
                                   device=self.device, model_state_specs=getattr(self.model, "state_specs", None))
         self.runner = StepRunner(self.model, self.cache)
         self.runner.use_graphs = self.runner.use_graphs and o.cuda_graphs
+        self.runner.small_products = True
         self.scheduler = Scheduler(self.cache, max_batch=o.max_batch, max_tokens_per_step=o.max_tokens_per_step,
                                    max_positions=getattr(self.model, "max_positions", None))
         self.sampler = Sampler(self.device)

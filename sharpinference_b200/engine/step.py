@@ -25,6 +25,7 @@ import torch
 from ..cache.manager import CacheManager
 from ..kernels import library, ops
 from ..parts.base import StepContext
+from ..parts.linear import engine_step
 
 
 class StepError(ValueError):
@@ -75,6 +76,7 @@ class StepRunner:
             for planner in made:
                 if planner is not None:
                     self.planners.setdefault(planner.key, planner)
+        self.small_products = False          # small dense products on the weight-streaming kernel (parts/linear.py)
         self.steps_run = 0
         self.rows_run = 0
         # Tracing, for hunting the first difference: when `trace_router` is set, every routed
@@ -292,7 +294,8 @@ class StepRunner:
                 ctx.extras["layer_norms"] = []
             if self.trace_streams:
                 ctx.extras["layer_streams"] = []
-            logits = self.model.forward(ctx)
+            with engine_step(self.small_products):
+                logits = self.model.forward(ctx)
             self.last_router_choices = ctx.extras.get("router_choices", [])
             self.last_layer_norms = ctx.extras.get("layer_norms", [])
             self.last_layer_streams = ctx.extras.get("layer_streams", [])
@@ -410,7 +413,7 @@ class StepRunner:
         torch.cuda.synchronize(self.device)
         graph = torch.cuda.CUDAGraph()
         before = library.launch_count
-        with torch.cuda.graph(graph, pool=self._graph_pool):
+        with torch.cuda.graph(graph, pool=self._graph_pool), engine_step(self.small_products):
             logits = self.model.forward(ctx)
         launches = library.launch_count - before
         library.launch_count = before                # recorded, not run: replays do the counting

@@ -712,8 +712,7 @@ def dense_rows(a: torch.Tensor, w: torch.Tensor, *, swiglu: bool = False, out: O
     """``a . w^T`` for up to 16 bfloat16 rows against a bfloat16 weight ``[N, K]`` that streams in once
     (``dense_rows.cu``): float32 ``[M, N]`` (plus ``bias``), added into ``out`` with reductions when
     ``accumulate``, or with ``swiglu`` (``w`` = gate rows then up rows) ``silu(g) * u`` in bfloat16 ``[M, N / 2]``.
-    ``early``: weight and bias were there before the kernel in front of this one, whose end the product need not await to
-    read them."""
+    ``early``: weight and bias may be read before the kernels in front of this one have ended (see dense_rows.cu)."""
     _need(a, "a", torch.bfloat16)
     _need(w, "w", torch.bfloat16)
     M, K = a.shape

@@ -9,15 +9,17 @@ Which routine runs is decided by the weight's dtype and the number of rows, not 
   batched projections, src/SharpInference.Cuda/CudaBackend.cs:2083-2117).  With few rows (decode), where the
   reference runs matvec kernels of its own (llm_matvec_*, src/SharpInference.Cuda/CudaTextKernels.cs:1325),
   they can run the engine's weight-streaming kernel instead (``stream_rows``; ``dense_rows.cu``: the weight is
-  read once, rows dealt evenly over the SMs, bias, add-in or SwiGLU in its epilogue).  In a model that an engine
-  holds small products run there by default (``stream_small``); for large ones it is the faster kernel alone (see
-  DEFAULT_STREAM_ROWS) but not inside a decode step, so they stay with the library.
+  read once, rows dealt evenly over the SMs, bias, add-in or SwiGLU in its epilogue).  In an engine's steps small products
+  run there by default (:func:`engine_step`); for large ones it is the faster kernel alone (see DEFAULT_STREAM_ROWS) but
+  not inside a decode step, so they stay with the library.
 * sizes neither takes (an inner size that is no multiple of 8) use the CUDA-core kernel.
 
 The grouped (per-expert) product has no library counterpart and always runs our own kernels.
 """
 from __future__ import annotations
 
+import contextlib
+import threading
 from typing import Optional
 
 import torch
@@ -34,13 +36,33 @@ from ..kernels import ops
 # kernel of another stream (the router beside the shared expert) or a block of a neighbour that is still or
 # already there delays one of its CTAs by up to the whole product.
 DEFAULT_STREAM_ROWS = 0
-# Small products (``stream_small``): up to this many rows against a weight of up to this many elements, the weight-streaming kernel,
+# Small products (:func:`engine_step`): up to this many rows against a weight of up to this many elements, the weight-streaming kernel,
 # which may start while the kernel before it ends (the library's kernels take 8 to 13 us where reading the weight takes 1 to 3).
 # Library / own kernel between two other kernels of a captured graph, us, weights from memory, at 1, 8 and 16 rows: 1024 x 1024
 # 5.7 / 3.9, 6.1 / 4.5, 6.1 / 4.5; 2048 x 2048 9.3 / 5.3, 8.2 / 5.7, 7.1 / 6.3; 2048 x 4096 13.3 / 6.7, 12.1 / 7.4, 9.8 / 9.0; 4096 x
 # 4096 14.5 / 10.0, 13.2 / 10.2, 10.9 / 10.8; 8192 x 2048 10.0 / 9.2, 9.5 / 9.6, 9.9 / 10.1; 16384 x 2048 15.0 / 15.0, 14.7 / 15.3,
 # 14.9 / 17.1; 5120 x 5120 13.5 / 12.6, 13.5 / 12.8, 14.8 / 14.2.
 SMALL_PRODUCTS = ((8, 1 << 24), (16, 1 << 23))
+
+
+class _Step(threading.local):
+    small_products = False
+
+
+_step = _Step()
+
+
+@contextlib.contextmanager
+def engine_step(small_products: bool):
+    """While an engine launches a step in this thread: whether small products run on the weight-streaming kernel, which may
+    read a weight before the kernels in front of it have ended.  A step begins behind a copy, which waits for all that the
+    stream was given before, so whatever a program wrote into its weights by then is there; outside of a step nothing is known
+    of what wrote them last, and the same :class:`Linear` goes to the library."""
+    before, _step.small_products = _step.small_products, small_products
+    try:
+        yield
+    finally:
+        _step.small_products = before
 
 
 class Linear:
@@ -63,8 +85,8 @@ class Linear:
         # Up to this many rows (at most ops.DENSE_ROWS_MAX) the product runs on the weight-streaming kernel
         # instead of the library; 0: the library at every size.
         self.stream_rows = stream_rows
-        # Whether small products (SMALL_PRODUCTS) run there too.  Set by an engine for the weights of its model, which are written
-        # once, before its first step: such a product may read them before the kernel in front of it has ended.
+        # Whether small products (SMALL_PRODUCTS) run there outside of an engine's steps too: for a program whose stream has waited
+        # for what wrote the weight since (see engine_step).
         self.stream_small = False
         # Up to this many rows an add-in (``accumulate``) runs on the grouped tensor-core kernel with one group
         # and K cut over CTAs: small CTAs that add with reductions and run well beside other kernels.
@@ -106,9 +128,9 @@ class Linear:
                     and (a.data_ptr() | self.weight.data_ptr()) % 16 == 0))
 
     def small(self, rows: int, fused: bool = False) -> bool:
-        """Whether a product of this many rows is one of the small ones that ``stream_small`` means.  With SwiGLU in its epilogue,
+        """Whether a product of this many rows is a small one that runs on the weight-streaming kernel.  With SwiGLU in its epilogue,
         which saves a kernel of 2 to 3 us, weights may have twice as many elements."""
-        return self.stream_small and any(0 < rows <= most and self.weight.numel() <= size << fused for most, size in SMALL_PRODUCTS)
+        return (self.stream_small or _step.small_products) and any(0 < rows <= most and self.weight.numel() <= size << fused for most, size in SMALL_PRODUCTS)
 
     def adds_with_reductions(self, a: torch.Tensor) -> bool:
         """Whether ``accumulate`` adds this product of ``a`` into the output element by element with reductions

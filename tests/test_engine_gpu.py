@@ -180,6 +180,23 @@ def test_dense_products_on_the_engines_own_kernel(large_shapes, rows):
     assert err < TOL["bfloat16"], (err, where)
 
 
+def test_small_products_run_on_the_own_kernel_inside_of_steps_only(model_dirs, monkeypatch):
+    """A model's small products are on the weight-streaming kernel in the engine's steps; called by the program, the same weights go
+    to the library as before it had an engine."""
+    from sharpinference_b200 import StepEntry
+    from sharpinference_b200.kernels import ops
+    calls, kernel = [], ops.dense_rows
+    monkeypatch.setattr(ops, "dense_rows", lambda *a, **kw: (calls.append(1), kernel(*a, **kw))[1])
+    engine = make_engine(model_dirs["A"], "bfloat16", 64)
+    lin = engine.model.blocks[0].mixer.qkv
+    a = torch.randn(3, lin.in_features, device="cuda:0").to(torch.bfloat16)
+    engine.open_request(0)
+    engine.forward_step([StepEntry(0, [1, 2, 3], [2])])
+    assert calls
+    calls.clear()
+    assert not lin.streams(a) and torch.equal(lin(a), torch.mm(a, lin.weight.t(), out_dtype=torch.float32)) and not calls
+
+
 @pytest.mark.parametrize("name", list(TINY))
 def test_float32_cuts_agree_with_each_other_tightly(model_dirs, name):
     """In 32-bit every kernel sums in an order that depends on the row alone, so a row's logits

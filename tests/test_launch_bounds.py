@@ -100,3 +100,26 @@ def test_chunk_kernels_are_left_alone_beyond_their_sizes():
     assert ops._chunks("mlstm", 4096, 1, None, 1, 128, 1 << 17) > 0 and ops._chunks("mlstm", 4096, 1, None, 1, 128, (1 << 17) + 4) == 0
     assert ops._chunks("mlstm", 4096, 1, None, 8, 130, 64) == 0 and ops._chunks("mlstm", 4096, 1, None, 8, 128, 66) == 0
     assert ops._chunks("ssd", 4096, 1, None, 8, 64, 64, 4, 1) == 0
+
+
+def test_small_products_are_an_engine_steps_own():
+    """Inside of an engine's step, and in its thread alone, small products may run on the weight-streaming kernel; the model's
+    weights carry no mark of it afterwards, also when the step failed."""
+    import threading
+
+    import pytest
+    import torch
+    from sharpinference_b200.parts.linear import Linear, engine_step
+    lin = Linear(torch.zeros(16, 8, dtype=torch.bfloat16))
+    seen = []
+    with pytest.raises(ValueError):
+        with engine_step(True):
+            assert lin.small(1) and lin.small(16) and not lin.small(17)
+            other = threading.Thread(target=lambda: seen.append(lin.small(1)))
+            other.start()
+            other.join()
+            with engine_step(False):
+                assert not lin.small(1)
+            assert lin.small(1)
+            raise ValueError
+    assert seen == [False] and not lin.small(1) and not lin.stream_small
