@@ -9,7 +9,7 @@ Kept with the same spelling, meaning and default: ``-m|--model`` (here a model f
 ``--verbose-prompt``, ``--no-display-prompt``, ``--device`` (an index or a name such as CUDA0; one GPU, and
 no CPU), ``--min-batch-blas`` (the smallest step whose dense products go to the library's GEMM: below it the
 engine's own weight-streaming kernel runs them, as the reference's matvec kernels do below its threshold,
-src/SharpInference.Cli/RunCommand.cs:179-182; here 0 means that for small weights only).  There is no tokenizer in this engine (random-weight
+src/SharpInference.Cli/RunCommand.cs:179-182; here 0 means that for small weights only, 1 the library for all).  There is no tokenizer in this engine (random-weight
 models have no vocabulary), so a prompt is a list of token ids: ``-p "5 17 3"`` or ``--tokens
 5,17,3``; several prompts are separated by ``;`` and are served as one continuous batch.  Added:
 ``--dtype``, ``--random-weights SEED`` with ``--config`` (writes a model folder first),
@@ -71,7 +71,8 @@ def build_parser() -> argparse.ArgumentParser:
     ap.add_argument("--min-batch-blas", type=int, default=0,
                     help="smallest step (rows) whose dense products go to the library's GEMM; smaller steps run them on "
                          "the engine's own weight-streaming kernel (at most 17: that kernel takes up to 16 rows).  "
-                         "0 (default): small weights only, the library for the others, which is the faster step on B200")
+                         "0 (default): small weights only, the library for the others, which is the faster step on B200; "
+                         "1: the library at every size and weight")
     ap.add_argument("--json", action="store_true", help="print the result as one JSON object")
     ap.add_argument("--trace-layers", action="store_true",
                     help="after every step print, per layer, the L2 norm of the last row's residual and the expert "
@@ -128,7 +129,8 @@ def main(argv=None) -> int:
         return 2
     engine = Engine(model_dir, dtype=ns.dtype, device=device, options=EngineOptions(
         page_size=ns.page_size, max_cache_tokens=cache_tokens, max_batch=ns.max_batch,
-        max_tokens_per_step=ns.max_tokens_per_step, own_dense_rows=max(0, min(ns.min_batch_blas, 17) - 1)))
+        max_tokens_per_step=ns.max_tokens_per_step, own_dense_rows=max(0, min(ns.min_batch_blas, 17) - 1),
+        own_small_products=ns.min_batch_blas != 1))
     params = [SamplingParams(temperature=ns.temp, top_k=ns.top_k, top_p=ns.top_p, min_p=ns.min_p,
                              repetition_penalty=ns.repeat_penalty, penalty_last_n=ns.repeat_last_n,
                              frequency_penalty=ns.frequency_penalty, presence_penalty=ns.presence_penalty,

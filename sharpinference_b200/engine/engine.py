@@ -46,10 +46,9 @@ class EngineOptions:
     cuda_graphs: bool = True            # capture decode-only steps as CUDA graphs (when the model's parts allow)
     # Dense bfloat16 products of steps of up to this many rows (at most 16) run on the engine's own
     # weight-streaming kernel instead of the vendor library (which the reference also uses only for batched
-    # projections, its single-token products being kernels of its own).  0: small products only
-    # (parts/linear.py, SMALL_PRODUCTS), the library for the others, which is the faster step on B200 (Scout sizes, 8
-    # layers, batch 1: 614 against 593 tok/s) although the own kernel is the faster product alone (parts/linear.py has
-    # the figures).  The LM head keeps the library either way (2 GB of weights: 322 against 299 us) unless it is small.
+    # projections, its single-token products being kernels of its own).  0: the library, but for small products
+    # (own_small_products), which is the faster step on B200 (Scout sizes, 8 layers, batch 1: 614 against 593 tok/s)
+    # although the own kernel is the faster product alone (parts/linear.py has the figures).  The LM head keeps the library either way (2 GB of weights: 322 against 299 us) unless it is small.
     # The results differ by rounding only.
     own_dense_rows: int = 0
     # Launch kernels with programmatic stream serialization: a kernel's set-up overlaps the tail of the one
@@ -57,6 +56,10 @@ class EngineOptions:
     # are shared by every engine in it).
     programmatic_launch: bool = True
     keep_finished: int = 1024           # finished requests whose output `output()` can still give
+    # Small dense products of few rows (parts/linear.py, SMALL_PRODUCTS) on the weight-streaming kernel whatever own_dense_rows
+    # says, where it is the faster step (4 layers of width 2048 at batch 1: 178 against 283 us).  False, with own_dense_rows
+    # = 0: the library for every dense product.
+    own_small_products: bool = True
 
 
 @dataclass
@@ -116,7 +119,7 @@ class Engine:
                                   device=self.device, model_state_specs=getattr(self.model, "state_specs", None))
         self.runner = StepRunner(self.model, self.cache)
         self.runner.use_graphs = self.runner.use_graphs and o.cuda_graphs
-        self.runner.small_products = True
+        self.runner.small_products = o.own_small_products
         self.scheduler = Scheduler(self.cache, max_batch=o.max_batch, max_tokens_per_step=o.max_tokens_per_step,
                                    max_positions=getattr(self.model, "max_positions", None))
         self.sampler = Sampler(self.device)

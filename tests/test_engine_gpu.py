@@ -197,6 +197,23 @@ def test_small_products_run_on_the_own_kernel_inside_of_steps_only(model_dirs, m
     assert not lin.streams(a) and torch.equal(lin(a), torch.mm(a, lin.weight.t(), out_dtype=torch.float32)) and not calls
 
 
+def test_the_library_can_have_every_dense_product(model_dirs, monkeypatch):
+    """own_small_products=False with own_dense_rows=0: no dense product of a step, eager or replayed, is on the weight-streaming
+    kernel; by default the small ones are."""
+    from sharpinference_b200 import Engine, EngineOptions, StepEntry
+    from sharpinference_b200.kernels import ops
+    calls, kernel = [], ops.dense_rows
+    monkeypatch.setattr(ops, "dense_rows", lambda *a, **kw: (calls.append(1), kernel(*a, **kw))[1])
+    for own in (True, False):
+        calls.clear()
+        engine = Engine(model_dirs["A"], dtype="bfloat16", device="cuda:0",
+                        options=EngineOptions(page_size=16, max_cache_tokens=64, max_batch=2, own_small_products=own))
+        engine.open_request(0)
+        for toks in ([1, 2, 3], [4], [5], [6]):
+            engine.forward_step([StepEntry(0, toks, [len(toks) - 1])])
+        assert bool(calls) == own and engine.runner.graph_replays > 0
+
+
 @pytest.mark.parametrize("name", list(TINY))
 def test_float32_cuts_agree_with_each_other_tightly(model_dirs, name):
     """In 32-bit every kernel sums in an order that depends on the row alone, so a row's logits
