@@ -231,7 +231,7 @@ def wkv(ns) -> None:
 
 
 def scan(ns) -> None:
-    """The causal convolution (with the gate's silu), the softplus of the step sizes and the selective scan for `batch`
+    """The causal convolution and the selective scan with its softplus and silu, as the mixer calls them, for `batch`
     requests of `tokens` rows each: per row, channel and state one exponential and four flops; decode streams the
     state once."""
     B, n, C, N, R = ns.batch, ns.tokens, ns.channels, ns.states, ns.dt_rank
@@ -246,16 +246,14 @@ def scan(ns) -> None:
     rr = torch.arange(T, dtype=torch.int32, device=DEV) // n
     slot_sets = [torch.arange(c * B, (c + 1) * B, dtype=torch.int32, device=DEV) for c in range(copies)]
     it = {"i": 0}
-    dtwork = torch.empty_like(dtraw)
 
     def fn():
         slots = slot_sets[it["i"] % copies]
         it["i"] += 1
         x32, _ = ops.causal_conv(xz, C, conv_w, conv_b, conv_state, row_request=rr, row_offsets=offs, state_slots=slots,
-                                 act_dtype=torch.bfloat16, gate_col=C)
-        dt = ops.bias_act(dtraw, dt_b, ops.ACT_SOFTPLUS, torch.float32, out=dtwork)
-        ops.selective_scan(x32, dt, dbc, R, R + N, a_log, dsk, xz, C, row_offsets=offs, state_slots=slots,
-                           state=state, out_dtype=torch.bfloat16)
+                                 act_dtype=torch.bfloat16)
+        ops.selective_scan(x32, dtraw, dbc, R, R + N, a_log, dsk, xz, C, row_offsets=offs, state_slots=slots,
+                           state=state, out_dtype=torch.bfloat16, dt_bias=dt_b, max_rows=n)
     ms = _time(fn, max(ns.iters, copies))
     print(f"scan batch={B} tokens={n} channels={C} states={N}: {ms * 1e3:.1f} us, state {2 * B * C * N * 4 / ms / 1e6:.0f} GB/s "
           f"(read and written once), {T * C * N / ms / 1e6:.1f} G state updates/s (an exponential and four flops each)")

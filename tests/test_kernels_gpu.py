@@ -346,6 +346,30 @@ def test_gemm_nt_kernels_form_the_same_numbers(ops, N, K):
     assert shifted.data_ptr() % 16 and torch.equal(full, ops.gemm_nt(shifted, w))
 
 
+def test_gemm_nt_wide_tiles_form_the_same_numbers(ops):
+    """Products that fill the GPU take tiles of 128 rows (from 148 tiles on): the bits of the few-row kernel, of tiles of 64 and
+    of the general kernel, with remainders on all sides; grouped, with an empty group, groups that end inside a tile and one row."""
+    M, N, K = 1203, 1000, 132
+    assert -(-M // 128) * -(-N // 64) >= 148
+    a, w = rnd(M, K, seed=13), rnd(N, K, seed=14)
+    full = ops.gemm_nt(a, w)
+    ref, mag = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    assert bool(((full.double() - ref).abs() <= (65 + K / 128) * 2.0 ** -24 * mag).all())
+    for at, m in ((0, 1), (120, 16), (1100, 103), (700, 300)):                     # few rows, and tiles of 64
+        assert torch.equal(full[at:at + m], ops.gemm_nt(a[at:at + m].contiguous(), w)), (at, m)
+    shifted = torch.empty(M * K + 1, device=DEV)[1:].view(M, K).copy_(a)
+    assert shifted.data_ptr() % 16 and torch.equal(full, ops.gemm_nt(shifted, w))
+    counts = [300, 0, 1, 128, 129, 645]
+    assert sum(counts) == M
+    offsets = torch.tensor([sum(counts[:i]) for i in range(7)], dtype=torch.int32, device=DEV)
+    we = rnd(6, N, K, seed=15)
+    got = ops.gemm_nt(a, we, group_offsets=offsets, rows=M)
+    for e, n in enumerate(counts):
+        lo = int(offsets[e])
+        if n:
+            assert torch.equal(got[lo:lo + n], ops.gemm_nt(a[lo:lo + n].contiguous(), we[e])), e
+
+
 def test_gemm_nt_few_rows_grouped(ops):
     E, N, K, T = 6, 70, 388, 19
     w, a = rnd(E, N, K, seed=5), rnd(T, K, seed=6)

@@ -223,6 +223,27 @@ def test_state_space_duality_in_chunks(monkeypatch, heads, groups, N, P):
         assert float((torch.cat(got[b]) - want[b]).abs().max()) < 2e-5 * max(float(want[b].abs().max()), 1.0)
 
 
+@pytest.mark.parametrize("heads,groups,N,P,lens", [(64, 1, 128, 100, [700]), (64, 2, 64, 64, [300, 200, 650, 1])])
+def test_state_space_duality_in_chunks_many_tiles_a_cta(heads, groups, N, P, lens):
+    """Steps whose CTAs work through several tiles: more than one of a head, from the middle of a head on, over heads, with a short
+    last group; against the walk (sums of up to 700 products rounded in another order, 1e-5 of the largest)."""
+    from sharpinference_b200.kernels import ops
+    assert heads // groups * -(-P // 64) * groups * (sum(lens) // 64) > 2 * 296
+    g = torch.Generator().manual_seed(P)
+    T, inner, bc = sum(lens), heads * P, groups * N
+    xbc, dt, params = 0.7 * torch.randn(T, inner + 2 * bc, generator=g), torch.randn(T, heads, generator=g), torch.randn(3, heads, generator=g)
+    _, off, sl = _step_meta(lens, list(range(len(lens))))
+    out = []
+    for split in (False, True):
+        state = torch.zeros(len(lens), heads * N * P, device=DEV)
+        y = ops.ssd_scan(xbc.to(DEV), dt.to(DEV), col_x=0, col_b=inner, col_c=inner + bc, col_dt=0, dt_bias=f32(params[0] - 2),
+                         a_log=f32(params[1]), dskip=f32(params[2]), row_offsets=off, state_slots=sl, state=state, heads=heads,
+                         groups=groups, states=N, vdim=P, split=split, max_rows=max(lens))
+        out.append((y, state))
+    for a, b in zip(*out):
+        assert float((a - b).abs().max()) <= 1e-5 * float(a.abs().max()) and not torch.equal(a, b)
+
+
 @pytest.mark.parametrize("bad", [math.nan, math.inf])
 @pytest.mark.parametrize("heads,groups,N,P", [(4, 2, 64, 8), (3, 1, 128, 100)])
 def test_state_space_duality_in_chunks_keeps_later_values_out(monkeypatch, heads, groups, N, P, bad):

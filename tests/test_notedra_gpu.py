@@ -321,6 +321,29 @@ def test_mlstm_recurrence_in_chunks(monkeypatch, heads, d, dv):
         assert torch.equal(out[0][0][short], out[1][0][short])
 
 
+@pytest.mark.parametrize("heads,d,dv,lens", [(8, 128, 256, [900, 700, 400]), (10, 64, 200, [2000])])
+def test_mlstm_recurrence_in_chunks_many_tiles_a_cta(heads, d, dv, lens):
+    """Steps whose CTAs work through several tiles of a head, the first of which also has the normaliser: numerators, n . q and state
+    as the walk leaves them (sums of up to 2000 decaying products rounded in another order, 1e-5 of the largest)."""
+    from sharpinference_b200.kernels import ops
+    from sharpinference_b200.parts.mlstm import fused_mlstm_columns
+    assert heads * -(-dv // 64) * (sum(lens) // 64) > 2 * 296
+    g = torch.Generator().manual_seed(dv)
+    cq, ck, cv, cg, ci, cf, width = fused_mlstm_columns(heads, d, dv)
+    T = sum(lens)
+    proj, bias = torch.randn(T, width, generator=g).to(DEV), torch.randn(2, heads, generator=g).to(DEV)
+    offs = torch.tensor([sum(lens[:i]) for i in range(len(lens) + 1)], dtype=torch.int32, device=DEV)
+    slots, out = torch.arange(len(lens), dtype=torch.int32, device=DEV), []
+    for split in (False, True):
+        state = torch.zeros(len(lens), ops.mlstm_state_floats(heads, d, dv)[1], device=DEV)
+        num, nq, _ = ops.mlstm_recurrence(proj, col_q=cq, col_k=ck, col_v=cv, col_i=ci, col_f=cf, bias_i=bias[0], bias_f=bias[1] + 3,
+                                          row_offsets=offs, state_slots=slots, state=state, heads=heads, d=d, dv=dv, cap=9.0,
+                                          q_scale=d ** -0.5, split=split, max_rows=max(lens))
+        out.append((num, nq, state))
+    for a, b in zip(*out):
+        assert float((a - b).abs().max()) <= 1e-5 * float(a.abs().max()) and not torch.equal(a, b)
+
+
 @pytest.mark.parametrize("bad", [float("nan"), float("inf")])
 @pytest.mark.parametrize("heads,d,dv", [(2, 24, 40), (1, 128, 132)])
 def test_mlstm_recurrence_in_chunks_keeps_later_values_out(monkeypatch, heads, d, dv, bad):

@@ -419,6 +419,31 @@ def test_selective_scan_raw_inputs_and_cuts(C, N):
     assert torch.equal(given, whole) and torch.equal(s_given, s_whole)
 
 
+def test_selective_scan_of_several_prompts_is_that_of_each_alone():
+    """Three walks of 3200 channels go at four states a lane without helpers, one alone at two with them; single rows beside a
+    prompt leave it at two: the same bits whatever serves a request."""
+    from sharpinference_b200.kernels import ops
+    g = torch.Generator().manual_seed(8)
+    C, N = 3200, 16
+    f = lambda *s: torch.randn(*s, generator=g).to(DEV)
+    bias, dsk, a_log = f(C), f(C), (-2.0 + 2.0 * torch.rand(C, N, generator=g)).to(DEV)
+    for lens in ([40, 40, 37], [90, 1, 1, 2], [20, 1]):
+        T, B = sum(lens), len(lens)
+        x, dt, bc, z = f(T, C), f(T, C), f(T, 2 * N), f(T, C)
+
+        def run(rows, lens, known):
+            state = torch.zeros(len(lens), C * N, device=DEV)
+            meta = _step_meta(lens, list(range(len(lens))))
+            return ops.selective_scan(x[rows], dt[rows], bc[rows], 0, N, a_log, dsk, z[rows], 0, row_offsets=meta[1], state_slots=meta[2],
+                                      state=state, out_dtype=torch.float32, dt_bias=bias, max_rows=max(lens) if known else None), state
+        for known in (True, False):
+            y, states = run(slice(0, T), lens, known)
+            for b, n in enumerate(lens):
+                rows = slice(sum(lens[:b]), sum(lens[:b]) + n)
+                y1, s1 = run(rows, [n], known)
+                assert torch.equal(y[rows], y1) and torch.equal(states[b], s1[0]), (lens, b, known)
+
+
 @pytest.mark.parametrize("layout", ["halves", "interleaved"])
 @pytest.mark.parametrize("nq,nkv,dk,dv,rot", [(4, 2, 16, 32, 8), (2, 1, 64, 64, 64), (3, 3, 24, 10, 0), (1, 1, 2, 2, 2)])
 def test_rotation_with_norm_first_and_rotated_values(layout, nq, nkv, dk, dv, rot):
