@@ -31,7 +31,7 @@
 // latent attention).  A key block is loaded once and is the right operand of both products, K-major for the scores and
 // MN-major for the sums: the same bytes in shared memory.  The tile list cuts 64 rows there, so a CTA serves two query heads of
 // one key head, rows 0-63 and 64-127 of the MMA.  One CTA an SM at the larger sizes (the queries alone take 80 KB at 320
-// elements), three key blocks in flight.  16 heads on one row of 320 with sums of 256, a prompt of 2048 rows: 54 us, 269 us
+// elements), three key blocks in flight.  16 heads on one row of 320 with sums of 256, a prompt of 2048 rows: 55 us, 269 us
 // with m16n8k16 (attention_keys.cu, which keeps the sizes, masks and biases that this form does not take).
 //
 // Sizes: head size 64 or 128, pages of a multiple of 64 positions, bf16.  Everything else takes the

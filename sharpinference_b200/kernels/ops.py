@@ -1215,7 +1215,8 @@ def causal_conv(xz: torch.Tensor, channels: int, weight: torch.Tensor, bias: Opt
     """``silu`` of the causal convolution of the first ``channels`` columns of ``xz`` (float32 ``[T, ld]``) with
     ``weight [channels, taps]`` (last column: the current token) and ``bias``; inputs before a portion come from
     ``state [slots, (taps - 1) * channels]``, which is moved on.  Returns ``(x32, x_act)``.  With ``gate_col`` the
-    columns ``gate_col .. gate_col + channels - 1`` of ``xz`` are replaced by their ``silu`` in the same pass."""
+    columns ``gate_col .. gate_col + channels - 1`` of ``xz`` are replaced by their ``silu`` in the same pass: for a program
+    that gives :func:`selective_scan` ready gates (the mixers leave the gate to the kernels behind)."""
     _need(xz, "xz", torch.float32)
     _need(weight, "weight", torch.float32)
     _need(state, "state", torch.float32)
@@ -1251,9 +1252,9 @@ def selective_scan(x: torch.Tensor, dt: torch.Tensor, bc: torch.Tensor, col_b: i
                    max_rows: Optional[int] = None) -> torch.Tensor:
     """The selective scan over the rows of every request from and into ``state [slots, channels * states]``:
     ``(S C + D x) * g`` in ``out_dtype``, with ``dt`` the step sizes themselves (after their softplus) and ``g`` the
-    gate (already ``silu(z)``) in the columns of ``xz`` from ``col_z``.  With ``dt_bias [channels]`` both come raw: the
-    step sizes are ``softplus(dt + dt_bias)`` and the gate ``silu`` of those columns.  ``max_rows``: the rows of the longest
-    request, if known (a choice of kernels, no result depends on it)."""
+    gate (already ``silu(z)``) in the columns of ``xz`` from ``col_z``, for programs that have them so.  With ``dt_bias
+    [channels]``, as in the mixer, both come raw: the step sizes are ``softplus(dt + dt_bias)`` and the gate ``silu`` of
+    those columns.  ``max_rows``: the rows of the longest request, if known (a choice of kernels, no result depends on it)."""
     if dt_bias is not None:
         _need(dt_bias, "dt_bias", torch.float32)
         if dt_bias.numel() != x.shape[1]:
