@@ -296,11 +296,12 @@ __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAtt
             m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
             m = fmaxf(m_run, fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2)));
             const float corr = m_run == -INFINITY ? 0.0f : expf(m_run - m);
+            const float base = m == -INFINITY ? 0.0f : m;         // (a score of minus infinity gives zero also where there is no other)
 #pragma unroll
             for (int i = 0; i < AR_BK; i += 16)
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
-                    const float v = p[i + c], e = __float_as_uint(v) == AR_HIDDEN ? -0.0f : v == -INFINITY ? 0.0f : expf(v - m);
+                    const float v = p[i + c], e = __float_as_uint(v) == AR_HIDDEN ? -0.0f : expf(v - base);
                     p[i + c] = e;
                     l = __fadd_rn(l, e);
                 }
