@@ -908,10 +908,10 @@ def _chunks(kind: str, T: int, B: int, max_rows: Optional[int], heads: int, d: i
     return chunks if max(chunks, B, heads) <= 65535 and d * dv <= 1 << 24 else 0
 
 
-def _others_walk(T: int, B: int, max_rows: Optional[int]) -> int:
-    """Whether requests beside those in chunks may have rows to walk: not where the one request is known to have all of the step's
-    rows (the row count alone does not say so: the rows may lie behind the last request's)."""
-    return int(not (B == 1 and max_rows == T))
+def _chunk_border(kind: str, T: int, B: int, max_rows: Optional[int], heads: int) -> tuple:
+    """For a step with chunks: the rows from which on a request runs so, and whether others may have rows to walk: not where the one
+    request is known to have all of the step's rows (the row count alone does not say so: rows may lie behind the last request's)."""
+    return chunked_least(kind, heads), int(not (B == 1 and max_rows == T))
 
 
 def mlstm_recurrence(proj: torch.Tensor, *, col_q: int, col_k: int, col_v: int, col_i: int, col_f: int,
@@ -950,8 +950,7 @@ def mlstm_recurrence(proj: torch.Tensor, *, col_q: int, col_k: int, col_v: int, 
                                             bias_f.data_ptr(), row_offsets.data_ptr(), state_slots.data_ptr(),
                                             state.data_ptr(), state.stride(0), per_head, B, T, heads, d, dv,
                                             float(cap), float(q_scale), coef.data_ptr(), o_raw.data_ptr(), nq.data_ptr(),
-                                            _ptr(sums), chunks, chunked_least("mlstm", heads),
-                                            _others_walk(T, B, max_rows), _stream()),
+                                            _ptr(sums), chunks, *(_chunk_border("mlstm", T, B, max_rows, heads) if chunks else (0, 1)), _stream()),
           "sharpi_mlstm_recurrence")
     return o_raw, nq, coef
 
@@ -1185,8 +1184,8 @@ def wkv_recurrence(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, wraw: torc
     check(kernel("sharpi_wkv_recurrence")(r.data_ptr(), k.data_ptr(), v.data_ptr(), wraw.data_ptr(), w0.data_ptr(),
                                           u.data_ptr(), row_offsets.data_ptr(), state_slots.data_ptr(),
                                           state.data_ptr(), state.stride(0), o.data_ptr(), bonus.data_ptr(), T,
-                                          B, heads, d, _ptr(sums), chunks, chunked_least("wkv", heads),
-                                          _others_walk(T, B, max_rows), _stream()),
+                                          B, heads, d, _ptr(sums), chunks,
+                                          *(_chunk_border("wkv", T, B, max_rows, heads) if chunks else (0, 1)), _stream()),
           "sharpi_wkv_recurrence")
     return o
 
@@ -1490,7 +1489,7 @@ def ssd_scan(xbc: torch.Tensor, proj: torch.Tensor, *, col_x: int, col_b: int, c
                                     dt_bias.data_ptr(), a_log.data_ptr(), dskip.data_ptr(), row_offsets.data_ptr(),
                                     state_slots.data_ptr(), state.data_ptr(), state.stride(0), y.data_ptr(), T,
                                     B, heads, groups, states, vdim, _ptr(sums), chunks,
-                                    chunked_least("ssd", heads), _others_walk(T, B, max_rows), _stream()),
+                                    *(_chunk_border("ssd", T, B, max_rows, heads) if chunks else (0, 1)), _stream()),
           "sharpi_ssd_scan")
     return y
 
