@@ -241,16 +241,19 @@ constexpr int WALK_STAGE = 8;                                  // rows staged to
 
 // A walk over many rows (LONG) starts on an empty GPU and lets nothing onto its SMs: its few blocks would otherwise land
 // several to an SM.
-template <int R4, bool LONG>                                   // float4 of a column a lane: 32 R4 >= d
-__global__ void __launch_bounds__(WALK_THREADS) delta_walk_kernel(DeltaArgs a) {
-    constexpr int DP = 32 * R4;
+// NC: columns that eight lanes hold, 32 apart.  Rows of many requests that each bring few are their states' bytes, read and
+// written once: with four columns a block has a whole head of 128 on its way at once, and its keys, queries and decays (two
+// exponentials and a logarithm each) are formed once instead of four times.  A column's operations are the same for every NC.
+template <int R4, int NC, bool LONG>                           // float4 of a column a lane: 32 R4 >= d
+__global__ void __launch_bounds__(WALK_THREADS, NC > 1 ? 2 : 0) delta_walk_kernel(DeltaArgs a) {
+    constexpr int DP = 32 * R4, COLS = WALK_COLS * NC;         // columns of a block
     extern __shared__ __align__(16) float walk_smem[];
     float* q_s = walk_smem;                                    // [STAGE][DP] each, zeros behind d
     float* k_s = q_s + WALK_STAGE * DP;
     float* g_s = k_s + WALK_STAGE * DP;
     float* v_s = g_s + WALK_STAGE * DP;                        // [STAGE][COLS]
-    float* o_s = v_s + WALK_STAGE * WALK_COLS;
-    float* b_s = o_s + WALK_STAGE * WALK_COLS;                 // [STAGE] beta, [STAGE] k . q
+    float* o_s = v_s + WALK_STAGE * COLS;
+    float* b_s = o_s + WALK_STAGE * COLS;                 // [STAGE] beta, [STAGE] k . q
     const int h = blockIdx.y, hk = h / (a.heads / a.kvh);
     const float rate = expf(a.a_log[h]);
     if (LONG) pdl_wait_only();
@@ -260,14 +263,17 @@ __global__ void __launch_bounds__(WALK_THREADS) delta_walk_kernel(DeltaArgs a) {
     if (rows <= 0) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int sub = threadIdx.x & (WALK_LANES - 1), col = threadIdx.x / WALK_LANES;
-    const int c0 = blockIdx.x * WALK_COLS, c = c0 + col;
+    const int c0 = blockIdx.x * COLS, c = c0 + col;
     float* st = a.state + (size_t)a.state_slots[req] * a.state_stride + ((size_t)h * a.dv + c) * a.dp;
-    float4 S[R4];
+    float4 S[NC][R4];
 #pragma unroll
-    for (int j = 0; j < R4; ++j) {
-        const int e = 4 * (sub + WALK_LANES * j);
-        S[j] = c < a.dv && e < a.dp ? *reinterpret_cast<const float4*>(st + e) : make_float4(0, 0, 0, 0);
-    }
+    for (int x = 0; x < NC; ++x)
+#pragma unroll
+        for (int j = 0; j < R4; ++j) {
+            const int e = 4 * (sub + WALK_LANES * j);
+            S[x][j] = c + x * WALK_COLS < a.dv && e < a.dp ? *reinterpret_cast<const float4*>(st + (size_t)x * WALK_COLS * a.dp + e)
+                                                            : make_float4(0, 0, 0, 0);
+        }
     for (int r0 = 0; r0 < rows; r0 += WALK_STAGE) {
         const int nr = min(WALK_STAGE, rows - r0);
         if (r0) __syncthreads();                               // the rows before are no longer read
@@ -283,8 +289,8 @@ __global__ void __launch_bounds__(WALK_THREADS) delta_walk_kernel(DeltaArgs a) {
             }
             q_s[i] = q; k_s[i] = k; g_s[i] = g;
         }
-        for (int i = threadIdx.x; i < nr * WALK_COLS; i += WALK_THREADS) {
-            const int r = i / WALK_COLS, cc = c0 + i % WALK_COLS;
+        for (int i = threadIdx.x; i < nr * COLS; i += WALK_THREADS) {
+            const int r = i / COLS, cc = c0 + i % COLS;
             v_s[i] = cc < a.dv ? a.qkv[(size_t)(first + r0 + r) * a.C + 2 * a.kvh * a.d + (size_t)h * a.dv + cc] : 0.0f;
         }
         if (threadIdx.x < nr) b_s[threadIdx.x] = a.beta[(size_t)(first + r0 + threadIdx.x) * a.heads + h];
@@ -300,42 +306,58 @@ __global__ void __launch_bounds__(WALK_THREADS) delta_walk_kernel(DeltaArgs a) {
             const float4* k4 = reinterpret_cast<const float4*>(k_s + r * DP) + sub;
             const float4* q4 = reinterpret_cast<const float4*>(q_s + r * DP) + sub;
             const float4* g4 = reinterpret_cast<const float4*>(g_s + r * DP) + sub;
-            float4 ak = make_float4(0, 0, 0, 0), aq = ak;
+            float4 ak[NC], aq[NC];
+#pragma unroll
+            for (int x = 0; x < NC; ++x) ak[x] = aq[x] = make_float4(0, 0, 0, 0);
 #pragma unroll
             for (int j = 0; j < R4; ++j) {
                 const float4 k = k4[WALK_LANES * j], q = q4[WALK_LANES * j], g = g4[WALK_LANES * j];
-                S[j].x *= g.x; S[j].y *= g.y; S[j].z *= g.z; S[j].w *= g.w;
-                ak.x = fmaf(S[j].x, k.x, ak.x); ak.y = fmaf(S[j].y, k.y, ak.y);
-                ak.z = fmaf(S[j].z, k.z, ak.z); ak.w = fmaf(S[j].w, k.w, ak.w);
-                aq.x = fmaf(S[j].x, q.x, aq.x); aq.y = fmaf(S[j].y, q.y, aq.y);
-                aq.z = fmaf(S[j].z, q.z, aq.z); aq.w = fmaf(S[j].w, q.w, aq.w);
-            }
-            float dk = (ak.x + ak.y) + (ak.z + ak.w), dq = (aq.x + aq.y) + (aq.z + aq.w);
 #pragma unroll
-            for (int o = WALK_LANES / 2; o > 0; o >>= 1) {
-                dk += __shfl_xor_sync(0xffffffffu, dk, o);
-                dq += __shfl_xor_sync(0xffffffffu, dq, o);
+                for (int x = 0; x < NC; ++x) {
+                    float4& s = S[x][j];
+                    s.x *= g.x; s.y *= g.y; s.z *= g.z; s.w *= g.w;
+                    ak[x].x = fmaf(s.x, k.x, ak[x].x); ak[x].y = fmaf(s.y, k.y, ak[x].y);
+                    ak[x].z = fmaf(s.z, k.z, ak[x].z); ak[x].w = fmaf(s.w, k.w, ak[x].w);
+                    aq[x].x = fmaf(s.x, q.x, aq[x].x); aq[x].y = fmaf(s.y, q.y, aq[x].y);
+                    aq[x].z = fmaf(s.z, q.z, aq[x].z); aq[x].w = fmaf(s.w, q.w, aq[x].w);
+                }
             }
-            const float u = b_s[r] * (v_s[r * WALK_COLS + col] - dk);
-            if (sub == 0) o_s[r * WALK_COLS + col] = fmaf(b_s[WALK_STAGE + r], u, dq);
+            float u[NC];
+#pragma unroll
+            for (int x = 0; x < NC; ++x) {
+                float dk = (ak[x].x + ak[x].y) + (ak[x].z + ak[x].w), dq = (aq[x].x + aq[x].y) + (aq[x].z + aq[x].w);
+#pragma unroll
+                for (int o = WALK_LANES / 2; o > 0; o >>= 1) {
+                    dk += __shfl_xor_sync(0xffffffffu, dk, o);
+                    dq += __shfl_xor_sync(0xffffffffu, dq, o);
+                }
+                u[x] = b_s[r] * (v_s[r * COLS + col + x * WALK_COLS] - dk);
+                if (sub == 0) o_s[r * COLS + col + x * WALK_COLS] = fmaf(b_s[WALK_STAGE + r], u[x], dq);
+            }
 #pragma unroll
             for (int j = 0; j < R4; ++j) {
                 const float4 k = k4[WALK_LANES * j];
-                S[j].x = fmaf(k.x, u, S[j].x); S[j].y = fmaf(k.y, u, S[j].y);
-                S[j].z = fmaf(k.z, u, S[j].z); S[j].w = fmaf(k.w, u, S[j].w);
+#pragma unroll
+                for (int x = 0; x < NC; ++x) {
+                    float4& s = S[x][j];
+                    s.x = fmaf(k.x, u[x], s.x); s.y = fmaf(k.y, u[x], s.y);
+                    s.z = fmaf(k.z, u[x], s.z); s.w = fmaf(k.w, u[x], s.w);
+                }
             }
         }
         __syncthreads();
-        for (int i = threadIdx.x; i < nr * WALK_COLS; i += WALK_THREADS) {
-            const int r = i / WALK_COLS, cc = c0 + i % WALK_COLS;
+        for (int i = threadIdx.x; i < nr * COLS; i += WALK_THREADS) {
+            const int r = i / COLS, cc = c0 + i % COLS;
             if (cc < a.dv) a.y[((size_t)(first + r0 + r) * a.heads + h) * a.dv + cc] = o_s[i];
         }
     }
 #pragma unroll
-    for (int j = 0; j < R4; ++j) {
-        const int e = 4 * (sub + WALK_LANES * j);
-        if (c < a.dv && e < a.dp) *reinterpret_cast<float4*>(st + e) = S[j];
-    }
+    for (int x = 0; x < NC; ++x)
+#pragma unroll
+        for (int j = 0; j < R4; ++j) {
+            const int e = 4 * (sub + WALK_LANES * j);
+            if (c + x * WALK_COLS < a.dv && e < a.dp) *reinterpret_cast<float4*>(st + (size_t)x * WALK_COLS * a.dp + e) = S[x][j];
+        }
 }
 
 static bool fill_delta(DeltaArgs& a, const float* qkv, const float* beta, const float* z, int ldz, const float* dt_bias,
@@ -351,24 +373,33 @@ static bool fill_delta(DeltaArgs& a, const float* qkv, const float* beta, const 
     return true;
 }
 
-template <int R4>
-static int launch_delta_walk(const DeltaArgs& a, int n, int max_rows, cudaStream_t stream) {
-    const dim3 grid((a.dv + WALK_COLS - 1) / WALK_COLS, a.heads, n);
-    const size_t smem = (size_t)(WALK_STAGE * (3 * 32 * R4 + 2 * WALK_COLS) + 2 * WALK_STAGE) * sizeof(float);
+template <int R4, int NC, bool LONG>
+static int launch_delta_walk(const DeltaArgs& a, int n, cudaStream_t stream) {
+    const dim3 grid((a.dv + WALK_COLS * NC - 1) / (WALK_COLS * NC), a.heads, n);
+    const size_t smem = (size_t)(WALK_STAGE * (3 * 32 * R4 + 2 * WALK_COLS * NC) + 2 * WALK_STAGE) * sizeof(float);
+    auto kern = delta_walk_kernel<R4, NC, LONG>;
     static bool configured = false;
     if (smem > 48 * 1024 && !configured) {
-        if (cudaFuncSetAttribute(delta_walk_kernel<R4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-            cudaFuncSetAttribute(delta_walk_kernel<R4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-            return SHARPI_LAUNCH_FAILED;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SHARPI_LAUNCH_FAILED;
         configured = true;
     }
-    if (max_rows > WALK_STAGE) {
-        delta_walk_kernel<R4, true><<<grid, WALK_THREADS, smem, stream>>>(a);
+    if (LONG) {
+        kern<<<grid, WALK_THREADS, smem, stream>>>(a);
         SHARPI_CHECK_LAUNCH();
     } else {
-        SHARPI_LAUNCH_PDL((delta_walk_kernel<R4, false>), grid, WALK_THREADS, smem, stream, a);
+        SHARPI_LAUNCH_PDL(kern, grid, WALK_THREADS, smem, stream, a);
     }
     return SHARPI_OK;
+}
+
+template <int R4>
+static int launch_delta_walk(const DeltaArgs& a, int n, int max_rows, cudaStream_t stream) {
+    if (max_rows > WALK_STAGE) return launch_delta_walk<R4, 1, true>(a, n, stream);
+    // Four columns where the blocks are many waves of the SMs (two blocks each): 128 x 128 heads, single rows, us with one / four
+    // columns: 16 heads of 8 requests 6.7 / 8.4, 40 20.9 / 21.0, 80 37.7 / 35.7, 200 94.0 / 84.4; 8 heads of 80 21.5 / 22.0, 200 48.7 / 44.9.
+    if constexpr (R4 <= 4)
+        if (a.dv > 3 * WALK_COLS && (long long)n * a.heads >= 1024) return launch_delta_walk<R4, 4, false>(a, n, stream);
+    return launch_delta_walk<R4, 1, false>(a, n, stream);
 }
 
 // `requests` (nullable): the `n` requests of the step to serve; null: requests 0 .. n - 1.  `max_rows`: the most rows one of
