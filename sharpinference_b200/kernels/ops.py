@@ -28,7 +28,8 @@ def dtype_code(dtype: torch.dtype) -> int:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # torch.cuda.current_stream().cuda_stream without the Stream object in between (a tenth of a launch's host time)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
