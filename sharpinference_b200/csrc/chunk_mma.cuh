@@ -10,13 +10,16 @@
 //                  D_ij = b_j a_(j+1) .. a_i
 //
 // Operands are float32 numbers in three bfloat16 pieces (24 bits together), products the six of nine piece products that
-// reach 24 bits, added in float32 (m16n8k16).  Decays are products of the a themselves, formed one factor after the other
-// as a walk over the rows would: differences of summed logarithms would lose what the sums have in common.
+// reach 24 bits, added in float32 (m16n8k16).  Decays are products of the a themselves: differences of summed
+// logarithms would lose what the sums have in common.
 // Several heads may share keys and queries (a key head); their scores q . k are then formed once.
 //
-// One prompt of 2048 rows, walked row by row / in chunks: matrix memory, 8 heads of 128 x 256, 321 / 126 us; state-space
-// duality, 64 heads of 128 x 64 on one key head, 646 / 212 us.  The chunk kernels wait for their tiles from L2 and for the
-// tensor core's latency (two CTAs of four warps an SM; the tensor pipe is busy a fifth of the time).
+// One prompt of 2048 rows, walked row by row / in chunks: matrix memory, 8 heads of 128 x 256, 321 / 120 us; state-space
+// duality, 64 heads of 128 x 64 on one key head, 646 / 180 us.  Two CTAs of four warps an SM (255 registers hold the queries' or keys'
+// pieces); the chunk kernels wait for one warp's products, conversions and barriers in turn (a fifth to a quarter of the issue
+// slots, the tensor pipe a third of the time).  1777 rows of the duality, outputs / sums: 113 / 52 us when a tile's values were fetched
+// as it began, a head's 64 x 64 decays formed by chains of 64 products, and what joins an output was read behind a store
+// (which it might alias: sixteen trips to L2, one after the other); 86 / 46 us now.
 #pragma once
 
 #include "common.cuh"
@@ -27,7 +30,8 @@ namespace chunked {
 constexpr int ROWS = 64;          // rows of a chunk
 constexpr int COLS = 64;          // value columns of a tile
 constexpr int THREADS = 128;
-constexpr int LD_D = ROWS + 1;    // floats between two rows of D in shared memory
+constexpr int BLOCK = 16;         // rows of a block of a chunk (a warp's)
+constexpr int LD_D = BLOCK + 1;   // floats between two rows of a block's D in shared memory
 constexpr int CARRY_THREADS = 256;
 
 struct Args {
@@ -121,6 +125,34 @@ __device__ __forceinline__ bool load_split(bf16* dst, const float* src, size_t l
     return zero == 0.0f;
 }
 
+// The same in two parts: R x C floats on their way into shared memory (a thread's pieces of four lie where it alone reads them: no
+// barrier), and, when they are there, their pieces; a row of block b times f(r).
+template <int R, int C>
+__device__ __forceinline__ void fetch_raw(float* raw, const float* src, size_t ld, int rows, int cols) {
+#pragma unroll
+    for (int p = 0; p < R * C / 4 / THREADS; ++p) {
+        const int i = threadIdx.x + p * THREADS, r = i / (C / 4), e = (i % (C / 4)) * 4;
+        const bool ok = r < rows && e < cols;
+        mma16::cp_async_16(raw + 4 * i, ok ? src + (size_t)r * ld + e : src, ok ? 16 : 0);
+    }
+}
+template <int R, int C, class W>
+__device__ __forceinline__ bool split_raw(bf16* dst, const float* raw, const W& f) {
+    constexpr int LD = C + 8, PLANE = R * LD;
+    float zero = 0.0f;
+#pragma unroll
+    for (int p = 0; p < R * C / 4 / THREADS; ++p) {
+        const int i = threadIdx.x + p * THREADS, r = i / (C / 4), e = (i % (C / 4)) * 4;
+        float4 x = *reinterpret_cast<const float4*>(raw + 4 * i);
+        zero = fmaf(x.x, 0.0f, fmaf(x.y, 0.0f, fmaf(x.z, 0.0f, fmaf(x.w, 0.0f, zero))));
+        const float s = f(p, r);
+        const mma16::Pieces lo = mma16::split3(x.x * s, x.y * s), hi = mma16::split3(x.z * s, x.w * s);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(dst + q * PLANE + r * LD + e) = make_uint2(lo.v[q], hi.v[q]);
+    }
+    return zero == 0.0f;
+}
+
 // x b[n] for N neighbouring n-tiles, all pieces, a tile after the other for each.  The tensor core's own additions cut off what
 // does not fit: over the 72 of a row's sums that was the largest error (5.3e-7 of the result against 7.7e-8 of a float32 walk).
 // So the large product of a step starts from zero and joins `acc` by a rounded addition; the five small ones, which start 8 bits
@@ -193,31 +225,52 @@ __device__ __forceinline__ void own_rows_exact(float (&acc)[8][4], const float (
     }
 }
 
-// a_t and b_t of the chunk's rows for head h into shared memory (1 and 0 behind the last row)
+// a_t and b_t of row threadIdx.x of the chunk for head h, in the threads of the first two warps (1 and 0 behind the last row)
 template <class F>
-__device__ __forceinline__ void load_decays(const F& f, const Place& p, int h, float* a_s, float* b_s) {
-    if (threadIdx.x < ROWS) {
-        float al = 1.0f, be = 0.0f;
-        if (threadIdx.x < p.rows) f.decay(p.row0 + threadIdx.x, h, al, be);
-        a_s[threadIdx.x] = al;
-        b_s[threadIdx.x] = be;
+__device__ __forceinline__ void load_decays(const F& f, const Place& p, int h, float& al, float& be) {
+    al = 1.0f; be = 0.0f;
+    if ((int)threadIdx.x < p.rows) f.decay(p.row0 + threadIdx.x, h, al, be);
+}
+
+// In the first two warps, a row a thread: b of the row times the decays behind it in its block of 16 rows, and every block's decay.
+// With them D_ij of rows in different blocks is three factors: the decays up to i in its block, those of the blocks between, and
+// this.  (All factors are at most 1, so none is zero where their product is not.)
+__device__ __forceinline__ void block_tails(float al, float be, float* tail_s, float* block_s) {
+    const int l = threadIdx.x % BLOCK;
+    float z = al;
+#pragma unroll
+    for (int o = 1; o < BLOCK; o <<= 1) {
+        const float y = __shfl_down_sync(0xffffffffu, z, o, BLOCK);
+        if (l + o < BLOCK) z *= y;
     }
+    const float behind = __shfl_down_sync(0xffffffffu, z, 1, BLOCK);
+    tail_s[threadIdx.x] = l == BLOCK - 1 ? be : be * behind;
+    if (l == 0) block_s[threadIdx.x / BLOCK] = z;
 }
 
 // DP: the key size padded to 64 or 128.  A CTA holds the chunk's keys as left operands in registers (warp w: DP / 4 of the
-// state's rows) and works through `group` tiles of the key head's heads.
+// state's rows) and works through `group` tiles of the key head's heads; a tile's values come in while the one before is multiplied.
 template <class F, int DP>
 __global__ void __launch_bounds__(THREADS, 2) sums_kernel(Args a, F f) {
     extern __shared__ __align__(16) uint8_t chunk_smem[];
     constexpr int LDK = DP + 8, PLANE_K = ROWS * LDK, LDV = COLS + 8, PLANE_V = ROWS * LDV, MT = DP / 64;
     bf16* k_s = reinterpret_cast<bf16*>(chunk_smem);
     bf16* v_s = k_s + 3 * PLANE_K;
-    __shared__ float a_s[ROWS], b_s[ROWS], w_s[ROWS];
+    float* raw = reinterpret_cast<float*>(v_s + 3 * PLANE_V);
+    __shared__ float tail_s[ROWS], block_s[ROWS / BLOCK];
     Place p;
     if (!find_chunk(a.row_offsets, a.B, a.least, blockIdx.z, p)) return;
     const int kh = blockIdx.y, per = a.heads / a.key_heads, tiles = (a.dv + COLS - 1) / COLS;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const float* keys = a.k + (size_t)p.row0 * a.ld_k + (size_t)kh * a.d;
+    const int first = blockIdx.x * a.group, last = min(first + a.group, per * tiles);
+    auto fetch = [&](int tl) {
+        const int h = kh * per + tl / tiles, c0 = (tl % tiles) * COLS;
+        fetch_raw<ROWS, COLS>(raw, a.v + (size_t)p.row0 * a.ld_v + (size_t)h * a.dv + c0, a.ld_v, p.rows, a.dv - c0);
+    };
+    float al = 1.0f, be = 0.0f;
+    fetch(first);
+    if (warp < 2) load_decays(f, p, kh * per + first / tiles, al, be);
     load_split<ROWS, DP>(k_s, keys, a.ld_k, p.rows, a.d, nullptr);
     __syncthreads();
     uint32_t x[MT][4][3][4];
@@ -229,33 +282,32 @@ __global__ void __launch_bounds__(THREADS, 2) sums_kernel(Args a, F f) {
             for (int q = 0; q < 3; ++q)      // stored [row][key channel], taken transposed
                 mma16::ldmatrix_x4_trans(x[m][kk][q], k_s + q * PLANE_K + (kk * 16 + (lane / 16) * 8 + lane % 8) * LDK +
                                                           (warp * MT + m) * 16 + ((lane / 8) % 2) * 8);
-    const int last = min((int)(blockIdx.x + 1) * a.group, per * tiles);
     int have = -1;
-    for (int tl = blockIdx.x * a.group; tl < last; ++tl) {
+    for (int tl = first; tl < last; ++tl) {
         const int h = kh * per + tl / tiles, c0 = (tl % tiles) * COLS;
-        __syncthreads();
-        if (h != have) {
-            load_decays(f, p, h, a_s, b_s);
-            __syncthreads();
-            if (threadIdx.x <= ROWS) {       // thread j: what row j's term is worth behind the last row; thread 64: A
-                const int j = threadIdx.x;
-                float w = j < ROWS ? b_s[j] : 1.0f;
-#pragma unroll 8
-                for (int i = 0; i < ROWS; ++i)
-                    if (i > j || j == ROWS) w *= a_s[i];
-                if (j < ROWS) w_s[j] = w;
-                else if (tl % tiles == 0) a.total[(size_t)blockIdx.z * a.heads + h] = w;
-            }
-            __syncthreads();
-            have = h;
-        }
-        load_split<ROWS, COLS>(v_s, a.v + (size_t)p.row0 * a.ld_v + (size_t)h * a.dv + c0, a.ld_v, p.rows, a.dv - c0, w_s);
-        __syncthreads();
         const size_t head = (size_t)blockIdx.z * a.heads + h;
-        if (F::NORM && tl % tiles == 0 && (int)threadIdx.x < a.d) {
-            float n = 0.0f;
-            for (int j = 0; j < p.rows; ++j) n = fmaf(w_s[j], keys[(size_t)j * a.ld_k + threadIdx.x], n);
-            a.sums[a.norms + head * a.d + threadIdx.x] = n;
+        if (h != have && warp < 2) block_tails(al, be, tail_s, block_s);
+        have = h;
+        mma16::cp_async_wait_all();
+        __syncthreads();                     // the tails are here; the tile before has been multiplied
+        const float after[4] = {block_s[1] * block_s[2] * block_s[3], block_s[2] * block_s[3], block_s[3], 1.0f};
+        // rows 8 p + thread / 16: what the row's term is worth behind the last one
+        split_raw<ROWS, COLS>(v_s, raw, [&](int pc, int r) { return tail_s[r] * after[pc / 2]; });
+        if (tl % tiles == 0) {
+            if (threadIdx.x == 0) a.total[head] = block_s[0] * after[0];
+            if (F::NORM && (int)threadIdx.x < a.d) {
+                float n = 0.0f;
+#pragma unroll
+                for (int b = 0; b < ROWS / BLOCK; ++b)
+                    for (int j = b * BLOCK; j < min((b + 1) * BLOCK, p.rows); ++j)
+                        n = fmaf(tail_s[j] * after[b], keys[(size_t)j * a.ld_k + threadIdx.x], n);
+                a.sums[a.norms + head * a.d + threadIdx.x] = n;
+            }
+        }
+        __syncthreads();
+        if (tl + 1 < last) {
+            fetch(tl + 1);
+            if (warp < 2 && (tl + 1) % tiles == 0) load_decays(f, p, h + 1, al, be);
         }
         float* out = a.sums + head * a.d * a.dv;
 #pragma unroll
@@ -346,14 +398,23 @@ __global__ void __launch_bounds__(THREADS, 2) outs_kernel(Args a, F f) {
     constexpr int KS = 3 * (PLANE_K > PLANE_S ? PLANE_K : PLANE_S);
     bf16* k_s = reinterpret_cast<bf16*>(chunk_smem);           // the keys; then the state before the chunk
     bf16* v_s = k_s + KS;
-    float* D_s = reinterpret_cast<float*>(v_s + 3 * PLANE_V);   // [64][LD_D]
-    __shared__ float a_s[ROWS], b_s[ROWS], d0_s[ROWS];
+    float* raw = reinterpret_cast<float*>(v_s + 3 * PLANE_V);   // the next tile's values
+    float* D_s = raw + ROWS * COLS;                            // [block][16][LD_D]: D inside a block
+    __shared__ float head_s[ROWS], tail_s[ROWS], block_s[ROWS / BLOCK];   // decays from a block's first row up to a row; block_tails
     Place p;
     if (!find_chunk(a.row_offsets, a.B, a.least, blockIdx.z, p)) return;
     const int kh = blockIdx.y, per = a.heads / a.key_heads, tiles = (a.dv + COLS - 1) / COLS;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane / 4, t = lane % 4;
     const int i0 = warp * 16 + g, i1 = i0 + 8;                 // this lane's rows
     const float* queries = a.q + (size_t)p.row0 * a.ld_q + (size_t)kh * a.d;
+    const int first = blockIdx.x * a.group, last = min(first + a.group, per * tiles);
+    auto fetch_values = [&](int tl) {
+        const int h = kh * per + tl / tiles, c0 = (tl % tiles) * COLS;
+        fetch_raw<ROWS, COLS>(raw, a.v + (size_t)p.row0 * a.ld_v + (size_t)h * a.dv + c0, a.ld_v, p.rows, a.dv - c0);
+    };
+    float al = 1.0f, be = 0.0f;
+    fetch_values(first);
+    if (warp < 2) load_decays(f, p, kh * per + first / tiles, al, be);
     load_split<ROWS, DP>(k_s, a.k + (size_t)p.row0 * a.ld_k + (size_t)kh * a.d, a.ld_k, p.rows, a.d, nullptr);
     uint32_t x[KT][3][4];
 #pragma unroll
@@ -394,36 +455,33 @@ __global__ void __launch_bounds__(THREADS, 2) outs_kernel(Args a, F f) {
         }
         add_small(score + n, small);
     }
-    const int last = min((int)(blockIdx.x + 1) * a.group, per * tiles);
     int have = -1;
-    for (int tl = blockIdx.x * a.group; tl < last; ++tl) {
+    for (int tl = first; tl < last; ++tl) {
         const int h = kh * per + tl / tiles, c0 = (tl % tiles) * COLS;
         const size_t head = (size_t)blockIdx.z * a.heads + h;
-        __syncthreads();
-        if (h != have) {
-            load_decays(f, p, h, a_s, b_s);
-            __syncthreads();
-            const int j = threadIdx.x % ROWS;
-            if (threadIdx.x < ROWS) {                          // column j of D
-                float w = 0.0f;
-                const float own = b_s[j];
-#pragma unroll 8
-                for (int i = 0; i < ROWS; ++i) {
-                    w = i == j ? own : w * a_s[i];
-                    D_s[i * LD_D + j] = w;
-                }
-            } else {
-                float w = 1.0f;
-#pragma unroll 8
-                for (int i = 0; i < ROWS; ++i)
-                    if (i <= j) w *= a_s[i];
-                d0_s[j] = w;
-            }
-            have = h;
-        }
-        load_split<DP, COLS>(k_s, a.sums + head * a.d * a.dv + c0, a.dv, a.d, a.dv - c0, nullptr);
         const float* values = a.v + (size_t)p.row0 * a.ld_v + (size_t)h * a.dv + c0;
-        const bool odd = __syncthreads_or(!load_split<ROWS, COLS>(v_s, values, a.ld_v, p.rows, a.dv - c0, nullptr));
+        mma16::cp_async_wait_all();
+        __syncthreads();                                       // the keys, or the tile before: done with
+        load_split<DP, COLS>(k_s, a.sums + head * a.d * a.dv + c0, a.dv, a.d, a.dv - c0, nullptr);
+        const bool odd = __syncthreads_or(!split_raw<ROWS, COLS>(v_s, raw, [](int, int) { return 1.0f; }));
+        if (h != have && warp < 2) {
+            const int l = lane % BLOCK;
+            float z = al, w = 0.0f;
+#pragma unroll
+            for (int o = 1; o < BLOCK; o <<= 1) {
+                const float y = __shfl_up_sync(0xffffffffu, z, o, BLOCK);
+                if (l >= o) z *= y;
+            }
+            head_s[threadIdx.x] = z;
+            block_tails(al, be, tail_s, block_s);
+#pragma unroll
+            for (int i = 0; i < BLOCK; ++i) {                  // column l of the block's D
+                const float ai = __shfl_sync(0xffffffffu, al, i, BLOCK);
+                w = i == l ? be : w * ai;
+                D_s[(threadIdx.x / BLOCK * BLOCK + i) * LD_D + l] = w;
+            }
+        }
+        have = h;
         float acc[8][4];
         clear(acc);
 #pragma unroll
@@ -438,7 +496,16 @@ __global__ void __launch_bounds__(THREADS, 2) outs_kernel(Args a, F f) {
             }
             add_small(acc + n, small);
         }
-        const float p0 = d0_s[i0], p1 = d0_s[i1];
+        __syncthreads();                                       // D is here
+        if (tl + 1 < last) {
+            fetch_values(tl + 1);
+            if (warp < 2 && (tl + 1) % tiles == 0) load_decays(f, p, h + 1, al, be);
+        }
+        float before = 1.0f;                                   // the decays of the blocks in front of this warp's
+#pragma unroll
+        for (int b = 0; b < 3; ++b)
+            if (b < warp) before *= block_s[b];
+        const float h0 = head_s[i0], h1 = head_s[i1], p0 = before * h0, p1 = before * h1;
 #pragma unroll
         for (int n = 0; n < 8; ++n) {
             acc[n][0] *= p0; acc[n][1] *= p0;
@@ -449,14 +516,24 @@ __global__ void __launch_bounds__(THREADS, 2) outs_kernel(Args a, F f) {
         for (int kk = 0; kk < 4; ++kk) {
             if (kk > warp) continue;
             uint32_t w[3][4];
-            float u[4][2];
+            float u[4][2], m = 1.0f;                           // the decays of the blocks between
+#pragma unroll
+            for (int b = kk + 1; b < 3; ++b)
+                if (b < warp) m *= block_s[b];
+            const float m0 = m * h0, m1 = m * h1;
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int r = e & 1 ? i1 : i0, n = 2 * kk + (e >> 1), c = n * 8 + 2 * t;
+                float d0, d1;
+                if (kk == warp) {
+                    d0 = D_s[r * LD_D + c % BLOCK]; d1 = D_s[r * LD_D + c % BLOCK + 1];
+                } else {
+                    d0 = (e & 1 ? m1 : m0) * tail_s[c]; d1 = (e & 1 ? m1 : m0) * tail_s[c + 1];
+                }
                 // (selected, not multiplied by zero: what a later row's key brings must not reach this one through a NaN; for its
                 // values see own_rows_exact)
-                const float u0 = c <= r ? score[n][2 * (e & 1)] * D_s[r * LD_D + c] : 0.0f;
-                const float u1 = c + 1 <= r ? score[n][2 * (e & 1) + 1] * D_s[r * LD_D + c + 1] : 0.0f;
+                const float u0 = c <= r ? score[n][2 * (e & 1)] * d0 : 0.0f;
+                const float u1 = c + 1 <= r ? score[n][2 * (e & 1) + 1] * d1 : 0.0f;
                 if (F::NORM) (e & 1 ? row1 : row0) += u0 + u1;
                 u[e][0] = u0; u[e][1] = u1;
                 const mma16::Pieces s = mma16::split3(u0, u1);
@@ -503,11 +580,15 @@ __global__ void __launch_bounds__(THREADS, 2) outs_kernel(Args a, F f) {
             const int r = e ? i1 : i0;
             if (r >= p.rows) continue;
 #pragma unroll
+            for (int n = 0; n < 8; ++n) {                      // (what joins is read before the first store: a load behind one waits for it)
+                const int c = c0 + n * 8 + 2 * t;
+                if (c < a.dv) f.finish(p.row0 + r, h, c, acc[n][2 * e], acc[n][2 * e + 1]);
+            }
+#pragma unroll
             for (int n = 0; n < 8; ++n) {
                 const int c = c0 + n * 8 + 2 * t;
                 if (c < a.dv)
-                    *reinterpret_cast<float2*>(a.out + ((size_t)(p.row0 + r) * a.heads + h) * a.dv + c) =
-                        f.finish(p.row0 + r, h, c, make_float2(acc[n][2 * e], acc[n][2 * e + 1]));
+                    *reinterpret_cast<float2*>(a.out + ((size_t)(p.row0 + r) * a.heads + h) * a.dv + c) = make_float2(acc[n][2 * e], acc[n][2 * e + 1]);
             }
         }
     }
@@ -524,8 +605,8 @@ inline bool takes(const Args& a) {
 template <class F, int DP>
 static int launch(Args a, const F& f, int chunks, cudaStream_t stream) {
     constexpr int LDV = COLS + 8, KS = 3 * (ROWS * (DP + 8) > DP * LDV ? ROWS * (DP + 8) : DP * LDV);
-    constexpr size_t smem_sums = (size_t)(3 * ROWS * (DP + 8) + 3 * ROWS * LDV) * sizeof(bf16);
-    constexpr size_t smem_outs = (size_t)(KS + 3 * ROWS * LDV) * sizeof(bf16) + ROWS * LD_D * sizeof(float);
+    constexpr size_t smem_sums = (size_t)(3 * ROWS * (DP + 8) + 3 * ROWS * LDV) * sizeof(bf16) + ROWS * COLS * sizeof(float);
+    constexpr size_t smem_outs = (size_t)(KS + 3 * ROWS * LDV) * sizeof(bf16) + (ROWS * COLS + ROWS * LD_D) * sizeof(float);
     if (cudaFuncSetAttribute(sums_kernel<F, DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_sums) != cudaSuccess ||
         cudaFuncSetAttribute(outs_kernel<F, DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_outs) != cudaSuccess)
         return SHARPI_LAUNCH_FAILED;

@@ -195,10 +195,10 @@ struct SsdChunks {
     }
     __device__ __forceinline__ float* norm(int, int, int) const { return nullptr; }
     __device__ __forceinline__ void store_norm(int, int, float) const {}
-    __device__ __forceinline__ float2 finish(int t, int h, int c, float2 o) const {
+    __device__ __forceinline__ void finish(int t, int h, int c, float& o0, float& o1) const {
         const float2 x = *reinterpret_cast<const float2*>(s.xbc + (size_t)t * s.ld_x + s.col_x + h * s.P + c);
         const float d = s.dskip[h];
-        return make_float2(o.x + d * x.x, o.y + d * x.y);
+        o0 += d * x.x; o1 += d * x.y;
     }
 };
 

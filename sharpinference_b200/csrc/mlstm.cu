@@ -352,7 +352,7 @@ struct MlstmChunks {
     }
     __device__ __forceinline__ float* norm(int slot, int h, int i) const { return head(slot, h) + (size_t)m.slices * m.d * 32 + i; }
     __device__ __forceinline__ void store_norm(int t, int h, float s) const { m.nq[(size_t)t * m.heads + h] = s * m.q_scale; }
-    __device__ __forceinline__ float2 finish(int, int, int, float2 o) const { return make_float2(o.x * m.q_scale, o.y * m.q_scale); }
+    __device__ __forceinline__ void finish(int, int, int, float& o0, float& o1) const { o0 *= m.q_scale; o1 *= m.q_scale; }
 };
 
 // `sums` (nullable; `chunks` * heads * (d * dv + d + 1) floats): requests of at least `least` rows run in chunks, `chunks` of
