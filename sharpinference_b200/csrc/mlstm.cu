@@ -64,94 +64,124 @@ __device__ __forceinline__ float log_sigmoid(float x) {
 }
 
 // ---------------------------------------------------------------------------------------
-// gates: grid (B, heads), one warp.  PRE: the capped gates of every row were formed by gate_values_kernel (all rows
-// in parallel) and lie in coef[.., 0] and coef[.., 1]; otherwise the warp forms them itself (steps of few rows: one
-// launch fewer).  The arithmetic is the same either way.
+// gates: grid (B, heads).  Steps of few rows: one warp forms the gates of 32 rows and walks them.  Steps of many: one warp walks,
+// four others form the gates of the rows ahead and what follows from the rows behind.  The arithmetic is the same either way.
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ void capped_gates(float zi, float zf, float bi, float bf, float cap, float& ig, float& fg) {
     ig = cap * tanhf((zi + bi) / cap);
     fg = log_sigmoid(cap * tanhf((zf + bf) / cap));
 }
 
-__global__ void gate_values_kernel(MlstmArgs a, long long items) {
-    const long long item = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (item >= items) return;
-    const long long t = item / a.heads;
-    const int h = (int)(item - t * a.heads);
-    float ig, fg;
-    capped_gates(a.proj[(size_t)t * a.ld + a.col_i + h], a.proj[(size_t)t * a.ld + a.col_f + h], a.bias_i[h], a.bias_f[h],
-                 a.cap, ig, fg);
-    a.coef[item * 4] = ig;
-    a.coef[item * 4 + 1] = fg;
+__device__ __forceinline__ float* running_maximum(const MlstmArgs& a, int b, int h) {
+    return a.state + (size_t)a.state_slots[b] * a.state_stride + (size_t)h * a.head_stride + (size_t)a.slices * a.d * 32 + a.d;
 }
 
-template <bool PRE>
+__device__ __forceinline__ void store_coef(const MlstmArgs& a, int t, int h, float ig, float fg, float m_before, float m_after) {
+    float* c = a.coef + ((size_t)t * a.heads + h) * 4;
+    c[0] = fg + m_before - m_after;
+    c[1] = ig - m_after;
+    c[2] = m_after;
+}
+
 __global__ void __launch_bounds__(32) mlstm_gates_kernel(MlstmArgs a) {
-    __shared__ __align__(16) float2 gates_s[32];
-    __shared__ float m_s[33];
     const int b = blockIdx.x, h = blockIdx.y, lane = threadIdx.x;
     const int r0 = a.row_offsets[b], r1 = a.row_offsets[b + 1];
     if (r1 <= r0) return;
-    float* m_state = a.state + (size_t)a.state_slots[b] * a.state_stride + (size_t)h * a.head_stride +
-                     (size_t)a.slices * a.d * 32 + a.d;
+    float* m_state = running_maximum(a, b, h);
     float m = *m_state;
     const float bi = a.bias_i[h], bf = a.bias_f[h];
-    // x, y: the raw gate projections of this lane's row, or (PRE) its finished gates
-    auto fetch = [&](int r, float& x, float& y) {
-        x = 0.0f;
-        y = 0.0f;
-        if (r < r1) {
-            if (PRE) {
-                x = a.coef[((size_t)r * a.heads + h) * 4];
-                y = a.coef[((size_t)r * a.heads + h) * 4 + 1];
-            } else {
-                x = a.proj[(size_t)r * a.ld + a.col_i + h];
-                y = a.proj[(size_t)r * a.ld + a.col_f + h];
-            }
-        }
-    };
-    // A block of 32 rows takes 600 cycles, its gates as long to arrive: four blocks are on their way.
-    constexpr int AHEAD = 4;
-    float xs[AHEAD], ys[AHEAD];
-#pragma unroll
-    for (int k = 0; k < AHEAD; ++k) fetch(r0 + 32 * k + lane, xs[k], ys[k]);
-    for (int u0 = r0; u0 < r1; u0 += 32 * AHEAD)
-#pragma unroll
-    for (int k = 0; k < AHEAD; ++k) {
-        const int t0 = u0 + 32 * k;
-        if (t0 >= r1) break;
+    for (int t0 = r0; t0 < r1; t0 += 32) {
         const int n = min(32, r1 - t0);
-        const float x = xs[k], y = ys[k];
-        float ig = x, fg = y;
-        if (!PRE) capped_gates(x, y, bi, bf, a.cap, ig, fg);
-        fetch(t0 + 32 * AHEAD + lane, xs[k], ys[k]);
-        // The chain is one addition and one maximum a row.  The gates go through shared memory, so that they are in registers
-        // two rows a load before the chain needs them and a row costs three instructions (shuffles and selects took ten:
-        // 2048 rows of 8 heads: 24.7 us so, 20.6 us now).  Rows beyond the request's end come behind the last m that is used.
-        gates_s[lane] = make_float2(fg, ig);
-        __syncwarp();
-        float4 g[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) g[j] = reinterpret_cast<const float4*>(gates_s)[j];
-        if (lane == 0) m_s[0] = m;
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            const float m1 = fmaxf(g[j].x + m, g[j].y);
-            m = fmaxf(g[j].z + m1, g[j].w);
-            if (lane == 0) { m_s[2 * j + 1] = m1; m_s[2 * j + 2] = m; }
+        float ig = 0.0f, fg = 0.0f, m_before = 0.0f, m_after = 0.0f;
+        if (lane < n)
+            capped_gates(a.proj[(size_t)(t0 + lane) * a.ld + a.col_i + h], a.proj[(size_t)(t0 + lane) * a.ld + a.col_f + h], bi, bf, a.cap, ig, fg);
+        for (int j = 0; j < n; ++j) {
+            const float next = fmaxf(__shfl_sync(0xffffffffu, fg, j) + m, __shfl_sync(0xffffffffu, ig, j));
+            if (lane == j) { m_before = m; m_after = next; }
+            m = next;
         }
-        __syncwarp();
-        const float m_before = m_s[lane], m_after = m_s[lane + 1];
-        m = m_s[n];
-        if (lane < n) {
-            float* c = a.coef + ((size_t)(t0 + lane) * a.heads + h) * 4;
-            c[0] = fg + m_before - m_after;
-            c[1] = ig - m_after;
-            c[2] = m_after;
-        }
-        __syncwarp();
+        if (lane < n) store_coef(a, t0 + lane, h, ig, fg, m_before, m_after);
     }
     if (lane == 0) *m_state = m;
+}
+
+// Many rows, GATE_ROWS at a time.  The chain is one addition and one maximum a row, and nothing else may stand in its way: its warp
+// reads finished gates (two rows a load, in registers before the chain needs them) and stores the maxima four rows at a time,
+// while the others, a row a thread, store the coefficients of the rows before, form the gates of the rows after (tanh and
+// logsigmoid) and have the projections behind those on their way.  8 heads, 2048 rows / three requests of at most 1118: 42 / 22 us when the
+// walking warp did the rest too (the gates in a kernel of their own), 16 / 10 us so.
+constexpr int GATE_ROWS = 128;
+
+__global__ void __launch_bounds__(GATE_ROWS + 32) mlstm_gates_long_kernel(MlstmArgs a) {
+    __shared__ __align__(16) float2 gates_s[3][GATE_ROWS];     // (forget, input): the rows before, of now, after
+    __shared__ __align__(16) float m_s[2][GATE_ROWS + 4];      // [3]: the maximum before the first row; [4 + j]: behind row j
+    const int b = blockIdx.x, h = blockIdx.y, row = (int)threadIdx.x - 32;
+    const int r0 = a.row_offsets[b], r1 = a.row_offsets[b + 1];
+    if (r1 <= r0) return;
+    float* m_state = running_maximum(a, b, h);
+    const float bi = a.bias_i[h], bf = a.bias_f[h];
+    float m = *m_state, x = 0.0f, y = 0.0f;
+    auto fetch = [&](int t) {
+        if (t < r1) {
+            x = a.proj[(size_t)t * a.ld + a.col_i + h];
+            y = a.proj[(size_t)t * a.ld + a.col_f + h];
+        }
+    };
+    auto form = [&](int k) {
+        float ig, fg;
+        capped_gates(x, y, bi, bf, a.cap, ig, fg);
+        gates_s[k % 3][row] = make_float2(fg, ig);
+    };
+    auto finish = [&](int k) {                                 // the coefficients of block k
+        const int t = r0 + k * GATE_ROWS + row;
+        const float2 g = gates_s[k % 3][row];
+        if (t < r1) store_coef(a, t, h, g.y, g.x, m_s[k & 1][3 + row], m_s[k & 1][4 + row]);
+    };
+    const int blocks = (r1 - r0 + GATE_ROWS - 1) / GATE_ROWS;
+    if (row >= 0) {
+        fetch(r0 + row);
+        form(0);
+        fetch(r0 + GATE_ROWS + row);
+    }
+    for (int k = 0; k < blocks; ++k) {
+        __syncthreads();
+        if (row >= 0) {
+            if (k > 0) finish(k - 1);
+            if (k + 1 < blocks) form(k + 1);
+            fetch(r0 + (k + 2) * GATE_ROWS + row);
+        } else {
+            const float4* g = reinterpret_cast<const float4*>(gates_s[k % 3]);
+            float4* out = reinterpret_cast<float4*>(m_s[k & 1]);
+            if (threadIdx.x == 0) m_s[k & 1][3] = m;
+            // (rows beyond the request's end come behind the last m that is used)
+            constexpr int STEP = 8;                            // pieces of two rows read ahead of the chain
+            float4 now[STEP], next[STEP];
+#pragma unroll
+            for (int j = 0; j < STEP; ++j) now[j] = g[j];
+#pragma unroll
+            for (int q = 0; q < GATE_ROWS / 2; q += STEP) {
+#pragma unroll
+                for (int j = 0; j < STEP; ++j) next[j] = g[(q + STEP + j) % (GATE_ROWS / 2)];
+#pragma unroll
+                for (int j = 0; j < STEP; j += 2) {
+                    float4 w;
+                    w.x = fmaxf(now[j].x + m, now[j].y);
+                    w.y = fmaxf(now[j].z + w.x, now[j].w);
+                    w.z = fmaxf(now[j + 1].x + w.y, now[j + 1].y);
+                    w.w = fmaxf(now[j + 1].z + w.z, now[j + 1].w);
+                    m = w.w;
+                    if (threadIdx.x == 0) out[1 + (q + j) / 2] = w;
+                }
+#pragma unroll
+                for (int j = 0; j < STEP; ++j) now[j] = next[j];
+            }
+        }
+    }
+    __syncthreads();
+    if (row >= 0) {
+        finish(blocks - 1);
+        if (row == r1 - r0 - 1 - (blocks - 1) * GATE_ROWS) *m_state = m_s[(blocks - 1) & 1][4 + row];
+    }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -374,14 +404,8 @@ SHARPI_API int sharpi_mlstm_recurrence(const float* proj, int ld, int col_q, int
     a.state = state; a.state_stride = state_stride; a.head_stride = head_stride; a.heads = heads; a.d = d; a.dv = dv;
     a.slices = (dv + 31) / 32; a.cap = cap; a.q_scale = q_scale; a.coef = coef; a.o_raw = o_raw; a.nq = nq; a.skip = 0x7fffffff;
     if ((long long)head_stride < (long long)a.slices * d * 32 + d + 1) return SHARPI_BAD_ARGUMENT;
-    if (T > 256) {                   // many rows: the gates' tanh and logsigmoid for all rows at once, ahead of the walk
-        const long long items = (long long)T * heads;
-        gate_values_kernel<<<(unsigned)((items + 255) / 256), 256, 0, stream>>>(a, items);
-        SHARPI_CHECK_LAUNCH();
-        mlstm_gates_kernel<true><<<dim3(B, heads), 32, 0, stream>>>(a);
-    } else {
-        mlstm_gates_kernel<false><<<dim3(B, heads), 32, 0, stream>>>(a);
-    }
+    if (T - B + 1 > 32) mlstm_gates_long_kernel<<<dim3(B, heads), GATE_ROWS + 32, 0, stream>>>(a);
+    else mlstm_gates_kernel<<<dim3(B, heads), 32, 0, stream>>>(a);
     SHARPI_CHECK_LAUNCH();
     if (sums) {
         if (least < 1 || (reinterpret_cast<uintptr_t>(state) & 15) != 0 || state_stride % 4 != 0 || head_stride % 4 != 0)
