@@ -51,6 +51,7 @@ struct Args {
 // Chunk number `want` of the step: the chunks of the requests that are served, one request after the other.
 struct Place { int req, row0, rows; };
 
+template <int LEN = ROWS>                 // rows of a chunk
 __device__ __forceinline__ bool find_chunk(const int* row_offsets, int B, int least, int want, Place& p) {
     __shared__ int place_s[3];
     if (threadIdx.x < 32) {
@@ -58,7 +59,7 @@ __device__ __forceinline__ bool find_chunk(const int* row_offsets, int B, int le
         int base = 0, found = 0;
         for (int b0 = 0; b0 < B && !found; b0 += 32) {
             const int b = b0 + lane, first = b < B ? row_offsets[b] : 0, n = b < B ? row_offsets[b + 1] - first : 0;
-            const int c = n >= least ? (n + ROWS - 1) / ROWS : 0;
+            const int c = n >= least ? (n + LEN - 1) / LEN : 0;
             int upto = c;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -67,7 +68,7 @@ __device__ __forceinline__ bool find_chunk(const int* row_offsets, int B, int le
             }
             const int mine = want - (base + upto - c);
             if (mine >= 0 && mine < c) {
-                place_s[0] = b; place_s[1] = first + mine * ROWS; place_s[2] = min(ROWS, n - mine * ROWS);
+                place_s[0] = b; place_s[1] = first + mine * LEN; place_s[2] = min(LEN, n - mine * LEN);
                 found = 1;
             }
             found = __any_sync(0xffffffffu, found);
@@ -81,13 +82,14 @@ __device__ __forceinline__ bool find_chunk(const int* row_offsets, int B, int le
 }
 
 // The chunks in front of request b's, for every thread of a block
+template <int LEN = ROWS>
 __device__ __forceinline__ int chunks_before(const int* row_offsets, int b, int least) {
     __shared__ int base_s;
     if (threadIdx.x < 32) {
         int c = 0;
         for (int i = threadIdx.x; i < b; i += 32) {
             const int n = row_offsets[i + 1] - row_offsets[i];
-            c += n >= least ? (n + ROWS - 1) / ROWS : 0;
+            c += n >= least ? (n + LEN - 1) / LEN : 0;
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);

@@ -17,6 +17,7 @@
 //                        and the walk over a request's rows is sequential, so a row's result does not depend on how
 //                        the prompt was cut or batched.
 #include "common.cuh"
+#include "chunk_mma.cuh"
 
 __device__ __forceinline__ float silu_f(float z) { return z / (1.0f + expf(-z)); }
 
@@ -210,6 +211,7 @@ struct ScanArgs {
     int vec_ch, vec_bc;      // whether the channel arrays / B and C may be fetched 16 bytes at a time
     int ch;                  // rows a chunk (at most SCAN_CH; fewer when no request brings that many)
     int alone;               // a long walk: the next kernel's blocks stay off the SMs until it ends
+    int skip;                // requests of this many rows or more are not walked (the chunk kernels serve them)
 };
 
 constexpr int SCAN_CH = 16;      // rows a chunk at most
@@ -263,6 +265,7 @@ __global__ void __launch_bounds__(SPLIT ? 64 * (1 + SCAN_HELPERS) : 128) selecti
     const int c = live ? c0 + cl : a.C - 1;
     const int b = blockIdx.y;
     const int first = a.row_offsets[b], end = a.row_offsets[b + 1];
+    if (end - first >= a.skip) return;
     const int N = a.N;
     auto n_of = [&](int i) { return 2 * (sub + (i >> 1) * G) + (i & 1); };      // the state behind register i
     // one buffer: [CH] rows of dt | x | gate [CPB each], (dt, dt x) [CPB pairs], B | C [NP each]
@@ -514,18 +517,304 @@ static int launch_scan(const ScanArgs& a, int B, int T, int longest, cudaStream_
     }
 }
 
-// `longest`: the rows of the longest request, 0 where it is not known (a choice of kernels, no result depends on it).
+// -------------------------------------------------------------------------------------------------------------
+// The scan in chunks of 64 rows that work side by side, for up to 16 states:
+//   scan_sums_kernel   per chunk and channel: the step sizes (softplus), the state that the chunk's own inputs leave behind it, and the
+//                      sum of its step sizes, of which exp(A sum) is the decay over the chunk
+//   scan_carry_kernel  over the chunks of a request: the state before each chunk in the place of what it leaves
+//   scan_outs_kernel   per chunk and channel: the rows from the state before the chunk, as the walk forms them
+// A lane is a channel with all its states, two of them an instruction (f32x2); nothing is exchanged between lanes, a row's B and C are
+// read by all lanes of a warp at once, and a lane's own numbers of the next rows are on their way into shared memory, where it alone
+// reads them.  The exponentials are formed twice, and still the walk, whose rows follow one another, is the slower form for one long
+// prompt (us, walked / in chunks, 16 states: 2048 rows of 4096 channels 155 / 111, of 2048 channels 121 / 70; 400 rows of 4096
+// channels 35 / 41).  Bound by the special-function unit (two thirds busy: 36 operations a row and channel) and the last wave;
+// an eighth to a half of the exponentials as polynomials on the multiply-add pipe instead were slower (115 to 135 us).
+// -------------------------------------------------------------------------------------------------------------
+constexpr int SC_THREADS = 128, SC_ROWS = 64, SC_AHEAD = 8;
+
+struct ScanChunks {
+    ScanArgs s;
+    int B, least;
+    float* dt;               // [T, C]: the step sizes
+    float* sums;             // [chunks][C][N]
+    float* total;            // [chunks][C]
+};
+
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair2(float lo, float hi) { return (f32x2)__float_as_uint(lo) | ((f32x2)__float_as_uint(hi) << 32); }
+__device__ __forceinline__ float low2(f32x2 v) { return __uint_as_float((unsigned)v); }
+__device__ __forceinline__ float high2(f32x2 v) { return __uint_as_float((unsigned)(v >> 32)); }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f32x2 ex2_pair(f32x2 v) { return pair2(ex2_approx(low2(v)), ex2_approx(high2(v))); }
+
+// A thread's own numbers of the rows ahead, in shared memory: V floats a row, SC_AHEAD rows a group, two groups on their way
+template <int V>
+struct ScanRing {
+    static constexpr int GROUP = SC_AHEAD * V * SC_THREADS;
+    float* mine;                                           // [2][SC_AHEAD][V] of this thread, SC_THREADS floats apart
+    __device__ __forceinline__ float at(int group, int j, int v) const { return mine[group * GROUP + (j * V + v) * SC_THREADS]; }
+    // rows r0 .. of a chunk of `rows`: source[v] + row * ld[v]
+    __device__ __forceinline__ void fetch(int group, int r0, int rows, const float* const (&source)[V], const unsigned (&ld)[V]) const {
+        unsigned off[V];
+#pragma unroll
+        for (int v = 0; v < V; ++v) off[v] = r0 * ld[v];
+#pragma unroll
+        for (int j = 0; j < SC_AHEAD; ++j)
+            if (r0 + j < rows)
+#pragma unroll
+                for (int v = 0; v < V; ++v) {
+                    cp_async4(mine + group * GROUP + (j * V + v) * SC_THREADS, source[v] + off[v]);
+                    off[v] += ld[v];
+                }
+        cp_async_commit();
+    }
+};
+
+// softplus(v) = max(v, 0) + log(1 + w), w = exp(-|v|) in [0, 1]; log(1 + w) / w as the polynomial through its Chebyshev points of
+// degree 9 (5e-9 of the value; one unit in the last place with the roundings).  Two at a time.
+__device__ __forceinline__ f32x2 softplus2(float v0, float v1) {
+    constexpr float P[10] = {1.0f, -0.49999892711639404f, 0.33329710364341736f, -0.24951615929603577f, 0.1966327428817749f,
+                             -0.1526966691017151f, 0.10543623566627502f, -0.05637361481785774f, 0.019542528316378593f, -0.0031760570127516985f};
+    const f32x2 w = pair2(ex2_approx(fabsf(v0) * -1.4426950408889634f), ex2_approx(fabsf(v1) * -1.4426950408889634f));
+    f32x2 p = pair2(P[9], P[9]);
+#pragma unroll
+    for (int i = 8; i >= 0; --i) p = fma2(p, w, pair2(P[i], P[i]));
+    return fma2(p, w, pair2(fmaxf(v0, 0.0f), fmaxf(v1, 0.0f)));
+}
+
+// Columns col .. col + N - 1 of the chunk's rows of B or C, zeros behind N
+template <int NP>
+__device__ __forceinline__ void scan_stage(const ScanArgs& a, const chunked::Place& p, int col, float* dst) {
+    for (int i = threadIdx.x; i < p.rows * NP; i += SC_THREADS) {
+        const int r = i / NP, n = i % NP;
+        dst[i] = n < a.N ? a.bc[(size_t)(p.row0 + r) * a.ld_bc + col + n] : 0.0f;
+    }
+}
+
+// A log2(e) of a channel's states (0 behind N: what is there stays zero)
+template <int NP>
+__device__ __forceinline__ void scan_rates(const ScanArgs& a, int c, f32x2 (&A)[NP / 2]) {
+#pragma unroll
+    for (int i = 0; i < NP / 2; ++i) {
+        float v[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) v[e] = 2 * i + e < a.N ? -expf(a.a_log[(size_t)c * a.N + 2 * i + e]) * 1.4426950408889634f : 0.0f;
+        A[i] = pair2(v[0], v[1]);
+    }
+}
+
+template <int NP, bool RAW>
+__global__ void __launch_bounds__(SC_THREADS, 5) scan_sums_kernel(ScanChunks q) {
+    __shared__ __align__(16) float B_s[SC_ROWS * NP];
+    __shared__ float ring_s[2 * SC_AHEAD * 2 * SC_THREADS];
+    const ScanArgs& a = q.s;
+    chunked::Place p;
+    if (!chunked::find_chunk<SC_ROWS>(a.row_offsets, q.B, q.least, blockIdx.y, p)) return;
+    scan_stage<NP>(a, p, a.col_b, B_s);
+    __syncthreads();
+    const int c = blockIdx.x * SC_THREADS + threadIdx.x;
+    if (c >= a.C) return;
+    f32x2 A[NP / 2], S[NP / 2];
+    scan_rates<NP>(a, c, A);
+#pragma unroll
+    for (int i = 0; i < NP / 2; ++i) S[i] = 0;
+    const float bias = RAW ? a.dt_bias[c] : 0.0f;
+    const size_t at0 = (size_t)p.row0 * a.C + c;
+    const ScanRing<2> ring{ring_s + threadIdx.x};
+    const float* const source[2] = {a.dtraw + at0, a.x + at0};
+    const unsigned ld[2] = {(unsigned)a.C, (unsigned)a.C};
+    ring.fetch(0, 0, p.rows, source, ld);
+    ring.fetch(1, SC_AHEAD, p.rows, source, ld);
+    float* dt = q.dt + at0;
+    float sum = 0.0f;
+    auto walk = [&](int g, int r0, int n) {
+        float d[SC_AHEAD], dx[SC_AHEAD];
+#pragma unroll
+        for (int j = 0; j < SC_AHEAD; j += 2) {
+            f32x2 v = pair2(ring.at(g, j, 0), ring.at(g, j + 1, 0));
+            if (RAW) v = softplus2(low2(v) + bias, high2(v) + bias);
+            d[j] = low2(v); d[j + 1] = high2(v);
+            dx[j] = d[j] * ring.at(g, j, 1); dx[j + 1] = d[j + 1] * ring.at(g, j + 1, 1);
+        }
+#pragma unroll
+        for (int j = 0; j < SC_AHEAD; ++j) {
+            if (j >= n) break;
+            dt[(unsigned)(r0 + j) * (unsigned)a.C] = d[j];
+            sum += d[j];
+            const f32x2 dd = pair2(d[j], d[j]), ee = pair2(dx[j], dx[j]);
+            const ulonglong2* B = reinterpret_cast<const ulonglong2*>(B_s + (r0 + j) * NP);
+#pragma unroll
+            for (int i = 0; i < NP / 4; ++i) {
+                const ulonglong2 b = B[i];
+                S[2 * i] = fma2(ex2_pair(mul2(dd, A[2 * i])), S[2 * i], mul2(ee, b.x));
+                S[2 * i + 1] = fma2(ex2_pair(mul2(dd, A[2 * i + 1])), S[2 * i + 1], mul2(ee, b.y));
+            }
+        }
+    };
+    int r0 = 0, g = 0;
+    for (; r0 + SC_AHEAD <= p.rows; r0 += SC_AHEAD, g ^= 1) {
+        cp_async_wait<1>();
+        walk(g, r0, SC_AHEAD);
+        ring.fetch(g, r0 + 2 * SC_AHEAD, p.rows, source, ld);
+    }
+    cp_async_wait<0>();
+    if (r0 < p.rows) walk(g, r0, p.rows - r0);
+    float* out = q.sums + ((size_t)blockIdx.y * a.C + c) * a.N;
+#pragma unroll
+    for (int i = 0; i < NP / 2; ++i) {
+        if (2 * i < a.N) out[2 * i] = low2(S[i]);
+        if (2 * i + 1 < a.N) out[2 * i + 1] = high2(S[i]);
+    }
+    q.total[(size_t)blockIdx.y * a.C + c] = sum;
+}
+
+__global__ void __launch_bounds__(256) scan_carry_kernel(ScanChunks q) {
+    const ScanArgs& a = q.s;
+    const int b = blockIdx.y, rows = a.row_offsets[b + 1] - a.row_offsets[b];
+    if (rows < q.least) return;
+    const int base = chunked::chunks_before<SC_ROWS>(a.row_offsets, b, q.least), n = (rows + SC_ROWS - 1) / SC_ROWS;
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x, size = (long long)a.C * a.N;
+    if (i >= size) return;
+    const int c = (int)(i / a.N);
+    const float A = -expf(a.a_log[i]) * 1.4426950408889634f;
+    float* state = a.state + (size_t)a.state_slots[b] * a.state_stride + i;
+    float* u = q.sums + base * size + i;
+    const float* total = q.total + (size_t)base * a.C + c;
+    float S = *state, own[SC_AHEAD], dt[SC_AHEAD];
+    auto fetch = [&](int k) {
+#pragma unroll
+        for (int j = 0; j < SC_AHEAD; ++j)
+            if (k + j < n) { own[j] = u[(k + j) * size]; dt[j] = total[(size_t)(k + j) * a.C]; }
+    };
+    fetch(0);
+    for (int k = 0; k < n; k += SC_AHEAD) {
+        float o[SC_AHEAD], e[SC_AHEAD];
+#pragma unroll
+        for (int j = 0; j < SC_AHEAD; ++j) { o[j] = own[j]; e[j] = ex2_approx(dt[j] * A); }
+        fetch(k + SC_AHEAD);
+#pragma unroll
+        for (int j = 0; j < SC_AHEAD; ++j) {
+            if (k + j >= n) break;
+            u[(k + j) * size] = S;
+            S = fmaf(e[j], S, o[j]);
+        }
+    }
+    *state = S;
+}
+
+template <typename TO, int NP, bool RAW>
+__global__ void __launch_bounds__(SC_THREADS, 5) scan_outs_kernel(ScanChunks q) {
+    __shared__ __align__(16) float B_s[SC_ROWS * NP], C_s[SC_ROWS * NP];
+    __shared__ float ring_s[2 * SC_AHEAD * 3 * SC_THREADS];
+    const ScanArgs& a = q.s;
+    chunked::Place p;
+    if (!chunked::find_chunk<SC_ROWS>(a.row_offsets, q.B, q.least, blockIdx.y, p)) return;
+    scan_stage<NP>(a, p, a.col_b, B_s);
+    scan_stage<NP>(a, p, a.col_c, C_s);
+    __syncthreads();
+    const int c = blockIdx.x * SC_THREADS + threadIdx.x;
+    if (c >= a.C) return;
+    f32x2 A[NP / 2], S[NP / 2];
+    scan_rates<NP>(a, c, A);
+    const float* before = q.sums + ((size_t)blockIdx.y * a.C + c) * a.N;
+#pragma unroll
+    for (int i = 0; i < NP / 2; ++i) S[i] = pair2(2 * i < a.N ? before[2 * i] : 0.0f, 2 * i + 1 < a.N ? before[2 * i + 1] : 0.0f);
+    const float dsk = a.dskip[c];
+    const size_t at0 = (size_t)p.row0 * a.C + c;
+    const ScanRing<3> ring{ring_s + threadIdx.x};
+    const float* const source[3] = {q.dt + at0, a.x + at0, a.z + (size_t)p.row0 * a.ld_z + c};
+    const unsigned ld[3] = {(unsigned)a.C, (unsigned)a.C, (unsigned)a.ld_z};
+    ring.fetch(0, 0, p.rows, source, ld);
+    ring.fetch(1, SC_AHEAD, p.rows, source, ld);
+    TO* out = reinterpret_cast<TO*>(a.out) + at0;
+    auto walk = [&](int g, int r0, int n) {
+#pragma unroll
+        for (int j = 0; j < SC_AHEAD; ++j) {
+            if (j >= n) break;
+            const float d = ring.at(g, j, 0), x = ring.at(g, j, 1), z = ring.at(g, j, 2), dx = d * x;
+            const f32x2 dd = pair2(d, d), ee = pair2(dx, dx);
+            const ulonglong2* B = reinterpret_cast<const ulonglong2*>(B_s + (r0 + j) * NP);
+            const ulonglong2* Cn = reinterpret_cast<const ulonglong2*>(C_s + (r0 + j) * NP);
+            f32x2 y0 = 0, y1 = 0;
+#pragma unroll
+            for (int i = 0; i < NP / 4; ++i) {
+                const ulonglong2 b = B[i], cn = Cn[i];
+                S[2 * i] = fma2(ex2_pair(mul2(dd, A[2 * i])), S[2 * i], mul2(ee, b.x));
+                S[2 * i + 1] = fma2(ex2_pair(mul2(dd, A[2 * i + 1])), S[2 * i + 1], mul2(ee, b.y));
+                y0 = fma2(S[2 * i], cn.x, y0);
+                y1 = fma2(S[2 * i + 1], cn.y, y1);
+            }
+            const float y = (low2(y0) + low2(y1)) + (high2(y0) + high2(y1));
+            out[(unsigned)(r0 + j) * (unsigned)a.C] = from_float<TO>(fmaf(dsk, x, y) * (RAW ? silu_f(z) : z));
+        }
+    };
+    int r0 = 0, g = 0;
+    for (; r0 + SC_AHEAD <= p.rows; r0 += SC_AHEAD, g ^= 1) {
+        cp_async_wait<1>();
+        walk(g, r0, SC_AHEAD);
+        ring.fetch(g, r0 + 2 * SC_AHEAD, p.rows, source, ld);
+    }
+    cp_async_wait<0>();
+    if (r0 < p.rows) walk(g, r0, p.rows - r0);
+}
+
+template <typename TO, int NP, bool RAW>
+static int launch_scan_chunks(const ScanChunks& q, int chunks, cudaStream_t stream) {
+    const dim3 grid((q.s.C + SC_THREADS - 1) / SC_THREADS, chunks);
+    scan_sums_kernel<NP, RAW><<<grid, SC_THREADS, 0, stream>>>(q);
+    SHARPI_CHECK_LAUNCH();
+    scan_carry_kernel<<<dim3((unsigned)(((long long)q.s.C * q.s.N + 255) / 256), q.B), 256, 0, stream>>>(q);
+    SHARPI_CHECK_LAUNCH();
+    scan_outs_kernel<TO, NP, RAW><<<grid, SC_THREADS, 0, stream>>>(q);
+    SHARPI_CHECK_LAUNCH();
+    return SHARPI_OK;
+}
+
+template <typename TO, int NP>
+static int launch_scan_chunks(const ScanChunks& q, int chunks, cudaStream_t stream) {
+    return q.s.dt_bias ? launch_scan_chunks<TO, NP, true>(q, chunks, stream) : launch_scan_chunks<TO, NP, false>(q, chunks, stream);
+}
+
+template <typename TO>
+static int launch_scan_chunks(const ScanChunks& q, int chunks, cudaStream_t stream) {
+    return q.s.N <= 4 ? launch_scan_chunks<TO, 4>(q, chunks, stream)
+                      : q.s.N <= 8 ? launch_scan_chunks<TO, 8>(q, chunks, stream) : launch_scan_chunks<TO, 16>(q, chunks, stream);
+}
+
+// `longest`: the rows of the longest request, 0 where it is not known (a choice of kernels, no result depends on it).  `work`
+// (nullable; T * C + `chunks` * C * (N + 1) floats): requests of at least `least` rows run in chunks, `chunks` of them at most; the
+// others, and without it all, are walked (`walk` = 0: there are no others).
 SHARPI_API int sharpi_selective_scan(const float* x, const float* dtraw, const float* dt_bias, const float* bc,
                                      int ld_bc, int col_b, int col_c, const float* a_log, const float* dskip,
                                      const float* z, int ld_z, const int* row_offsets, const int* state_slots,
                                      float* state, long long state_stride, void* out, int out_dtype, int T, int B,
-                                     int C, int N, int longest, cudaStream_t stream) {
+                                     int C, int N, int longest, float* work, int chunks, int least, int walk, cudaStream_t stream) {
     if (B <= 0) return SHARPI_OK;
     if (C <= 0 || N <= 0 || N > 256) return SHARPI_BAD_ARGUMENT;
     ScanArgs a;
     a.x = x; a.dtraw = dtraw; a.dt_bias = dt_bias; a.bc = bc; a.ld_bc = ld_bc; a.col_b = col_b; a.col_c = col_c;
     a.a_log = a_log; a.dskip = dskip; a.z = z; a.ld_z = ld_z; a.row_offsets = row_offsets; a.state_slots = state_slots;
-    a.state = state; a.state_stride = state_stride; a.out = out; a.C = C; a.N = N;
+    a.state = state; a.state_stride = state_stride; a.out = out; a.C = C; a.N = N; a.skip = 0x7fffffff;
+    if (work) {
+        if (N > 16 || chunks < 1 || chunks > 65535 || B > 65535 || least < 1) return SHARPI_BAD_ARGUMENT;
+        ScanChunks q;
+        q.s = a; q.B = B; q.least = least; q.dt = work; q.sums = work + (size_t)T * C; q.total = q.sums + (size_t)chunks * C * N;
+        int rc = SHARPI_BAD_ARGUMENT;
+        if (out_dtype == SHARPI_F32) rc = launch_scan_chunks<float>(q, chunks, stream);
+        if (out_dtype == SHARPI_BF16) rc = launch_scan_chunks<bf16>(q, chunks, stream);
+        if (rc != SHARPI_OK || !walk) return rc;
+        a.skip = least;
+        if (longest >= least) longest = least - 1;
+    }
     if (out_dtype == SHARPI_F32) return launch_scan<float>(a, B, T, longest, stream);
     if (out_dtype == SHARPI_BF16) return launch_scan<bf16>(a, B, T, longest, stream);
     return SHARPI_BAD_ARGUMENT;

@@ -888,7 +888,9 @@ CHUNKED_LEAST = 128
 #   wkv   32 heads of 64        33 / 27, 63 / 28, 390 / 120;  40 / 70, 77 / 138, 134 / 135
 #         16 heads of 64        33 / 27, 61 / 27, 367 / 62;   36 / 39, 68 / 68, 124 / 67
 #         64 heads of 64        35 / 28, 64 / 31, 488 / 209;  80 / 144, 163 / 257, 160 / 252
-_WALK_OR_CHUNKS = {"mlstm": (0.16, 30, 0.0), "ssd": (0.32, 30, 0.0), "wkv": (0.21, 15, 0.8)}
+#   scan  4096 channels of 16   250 rows 24 / 30, 400 35 / 41, 2048 155 / 111; 2048 channels 19 / 29, -, 121 / 70; 1117, 558 and 372 rows of
+#         4096 in a step 120 / 120, 576, 288, 192 and 144 rows 73 / 107: the walk takes several requests side by side
+_WALK_OR_CHUNKS = {"mlstm": (0.16, 30, 0.0), "ssd": (0.32, 30, 0.0), "wkv": (0.21, 15, 0.8), "scan": (0.028, 20, 0.0)}
 
 
 def chunked_least(kind: str, heads: int) -> int:
@@ -897,14 +899,15 @@ def chunked_least(kind: str, heads: int) -> int:
     return max(CHUNKED_LEAST, math.ceil((s + c * heads) / w))
 
 
-def _chunks(kind: str, T: int, B: int, max_rows: Optional[int], heads: int, d: int, dv: int, *aligned: int) -> int:
+def _chunks(kind: str, T: int, B: int, max_rows: Optional[int], heads: int, d: int, dv: int, *aligned: int, size: int = 64) -> int:
     """How many chunks the requests of a step that run in chunks can have together (each ends in one that may be short);
     0: none has the rows, or the sizes are not the chunk kernels'.  ``max_rows``: rows of the longest request (None or 0: at
-    most ``T - B + 1``); ``aligned``: column numbers, strides and addresses in floats, which the chunk kernels want on 16 bytes."""
+    most ``T - B + 1``); ``size``: rows of a chunk; ``aligned``: column numbers, strides and addresses in floats, which the chunk kernels want on
+    16 bytes."""
     least = chunked_least(kind, heads)
     if (max_rows or T - B + 1) < least or d > 128 or d % 4 or dv % 4 or any(x % 4 for x in aligned):
         return 0
-    chunks = (T + 63) // 64 if B == 1 else T // 64 + min(B, T // least)
+    chunks = (T + size - 1) // size if B == 1 else T // size + min(B, T // least)
     # what the chunk kernels' grids and offsets hold (the walks take more)
     return chunks if max(chunks, B, heads) <= 65535 and d * dv <= 1 << 24 else 0
 
@@ -1207,6 +1210,8 @@ def wkv_out(o: torch.Tensor, gate: torch.Tensor, weight: torch.Tensor, eps: floa
 # ---------------------------------------------------------------------------------------
 # Selective scan and its convolution (mamba.cu)
 SCAN_MAX_STATES = 256
+SCAN_CHUNK = 64              # rows of its chunks
+SCAN_CHUNK_STATES = 16       # states a channel up to which long portions are scanned in chunks
 
 
 def causal_conv(xz: torch.Tensor, channels: int, weight: torch.Tensor, bias: Optional[torch.Tensor],
@@ -1249,12 +1254,14 @@ def selective_scan(x: torch.Tensor, dt: torch.Tensor, bc: torch.Tensor, col_b: i
                    col_c: int, a_log: torch.Tensor, dskip: torch.Tensor, xz: torch.Tensor, col_z: int, *,
                    row_offsets: torch.Tensor, state_slots: torch.Tensor, state: torch.Tensor,
                    out_dtype: torch.dtype, dt_bias: Optional[torch.Tensor] = None,
-                   max_rows: Optional[int] = None) -> torch.Tensor:
+                   max_rows: Optional[int] = None, split: bool = False) -> torch.Tensor:
     """The selective scan over the rows of every request from and into ``state [slots, channels * states]``:
     ``(S C + D x) * g`` in ``out_dtype``, with ``dt`` the step sizes themselves (after their softplus) and ``g`` the
     gate (already ``silu(z)``) in the columns of ``xz`` from ``col_z``, for programs that have them so.  With ``dt_bias
     [channels]``, as in the mixer, both come raw: the step sizes are ``softplus(dt + dt_bias)`` and the gate ``silu`` of
-    those columns.  ``max_rows``: the rows of the longest request, if known (a choice of kernels, no result depends on it)."""
+    those columns.  ``max_rows``: the rows of the longest request, if known (a choice of kernels, no result depends on it).
+    ``split``: requests of many rows may run in chunks that work side by side, from a number of rows on that the sizes fix (the
+    sums are then rounded in another order than the walk's)."""
     if dt_bias is not None:
         _need(dt_bias, "dt_bias", torch.float32)
         if dt_bias.numel() != x.shape[1]:
@@ -1270,11 +1277,15 @@ def selective_scan(x: torch.Tensor, dt: torch.Tensor, bc: torch.Tensor, col_b: i
         raise KernelError("the gate's columns lie outside the fused projection")
     out = torch.empty((T, C), dtype=out_dtype, device=x.device)
     z = xz[:, col_z:]
+    B = state_slots.numel()
+    chunks = _chunks("scan", T, B, max_rows, C, 4, 4, size=SCAN_CHUNK) if split and N <= SCAN_CHUNK_STATES and max(C, xz.shape[1]) < 1 << 24 and T - B + 1 >= CHUNKED_LEAST else 0
+    work = torch.empty(T * C + chunks * C * (N + 1), dtype=torch.float32, device=x.device) if chunks else None
     check(kernel("sharpi_selective_scan")(x.data_ptr(), dt.data_ptr(), _ptr(dt_bias), bc.data_ptr(),
                                           bc.shape[1], col_b, col_c, a_log.data_ptr(), dskip.data_ptr(), z.data_ptr(),
                                           xz.shape[1], row_offsets.data_ptr(), state_slots.data_ptr(), state.data_ptr(),
-                                          state.stride(0), out.data_ptr(), dtype_code(out_dtype), T, state_slots.numel(),
-                                          C, N, int(max_rows or 0), _stream()), "sharpi_selective_scan")
+                                          state.stride(0), out.data_ptr(), dtype_code(out_dtype), T, B, C, N, int(max_rows or 0),
+                                          _ptr(work), chunks, *(_chunk_border("scan", T, B, max_rows, C) if chunks else (0, 1)),
+                                          _stream()), "sharpi_selective_scan")
     return out
 
 

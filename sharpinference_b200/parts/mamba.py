@@ -72,7 +72,7 @@ class SelectiveScanMixer(Mixer):
         y = ops.selective_scan(x32, dt, dbc, self.dt_rank, self.dt_rank + self.states, self.a_log,
                                self.d_skip, xz, self.inner, row_offsets=ctx.row_offsets, state_slots=ctx.state_slots,
                                state=slot.states["S"], out_dtype=self.act_dtype, dt_bias=self.dt_bias,
-                               max_rows=ctx.max_rows_per_request)
+                               max_rows=ctx.max_rows_per_request, split=self.act_dtype == torch.bfloat16)
         return self.out(y)
 
 
