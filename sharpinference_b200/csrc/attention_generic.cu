@@ -151,8 +151,13 @@ __global__ void paged_attention_generic_kernel(PagedAttnArgs a) {
 // of the group sees are not loaded (zeros in their place), and in tiles that some of its rows see and others do not a
 // hidden value is left out of the sum (zero times a NaN would be NaN); a hidden probability is minus zero there, which no
 // exponential is.  Bound by the multiply-adds and the barriers between a tile's parts.
+//   SPLIT: where the CTAs are few, a cluster of `ctas` of them shares the key tiles, tile it in CTA it % ctas.  What follows from tile to
+// tile (the running maximum, the factors, the sums) is then a chain over numbers that the CTAs leave in shared memory: every CTA's
+// maxima first, then, with them, its probabilities and sums, which all CTAs add up in the tiles' order, each for its share of the
+// elements.  The operations and their order are those of one CTA.  4 decode rows at 300 keys: 47 us with a CTA a row and key
+// head, 15.5 us so; at 4000 keys 555 and 103 us.
 // 980 rows of 4 requests, 8 heads on 2, head size 128: 556 -> 95 us (before: a block a row and head, one key a thread read
-// element by element); 4 decode rows at 300 keys: 69 -> 48 us.
+// element by element); 
 constexpr int AR_BK = 64, AR_THREADS = 128, AR_MAX_D = 256;
 
 typedef unsigned long long f32x2;
@@ -171,8 +176,31 @@ constexpr unsigned AR_HIDDEN = 0x7fa51dedu;
 // Floats a row takes in shared memory: an odd number of 16-byte pieces, so that neighbouring rows start in other banks.
 __host__ __device__ __forceinline__ int ar_ld(int d) { return (d / 4) % 2 ? d + 8 : d + 4; }
 
-template <int R, int JJ>
+// All threads of the cluster: what one wrote into its shared memory before, the others may read behind it.
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The same place in the shared memory of CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t in_cta(const void* p, int rank) {
+    uint32_t at;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(mma16::smem_addr(p)), "r"(rank));
+    return at;
+}
+__device__ __forceinline__ float load_cluster(uint32_t at) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
+    return v;
+}
+__device__ __forceinline__ float4 load_cluster4(uint32_t at) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
+    return v;
+}
+
+template <int R, int JJ, bool SPLIT>
 __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAttnArgs a, int heads_cta, int tokens) {
+    static_assert(!SPLIT || R == 8, "a thread has four neighbouring elements of the cluster's sums at most");
+    const int ctas = SPLIT ? (int)gridDim.z : 1, rank = SPLIT ? (int)blockIdx.z : 0;
     extern __shared__ __align__(16) float ar_smem[];
     __shared__ long long off_s[2][AR_BK];                // where the keys of two tiles lie, -1: not there
     constexpr int RT = R / 8;                            // rows a thread
@@ -182,6 +210,9 @@ __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAtt
     float* v_s = k_s + AR_BK * ld;                       // [64][ld] (keys-only pages: none)
     float* p_s = v_s + (a.kv_planes == 2 ? AR_BK * ld : 0);   // [R][68]: scores, then probabilities
     float* corr_s = p_s + R * (AR_BK + 4);               // [R]
+    float* top_s = corr_s + R;                           // SPLIT: [R] a tile's maxima, [R] its probabilities' sums, [R][d] its weighted values
+    float* l_s = top_s + R;
+    float* sum_s = l_s + R;
 
     const int t = blockIdx.x, pos0 = a.positions[t], req = a.row_req[t];
     if (t > 0 && pos0 % tokens != 0 && a.row_req[t - 1] == req && a.positions[t - 1] == pos0 - 1) return;
@@ -211,16 +242,16 @@ __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAtt
         const int page = key <= p_last && (key >= lo_first || key < keep) ? table[key / a.page_size] : -1;
         return page >= 0 ? (long long)page * a.kv_planes * plane + ((long long)kvh * a.page_size + key % a.page_size) * d : -1;
     };
-    auto load = [&](float* dst, int it, size_t second) {  // a warp copies every fourth row
+    auto load = [&](float* dst, int at, size_t second) {  // a warp copies every fourth row of the tile whose places are off_s[at]
 #pragma unroll 4
         for (int r = warp; r < AR_BK; r += AR_THREADS / 32) {
-            const long long off = off_s[it & 1][r];
+            const long long off = off_s[at][r];
             const float* src = kv + (off >= 0 ? off + second : 0);
             for (int c = lane; c < vec; c += 32) mma16::cp_async_16(dst + r * ld + c * 4, src + (off >= 0 ? c * 4 : 0), off >= 0 ? 16 : 0);
         }
         mma16::cp_async_commit();
     };
-    if (tid < AR_BK) off_s[0][tid] = place(0);
+    if (tid < AR_BK) off_s[0][tid] = rank < n_iter ? place(rank) : -1;
     __syncthreads();
     load(k_s, 0, 0);
     if (a.kv_planes == 2) load(v_s, 0, plane);
@@ -237,10 +268,15 @@ __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAtt
 #pragma unroll
         for (int j = 0; j < JJ; ++j) acc[i][j][0] = acc[i][j][1] = 0;
     float m_run = -INFINITY, l_run = 0.0f;               // of row tid / 4 (four threads a row)
+    // SPLIT: this thread's four elements of the cluster's sums
+    const int unit = rank + ctas * tid, unit_r = unit / vec, unit_c = unit % vec * 4;
+    float4 joint = make_float4(0.f, 0.f, 0.f, 0.f);
 
-    for (int it = 0; it < n_iter; ++it) {
-        const int key0 = key0_of(it);
-        const long long next = tid < AR_BK && it + 1 < n_iter ? place(it + 1) : -1;      // arrives while the scores are formed
+    for (int it0 = 0, at = 0; it0 < n_iter; it0 += ctas, at ^= 1) {
+        const int it = it0 + rank;
+        const bool have = !SPLIT || it < n_iter, more = it0 + ctas < n_iter;      // (a CTA without a tile in the last round goes along)
+        const int key0 = key0_of(have ? it : 0);
+        const long long next = tid < AR_BK && it + ctas < n_iter ? place(it + ctas) : -1;      // arrives while the scores are formed
         if (a.kv_planes == 2) mma16::cp_async_wait<1>(); else mma16::cp_async_wait<0>();
         __syncthreads();                                 // the keys are here (and the queries); p_s is free
         {
@@ -274,7 +310,7 @@ __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAtt
                 for (int j = 0; j < 4; ++j) {
                     const int key = key0 + tx + 16 * j;
                     float v = __uint_as_float(AR_HIDDEN);
-                    if (key <= pos && (key >= lo || key < keep) && off_s[it & 1][tx + 16 * j] >= 0) {
+                    if (key <= pos && (key >= lo || key < keep) && off_s[at][tx + 16 * j] >= 0) {
                         v = __fmul_rn(__fadd_rn(lo2(s[i][j]), hi2(s[i][j])), a.scale);
                         if (a.softcap > 0.0f) v = a.softcap * tanhf(v / a.softcap);
                         if (a.dist_bias) v += a.dist_bias[(size_t)min(pos - key, a.dist_far) * a.nq + h];
@@ -283,10 +319,46 @@ __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAtt
                 }
             }
         }
-        if (tid < AR_BK) off_s[(it + 1) & 1][tid] = next;
+        if (tid < AR_BK) off_s[at ^ 1][tid] = next;
         __syncthreads();                                 // the scores are here; keys are free
-        if (a.kv_planes == 2 && it + 1 < n_iter) load(k_s, it + 1, 0);
-        if (tid < 4 * R) {
+        if (a.kv_planes == 2 && more) load(k_s, at ^ 1, 0);
+        if constexpr (SPLIT) {
+            float* p = p_s + (tid >> 2) * (AR_BK + 4) + (tid & 3) * 4;
+            if (tid < 4 * R) {
+                float m = -INFINITY;
+#pragma unroll
+                for (int i = 0; i < AR_BK; i += 16)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) m = fmaxf(m, p[i + c]);
+                m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+                m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+                if ((tid & 3) == 0) top_s[tid >> 2] = have ? m : -INFINITY;
+            }
+            cluster_sync();
+            if (tid < 4 * R) {
+                float before = m_run, m = m_run, all = m_run, l = 0.0f;
+                for (int q = 0; q < ctas; ++q) {
+                    const float top = load_cluster(in_cta(top_s + (tid >> 2), q));
+                    all = fmaxf(all, top);
+                    if (q < rank) before = all;
+                    if (q <= rank) m = all;
+                }
+                const float corr = before == -INFINITY ? 0.0f : expf(before - m);
+                const float base = m == -INFINITY ? 0.0f : m;
+                m_run = all;
+#pragma unroll
+                for (int i = 0; i < AR_BK; i += 16)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const float v = p[i + c], e = __float_as_uint(v) == AR_HIDDEN ? -0.0f : expf(v - base);
+                        p[i + c] = e;
+                        l = __fadd_rn(l, e);
+                    }
+                l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 1));
+                l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 2));
+                if ((tid & 3) == 0) { corr_s[tid >> 2] = corr; l_s[tid >> 2] = l; }
+            }
+        } else if (tid < 4 * R) {
             float* p = p_s + (tid >> 2) * (AR_BK + 4) + (tid & 3) * 4;
             float m = -INFINITY, l = 0.0f;
 #pragma unroll
@@ -312,7 +384,7 @@ __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAtt
             if ((tid & 3) == 0) corr_s[tid >> 2] = corr;
         }
         if (a.kv_planes == 2) {
-            if (it + 1 < n_iter) mma16::cp_async_wait<1>(); else mma16::cp_async_wait<0>();
+            if (more) mma16::cp_async_wait<1>(); else mma16::cp_async_wait<0>();
         }
         __syncthreads();                                 // values, probabilities and corrections are here
         {
@@ -354,6 +426,24 @@ __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAtt
             if constexpr (R == 8) weigh(mixed);
             else if (mixed) weigh(std::true_type{});
             else weigh(std::false_type{});
+            if constexpr (SPLIT) {
+#pragma unroll
+                for (int j = 0; j < JJ; ++j)
+                    if (tx * 4 + 64 * j < d)
+                        *reinterpret_cast<float4*>(sum_s + ty * d + tx * 4 + 64 * j) =
+                            make_float4(lo2(sum[0][j][0]), hi2(sum[0][j][0]), lo2(sum[0][j][1]), hi2(sum[0][j][1]));
+                cluster_sync();
+                const int tiles = min(ctas, n_iter - it0);
+                for (int q = 0; q < tiles; ++q) {
+                    if (unit_r < R) {
+                        const float corr = load_cluster(in_cta(corr_s + unit_r, q));
+                        const float4 v = load_cluster4(in_cta(sum_s + unit_r * d + unit_c, q));
+                        joint = make_float4(__fmaf_rn(joint.x, corr, v.x), __fmaf_rn(joint.y, corr, v.y),
+                                            __fmaf_rn(joint.z, corr, v.z), __fmaf_rn(joint.w, corr, v.w));
+                    }
+                    if (tid < 4 * R) l_run = __fmaf_rn(l_run, load_cluster(in_cta(corr_s + (tid >> 2), q)), load_cluster(in_cta(l_s + (tid >> 2), q)));
+                }
+            } else
 #pragma unroll
             for (int i = 0; i < RT; ++i) {
                 const float corr = corr_s[ty + i * 8];
@@ -365,12 +455,13 @@ __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAtt
                                              __fmaf_rn(hi2(acc[i][j][c]), corr, hi2(sum[i][j][c])));
             }
         }
-        if (it + 1 < n_iter) {
+        if (more) {
             __syncthreads();                             // the values are free
-            if (a.kv_planes == 2) load(v_s, it + 1, plane); else load(k_s, it + 1, 0);
+            if (a.kv_planes == 2) load(v_s, at ^ 1, plane); else load(k_s, at ^ 1, 0);
         }
     }
-    __syncthreads();
+    if constexpr (SPLIT) cluster_sync();                 // nobody reads this CTA's shared memory any more
+    else __syncthreads();
     if (tid < 4 * R && (tid & 3) == 0) {
         float shrink = 1.0f;
         const int r = tid >> 2, h = head0 + (r < n_rows ? r % heads_here : 0);
@@ -386,6 +477,14 @@ __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAtt
         corr_s[r] = shrink / l_run;
     }
     __syncthreads();
+    if constexpr (SPLIT) {
+        if (unit_r < n_rows) {
+            const float f = corr_s[unit_r];
+            float* out = (float*)a.out + ((size_t)(t + unit_r / heads_here) * a.nq + head0 + unit_r % heads_here) * d;
+            *reinterpret_cast<float4*>(out + unit_c) = make_float4(joint.x * f, joint.y * f, joint.z * f, joint.w * f);
+        }
+        return;
+    }
 #pragma unroll
     for (int i = 0; i < RT; ++i) {
         const int r = ty + i * 8;
@@ -402,23 +501,33 @@ __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAtt
     }
 }
 
-template <int R, int JJ>
-static int launch_rows_f32(const PagedAttnArgs& a, cudaStream_t stream) {
+// `ctas`: of a cluster (1: none)
+template <int R, int JJ, bool SPLIT>
+static int launch_rows_f32(const PagedAttnArgs& a, int ctas, cudaStream_t stream) {
     const int G = a.nq / a.nkv, heads_cta = G < R ? G : R, tokens = R / heads_cta;
-    const size_t smem = ((size_t)(R + (a.kv_planes == 2 ? 2 : 1) * AR_BK) * ar_ld(a.d) + R * (AR_BK + 4) + R) * sizeof(float);
+    const size_t smem = ((size_t)(R + (a.kv_planes == 2 ? 2 : 1) * AR_BK) * ar_ld(a.d) + R * (AR_BK + 4) + R + (SPLIT ? R * (2 + a.d) : 0)) * sizeof(float);
+    auto kern = attention_rows_f32_kernel<R, JJ, SPLIT>;
     // (the same limit whatever the size: another thread's launch, or a captured one, must not find it lowered)
-    if (cudaFuncSetAttribute(attention_rows_f32_kernel<R, JJ>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess)
-        return SHARPI_LAUNCH_FAILED;
-    const dim3 grid(a.T, a.nkv * ((G + heads_cta - 1) / heads_cta));
-    attention_rows_f32_kernel<R, JJ><<<grid, AR_THREADS, smem, stream>>>(a, heads_cta, tokens);
-    SHARPI_CHECK_LAUNCH();
-    return SHARPI_OK;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess) return SHARPI_LAUNCH_FAILED;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(a.T, a.nkv * ((G + heads_cta - 1) / heads_cta), ctas);
+    cfg.blockDim = AR_THREADS;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = ctas;
+    cfg.attrs = attr;
+    cfg.numAttrs = SPLIT ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, a, heads_cta, tokens) == cudaSuccess ? SHARPI_OK : SHARPI_LAUNCH_FAILED;
 }
 
-template <int R>
-static int launch_rows_f32(const PagedAttnArgs& a, cudaStream_t stream) {
-    return a.d <= 64 ? launch_rows_f32<R, 1>(a, stream) : a.d <= 128 ? launch_rows_f32<R, 2>(a, stream)
-                                                                       : launch_rows_f32<R, 4>(a, stream);
+template <int R, bool SPLIT = false>
+static int launch_rows_f32(const PagedAttnArgs& a, int ctas, cudaStream_t stream) {
+    return a.d <= 64 ? launch_rows_f32<R, 1, SPLIT>(a, ctas, stream) : a.d <= 128 ? launch_rows_f32<R, 2, SPLIT>(a, ctas, stream)
+                                                                                   : launch_rows_f32<R, 4, SPLIT>(a, ctas, stream);
 }
 
 // Whether CTAs take 32 rows instead of 8.  A CTA of 8 walks its keys in two thirds of the time and three to six of them share an
@@ -426,14 +535,23 @@ static int launch_rows_f32(const PagedAttnArgs& a, cudaStream_t stream) {
 // (single rows beside a portion stay a CTA each).  us, 8 / 32 rows a CTA, head size 128, 400 positions: 8 heads on 2: 60 rows
 // 66 / 109, 300 rows 80 / 111, 60 rows and 63 single ones 75 / 118, four portions of 250 181 / 128; 32 heads on 8, 2500 positions:
 // 100 rows 475 / 645, 150 rows 900 / 647, 16 portions of 16 1372 / 1278, 64 of 3 1386 / 1294, 300 rows and 63 single ones 1840 / 1917.
-static bool rows_f32_wide(const PagedAttnArgs& a, int B) {
+static int launch_rows_f32(const PagedAttnArgs& a, int B, cudaStream_t stream) {
     const int G = a.nq / a.nkv, first = a.T < B ? a.T : B;       // rows that open a request's portion, at most
     auto ctas = [&](int R) {
         const int heads_cta = G < R ? G : R, tokens = R / heads_cta;
         return (long long)((a.T - first) / tokens + first) * a.nkv * ((G + heads_cta - 1) / heads_cta);
     };
     const int per_sm = a.d <= 64 ? 6 : a.d <= 128 ? 3 : 1;
-    return ctas(8) > 148 * per_sm && 2 * ctas(8) > 5 * ctas(32);
+    if (ctas(8) > 148 * per_sm && 2 * ctas(8) > 5 * ctas(32)) return launch_rows_f32<32>(a, 1, stream);
+    // CTAs of 8 rows that leave SMs empty share their tiles in clusters, as long as those fit two thirds of the places at once.  us,
+    // without / with clusters, 8 heads on 2, head size 128: one row at 30 keys 11.6 / 13.8, at 100 20.8 / 14.6; 16 rows at 400 65 / 18;
+    // 60 rows behind 300 57 / 30; 32 heads on 8, 16 rows at 2000 287 / 205; four portions of 40 rows behind 250 (pairs, three quarters
+    // of the places) 65 / 67.
+    const long long grid = (long long)a.T * a.nkv * ((G + 7) / 8);
+    const int tiles = (int)(((long long)a.max_blocks * a.page_size + AR_BK - 1) / AR_BK);
+    for (int n = 8; n > 1; n >>= 1)
+        if (ctas(8) * n * 3 <= 148 * per_sm * 2 && tiles >= n && n * 64 >= a.d && grid * n <= 1 << 30) return launch_rows_f32<8, true>(a, n, stream);
+    return launch_rows_f32<8>(a, 1, stream);
 }
 
 SHARPI_API int sharpi_paged_attention_generic(const void* q, const void* kv_base, const int* block_table,
@@ -457,7 +575,7 @@ SHARPI_API int sharpi_paged_attention_generic(const void* q, const void* kv_base
     // (16 bytes a lane: other row sizes, larger ones and bfloat16 stay with the general kernel)
     const uintptr_t bases = (uintptr_t)q | (uintptr_t)kv_base | (uintptr_t)out;
     if (dtype == SHARPI_F32 && d % 4 == 0 && d <= AR_MAX_D && (bases & 15) == 0)
-        return rows_f32_wide(a, B) ? launch_rows_f32<32>(a, stream) : launch_rows_f32<8>(a, stream);
+        return launch_rows_f32(a, B, stream);
     dim3 grid(T, nq);
     if (dtype == SHARPI_F32)
         paged_attention_generic_kernel<float><<<grid, ATT_THREADS, 0, stream>>>(a);

@@ -81,3 +81,49 @@ def test_selective_scan_in_chunks(ops, monkeypatch, C, N, lens, raw):
             assert float((one - want).abs().max()) < 2e-5 * float(want.abs().max()), b
         assert torch.equal(state, alone)
         assert float((state.view(B, C, N) - S).abs().max()) < 2e-5 * float(S.abs().max())
+
+
+# contexts of less, as many and more tiles of 64 keys than a cluster has CTAs, the last round without tiles for some; element groups of
+# every width; a window with kept positions; keys-only pages
+@pytest.mark.parametrize("d,planes,mask,span,keep", [(128, 2, 0, 1, 0), (64, 2, 1, 300, 0), (20, 1, 0, 1, 0), (256, 2, 2, 170, 70)])
+def test_float32_attention_in_clusters_is_one_cta_a_row(ops, d, planes, mask, span, keep):
+    """A few decode rows share their key tiles in clusters; the same rows in one launch with many more have a CTA each."""
+    nq, nkv, ps, pages = 6, 2, 16, 70
+    kv = rnd(pages, planes, nkv, ps, d, seed=d)
+    table = torch.arange(pages, dtype=torch.int32, device=DEV).view(1, -1)
+    some = [0, 63, 64, 130, 511, 512, 600, 1023, 1100]
+    many = some + [t % 40 for t in range(600)]
+    q = rnd(len(many), nq, d, seed=1)
+
+    def run(n):
+        pos = torch.tensor(many[:n], dtype=torch.int32, device=DEV)
+        return ops.paged_attention_generic(q[:n].contiguous(), kv, table, torch.zeros_like(pos), pos, nq=nq, nkv=nkv, d=d, page_size=ps,
+                                           mask_kind=mask, mask_span=span, scale=d ** -0.5, keep_first=keep)
+    want = run(len(many))
+    for n in (1, 3, len(some)):
+        assert torch.equal(run(n), want[:n]), n
+
+
+@pytest.mark.parametrize("sinks", [False, True])
+def test_decode_rows_of_one_split_need_no_merge(ops, sinks):
+    """bfloat16 decode rows of up to 256 keys: alone (they write their outputs themselves) and beside a longer row (a merge does)."""
+    nq, nkv, d, ps = 8, 2, 128, 64
+    kv = rnd(16, 2, nkv, ps, d, seed=1).bfloat16()
+    table, pos = torch.arange(16, dtype=torch.int32, device=DEV).view(1, -1), torch.tensor([0, 255, 100, 700], dtype=torch.int32, device=DEV)
+    q, sink = rnd(4, nq, d, seed=2).bfloat16(), rnd(nq, seed=3) * 4 if sinks else None
+    keys, values = (kv[:, i].float().permute(1, 0, 2, 3).reshape(nkv, -1, d).double() for i in range(2))
+
+    def run(n, context, most=None):
+        out = torch.zeros(n, nq * d, dtype=torch.bfloat16, device=DEV)
+        ops.attention_decode(q[:n].contiguous(), kv, table, torch.zeros(n, dtype=torch.int32, device=DEV), pos[:n].contiguous(), out, rows=None,
+                             num_rows=n, nq=nq, nkv=nkv, d=d, page_size=ps, mask_kind=0, mask_span=1, scale=d ** -0.5,
+                             max_context=context, max_keys=most, sinks=sink)
+        return out
+    full = run(4, 701)
+    assert torch.equal(run(3, 256), full[:3]) and torch.equal(run(3, 1024, 358), full[:3]) and torch.equal(run(1, 1024, 256), full[:1])
+    for r, p in enumerate(pos.tolist()):
+        for h in range(nq):
+            s = (keys[h // 4, : p + 1] @ q[r, h].double()) * d ** -0.5
+            s = s if sink is None else torch.cat([s, sink[h: h + 1].double()])
+            want = torch.softmax(s, dim=0)[: p + 1] @ values[h // 4, : p + 1]
+            assert torch.allclose(full[r].view(nq, d)[h].double(), want, rtol=2e-2, atol=2e-2)
