@@ -77,7 +77,8 @@ __device__ __forceinline__ void decode_load_chunk(const DecodeArgs& a, const int
 //                 of the head size, 128-byte swizzle) that complete on an mbarrier; ldmatrix undoes the
 //                 swizzle in its addresses.  Needs pages of a multiple of 16 positions and a head size of
 //                 64 or 128, and cuts the instructions spent on loading to a few per pass.
-template <int D, bool TMA, bool COMPACT>
+// ONE: every row has one split, whose CTA writes the row's output itself.
+template <int D, bool TMA, bool COMPACT, bool ONE>
 __global__ void __launch_bounds__(DEC_THREADS, 3) attn_decode_split_kernel(const __grid_constant__ CUtensorMap kv_map,
                                                                            DecodeArgs a) {
     constexpr int LD = TMA ? 64 : D + 8;   // row pitch in elements: swizzled 128-byte rows, or padded rows
@@ -356,6 +357,13 @@ __global__ void __launch_bounds__(DEC_THREADS, 3) attn_decode_split_kernel(const
             acc += f * base_o[w * warp_stride + g * D + dd];
             L += f * base_o[w * warp_stride + 16 * D + g * 2 + 1];
         }
+        if constexpr (ONE) {                 // as the merge forms it: the split's weight is 1, or next to a larger sink less
+            const float sink = a.sinks ? a.sinks[head0 + g] * 1.4426950408889634f : -INFINITY;
+            const float top = fmaxf(M, sink), w = exp2f(M - top);
+            const float inv = 1.0f / (w * L + (a.sinks ? exp2f(sink - top) : 0.0f));
+            a.out[((size_t)r * a.nq + head0 + g) * D + dd] = __float2bfloat16_rn(w * acc * inv);
+            continue;
+        }
         const size_t slot = ((size_t)ri * a.nq + head0 + g) * a.max_splits + split_in_row;
         a.part_o[slot * D + dd] = acc;
         if (dd == 0) {
@@ -440,29 +448,30 @@ __global__ void __launch_bounds__(MERGE_THREADS) attn_decode_merge_kernel(Decode
 
 // A grid over all rows' splits together pays when rows times the longest row's splits would leave a fifth of
 // the CTAs without work; otherwise the grid is (splits, kv heads, rows).
-template <int D, bool TMA, bool COMPACT>
+template <int D, bool TMA, bool COMPACT, bool ONE>
 static int launch_split(const CUtensorMap& map, const DecodeArgs& a, int R, int splits, int items, cudaStream_t stream) {
     constexpr int ROW = TMA ? D : D + 8;
     constexpr int SMEM = (DEC_WARPS * 2 * 2 * DEC_CHUNK * ROW + 16 * (D + 8)) * 2 + DEC_WARPS * 2 * 8;
     static_assert(2 * 2 * DEC_CHUNK * ROW * 2 >= (16 * D + 32) * 4, "a warp's staging area must hold its partial");
     static bool configured = false;
     if (!configured) {
-        if (cudaFuncSetAttribute(attn_decode_split_kernel<D, TMA, COMPACT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        if (cudaFuncSetAttribute(attn_decode_split_kernel<D, TMA, COMPACT, ONE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  SMEM) != cudaSuccess)
             return SHARPI_LAUNCH_FAILED;
         configured = true;
     }
     const int G = a.nq / a.nkv;
     const dim3 grid = COMPACT ? dim3(items, a.nkv * ((G + 15) / 16)) : dim3(splits, a.nkv * ((G + 15) / 16), R);
-    auto kern = attn_decode_split_kernel<D, TMA, COMPACT>;
+    auto kern = attn_decode_split_kernel<D, TMA, COMPACT, ONE>;
     SHARPI_LAUNCH_PDL(kern, grid, DEC_THREADS, SMEM, stream, map, a);
     return SHARPI_OK;
 }
 
 template <int D, bool TMA>
 static int launch_split(const CUtensorMap& map, const DecodeArgs& a, int R, int splits, int items, cudaStream_t stream) {
-    if ((long long)items * 5 < (long long)R * splits * 4) return launch_split<D, TMA, true>(map, a, R, splits, items, stream);
-    return launch_split<D, TMA, false>(map, a, R, splits, items, stream);
+    if (splits == 1) return launch_split<D, TMA, false, true>(map, a, R, splits, items, stream);
+    if ((long long)items * 5 < (long long)R * splits * 4) return launch_split<D, TMA, true, false>(map, a, R, splits, items, stream);
+    return launch_split<D, TMA, false, false>(map, a, R, splits, items, stream);
 }
 
 template <int D>
@@ -477,7 +486,7 @@ static int launch_decode(const DecodeArgs& a, int R, int splits, int items, long
     } else {
         rc = launch_split<D, false>(map, a, R, splits, items, stream);
     }
-    if (rc != SHARPI_OK) return rc;
+    if (rc != SHARPI_OK || splits == 1) return rc;          // nothing to merge (2.6 us less a layer in a decode step at batch 1)
     SHARPI_LAUNCH_PDL(attn_decode_merge_kernel<D>, dim3(R, a.nq), splits >= MERGE_WIDE_FROM ? MERGE_THREADS : MERGE_THREADS / 2, 0,
                       stream, a);
     return SHARPI_OK;

@@ -305,6 +305,8 @@ def attention_decode(q: torch.Tensor, kv_layer: torch.Tensor, block_table: torch
     if d not in FAST_ATTENTION_HEAD_SIZES:
         raise KernelError(f"head size {d} is not served by the tensor-core attention kernels "
                           f"({FAST_ATTENTION_HEAD_SIZES}); use the generic kernel")
+    if max_keys is not None:                   # the other rows have a key each at least
+        max_context = min(max_context, max(max_keys - num_rows + 1, 1))
     splits = decode_splits(max_context, mask_kind, mask_span)
     # a row at position p has at most p // 256 + 1 splits, so the rows together at most max_keys // 256 + rows
     items = num_rows * splits if max_keys is None else min(num_rows * splits, max_keys // DECODE_SPLIT + num_rows)
@@ -889,8 +891,9 @@ CHUNKED_LEAST = 128
 #         16 heads of 64        33 / 27, 61 / 27, 367 / 62;   36 / 39, 68 / 68, 124 / 67
 #         64 heads of 64        35 / 28, 64 / 31, 488 / 209;  80 / 144, 163 / 257, 160 / 252
 #   scan  4096 channels of 16   250 rows 24 / 30, 400 35 / 41, 2048 155 / 111; 2048 channels 19 / 29, -, 121 / 70; 1117, 558 and 372 rows of
-#         4096 in a step 120 / 120, 576, 288, 192 and 144 rows 73 / 107: the walk takes several requests side by side
-_WALK_OR_CHUNKS = {"mlstm": (0.16, 30, 0.0), "ssd": (0.32, 30, 0.0), "wkv": (0.21, 15, 0.8), "scan": (0.028, 20, 0.0)}
+#         4096 in a step 120 / 120, 576, 288, 192 and 144 rows 73 / 107: the walk takes several requests side by side, and one that
+#         runs in chunks has what is left walked behind it, so s is such that the request's gain pays for a walk of half its rows
+_WALK_OR_CHUNKS = {"mlstm": (0.16, 30, 0.0), "ssd": (0.32, 30, 0.0), "wkv": (0.21, 15, 0.8), "scan": (0.028, 36, 0.0)}
 
 
 def chunked_least(kind: str, heads: int) -> int:
