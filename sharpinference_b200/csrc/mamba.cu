@@ -252,6 +252,7 @@ __global__ void __launch_bounds__(SPLIT ? 64 * (1 + SCAN_HELPERS) : 128) selecti
     constexpr int SCAN_STAGES = SPLIT ? 4 : 3;         // chunks in shared memory: walked, (prepared,) two on their way
     extern __shared__ __align__(16) float sm[];
     if (a.alone) pdl_wait_only(); else pdl_wait();
+    if (a.row_offsets[blockIdx.y + 1] - a.row_offsets[blockIdx.y] >= a.skip) return;
     constexpr int CPW = 32 / G, NP = G * NPT;
     const int warps = (blockDim.x >> 5) / (SPLIT ? 1 + SCAN_HELPERS : 1), CPB = warps * CPW;
     const int lane = threadIdx.x & 31;
@@ -265,7 +266,6 @@ __global__ void __launch_bounds__(SPLIT ? 64 * (1 + SCAN_HELPERS) : 128) selecti
     const int c = live ? c0 + cl : a.C - 1;
     const int b = blockIdx.y;
     const int first = a.row_offsets[b], end = a.row_offsets[b + 1];
-    if (end - first >= a.skip) return;
     const int N = a.N;
     auto n_of = [&](int i) { return 2 * (sub + (i >> 1) * G) + (i & 1); };      // the state behind register i
     // one buffer: [CH] rows of dt | x | gate [CPB each], (dt, dt x) [CPB pairs], B | C [NP each]
