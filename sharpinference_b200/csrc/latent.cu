@@ -16,7 +16,8 @@
 //                            per-head (grouped) product.
 //   sharpi_head_minor        the way back: src float32 [heads, T, n] into columns [col0, col0 + n) of
 //                            dst [T, heads, stride] in the activation dtype.
-//   sharpi_latent_q_join     the query rows: dst[t, h] = [qa[h, t, :rank] | rotate(q[t, h, dim:dim + rot]) | 0].
+//   sharpi_latent_q_join     the query rows: dst[t, h] = [qa[h, t, :rank] | rotate(q[t, h, dim:dim + rot]) | 0].  Without qa the first
+//                            `rank` elements are there already (the product with W_uk wrote them in place).
 //
 // `ld` / `ldq`: the distance between two rows of the source when it is a column range of a wider product; `rot_amp`:
 // a factor on the rotation's cosines and sines (frequency scalings that also stretch the amplitude); `gate` of
@@ -224,11 +225,12 @@ __global__ void __launch_bounds__(256)
 latent_q_join_kernel(const float* qa, const float* q, const int* positions, const float* __restrict__ inv_freq, int T,
                      int heads, int dim, int rank, int rot, int rot_dims, int D, TO* dst, int ldq, float rot_amp) {
     pdl_wait();
-    const int t = blockIdx.x, i = blockIdx.y * blockDim.x + threadIdx.x, per = D / VEC;
-    const int h = i / per, c0 = i % per * VEC;
+    const int first = qa ? 0 : rank;
+    const int t = blockIdx.x, i = blockIdx.y * blockDim.x + threadIdx.x, per = (D - first) / VEC;
+    const int h = i / per, c0 = first + i % per * VEC;
     if (h >= heads) return;
     float v[VEC];
-    if (c0 + VEC <= rank) {
+    if (qa && c0 + VEC <= rank) {
         load_vec<VEC>(qa + ((size_t)h * T + t) * rank + c0, v);
     } else {
 #pragma unroll
@@ -259,7 +261,8 @@ SHARPI_API int sharpi_latent_q_join(const float* qa, const float* q, const int* 
         rank + rot > D)
         return SHARPI_BAD_ARGUMENT;
     const bool vec = fours({rank, rot, D}, {qa, dst});
-    const dim3 grid(T, ((long long)heads * (D / (vec ? 4 : 1)) + 255) / 256);
+    if (!qa && D == rank) return SHARPI_OK;
+    const dim3 grid(T, ((long long)heads * ((qa ? D : D - rank) / (vec ? 4 : 1)) + 255) / 256);
 #define JOIN_CASE(TO)                                                                                                            \
     do {                                                                                                                         \
         if (vec) SHARPI_LAUNCH_PDL((latent_q_join_kernel<TO, 4>), grid, 256, 0, stream, qa, q, positions, inv_freq, T, heads, dim, rank, rot, rot_dims, D, (TO*)dst, ldq, rot_amp); \

@@ -42,7 +42,8 @@ constexpr int TC_BK = 64;    // K elements per stage: 128 bytes, one swizzle row
 constexpr int TC_THREADS = 192;
 
 struct TcGemmParams {
-    const int* group_offsets;   // [E + 1]
+    const int* group_offsets;   // [E + 1]; null: every group has `group_rows` rows
+    int group_rows;
     const int* out_rows;        // MODE_STORE: nullable
     const float* row_scale;     // nullable
     const int* scale_rows;      // nullable
@@ -52,7 +53,9 @@ struct TcGemmParams {
     int accumulate;
     float gate_limit;           // MODE_SWIGLU: > 0 = the clamped gate with this limit in place of silu(g) * u
     int store_act;              // MODE_STORE: 0 = float32 out as above; 1 / 2 / 3 = bf16 out [rows, N] (sorted rows) of
-                                // relu(x)^2 / tanh-GELU(x) / SiLU(x): the first product of a two-layer expert
+                                // relu(x)^2 / tanh-GELU(x) / SiLU(x): the first product of a two-layer expert; 4 = bf16 out
+                                // [group_rows][E][out_ld], row t of group e at [t][e]: a product a head whose heads become minor
+    int out_ld;
     // K split over gridDim.z CTAs (few rows and few experts: not enough tiles to fill the GPU otherwise).
     // Each CTA then leaves its raw fp32 accumulators in partial[z][sorted row][N]; the one that finishes last
     // adds the parts in the order of z and applies the epilogue.
@@ -143,6 +146,17 @@ __device__ __forceinline__ void tc_epilogue_chunk(const TcGemmParams& p, const f
         const bool scaled = p.row_scale != nullptr;      // a router that weights the experts' outputs
         if (p.store_act) {                               // activation in the epilogue, bf16 rows in sorted order
             bf16* A = reinterpret_cast<bf16*>(p.out);
+            if (p.store_act == 4) {                      // (a tile's rows are one group's)
+                const int e = r_first / p.group_rows;
+                bf16* dst = A + ((size_t)(r_first - e * p.group_rows) * p.E + e) * p.out_ld + n;
+#pragma unroll
+                for (int j = 0; j < 16; ++j, dst += (size_t)p.E * p.out_ld) {
+                    if (j >= count) break;
+                    if (n_ok) *dst = __float2bfloat16_rn(g[j]);
+                    if (nb_ok) dst[TC_BM] = __float2bfloat16_rn(u[j]);
+                }
+                return;
+            }
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
                 if (j < count) {
@@ -249,8 +263,8 @@ tc_grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             const int e = e0 + lane;
             int start = 0, end = 0;
             if (e < p.E) {
-                start = p.group_offsets[e];
-                end = p.group_offsets[e + 1];
+                start = p.group_offsets ? p.group_offsets[e] : e * p.group_rows;
+                end = p.group_offsets ? p.group_offsets[e + 1] : start + p.group_rows;
             }
             const int tiles = (end - start + NT - 1) / NT;
             int incl = tiles;
@@ -744,14 +758,14 @@ static int tc_grouped_gemm_impl(const void* A, const void* W, const int* group_o
                                const int* out_rows, const float* row_scale, const int* scale_rows,
                                int* status, float* partial, int* tickets, int rows, int N, int K, int E, int mode,
                                int row_tile, int accumulate, int k_split, int max_ctas, int store_act,
-                               float gate_limit, cudaStream_t stream) {
+                               float gate_limit, cudaStream_t stream, int group_rows = 0, int out_ld = 0) {
     if (rows <= 0 || N <= 0) return SHARPI_OK;
-    if (store_act < 0 || store_act > 3 || (store_act && (mode != MODE_STORE || accumulate || out_rows)))
+    if (store_act < 0 || store_act > 4 || (store_act && (mode != MODE_STORE || accumulate || out_rows)))
         return SHARPI_BAD_ARGUMENT;
     if (K <= 0 || E <= 0 || K % 8 != 0) return SHARPI_BAD_ARGUMENT;          // TMA: rows 16-byte aligned
     if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) return SHARPI_UNALIGNED;
     if (mode == MODE_SWIGLU && (N % 2 != 0)) return SHARPI_BAD_ARGUMENT;
-    if (!status || !group_offsets) return SHARPI_BAD_ARGUMENT;
+    if (!status || (!group_offsets && (group_rows <= 0 || row_tile == 0))) return SHARPI_BAD_ARGUMENT;
     CUtensorMap mw, ma;
     if (!tmap::make_bf16_map(&mw, W, (uint64_t)K, (uint64_t)N, (uint64_t)E, TC_BK, TC_BM)) return SHARPI_LAUNCH_FAILED;
     if (!tmap::make_bf16_map(&ma, A, (uint64_t)K, (uint64_t)rows, 0, TC_BK, (uint32_t)(row_tile ? row_tile : 128)))
@@ -759,7 +773,7 @@ static int tc_grouped_gemm_impl(const void* A, const void* W, const int* group_o
     TcGemmParams p;
     p.group_offsets = group_offsets; p.out_rows = out_rows; p.row_scale = row_scale; p.scale_rows = scale_rows;
     p.out = out; p.status = status; p.rows = rows; p.N = N; p.K = K; p.E = E; p.accumulate = accumulate;
-    p.store_act = store_act;
+    p.store_act = store_act; p.group_rows = group_rows; p.out_ld = out_ld;
     if (!(gate_limit >= 0.0f)) return SHARPI_BAD_ARGUMENT;
     p.gate_limit = gate_limit;
     if (k_split < 1 || k_split > 16 || (k_split > 1 && (!partial || !tickets))) return SHARPI_BAD_ARGUMENT;
@@ -816,6 +830,18 @@ SHARPI_API int sharpi_tc_grouped_gemm_act(const void* A, const void* W, const in
     if (act < 1 || act > 3) return SHARPI_BAD_ARGUMENT;
     return tc_grouped_gemm_impl(A, W, group_offsets, out, nullptr, nullptr, nullptr, status, partial, tickets, rows, N, K,
                                 E, MODE_STORE, row_tile, 0, k_split, 0, act, 0.0f, stream);
+}
+
+// A product a head, `T` rows each: A [E * T, K] holds every head's rows one head after the other; bf16 out[t][e][n] =
+// A[e T + t] . W[e][n] with heads `out_ld` elements apart (rounded as a conversion of the float32 product would): the result where
+// the next kernel reads it, without a float32 copy and a pass that turns it (2048 rows of 16 heads, 128 -> 256 and 256 -> 128: 17 us a
+// product and two passes behind them, 12 us a product and a pass over the rotated columns now; the mixer 206 -> 158 us).
+SHARPI_API int sharpi_tc_per_head(const void* A, const void* W, void* out, int* status, int T, int N, int K, int E, int out_ld,
+                                  int row_tile, cudaStream_t stream) {
+    if (T <= 0) return SHARPI_OK;
+    if (E <= 0 || out_ld < N || (long long)T * E > 0x7fffffff || row_tile == 0) return SHARPI_BAD_ARGUMENT;
+    return tc_grouped_gemm_impl(A, W, nullptr, out, nullptr, nullptr, nullptr, status, nullptr, nullptr, T * E, N, K, E, MODE_STORE, row_tile,
+                                0, 1, 0, 4, 0.0f, stream, T, out_ld);
 }
 
 // The gate|up mode with the clamped gate in the epilogue: bf16 out[r, i] = g sigmoid(1.702 g) (u + 1) with g cut off above

@@ -636,6 +636,21 @@ def tc_grouped_gemm(a: torch.Tensor, w: torch.Tensor, group_offsets: torch.Tenso
     return out
 
 
+def tc_per_head(a: torch.Tensor, w: torch.Tensor, T: int, out: torch.Tensor) -> torch.Tensor:
+    """A product a head on the tensor cores, the heads minor in the result: ``a`` bfloat16 ``[E * T, K]`` (every head's rows one head
+    after the other), ``w`` bfloat16 ``[E, N, K]``; ``out`` bfloat16 ``[T, E, ld]``, of which the first ``N`` columns are written."""
+    for name, t in (("a", a), ("w", w), ("out", out)):
+        _need(t, name, torch.bfloat16)
+    E, N, K = w.shape
+    if tuple(a.shape) != (E * T, K) or out.dim() != 3 or tuple(out.shape[:2]) != (T, E) or out.shape[2] < N:
+        raise KernelError(f"shapes disagree: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}, {T} rows a head")
+    if K % 8 != 0:
+        raise KernelError(f"the tensor-core product needs an inner size that is a multiple of 8, found {K}")
+    check(kernel("sharpi_tc_per_head")(a.data_ptr(), w.data_ptr(), out.data_ptr(), status_word(a.device).data_ptr(), T, N, K, E,
+                                       out.shape[2], tc_row_tile(E * T), _stream()), "sharpi_tc_per_head")
+    return out
+
+
 _TC_STORE_ACT = {ACT_RELU2: 1, ACT_GELU_TANH: 2, ACT_SILU: 3}
 
 
@@ -1461,19 +1476,27 @@ def head_minor(src: torch.Tensor, *, heads: int, out_dtype: torch.dtype, gate: O
     return out
 
 
-def latent_q_join(qa: torch.Tensor, q: torch.Tensor, positions: torch.Tensor, inv_freq: Optional[torch.Tensor], *,
+def latent_q_join(qa: Optional[torch.Tensor], q: torch.Tensor, positions: torch.Tensor, inv_freq: Optional[torch.Tensor], *,
                   heads: int, dim: int, rank: int, rot: int, rot_dims: int, D: int, out_dtype: torch.dtype,
-                  rot_amplitude: float = 1.0) -> torch.Tensor:
+                  rot_amplitude: float = 1.0, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """The query rows of latent attention, ``[T, heads, D]``: ``[qa[h, t] | rotate(q[t, h, dim:]) | 0]`` with ``qa``
     float32 ``[heads * T, rank]`` (head by head) and ``q`` float32 ``[T, heads * (dim + rot)]`` (possibly a column range
-    of a wider product); ``rot_amplitude`` multiplies the rotation's cosines and sines."""
-    _need(qa, "qa", torch.float32)
+    of a wider product); ``rot_amplitude`` multiplies the rotation's cosines and sines.  Without ``qa`` the first ``rank`` columns
+    of ``out`` are there already and the others are written."""
+    if qa is not None:
+        _need(qa, "qa", torch.float32)
+    elif out is None:
+        raise KernelError("without qa the rows need an output that holds their first columns")
     ldq = _need_columns(q, "q", torch.float32)
     T = q.shape[0]
-    if q.shape[1] != heads * (dim + rot) or tuple(qa.shape) != (heads * T, rank):
-        raise KernelError(f"q {tuple(q.shape)} or qa {tuple(qa.shape)} disagree with the sizes")
-    out = torch.empty((T, heads, D), dtype=out_dtype, device=q.device)
-    check(kernel("sharpi_latent_q_join")(qa.data_ptr(), q.data_ptr(), positions.data_ptr(), _ptr(inv_freq), T, heads, dim,
+    if q.shape[1] != heads * (dim + rot) or (qa is not None and tuple(qa.shape) != (heads * T, rank)):
+        raise KernelError(f"q {tuple(q.shape)} or qa {None if qa is None else tuple(qa.shape)} disagree with the sizes")
+    if out is None:
+        out = torch.empty((T, heads, D), dtype=out_dtype, device=q.device)
+    _need(out, "out", out_dtype)
+    if tuple(out.shape) != (T, heads, D):
+        raise KernelError(f"out is {tuple(out.shape)}, expected {(T, heads, D)}")
+    check(kernel("sharpi_latent_q_join")(_ptr(qa), q.data_ptr(), positions.data_ptr(), _ptr(inv_freq), T, heads, dim,
                                          rank, rot, rot_dims if inv_freq is not None else 0, D, out.data_ptr(),
                                          dtype_code(out_dtype), ldq, float(rot_amplitude), _stream()), "sharpi_latent_q_join")
     return out

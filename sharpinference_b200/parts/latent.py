@@ -135,10 +135,12 @@ class LatentAttention(Mixer):
         # [T, H (dim + rot)] float32: from the query latent, or leading the fused product
         q = self.up_q(cq) if self.q_rank > 0 else down[:, : self._lead]
         q_plain = ops.head_major(q, heads=H, stride=self.dim + self.rot_dim, col0=0, n=self.dim, out_dtype=act)
-        qa = self.up_k.per_group(q_plain, T)                                  # [H T, kv_rank] float32
-        qj = ops.latent_q_join(qa, q, ctx.positions, self.inv_freq, heads=H, dim=self.dim, rank=self.kv_rank,
-                               rot=self.rot_dim, rot_dims=self.rot_dims, D=D, out_dtype=act,
-                               rot_amplitude=self.rot_amplitude)
+        # into the query rows at once where the product can; else float32 [H T, kv_rank] beside them
+        qj = torch.empty((T, H, D), dtype=act, device=h.device)
+        qa = None if self.up_k.per_group_minor(q_plain, T, qj) else self.up_k.per_group(q_plain, T)
+        ops.latent_q_join(qa, q, ctx.positions, self.inv_freq, heads=H, dim=self.dim, rank=self.kv_rank,
+                          rot=self.rot_dim, rot_dims=self.rot_dims, D=D, out_dtype=act,
+                          rot_amplitude=self.rot_amplitude, out=qj)
         dv = (self.kv_rank + 15) // 16 * 16
         if ops.keys_attention_supported(act, D, dv) and slot.kv.shape[1] == 1:
             # the tensor-core kernels for keys-only pages: the value sum is taken over the latent's columns only
@@ -157,5 +159,9 @@ class LatentAttention(Mixer):
                                             page_size=slot.page_size, mask_kind=mask_kind, mask_span=mask_span,
                                             scale=self.softmax_scale)
             o_lat = ops.head_major(o, heads=H, stride=D, col0=0, n=self.kv_rank, out_dtype=act)
+        if gate is None:
+            v = torch.empty((T, H, self.value_dim), dtype=act, device=h.device)
+            if self.up_v.per_group_minor(o_lat, T, v):
+                return self.out(v.view(T, -1))
         v = self.up_v.per_group(o_lat, T)                                     # [H T, value_dim] float32
         return self.out(ops.head_minor(v, heads=H, out_dtype=act, gate=gate))

@@ -157,6 +157,14 @@ class GroupedLinear:
         return ops.gemm_nt(a, self.weight, out=out, group_offsets=group_offsets, a_rows=a_rows, out_rows=out_rows,
                            rows=rows, accumulate=accumulate)
 
+    def per_group_minor(self, a: torch.Tensor, rows_per_group: int, out: torch.Tensor) -> bool:
+        """:meth:`per_group` in bfloat16 with the groups minor, ``out [rows_per_group, groups, ld]``, where the tensor-core product
+        takes it (more than 16 rows in all: with fewer it cuts K over CTAs); False: nothing was written."""
+        if not (self.weight.dtype == torch.bfloat16 == a.dtype and self.in_features % 8 == 0 and a.shape[0] > 16):
+            return False
+        ops.tc_per_head(a, self.weight, rows_per_group, out)
+        return True
+
     def per_group(self, a: torch.Tensor, rows_per_group: int) -> torch.Tensor:
         """The product for ``a [groups * rows_per_group, in]`` that holds every group's rows one group after the
         other, the same number each (one weight a head: heads are the groups): float32 ``[groups * rows_per_group,

@@ -127,3 +127,15 @@ def test_decode_rows_of_one_split_need_no_merge(ops, sinks):
             s = s if sink is None else torch.cat([s, sink[h: h + 1].double()])
             want = torch.softmax(s, dim=0)[: p + 1] @ values[h // 4, : p + 1]
             assert torch.allclose(full[r].view(nq, d)[h].double(), want, rtol=2e-2, atol=2e-2)
+
+
+# rows that fill a tile of activations and that do not, one and two weight tiles a CTA, output rows wider than the product, one head
+@pytest.mark.parametrize("E,T,N,K,ld", [(3, 6, 40, 64, 48), (2, 130, 256, 128, 320), (8, 257, 300, 72, 300), (1, 33, 128, 256, 128)])
+def test_product_a_head_with_the_heads_minor(ops, E, T, N, K, ld):
+    """The bits of the float32 product turned and rounded; the columns behind the product stay as they are."""
+    a, w = rnd(E * T, K, seed=1).bfloat16(), rnd(E, N, K, seed=2).bfloat16()
+    out = torch.full((T, E, ld), 7.0, dtype=torch.bfloat16, device=DEV)
+    ops.tc_per_head(a, w, T, out)
+    offsets = torch.arange(E + 1, dtype=torch.int32, device=DEV) * T
+    want = ops.tc_grouped_gemm(a, w, offsets, mode=ops.TC_MODE_STORE).view(E, T, N).transpose(0, 1).to(torch.bfloat16)
+    assert torch.equal(out[..., :N], want) and bool((out[..., N:] == 7.0).all())
