@@ -44,6 +44,7 @@ constexpr int TC_THREADS = 192;
 struct TcGemmParams {
     const int* group_offsets;   // [E + 1]; null: every group has `group_rows` rows
     int group_rows;
+    int a_minor;                // A is [group_rows][E][a row's distance]: row t of group e at [t][e]
     const int* out_rows;        // MODE_STORE: nullable
     const float* row_scale;     // nullable
     const int* scale_rows;      // nullable
@@ -314,7 +315,8 @@ tc_grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                     tma_load_3d(stage, &map_w, &full_bar[s], kx, n0, expert);
                     if (WT == 2) tma_load_3d(stage + Cfg::W_BYTES, &map_w, &full_bar[s], kx, n1, expert);
                 }
-                tma_load_2d(stage + Cfg::W_TILES * Cfg::W_BYTES, &map_a, &full_bar[s], kx, row0);
+                if (p.a_minor) tma_load_3d(stage + Cfg::W_TILES * Cfg::W_BYTES, &map_a, &full_bar[s], kx, expert, row0 - expert * p.group_rows);
+                else tma_load_2d(stage + Cfg::W_TILES * Cfg::W_BYTES, &map_a, &full_bar[s], kx, row0);
                 issued = kb + 1;
             }
             if (!ok) {
@@ -758,7 +760,7 @@ static int tc_grouped_gemm_impl(const void* A, const void* W, const int* group_o
                                const int* out_rows, const float* row_scale, const int* scale_rows,
                                int* status, float* partial, int* tickets, int rows, int N, int K, int E, int mode,
                                int row_tile, int accumulate, int k_split, int max_ctas, int store_act,
-                               float gate_limit, cudaStream_t stream, int group_rows = 0, int out_ld = 0) {
+                               float gate_limit, cudaStream_t stream, int group_rows = 0, int out_ld = 0, int a_ld = 0) {
     if (rows <= 0 || N <= 0) return SHARPI_OK;
     if (store_act < 0 || store_act > 4 || (store_act && (mode != MODE_STORE || accumulate || out_rows)))
         return SHARPI_BAD_ARGUMENT;
@@ -768,12 +770,13 @@ static int tc_grouped_gemm_impl(const void* A, const void* W, const int* group_o
     if (!status || (!group_offsets && (group_rows <= 0 || row_tile == 0))) return SHARPI_BAD_ARGUMENT;
     CUtensorMap mw, ma;
     if (!tmap::make_bf16_map(&mw, W, (uint64_t)K, (uint64_t)N, (uint64_t)E, TC_BK, TC_BM)) return SHARPI_LAUNCH_FAILED;
-    if (!tmap::make_bf16_map(&ma, A, (uint64_t)K, (uint64_t)rows, 0, TC_BK, (uint32_t)(row_tile ? row_tile : 128)))
+    if (a_ld ? !tmap::make_bf16_rows_map(&ma, A, (uint64_t)K, (uint64_t)E, (uint64_t)group_rows, (uint64_t)a_ld, TC_BK, (uint32_t)row_tile)
+             : !tmap::make_bf16_map(&ma, A, (uint64_t)K, (uint64_t)rows, 0, TC_BK, (uint32_t)(row_tile ? row_tile : 128)))
         return SHARPI_LAUNCH_FAILED;
     TcGemmParams p;
     p.group_offsets = group_offsets; p.out_rows = out_rows; p.row_scale = row_scale; p.scale_rows = scale_rows;
     p.out = out; p.status = status; p.rows = rows; p.N = N; p.K = K; p.E = E; p.accumulate = accumulate;
-    p.store_act = store_act; p.group_rows = group_rows; p.out_ld = out_ld;
+    p.store_act = store_act; p.group_rows = group_rows; p.out_ld = out_ld; p.a_minor = a_ld > 0;
     if (!(gate_limit >= 0.0f)) return SHARPI_BAD_ARGUMENT;
     p.gate_limit = gate_limit;
     if (k_split < 1 || k_split > 16 || (k_split > 1 && (!partial || !tickets))) return SHARPI_BAD_ARGUMENT;
@@ -832,16 +835,17 @@ SHARPI_API int sharpi_tc_grouped_gemm_act(const void* A, const void* W, const in
                                 E, MODE_STORE, row_tile, 0, k_split, 0, act, 0.0f, stream);
 }
 
-// A product a head, `T` rows each: A [E * T, K] holds every head's rows one head after the other; bf16 out[t][e][n] =
+// A product a head, `T` rows each: A [E * T, K] holds every head's rows one head after the other, or (a_ld, a multiple of 8) is
+// [T][E][a_ld] with the heads minor; bf16 out[t][e][n] =
 // A[e T + t] . W[e][n] with heads `out_ld` elements apart (rounded as a conversion of the float32 product would): the result where
 // the next kernel reads it, without a float32 copy and a pass that turns it (2048 rows of 16 heads, 128 -> 256 and 256 -> 128: 17 us a
 // product and two passes behind them, 12 us a product and a pass over the rotated columns now; the mixer 206 -> 158 us).
-SHARPI_API int sharpi_tc_per_head(const void* A, const void* W, void* out, int* status, int T, int N, int K, int E, int out_ld,
+SHARPI_API int sharpi_tc_per_head(const void* A, int a_ld, const void* W, void* out, int* status, int T, int N, int K, int E, int out_ld,
                                   int row_tile, cudaStream_t stream) {
     if (T <= 0) return SHARPI_OK;
-    if (E <= 0 || out_ld < N || (long long)T * E > 0x7fffffff || row_tile == 0) return SHARPI_BAD_ARGUMENT;
+    if (E <= 0 || out_ld < N || a_ld < 0 || (a_ld && (a_ld < K || a_ld % 8 != 0)) || (long long)T * E > 0x7fffffff || row_tile == 0) return SHARPI_BAD_ARGUMENT;
     return tc_grouped_gemm_impl(A, W, nullptr, out, nullptr, nullptr, nullptr, status, nullptr, nullptr, T * E, N, K, E, MODE_STORE, row_tile,
-                                0, 1, 0, 4, 0.0f, stream, T, out_ld);
+                                0, 1, 0, 4, 0.0f, stream, T, out_ld, a_ld);
 }
 
 // The gate|up mode with the clamped gate in the epilogue: bf16 out[r, i] = g sigmoid(1.702 g) (u + 1) with g cut off above

@@ -40,4 +40,18 @@ inline bool make_bf16_map(CUtensorMap* map, const void* base, uint64_t d0, uint6
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// bf16 tensor [d2][d1][ld], of which the first d0 of every ld elements are read (ld a multiple of 8): boxes of [box2, 1, box0],
+// 128-byte swizzle as above, out-of-range elements read as zero.
+inline bool make_bf16_rows_map(CUtensorMap* map, const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t ld, uint32_t box0,
+                               uint32_t box2) {
+    EncodeTiledFn fn = encode_tiled();
+    if (!fn) return false;
+    cuuint64_t dims[3] = {d0, d1, d2};
+    cuuint64_t strides[2] = {ld * 2, d1 * ld * 2};
+    cuuint32_t box[3] = {box0, 1, box2};
+    cuuint32_t elem[3] = {1, 1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 }  // namespace tmap

@@ -46,7 +46,7 @@ SIGNATURES: Dict[str, Tuple[str, list]] = {
     "sharpi_router_top1": ("moe", [P, P, I, I, I, I, P, P, P, P, P, P, P]),
     "sharpi_moe_sort": ("moe", [P, I, I, P, P, P]),
     "sharpi_tc_grouped_gemm": ("tc_gemm", [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, P]),
-    "sharpi_tc_per_head": ("tc_gemm", [P, P, P, P, I, I, I, I, I, I, P]),
+    "sharpi_tc_per_head": ("tc_gemm", [P, I, P, P, P, I, I, I, I, I, I, P]),
     "sharpi_tc_grouped_gemm_act": ("tc_gemm", [P, P, P, P, P, P, P, I, I, I, I, I, I, I, P]),
     "sharpi_gather_rows_bf16": ("tc_gemm", [P, P, P, I, I, P]),
     "sharpi_dense_rows": ("dense_rows", [P, P, P, P, I, I, I, I, I, P]),

@@ -638,15 +638,17 @@ def tc_grouped_gemm(a: torch.Tensor, w: torch.Tensor, group_offsets: torch.Tenso
 
 def tc_per_head(a: torch.Tensor, w: torch.Tensor, T: int, out: torch.Tensor) -> torch.Tensor:
     """A product a head on the tensor cores, the heads minor in the result: ``a`` bfloat16 ``[E * T, K]`` (every head's rows one head
-    after the other), ``w`` bfloat16 ``[E, N, K]``; ``out`` bfloat16 ``[T, E, ld]``, of which the first ``N`` columns are written."""
+    after the other) or ``[T, E, ld]`` (heads minor, ld a multiple of 8 of which the first ``K`` are read), ``w`` bfloat16 ``[E, N, K]``;
+    ``out`` bfloat16 ``[T, E, ld]``, of which the first ``N`` columns are written."""
     for name, t in (("a", a), ("w", w), ("out", out)):
         _need(t, name, torch.bfloat16)
     E, N, K = w.shape
-    if tuple(a.shape) != (E * T, K) or out.dim() != 3 or tuple(out.shape[:2]) != (T, E) or out.shape[2] < N:
+    a_ld = a.shape[2] if a.dim() == 3 else 0
+    if (tuple(a.shape[:2]) != (T, E) or a_ld < K if a_ld else tuple(a.shape) != (E * T, K)) or out.dim() != 3 or tuple(out.shape[:2]) != (T, E) or out.shape[2] < N:
         raise KernelError(f"shapes disagree: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}, {T} rows a head")
-    if K % 8 != 0:
-        raise KernelError(f"the tensor-core product needs an inner size that is a multiple of 8, found {K}")
-    check(kernel("sharpi_tc_per_head")(a.data_ptr(), w.data_ptr(), out.data_ptr(), status_word(a.device).data_ptr(), T, N, K, E,
+    if K % 8 != 0 or a_ld % 8 != 0:
+        raise KernelError(f"the tensor-core product needs an inner size that is a multiple of 8, found {K} in rows of {a_ld or K}")
+    check(kernel("sharpi_tc_per_head")(a.data_ptr(), a_ld, w.data_ptr(), out.data_ptr(), status_word(a.device).data_ptr(), T, N, K, E,
                                        out.shape[2], tc_row_tile(E * T), _stream()), "sharpi_tc_per_head")
     return out
 

@@ -153,15 +153,16 @@ class LatentAttention(Mixer):
             if plan.num_decode_rows:
                 ops.attention_keys_decode(qj, slot.kv, table, ctx.row_request, ctx.positions, o, rows=plan.decode_rows,
                                           num_rows=plan.num_decode_rows, max_context=ctx.max_context, **kw)
-            o_lat = ops.head_major(o, heads=H, stride=dv, col0=0, n=self.kv_rank, out_dtype=act)
+            stride = dv
         else:
             o = ops.paged_attention_generic(qj, slot.kv, table, ctx.row_request, ctx.positions, nq=H, nkv=1, d=D,
                                             page_size=slot.page_size, mask_kind=mask_kind, mask_span=mask_span,
                                             scale=self.softmax_scale)
-            o_lat = ops.head_major(o, heads=H, stride=D, col0=0, n=self.kv_rank, out_dtype=act)
+            stride = D
         if gate is None:
             v = torch.empty((T, H, self.value_dim), dtype=act, device=h.device)
-            if self.up_v.per_group_minor(o_lat, T, v):
+            if self.up_v.per_group_minor(o.view(T, H, stride), T, v):
                 return self.out(v.view(T, -1))
+        o_lat = ops.head_major(o, heads=H, stride=stride, col0=0, n=self.kv_rank, out_dtype=act)
         v = self.up_v.per_group(o_lat, T)                                     # [H T, value_dim] float32
         return self.out(ops.head_minor(v, heads=H, out_dtype=act, gate=gate))

@@ -159,8 +159,10 @@ class GroupedLinear:
 
     def per_group_minor(self, a: torch.Tensor, rows_per_group: int, out: torch.Tensor) -> bool:
         """:meth:`per_group` in bfloat16 with the groups minor, ``out [rows_per_group, groups, ld]``, where the tensor-core product
-        takes it (more than 16 rows in all: with fewer it cuts K over CTAs); False: nothing was written."""
-        if not (self.weight.dtype == torch.bfloat16 == a.dtype and self.in_features % 8 == 0 and a.shape[0] > 16):
+        takes it (more than 16 rows in all: with fewer it cuts K over CTAs); False: nothing was written.  ``a`` as there, or with the
+        groups minor, ``[rows_per_group, groups, ld]``, of which the first ``in`` columns are read."""
+        if not (self.weight.dtype == torch.bfloat16 == a.dtype and self.in_features % 8 == 0 and self.num_groups * rows_per_group > 16
+                and (a.dim() == 2 or a.shape[2] % 8 == 0)):
             return False
         ops.tc_per_head(a, self.weight, rows_per_group, out)
         return True

@@ -139,3 +139,7 @@ def test_product_a_head_with_the_heads_minor(ops, E, T, N, K, ld):
     offsets = torch.arange(E + 1, dtype=torch.int32, device=DEV) * T
     want = ops.tc_grouped_gemm(a, w, offsets, mode=ops.TC_MODE_STORE).view(E, T, N).transpose(0, 1).to(torch.bfloat16)
     assert torch.equal(out[..., :N], want) and bool((out[..., N:] == 7.0).all())
+    wide = torch.full((T, E, K + 16), float("nan"), dtype=torch.bfloat16, device=DEV)          # operand rows with the heads minor too
+    wide[..., :K] = a.view(E, T, K).transpose(0, 1)
+    again = torch.empty(T, E, N, dtype=torch.bfloat16, device=DEV)
+    assert torch.equal(ops.tc_per_head(wide, w, T, again), want)
