@@ -146,9 +146,11 @@ __global__ void __launch_bounds__(256) gemm_nt_kernel(GemmArgs g) {
 
 // float32 operands, rows on 16 bytes.  A thread has rows ty + i BM / 8 and columns tx + 16 j of the tile; a stage is 32 k of
 // the tile's rows as they lie in memory (k in front), 4 floats of padding a row, so that neighbouring rows start in other
-// banks: 12 reads of 16 bytes serve 64 paired multiply-adds.  Bound by the multiply-adds: 37 TFLOP/s at 2048 rows of 5120 x
-// 5120, and no more with single instead of paired ones, 8 x 8 outputs a thread or another order of lanes.  980 rows of
-// 8192 x 1024: 467 us = 35 TFLOP/s; 694 us with 4 x 4 outputs a thread and scalar strided loads.
+// banks: 12 reads of 16 bytes serve 64 paired multiply-adds, eight of which in a row take the same weights (an operand that
+// the register file need not give again).  A stage is written out in full: the reads of the next k are then under way before
+// the products of these (219 registers, so one CTA of 256 threads an SM; two of 128 registers each were no faster: the
+// multiply-adds themselves are the bound, 58 TFLOP/s of them alone).  2048 rows of 5120 x 5120: 37.3 -> 41.3 TFLOP/s, 980 rows of
+// 8192 x 1024 470 -> 428 us, 300 rows of 8192 x 1024 199 -> 181 us, 64 rows of 1024 x 1024 46 -> 40 us.
 constexpr int GT_N = 64, GT_K = 32, GT_LD = GT_K + 4, GT_STAGES = 3;
 
 template <int BM>
@@ -206,19 +208,18 @@ __global__ void __launch_bounds__(2 * BM) gemm_tile_kernel(GemmArgs g) {
         mma16::cp_async_commit();
         const float* a_s = gt_smem + (s % GT_STAGES) * STAGE + ty * GT_LD;
         const float* w_s = gt_smem + (s % GT_STAGES) * STAGE + (BM + tx) * GT_LD;
-#pragma unroll 4
+#pragma unroll
         for (int k = 0; k < GT_K; k += 4) {
-            ulonglong2 w[4];
+            ulonglong2 a[8];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) w[j] = *reinterpret_cast<const ulonglong2*>(w_s + j * 16 * GT_LD + k);
+            for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(a_s + i * (BM / 8) * GT_LD + k);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(a_s + i * (BM / 8) * GT_LD + k);
+            for (int j = 0; j < 4; ++j) {
+                const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(w_s + j * 16 * GT_LD + k);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    fma2(acc[i][j], a.x, w[j].x);
-                    fma2(acc[i][j], a.y, w[j].y);
-                }
+                for (int i = 0; i < 8; ++i) fma2(acc[i][j], a[i].x, w.x);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) fma2(acc[i][j], a[i].y, w.y);
             }
         }
         if ((s + 1) % (GB_SEG / GT_K) == 0 || s + 1 == stages) {
