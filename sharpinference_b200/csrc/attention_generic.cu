@@ -200,6 +200,7 @@ __device__ __forceinline__ float4 load_cluster4(uint32_t at) {
 template <int R, int JJ, bool SPLIT>
 __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAttnArgs a, int heads_cta, int tokens) {
     static_assert(!SPLIT || R == 8, "a thread has four neighbouring elements of the cluster's sums at most");
+    if (SPLIT) pdl_wait();
     const int ctas = SPLIT ? (int)gridDim.z : 1, rank = SPLIT ? (int)blockIdx.z : 0;
     extern __shared__ __align__(16) float ar_smem[];
     __shared__ long long off_s[2][AR_BK];                // where the keys of two tiles lie, -1: not there
@@ -242,19 +243,20 @@ __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAtt
         const int page = key <= p_last && (key >= lo_first || key < keep) ? table[key / a.page_size] : -1;
         return page >= 0 ? (long long)page * a.kv_planes * plane + ((long long)kvh * a.page_size + key % a.page_size) * d : -1;
     };
-    auto load = [&](float* dst, int at, size_t second) {  // a warp copies every fourth row of the tile whose places are off_s[at]
+    auto side = [&](int it) { return it / ctas & 1; };    // which of off_s is tile it's
+    auto load = [&](float* dst, int it, size_t second) {  // a warp copies every fourth row
 #pragma unroll 4
         for (int r = warp; r < AR_BK; r += AR_THREADS / 32) {
-            const long long off = off_s[at][r];
+            const long long off = off_s[side(it)][r];
             const float* src = kv + (off >= 0 ? off + second : 0);
             for (int c = lane; c < vec; c += 32) mma16::cp_async_16(dst + r * ld + c * 4, src + (off >= 0 ? c * 4 : 0), off >= 0 ? 16 : 0);
         }
         mma16::cp_async_commit();
     };
-    if (tid < AR_BK) off_s[0][tid] = rank < n_iter ? place(rank) : -1;
+    if (tid < AR_BK) off_s[0][tid] = SPLIT && rank >= n_iter ? -1 : place(rank);
     __syncthreads();
-    load(k_s, 0, 0);
-    if (a.kv_planes == 2) load(v_s, 0, plane);
+    load(k_s, rank, 0);
+    if (a.kv_planes == 2) load(v_s, rank, plane);
     for (int r = warp; r < R; r += AR_THREADS / 32) {
         const bool ok = r < n_rows;
         const float* src = (const float*)a.q + ((size_t)(t + (ok ? r / heads_here : 0)) * a.nq + head0 + (ok ? r % heads_here : 0)) * d;
@@ -272,7 +274,7 @@ __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAtt
     const int unit = rank + ctas * tid, unit_r = unit / vec, unit_c = unit % vec * 4;
     float4 joint = make_float4(0.f, 0.f, 0.f, 0.f);
 
-    for (int it0 = 0, at = 0; it0 < n_iter; it0 += ctas, at ^= 1) {
+    for (int it0 = 0; it0 < n_iter; it0 += ctas) {
         const int it = it0 + rank;
         const bool have = !SPLIT || it < n_iter, more = it0 + ctas < n_iter;      // (a CTA without a tile in the last round goes along)
         const int key0 = key0_of(have ? it : 0);
@@ -310,7 +312,7 @@ __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAtt
                 for (int j = 0; j < 4; ++j) {
                     const int key = key0 + tx + 16 * j;
                     float v = __uint_as_float(AR_HIDDEN);
-                    if (key <= pos && (key >= lo || key < keep) && off_s[at][tx + 16 * j] >= 0) {
+                    if (key <= pos && (key >= lo || key < keep) && off_s[side(it)][tx + 16 * j] >= 0) {
                         v = __fmul_rn(__fadd_rn(lo2(s[i][j]), hi2(s[i][j])), a.scale);
                         if (a.softcap > 0.0f) v = a.softcap * tanhf(v / a.softcap);
                         if (a.dist_bias) v += a.dist_bias[(size_t)min(pos - key, a.dist_far) * a.nq + h];
@@ -319,9 +321,9 @@ __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAtt
                 }
             }
         }
-        if (tid < AR_BK) off_s[at ^ 1][tid] = next;
+        if (tid < AR_BK) off_s[side(it + ctas)][tid] = next;
         __syncthreads();                                 // the scores are here; keys are free
-        if (a.kv_planes == 2 && more) load(k_s, at ^ 1, 0);
+        if (a.kv_planes == 2 && more) load(k_s, it + ctas, 0);
         if constexpr (SPLIT) {
             float* p = p_s + (tid >> 2) * (AR_BK + 4) + (tid & 3) * 4;
             if (tid < 4 * R) {
@@ -457,7 +459,7 @@ __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAtt
         }
         if (more) {
             __syncthreads();                             // the values are free
-            if (a.kv_planes == 2) load(v_s, at ^ 1, plane); else load(k_s, at ^ 1, 0);
+            if (a.kv_planes == 2) load(v_s, it + ctas, plane); else load(k_s, it + ctas, 0);
         }
     }
     if constexpr (SPLIT) cluster_sync();                 // nobody reads this CTA's shared memory any more
@@ -514,13 +516,15 @@ static int launch_rows_f32(const PagedAttnArgs& a, int ctas, cudaStream_t stream
     cfg.blockDim = AR_THREADS;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 1;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = ctas;
     cfg.attrs = attr;
-    cfg.numAttrs = SPLIT ? 1 : 0;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = SPLIT ? 1 + sharpi_pdl_enabled() : 0;
     return cudaLaunchKernelEx(&cfg, kern, a, heads_cta, tokens) == cudaSuccess ? SHARPI_OK : SHARPI_LAUNCH_FAILED;
 }
 

@@ -252,6 +252,7 @@ template <int MR>
 __global__ void __launch_bounds__(32 * GF_MAX_WARPS) gemm_few_kernel(GemmArgs g, int passes) {
     extern __shared__ __align__(16) float gf_smem[];
     constexpr int STAGE = (32 + 4 * MR) * GT_LD;
+    pdl_wait();
     const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int e = blockIdx.y / passes;
     const int m0 = (g.group_offsets ? g.group_offsets[e] : 0) + (blockIdx.y % passes) * MR;
@@ -342,8 +343,8 @@ static int launch_few(const GemmArgs& g, cudaStream_t stream) {
     // (the same limit whatever the size: another thread's launch, or a captured one, must not find it lowered)
     if (cudaFuncSetAttribute(gemm_few_kernel<MR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess)
         return SHARPI_LAUNCH_FAILED;
-    gemm_few_kernel<MR><<<dim3((unsigned)((g.N + GF_N - 1) / GF_N), (unsigned)(passes * g.E)), 32 * warps, smem, stream>>>(g, passes);
-    SHARPI_CHECK_LAUNCH();
+    // (its set-up beside the tail of the kernel before it: the float32 decode step is a chain of 20 launches of 3 to 15 us)
+    SHARPI_LAUNCH_PDL(gemm_few_kernel<MR>, dim3((unsigned)((g.N + GF_N - 1) / GF_N), (unsigned)(passes * g.E)), 32 * warps, smem, stream, g, passes);
     return SHARPI_OK;
 }
 
