@@ -373,21 +373,21 @@ __global__ void __launch_bounds__(DEC_THREADS, 3) attn_decode_split_kernel(const
     }
 }
 
-// One block per (row, query head): the row's partials, weighted by exp2(max_s - max) and normalised.  A warp
-// takes one split at a time (its D floats are one coalesced read, four per lane) and every n-th (n warps a block)
-// split after it, several loads in flight; the warps' sums are then added in warp order, so the result
-// depends on the row's position alone.
-constexpr int MERGE_WARPS = 32;          // at most; the launch takes half of them for rows of few splits
-constexpr int MERGE_THREADS = MERGE_WARPS * 32;
-constexpr int MERGE_UNROLL = 4;
-constexpr int MERGE_WIDE_FROM = 256;     // splits from which a block of MERGE_WARPS warps pays
+// One block per (row, query head): the row's partials, weighted by exp2(max_s - max) and normalised.  The splits are dealt to
+// `PARTS` parts, split s to part s % PARTS; a part is one sum in ascending order (a split's D floats are one coalesced read of a warp,
+// four per lane), and the parts are then added in order, so the result depends on the row's position alone.  PARTS is 16, for rows of
+// MERGE_WIDE_FROM splits and more 32; a warp has 4 parts, or 1, of which it asks for 2 splits each at once.  64 rows of 40 heads, 20
+// splits each: 14 us behind the
+// splits with four loads a part under way and a third of the blocks, 10 us so; blocks of 512 threads, a warp a part, that met twice for
+// the maximum took 18.
+constexpr int MERGE_UNROLL = 2;
+constexpr int MERGE_WIDE_FROM = 256;
 
-template <int D>
-__global__ void __launch_bounds__(MERGE_THREADS) attn_decode_merge_kernel(DecodeArgs a) {
+template <int D, int PARTS, int PER_WARP>
+__global__ void __launch_bounds__(PARTS / PER_WARP * 32) attn_decode_merge_kernel(DecodeArgs a) {
     static_assert(D % 4 == 0 && D <= 128, "a warp reads a split's D floats four per lane");
-    __shared__ float4 acc_s[MERGE_WARPS][D / 4];
-    __shared__ float l_s[MERGE_WARPS];
-    __shared__ float scratch[32];
+    __shared__ float4 acc_s[PARTS][D / 4];
+    __shared__ float l_s[PARTS];
     pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ri = blockIdx.x, head = blockIdx.y;
@@ -395,43 +395,58 @@ __global__ void __launch_bounds__(MERGE_THREADS) attn_decode_merge_kernel(Decode
     const int pos = a.positions[r];
     const int lo = visible_lo(pos, a.mask_kind, a.mask_span);
     const int n_s = pos / DEC_SPLIT - lo / DEC_SPLIT + 1;
-    // how many warps share a row is a matter of the row alone (the block may have more), as the order of the sum
-    const int warps = n_s >= MERGE_WIDE_FROM ? MERGE_WARPS : MERGE_WARPS / 2;
+    // how many parts share a row is a matter of the row alone (the launch goes by the longest one)
+    const int parts = n_s >= MERGE_WIDE_FROM ? 32 : 16;
     const size_t slot0 = ((size_t)ri * a.nq + head) * a.max_splits;
     const float2* ml = reinterpret_cast<const float2*>(a.part_ml) + slot0;
-    float m = -INFINITY;
-    for (int s = threadIdx.x; s < n_s; s += blockDim.x) m = fmaxf(m, ml[s].x);
-    // a sink is one more term of the denominator, exp2(sink - M), with M the larger of the sink and every split's maximum
-    const float sink = a.sinks ? a.sinks[head] * 1.4426950408889634f : -INFINITY;
-    const float M = fmaxf(block_max(m, scratch), sink);
     const bool active = lane < D / 4;
     const float4* po = reinterpret_cast<const float4*>(a.part_o + slot0 * D) + (active ? lane : 0);
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    float l = 0.0f;
-    for (int s0 = warp; s0 < n_s && warp < warps; s0 += warps * MERGE_UNROLL) {
-        float2 st[MERGE_UNROLL];
-        float4 v[MERGE_UNROLL];
+    float2 st[PER_WARP][MERGE_UNROLL];
+    float4 v[PER_WARP][MERGE_UNROLL];
+    auto load = [&](int s0) {
 #pragma unroll
-        for (int u = 0; u < MERGE_UNROLL; ++u) {
-            const int s = s0 + u * warps;
-            const bool ok = s < n_s;
-            st[u] = ok ? ml[s] : make_float2(-INFINITY, 0.0f);
-            v[u] = ok ? po[(size_t)s * (D / 4)] : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
+        for (int q = 0; q < PER_WARP; ++q)
 #pragma unroll
-        for (int u = 0; u < MERGE_UNROLL; ++u) {
-            const float w = exp2f(st[u].x - M);       // 0 for the splits past the end
-            l += w * st[u].y;
-            acc.x += w * v[u].x; acc.y += w * v[u].y; acc.z += w * v[u].z; acc.w += w * v[u].w;
-        }
+            for (int u = 0; u < MERGE_UNROLL; ++u) {
+                const int part = warp * PER_WARP + q, s = s0 + part + u * parts;
+                const bool ok = s < n_s && part < parts;
+                st[q][u] = ok ? ml[s] : make_float2(-INFINITY, 0.0f);
+                v[q][u] = ok ? po[(size_t)s * (D / 4)] : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+    };
+    load(0);
+    float m = -INFINITY;
+    for (int s = lane; s < n_s; s += 32) m = fmaxf(m, ml[s].x);
+    // a sink is one more term of the denominator, exp2(sink - M), with M the larger of the sink and every split's maximum
+    const float sink = a.sinks ? a.sinks[head] * 1.4426950408889634f : -INFINITY;
+    const float M = fmaxf(warp_max(m), sink);
+    float4 acc[PER_WARP];
+    float l[PER_WARP];
+#pragma unroll
+    for (int q = 0; q < PER_WARP; ++q) { acc[q] = make_float4(0.f, 0.f, 0.f, 0.f); l[q] = 0.0f; }
+    for (int s0 = 0; s0 < n_s;) {
+#pragma unroll
+        for (int q = 0; q < PER_WARP; ++q)
+#pragma unroll
+            for (int u = 0; u < MERGE_UNROLL; ++u) {
+                const float w = exp2f(st[q][u].x - M);       // 0 for the splits past the end
+                l[q] += w * st[q][u].y;
+                acc[q].x += w * v[q][u].x; acc[q].y += w * v[q][u].y; acc[q].z += w * v[q][u].z; acc[q].w += w * v[q][u].w;
+            }
+        s0 += parts * MERGE_UNROLL;
+        if (s0 < n_s) load(s0);
     }
-    if (active && warp < warps) acc_s[warp][lane] = acc;
-    if (lane == 0 && warp < warps) l_s[warp] = l;
+#pragma unroll
+    for (int q = 0; q < PER_WARP; ++q) {
+        const int part = warp * PER_WARP + q;
+        if (active && part < parts) acc_s[part][lane] = acc[q];
+        if (lane == 0 && part < parts) l_s[part] = l[q];
+    }
     __syncthreads();
     if (threadIdx.x < D / 4) {
         float4 o = acc_s[0][threadIdx.x];
         float L = l_s[0] + (a.sinks ? exp2f(sink - M) : 0.0f);
-        for (int w = 1; w < warps; ++w) {
+        for (int w = 1; w < parts; ++w) {
             const float4 t = acc_s[w][threadIdx.x];
             o.x += t.x; o.y += t.y; o.z += t.z; o.w += t.w;
             L += l_s[w];
@@ -487,8 +502,8 @@ static int launch_decode(const DecodeArgs& a, int R, int splits, int items, long
         rc = launch_split<D, false>(map, a, R, splits, items, stream);
     }
     if (rc != SHARPI_OK || splits == 1) return rc;          // nothing to merge (2.6 us less a layer in a decode step at batch 1)
-    SHARPI_LAUNCH_PDL(attn_decode_merge_kernel<D>, dim3(R, a.nq), splits >= MERGE_WIDE_FROM ? MERGE_THREADS : MERGE_THREADS / 2, 0,
-                      stream, a);
+    if (splits >= MERGE_WIDE_FROM) SHARPI_LAUNCH_PDL((attn_decode_merge_kernel<D, 32, 1>), dim3(R, a.nq), 32 * 32, 0, stream, a);
+    else SHARPI_LAUNCH_PDL((attn_decode_merge_kernel<D, 16, 4>), dim3(R, a.nq), 4 * 32, 0, stream, a);
     return SHARPI_OK;
 }
 
