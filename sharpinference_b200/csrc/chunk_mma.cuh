@@ -260,6 +260,7 @@ __global__ void __launch_bounds__(THREADS, 2) sums_kernel(Args a, F f) {
     bf16* v_s = k_s + 3 * PLANE_K;
     float* raw = reinterpret_cast<float*>(v_s + 3 * PLANE_V);
     __shared__ float tail_s[ROWS], block_s[ROWS / BLOCK];
+    pdl_wait();
     Place p;
     if (!find_chunk(a.row_offsets, a.B, a.least, blockIdx.z, p)) return;
     const int kh = blockIdx.y, per = a.heads / a.key_heads, tiles = (a.dv + COLS - 1) / COLS;
@@ -347,6 +348,7 @@ __global__ void __launch_bounds__(THREADS, 2) sums_kernel(Args a, F f) {
 // the normaliser, a thread an element.
 template <class F>
 __global__ void __launch_bounds__(CARRY_THREADS) carry_kernel(Args a, F f) {
+    pdl_wait();
     const int b = blockIdx.z, h = blockIdx.y, rows = a.row_offsets[b + 1] - a.row_offsets[b];
     if (rows < a.least) return;
     const int base = chunks_before(a.row_offsets, b, a.least);
@@ -403,6 +405,7 @@ __global__ void __launch_bounds__(THREADS, 2) outs_kernel(Args a, F f) {
     float* raw = reinterpret_cast<float*>(v_s + 3 * PLANE_V);   // the next tile's values
     float* D_s = raw + ROWS * COLS;                            // [block][16][LD_D]: D inside a block
     __shared__ float head_s[ROWS], tail_s[ROWS], block_s[ROWS / BLOCK];   // decays from a block's first row up to a row; block_tails
+    pdl_wait();
     Place p;
     if (!find_chunk(a.row_offsets, a.B, a.least, blockIdx.z, p)) return;
     const int kh = blockIdx.y, per = a.heads / a.key_heads, tiles = (a.dv + COLS - 1) / COLS;
@@ -624,13 +627,11 @@ static int launch(Args a, const F& f, int chunks, cudaStream_t stream) {
         if (g == 1 || cost < best) { best = cost; a.group = g; }
     }
     const dim3 grid((tiles + a.group - 1) / a.group, a.key_heads, chunks);
-    sums_kernel<F, DP><<<grid, THREADS, smem_sums, stream>>>(a, f);
-    SHARPI_CHECK_LAUNCH();
+    // (each may start beside the tail of the one before: 2 us less a kernel)
+    SHARPI_LAUNCH_PDL((sums_kernel<F, DP>), grid, THREADS, smem_sums, stream, a, f);
     const dim3 carry((a.d * a.dv / 4 + CARRY_THREADS - 1) / CARRY_THREADS + (F::NORM ? 1 : 0), a.heads, a.B);
-    carry_kernel<F><<<carry, CARRY_THREADS, 0, stream>>>(a, f);
-    SHARPI_CHECK_LAUNCH();
-    outs_kernel<F, DP><<<grid, THREADS, smem_outs, stream>>>(a, f);
-    SHARPI_CHECK_LAUNCH();
+    SHARPI_LAUNCH_PDL(carry_kernel<F>, carry, CARRY_THREADS, 0, stream, a, f);
+    SHARPI_LAUNCH_PDL((outs_kernel<F, DP>), grid, THREADS, smem_outs, stream, a, f);
     return SHARPI_OK;
 }
 

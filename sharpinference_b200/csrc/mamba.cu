@@ -116,6 +116,7 @@ causal_conv_rows_kernel(const float* in, int ld, const float* __restrict__ w, co
 __global__ void __launch_bounds__(256)
 causal_conv_state_kernel(const float* in, int ld, float* state, long long state_stride, const int* row_offsets,
                          const int* state_slots, int C, int taps) {
+    pdl_wait();
     const int b = blockIdx.y;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C) return;
@@ -159,9 +160,8 @@ SHARPI_API int sharpi_causal_conv(const float* in, int ld, const float* w, const
         SHARPI_LAUNCH_PDL(causal_conv_kernel<bf16>, grid, 256, 0, stream, in, ld, w, bias, (const float*)state,
                           state_stride, row_request, row_offsets, state_slots, x32, (bf16*)xact, C, taps, gate);
     if (taps > 1) {
-        causal_conv_state_kernel<<<dim3((C + 255) / 256, B), 256, 0, stream>>>(in, ld, state, state_stride, row_offsets,
-                                                                               state_slots, C, taps);
-        SHARPI_CHECK_LAUNCH();
+        SHARPI_LAUNCH_PDL(causal_conv_state_kernel, dim3((C + 255) / 256, B), 256, 0, stream, in, ld, state, state_stride, row_offsets,
+                          state_slots, C, taps);
     }
     return SHARPI_OK;
 }
@@ -617,6 +617,7 @@ __global__ void __launch_bounds__(SC_THREADS, 5) scan_sums_kernel(ScanChunks q) 
     __shared__ __align__(16) float B_s[SC_ROWS * NP];
     __shared__ float ring_s[2 * SC_AHEAD * 2 * SC_THREADS];
     const ScanArgs& a = q.s;
+    pdl_wait();
     chunked::Place p;
     if (!chunked::find_chunk<SC_ROWS>(a.row_offsets, q.B, q.least, blockIdx.y, p)) return;
     scan_stage<NP>(a, p, a.col_b, B_s);
@@ -679,6 +680,7 @@ __global__ void __launch_bounds__(SC_THREADS, 5) scan_sums_kernel(ScanChunks q) 
 
 __global__ void __launch_bounds__(256) scan_carry_kernel(ScanChunks q) {
     const ScanArgs& a = q.s;
+    pdl_wait();
     const int b = blockIdx.y, rows = a.row_offsets[b + 1] - a.row_offsets[b];
     if (rows < q.least) return;
     const int base = chunked::chunks_before<SC_ROWS>(a.row_offsets, b, q.least), n = (rows + SC_ROWS - 1) / SC_ROWS;
@@ -716,6 +718,7 @@ __global__ void __launch_bounds__(SC_THREADS, 5) scan_outs_kernel(ScanChunks q) 
     __shared__ __align__(16) float B_s[SC_ROWS * NP], C_s[SC_ROWS * NP];
     __shared__ float ring_s[2 * SC_AHEAD * 3 * SC_THREADS];
     const ScanArgs& a = q.s;
+    pdl_wait();
     chunked::Place p;
     if (!chunked::find_chunk<SC_ROWS>(a.row_offsets, q.B, q.least, blockIdx.y, p)) return;
     scan_stage<NP>(a, p, a.col_b, B_s);
@@ -770,12 +773,9 @@ __global__ void __launch_bounds__(SC_THREADS, 5) scan_outs_kernel(ScanChunks q) 
 template <typename TO, int NP, bool RAW>
 static int launch_scan_chunks(const ScanChunks& q, int chunks, cudaStream_t stream) {
     const dim3 grid((q.s.C + SC_THREADS - 1) / SC_THREADS, chunks);
-    scan_sums_kernel<NP, RAW><<<grid, SC_THREADS, 0, stream>>>(q);
-    SHARPI_CHECK_LAUNCH();
-    scan_carry_kernel<<<dim3((unsigned)(((long long)q.s.C * q.s.N + 255) / 256), q.B), 256, 0, stream>>>(q);
-    SHARPI_CHECK_LAUNCH();
-    scan_outs_kernel<TO, NP, RAW><<<grid, SC_THREADS, 0, stream>>>(q);
-    SHARPI_CHECK_LAUNCH();
+    SHARPI_LAUNCH_PDL((scan_sums_kernel<NP, RAW>), grid, SC_THREADS, 0, stream, q);
+    SHARPI_LAUNCH_PDL(scan_carry_kernel, dim3((unsigned)(((long long)q.s.C * q.s.N + 255) / 256), q.B), 256, 0, stream, q);
+    SHARPI_LAUNCH_PDL((scan_outs_kernel<TO, NP, RAW>), grid, SC_THREADS, 0, stream, q);
     return SHARPI_OK;
 }
 

@@ -84,6 +84,7 @@ __device__ __forceinline__ void store_coef(const MlstmArgs& a, int t, int h, flo
 }
 
 __global__ void __launch_bounds__(32) mlstm_gates_kernel(MlstmArgs a) {
+    pdl_wait();
     const int b = blockIdx.x, h = blockIdx.y, lane = threadIdx.x;
     const int r0 = a.row_offsets[b], r1 = a.row_offsets[b + 1];
     if (r1 <= r0) return;
@@ -115,6 +116,7 @@ constexpr int GATE_ROWS = 128;
 __global__ void __launch_bounds__(GATE_ROWS + 32) mlstm_gates_long_kernel(MlstmArgs a) {
     __shared__ __align__(16) float2 gates_s[3][GATE_ROWS];     // (forget, input): the rows before, of now, after
     __shared__ __align__(16) float m_s[2][GATE_ROWS + 4];      // [3]: the maximum before the first row; [4 + j]: behind row j
+    pdl_wait();
     const int b = blockIdx.x, h = blockIdx.y, row = (int)threadIdx.x - 32;
     const int r0 = a.row_offsets[b], r1 = a.row_offsets[b + 1];
     if (r1 <= r0) return;
@@ -404,8 +406,8 @@ SHARPI_API int sharpi_mlstm_recurrence(const float* proj, int ld, int col_q, int
     a.state = state; a.state_stride = state_stride; a.head_stride = head_stride; a.heads = heads; a.d = d; a.dv = dv;
     a.slices = (dv + 31) / 32; a.cap = cap; a.q_scale = q_scale; a.coef = coef; a.o_raw = o_raw; a.nq = nq; a.skip = 0x7fffffff;
     if ((long long)head_stride < (long long)a.slices * d * 32 + d + 1) return SHARPI_BAD_ARGUMENT;
-    if (T - B + 1 > 32) mlstm_gates_long_kernel<<<dim3(B, heads), GATE_ROWS + 32, 0, stream>>>(a);
-    else mlstm_gates_kernel<<<dim3(B, heads), 32, 0, stream>>>(a);
+    if (T - B + 1 > 32) SHARPI_LAUNCH_PDL(mlstm_gates_long_kernel, dim3(B, heads), GATE_ROWS + 32, 0, stream, a);
+    else SHARPI_LAUNCH_PDL(mlstm_gates_kernel, dim3(B, heads), 32, 0, stream, a);
     SHARPI_CHECK_LAUNCH();
     if (sums) {
         if (least < 1 || (reinterpret_cast<uintptr_t>(state) & 15) != 0 || state_stride % 4 != 0 || head_stride % 4 != 0)
