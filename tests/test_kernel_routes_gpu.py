@@ -143,3 +143,29 @@ def test_product_a_head_with_the_heads_minor(ops, E, T, N, K, ld):
     wide[..., :K] = a.view(E, T, K).transpose(0, 1)
     again = torch.empty(T, E, N, dtype=torch.bfloat16, device=DEV)
     assert torch.equal(ops.tc_per_head(wide, w, T, again), want)
+
+
+# every lane count, value columns behind the last block's and of several blocks, states behind the last lane's, several groups
+@pytest.mark.parametrize("heads,groups,N,P", [(4, 1, 128, 64), (6, 3, 100, 36), (2, 2, 20, 100), (3, 1, 64, 4)])
+def test_state_space_duality_step_is_the_walk(ops, heads, groups, N, P):
+    """Rows that come one a step give the bits of the same rows in one portion, in the outputs and in the state."""
+    B, rows, inner = 5, 3, heads * P
+    xbc, dt = rnd(B * rows, inner + 2 * groups * N, seed=1), rnd(B * rows, heads, seed=2)
+    kw = dict(col_x=0, col_b=inner, col_c=inner + groups * N, col_dt=0, dt_bias=rnd(heads, seed=3) - 2, a_log=rnd(heads, seed=4),
+              dskip=rnd(heads, seed=5), heads=heads, groups=groups, states=N, vdim=P)
+    slots = torch.tensor([3, 0, 4, 1, 2], dtype=torch.int32, device=DEV)
+    whole = rnd(B, heads * N * P, seed=6)
+    single = whole.clone()
+    y = ops.ssd_scan(xbc, dt, row_offsets=torch.arange(B + 1, dtype=torch.int32, device=DEV) * rows, state_slots=slots, state=whole, **kw)
+    for r in range(rows):
+        at = torch.arange(B, device=DEV) * rows + r
+        one = ops.ssd_scan(xbc[at].contiguous(), dt[at].contiguous(), row_offsets=torch.arange(B + 1, dtype=torch.int32, device=DEV),
+                           state_slots=slots, state=single, **kw)
+        assert torch.equal(one, y[at]), r
+    assert torch.equal(single, whole)
+    # as many rows as requests, dealt otherwise: one request has two, another none
+    off = torch.tensor([0, 2, 2, 3, 4, 5], dtype=torch.int32, device=DEV)
+    a, b = whole.clone(), whole.clone()
+    got = ops.ssd_scan(xbc[:5], dt[:5], row_offsets=off, state_slots=slots, state=a, **kw)
+    want = ops.ssd_scan(xbc[:2], dt[:2], row_offsets=off[:2].contiguous(), state_slots=slots[:1], state=b, **kw)
+    assert torch.equal(got[:2], want) and torch.equal(a[3], b[3]) and torch.equal(a[0], whole[0])
