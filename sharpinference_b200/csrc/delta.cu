@@ -155,6 +155,14 @@ __global__ void __launch_bounds__(PREP_WARPS * 32) delta_prep_kernel(PrepArgs a)
     // move on now.  Every lane rewrites the channels it read.
     if (i0 == 0 && K > 0) {
         const int total = a.row_offsets[req + 1] - portion;
+        if (TAPS > 1 && rows == total) {                       // the window behind the last row is the state: nothing to read again
+#pragma unroll
+            for (int k = 0; k < WIN; ++k)
+#pragma unroll
+                for (int j = 0; j < NPL; ++j)
+                    if (lane + 32 * j < n) st[(size_t)k * a.C + c0 + lane + 32 * j] = win[k][j];
+            return;
+        }
         for (int j = 0; j < K; ++j)
             for (int e = lane; e < n; e += 32) {
                 const int i = total - K + j;                   // ascending j: place j + total is read before it is written

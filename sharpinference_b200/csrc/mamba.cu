@@ -122,6 +122,18 @@ causal_conv_state_kernel(const float* in, int ld, float* state, long long state_
     if (c >= C) return;
     const int first = row_offsets[b], n = row_offsets[b + 1] - first, K = taps - 1;
     float* st = state + (size_t)state_slots[b] * state_stride;
+    if (K <= 3) {                                      // read before the first store: a load behind one waits for it
+        float v[3];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const int src = n - K + j;
+            if (j < K) v[j] = src >= 0 ? in[(size_t)(first + src) * ld + c] : st[(size_t)(j + n) * C + c];
+        }
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+            if (j < K) st[(size_t)j * C + c] = v[j];
+        return;
+    }
     for (int j = 0; j < K; ++j) {                      // ascending: st[j + n] is read before it is overwritten
         const int src = n - K + j;
         st[(size_t)j * C + c] = src >= 0 ? in[(size_t)(first + src) * ld + c] : st[(size_t)(j + n) * C + c];
