@@ -507,7 +507,8 @@ static int launch_scan(const ScanArgs& a, int B, int T, int longest, cudaStream_
     const int NP = a.N <= 4 ? 4 : a.N <= 8 ? 8 : a.N <= 16 ? 16 : a.N <= 32 ? 32 : a.N <= 64 ? 64 : a.N <= 128 ? 128 : 256;
     // Rows to walk and fewer warps (of eight states a lane) than schedulers: two states a lane.  us, two split / four / eight
     // states a lane, 4096 channels of 16 states: one prompt of 2048 rows 152 / 296 / 455; two of 1024 133 / 165 / 230; three of
-    // 683 140 / 126 / 173; eight of 2048 909 / 765 / 1015.  Single rows (the state streams through): 200 requests 240 / 63 / 45.
+    // 683 140 / 126 / 173; eight of 2048 909 / 765 / 1015.  Single rows (the state streams through; of 16 states
+    // they have a kernel of their own where the strides allow 16-byte loads): 200 requests 240 / 63 / 45.
     // More than 16 states are more than 8 lanes of two, whose rows are walked and summed one by one: one prompt of 2048 rows, two /
     // eight states a lane, 2048 channels of 64 states 915 / 357, 1024 of 128 948 / 510, 4096 of 32 490 / 405.
     // Requests count as walks by their rows over those of the longest.  Every request, a single row too, costs a set of blocks
@@ -802,6 +803,74 @@ static int launch_scan_chunks(const ScanChunks& q, int chunks, cudaStream_t stre
                       : q.s.N <= 8 ? launch_scan_chunks<TO, 8>(q, chunks, stream) : launch_scan_chunks<TO, 16>(q, chunks, stream);
 }
 
+// Steps that bring about a row a request, 16 states a channel: the states' bytes and little else.  A warp is 32 channels of a
+// request; four lanes own four channels, four neighbouring states of each (a warp's load is 512 contiguous bytes), and what a
+// channel needs once a row (step size, gate, output) is formed by one of the four.  The operations of a channel and their order
+// are the walk's.  4096 channels: 200 requests 48 us with the walk (its blocks stage, prepare and meet for one row), 21 us so
+// (31 where every lane formed all of its channels' step sizes); 20 requests 8.4 and 4.1.  Two or four requests a warp, for one
+// set of decay rates: 22 us.
+constexpr int SS_THREADS = 128;
+
+template <typename TO, bool RAW>
+__global__ void __launch_bounds__(SS_THREADS) scan_step_kernel(ScanArgs a) {
+    constexpr int U = 4;                                   // channels of four lanes: c0, c0 + 8, c0 + 16 and c0 + 24
+    const int lane = threadIdx.x & 31, sub = lane % 4, c0 = (blockIdx.x * (SS_THREADS / 32) + (threadIdx.x >> 5)) * 8 * U + lane / 4;
+    const int own = c0 + 8 * sub, own_c = min(own, a.C - 1), b = blockIdx.y;
+    float4 A[U], S[U];
+    auto live = [&](int u) { return c0 + 8 * u < a.C; };
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const float4 l = *reinterpret_cast<const float4*>(a.a_log + (size_t)min(c0 + 8 * u, a.C - 1) * 16 + 4 * sub);
+        A[u] = make_float4(-expf(l.x) * 1.4426950408889634f, -expf(l.y) * 1.4426950408889634f, -expf(l.z) * 1.4426950408889634f,
+                           -expf(l.w) * 1.4426950408889634f);
+    }
+    const float bias = RAW ? a.dt_bias[own_c] : 0.0f, dsk = a.dskip[own_c];
+    pdl_wait();
+    const int first = a.row_offsets[b], end = a.row_offsets[b + 1];
+    if (first >= end || end - first >= a.skip) return;
+    float* st = a.state + (size_t)a.state_slots[b] * a.state_stride + (size_t)c0 * 16 + 4 * sub;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+        S[u] = live(u) ? *reinterpret_cast<const float4*>(st + u * 128) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int t = first; t < end; ++t) {
+        const float4 Bn = *reinterpret_cast<const float4*>(a.bc + (size_t)t * a.ld_bc + a.col_b + 4 * sub);
+        const float4 Cn = *reinterpret_cast<const float4*>(a.bc + (size_t)t * a.ld_bc + a.col_c + 4 * sub);
+        const float x = a.x[(size_t)t * a.C + own_c], z = a.z[(size_t)t * a.ld_z + own_c];
+        float d_own = a.dtraw[(size_t)t * a.C + own_c], y = 0.0f;
+        if (RAW) {
+            const float v = d_own + bias;
+            d_own = v > 20.0f ? v : log1pf(expf(v));
+        }
+        const float dx_own = d_own * x;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const float d = __shfl_sync(0xffffffffu, d_own, u, 4), dx = __shfl_sync(0xffffffffu, dx_own, u, 4);
+            S[u].x = fmaf(ex2_approx(d * A[u].x), S[u].x, __fmul_rn(dx, Bn.x));
+            S[u].y = fmaf(ex2_approx(d * A[u].y), S[u].y, __fmul_rn(dx, Bn.y));
+            S[u].z = fmaf(ex2_approx(d * A[u].z), S[u].z, __fmul_rn(dx, Bn.z));
+            S[u].w = fmaf(ex2_approx(d * A[u].w), S[u].w, __fmul_rn(dx, Bn.w));
+            // pairs of states, then the tree over the eight pairs (this lane has 2 sub and 2 sub + 1)
+            float p0 = fmaf(S[u].y, Cn.y, __fmul_rn(S[u].x, Cn.x)), p1 = fmaf(S[u].w, Cn.w, __fmul_rn(S[u].z, Cn.z));
+            p0 += __shfl_xor_sync(0xffffffffu, p0, 2); p1 += __shfl_xor_sync(0xffffffffu, p1, 2);
+            p0 += __shfl_xor_sync(0xffffffffu, p0, 1); p1 += __shfl_xor_sync(0xffffffffu, p1, 1);
+            if (sub == u) y = p0 + p1;
+        }
+        if (own < a.C)
+            reinterpret_cast<TO*>(a.out)[(size_t)t * a.C + own] = from_float<TO>(fmaf(dsk, x, y) * (RAW ? silu_f(z) : z));
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+        if (live(u)) *reinterpret_cast<float4*>(st + u * 128) = S[u];
+}
+
+template <typename TO>
+static int launch_scan_step(const ScanArgs& a, int B, cudaStream_t stream) {
+    const dim3 grid((a.C + SS_THREADS - 1) / SS_THREADS, B);
+    if (a.dt_bias) SHARPI_LAUNCH_PDL((scan_step_kernel<TO, true>), grid, SS_THREADS, 0, stream, a);
+    else SHARPI_LAUNCH_PDL((scan_step_kernel<TO, false>), grid, SS_THREADS, 0, stream, a);
+    return SHARPI_OK;
+}
+
 // `longest`: the rows of the longest request, 0 where it is not known (a choice of kernels, no result depends on it).  `work`
 // (nullable; T * C + `chunks` * C * (N + 1) floats): requests of at least `least` rows run in chunks, `chunks` of them at most; the
 // others, and without it all, are walked (`walk` = 0: there are no others).
@@ -826,6 +895,11 @@ SHARPI_API int sharpi_selective_scan(const float* x, const float* dtraw, const f
         if (rc != SHARPI_OK || !walk) return rc;
         a.skip = least;
         if (longest >= least) longest = least - 1;
+    }
+    const uintptr_t bases = (uintptr_t)state | (uintptr_t)bc | (uintptr_t)a_log;
+    if (T <= B && longest <= SCAN_CH && N == 16 && state_stride % 4 == 0 && ld_bc % 4 == 0 && col_b % 4 == 0 && col_c % 4 == 0 && (bases & 15) == 0) {
+        if (out_dtype == SHARPI_F32) return launch_scan_step<float>(a, B, stream);
+        if (out_dtype == SHARPI_BF16) return launch_scan_step<bf16>(a, B, stream);
     }
     if (out_dtype == SHARPI_F32) return launch_scan<float>(a, B, T, longest, stream);
     if (out_dtype == SHARPI_BF16) return launch_scan<bf16>(a, B, T, longest, stream);

@@ -169,3 +169,30 @@ def test_state_space_duality_step_is_the_walk(ops, heads, groups, N, P):
     got = ops.ssd_scan(xbc[:5], dt[:5], row_offsets=off, state_slots=slots, state=a, **kw)
     want = ops.ssd_scan(xbc[:2], dt[:2], row_offsets=off[:2].contiguous(), state_slots=slots[:1], state=b, **kw)
     assert torch.equal(got[:2], want) and torch.equal(a[3], b[3]) and torch.equal(a[0], whole[0])
+
+
+@pytest.mark.parametrize("C,raw", [(256, True), (100, False), (33, True)])
+def test_selective_scan_step_is_the_walk(ops, C, raw):
+    """Rows that come one a step give the bits of the same rows in one portion, in the outputs and in the state."""
+    B, rows, N = 7, 3, 16
+    x, z, dt, bc = rnd(B * rows, C, seed=1), rnd(B * rows, C, seed=2), rnd(B * rows, C, seed=3), rnd(B * rows, 2 * N, seed=4)
+    dt = dt if raw else torch.nn.functional.softplus(dt - 3.0)
+    a_log, dsk, bias = rnd(C, N, seed=5), rnd(C, seed=6), rnd(C, seed=7) - 3.0
+    slots = torch.tensor([3, 0, 6, 4, 1, 2, 5], dtype=torch.int32, device=DEV)
+
+    def run(rows_of, off, sl, state):
+        return ops.selective_scan(x[rows_of].contiguous(), dt[rows_of].contiguous(), bc[rows_of].contiguous(), 0, N, a_log, dsk,
+                                  z[rows_of].contiguous(), 0, row_offsets=off, state_slots=sl, state=state, out_dtype=torch.float32,
+                                  dt_bias=bias if raw else None)
+    whole = rnd(B, C * N, seed=8)
+    single, first = whole.clone(), torch.arange(B + 1, dtype=torch.int32, device=DEV)
+    y = run(slice(0, B * rows), first * rows, slots, whole)
+    for r in range(rows):
+        at = torch.arange(B, device=DEV) * rows + r
+        assert torch.equal(run(at, first, slots, single), y[at]), r
+    assert torch.equal(single, whole)
+    # as many rows as requests, dealt otherwise: one request has two, another none
+    off = torch.tensor([0, 2, 2, 3, 4, 5, 6, 7], dtype=torch.int32, device=DEV)
+    a, b = whole.clone(), whole.clone()
+    got, want = run(slice(0, 7), off, slots, a), run(slice(0, 2), off[:2].contiguous(), slots[:1], b)
+    assert torch.equal(got[:2], want) and torch.equal(a[3], b[3]) and torch.equal(a[0], whole[0])
