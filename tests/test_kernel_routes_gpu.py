@@ -196,3 +196,35 @@ def test_selective_scan_step_is_the_walk(ops, C, raw):
     a, b = whole.clone(), whole.clone()
     got, want = run(slice(0, 7), off, slots, a), run(slice(0, 2), off[:2].contiguous(), slots[:1], b)
     assert torch.equal(got[:2], want) and torch.equal(a[3], b[3]) and torch.equal(a[0], whole[0])
+
+
+@pytest.mark.parametrize("d,dv", [(128, 256), (40, 36), (132, 64), (256, 32)])
+def test_matrix_memory_step_is_the_walk(ops, d, dv):
+    """Rows that come one a step give the bits of the same rows in one portion, in the outputs and in the state."""
+    B, rows, heads = 5, 3, 2
+    ld = heads * (2 * d + dv) + 4
+    proj, bias = rnd(B * rows, ld, seed=1), rnd(heads, seed=2)
+    slots = torch.tensor([3, 0, 4, 1, 2], dtype=torch.int32, device=DEV)
+    first = torch.arange(B + 1, dtype=torch.int32, device=DEV)
+    floats = ops.mlstm_state_floats(heads, d, dv)[1]
+
+    def run(part, off, sl, state):
+        return ops.mlstm_recurrence(part.contiguous(), col_q=0, col_k=heads * d, col_v=2 * heads * d, col_i=ld - 4, col_f=ld - 2,
+                                    bias_i=bias, bias_f=bias + 1.0, row_offsets=off, state_slots=sl, state=state, heads=heads,
+                                    d=d, dv=dv, cap=15.0, q_scale=d ** -0.5)
+    whole = torch.zeros(B, floats, device=DEV)
+    run(rnd(2 * B, ld, seed=3), first * 2, slots, whole)          # (a state that has seen rows)
+    single, dealt = whole.clone(), whole.clone()
+    want = run(proj, first * rows, slots, whole)
+    for r in range(rows):
+        at = torch.arange(B, device=DEV) * rows + r
+        for g, w in zip(run(proj[at], first, slots, single), want):
+            assert torch.equal(g[..., :3], w[at][..., :3]), r
+    assert torch.equal(single, whole)
+    # as many rows as requests, dealt otherwise: one request has two, another none
+    off = torch.tensor([0, 2, 2, 3, 4, 5], dtype=torch.int32, device=DEV)
+    before = dealt.clone()
+    got = run(proj[:5], off, slots, dealt)
+    alone = before.clone()
+    want = run(proj[:2], off[:2].contiguous(), slots[:1].contiguous(), alone)
+    assert torch.equal(got[0][:2], want[0]) and torch.equal(dealt[3], alone[3]) and torch.equal(dealt[0], before[0])
