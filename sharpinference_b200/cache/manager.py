@@ -138,6 +138,8 @@ class CacheManager:
         self.state_slots = FreeList(max_requests)
         self._schedule = list(schedule)
         self._no_pages: Dict[int, int] = {}
+        self.ordered = allocate and self.device.type == "cuda"      # whether work on the memory goes by streams
+        self._last_stream = None                                    # where work on it was launched last
 
         by_spec: Dict[CacheSpec, CacheGroup] = {}
         for index, entry in enumerate(self._schedule):
@@ -196,6 +198,19 @@ class CacheManager:
             slots.append(slot)
         return slots
 
+    # -- streams -------------------------------------------------------------------------
+    def follow_stream(self) -> None:
+        """Called before work on the cache's memory is launched.  Pages, states and a captured step's static buffers belong to no
+        stream, and the host does not wait for one step before it launches the next: work from another stream than the last
+        (each thread has a current one of its own) goes behind everything on that one, a caller's reads of the step's
+        result among it.  Work that stays on its stream waits for nothing."""
+        if not self.ordered:
+            return
+        stream = torch.cuda.current_stream(self.device)
+        if self._last_stream is not None and stream != self._last_stream:
+            stream.wait_stream(self._last_stream)
+        self._last_stream = stream
+
     # -- requests ------------------------------------------------------------------------
     def add_request(self, request_id: Hashable) -> RequestCache:
         if request_id in self.requests:
@@ -203,13 +218,12 @@ class CacheManager:
         if self.state_slots.free_count == 0:
             raise OutOfSlots(f"all {self.max_requests} state slots are held")
         slot = self.state_slots.take()
-        for state in self._entry_state.values():
-            state[slot].zero_()
-        for named in self._entry_named.values():
-            for state in named.values():
+        states = [*self._entry_state.values(), *(s for named in self._entry_named.values() for s in named.values()),
+                  *self.model_states.values()]
+        if states:
+            self.follow_stream()
+            for state in states:
                 state[slot].zero_()
-        for state in self.model_states.values():
-            state[slot].zero_()
         rc = RequestCache(request_id, slot, tables={g.index: [] for g in self.groups}, version=self._next_version())
         self.requests[request_id] = rc
         return rc

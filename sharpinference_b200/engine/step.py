@@ -293,6 +293,7 @@ class StepRunner:
         self._read_status(self.STEPS_AHEAD)
         self.validate(entries)
         self.cache.reserve([(e.request_id, len(e.tokens)) for e in entries])
+        self.cache.follow_stream()
         logits, done, num_tokens = None, False, sum(len(e.tokens) for e in entries)
         if (self.use_graphs and not (self.trace_router or self.trace_layers or self.trace_streams)
                 and num_tokens == len(entries)):

@@ -617,6 +617,40 @@ def test_graphs_give_the_bits_of_eager_steps_in_bfloat16(folders, name):
     assert torch.equal(rows[True], rows[False])
 
 
+def test_steps_on_alternating_streams_give_the_bits_of_one_stream(folders):
+    """Portions with nothing wanted and decode steps (eager, captured and replayed), none read by the host before the last: from two
+    streams in turn, which know nothing of one another, and from one."""
+    from sharpinference_b200 import StepEntry
+    cfg, _ = plain.load_folder(folders["A"])
+    toks = {f"d{i}": traces.random_tokens(cfg["vocab"], 400, seed=420 + i) for i in range(2)}
+    streams, rows = [torch.cuda.Stream(), torch.cuda.Stream()], []
+    for used in (streams[:1], streams):
+        eng = engine_for(folders["A"], "bfloat16", 2 * 448)
+        torch.cuda.synchronize()
+        got, turn = [], 0
+
+        def step(entries):
+            nonlocal turn
+            with torch.cuda.stream(used[turn % len(used)]):
+                lg = eng.forward_step(entries)
+                if lg is not None:
+                    got.append(lg.clone())
+            turn += 1
+        for rid, t in toks.items():
+            with torch.cuda.stream(used[turn % len(used)]):
+                eng.open_request(rid)
+            step([StepEntry(rid, t[:180], [])])
+            step([StepEntry(rid, t[180:380], [])])
+            turn += 1
+        for at in range(380, 399):
+            step([StepEntry(rid, [t[at]], [0]) for rid, t in toks.items()])
+        torch.cuda.synchronize()
+        eng.runner.flush_status()
+        assert eng.runner.graph_replays > 10
+        rows.append(torch.stack(got))
+    assert torch.equal(rows[0], rows[1])
+
+
 @pytest.mark.parametrize("name", sorted(CASES))
 def test_greedy_generation_through_the_scheduler(folders, name):
     """``Engine.generate``: admission, portions under a small token budget, decoding in one batch, sampling (greedy) and the
