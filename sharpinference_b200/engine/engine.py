@@ -169,7 +169,9 @@ class Engine:
         self.cache.free_request(request_id)
 
     def forward_step(self, entries: Sequence[StepEntry]) -> Optional[torch.Tensor]:
-        """One step of the step function: float32 logits [wanted, vocab] on the device."""
+        """One step of the step function: float32 logits [wanted, vocab] on the device.  The host does not wait for the step: a
+        kernel that gave up raises at the call after the logits were read, or, where nothing is read between steps, at the
+        call after that or at ``runner.flush_status()``."""
         return self.runner.run(entries)
 
     # -- requests ----------------------------------------------------------------------------

@@ -93,8 +93,8 @@ class StepRunner:
         # `trace_streams`: the whole residual stream [T, H] after every scheduled block, in `last_layer_streams`
         self.trace_streams = False
         self.last_layer_streams: list = []
-        # after every step, read the word in which a tensor-core kernel records a wait that gave up
-        # (a 4-byte copy; the step's result is read by the host right after anyway)
+        # behind every step, copy the word in which a tensor-core kernel records a wait that gave up to the host (4 bytes), where
+        # a later step or flush_status looks at it
         self.check_kernel_status = True
         self._status_host, self._status_events, self._status_pending = None, None, []
         self.last_router_choices: List[torch.Tensor] = []
@@ -255,7 +255,9 @@ class StepRunner:
     # behind every step and looked at when the next step begins, if that step has ended by then (a caller that read
     # its result knows that it has), at the latest when the one after begins, or when flush_status is called.  So the
     # host lays out and launches one step while the GPU is at work on the one before: a decode step of 4 layers of
-    # width 1024 at batch 1 took 173 us when the host waited first, 135 us so.  A kernel that gave up raises there.
+    # width 1024 at batch 1 took 173 us when the host waited first, 135 us so.  A kernel that gave up raises there: for a caller
+    # who reads a step's result before the next one, before anything of that one runs; for one who does not, after one
+    # more step may have run on what it left.
     STEPS_AHEAD = 1            # steps that may be under way when another one is launched
 
     def _note_status(self) -> None:
@@ -279,6 +281,7 @@ class StepRunner:
             self._status_events[place].synchronize()
             if int(self._status_host[place]) != 0:
                 self._status_pending.clear()
+                self.cache.follow_stream()          # (a step under way on another stream ends first)
                 ops.check_status(self.device)       # raises, and puts the word and the counters back to zero
 
     def flush_status(self) -> None:
@@ -289,7 +292,9 @@ class StepRunner:
     def run(self, entries: Sequence[StepEntry]) -> Optional[torch.Tensor]:
         """Run one step.  Returns float32 logits ``[wanted, vocab]`` on the device, in the order of
         the entries and of each entry's ``want`` (None if nothing was wanted).  Raises
-        :class:`OutOfPages` before anything ran if the pages for the step cannot all be had."""
+        :class:`OutOfPages` before anything ran if the pages for the step cannot all be had.  The step may still be under way
+        when this returns, and so may the step before it; if a kernel of either gives up on a wait, a later call or
+        :meth:`flush_status` raises, which a caller who does not read the logits between steps calls before trusting them."""
         self._read_status(self.STEPS_AHEAD)
         self.validate(entries)
         self.cache.reserve([(e.request_id, len(e.tokens)) for e in entries])
