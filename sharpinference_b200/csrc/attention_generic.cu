@@ -157,7 +157,7 @@ __global__ void paged_attention_generic_kernel(PagedAttnArgs a) {
 // elements.  The operations and their order are those of one CTA.  4 decode rows at 300 keys: 47 us with a CTA a row and key
 // head, 15.5 us so; at 4000 keys 555 and 103 us.
 // 980 rows of 4 requests, 8 heads on 2, head size 128: 556 -> 95 us (before: a block a row and head, one key a thread read
-// element by element); 
+// element by element).
 constexpr int AR_BK = 64, AR_THREADS = 128, AR_MAX_D = 256;
 
 typedef unsigned long long f32x2;
@@ -201,7 +201,7 @@ template <int R, int JJ, bool SPLIT>
 __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAttnArgs a, int heads_cta, int tokens) {
     static_assert(!SPLIT || R == 8, "a thread has four neighbouring elements of the cluster's sums at most");
     if (SPLIT) pdl_wait();
-    const int ctas = SPLIT ? (int)gridDim.z : 1, rank = SPLIT ? (int)blockIdx.z : 0;
+    const int rank = SPLIT ? (int)blockIdx.z : 0;
     extern __shared__ __align__(16) float ar_smem[];
     __shared__ long long off_s[2][AR_BK];                // where the keys of two tiles lie, -1: not there
     constexpr int RT = R / 8;                            // rows a thread
@@ -235,6 +235,14 @@ __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAtt
     const int b_first = lo_first / AR_BK, b_last = p_last / AR_BK;
     const int n_keep = min((keep + AR_BK - 1) / AR_BK, b_first);   // tiles with kept positions below the others
     const int n_iter = n_keep + b_last - b_first + 1;
+    // How many CTAs of the cluster share the tiles goes by the tiles that there are (the launch knows the block table's width, which a
+    // captured step pads, and no window): the others end here, where none of them has met another one yet.  Together they have four
+    // elements of the sums a thread; a single one keeps its sums to itself.  Rows of 30 keys on a table of 1024, without clusters / with
+    // all CTAs of eight going along / so: 8 heads on 2 of 128, one row 11.6 / 12.1 / 11.6, 16 rows 12.2 / 15.0 / 13.5; 16 heads on 4
+    // of 64, 16 rows 10.3 / 16.8 / 15.1 (what is left is the launch of CTAs that end).
+    const int ctas = !SPLIT || n_iter == 1 ? 1 : min((int)gridDim.z, max(n_iter, (d + 63) / 64));
+    if (rank >= ctas) return;
+    const bool shared = SPLIT && ctas > 1;
     auto key0_of = [&](int it) { return (it < n_keep ? it : b_first + it - n_keep) * AR_BK; };
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, tx = tid & 15, ty = tid >> 4;
@@ -276,7 +284,7 @@ __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAtt
 
     for (int it0 = 0; it0 < n_iter; it0 += ctas) {
         const int it = it0 + rank;
-        const bool have = !SPLIT || it < n_iter, more = it0 + ctas < n_iter;      // (a CTA without a tile in the last round goes along)
+        const bool have = !shared || it < n_iter, more = it0 + ctas < n_iter;      // (a CTA without a tile in the last round goes along)
         const int key0 = key0_of(have ? it : 0);
         const long long next = tid < AR_BK && it + ctas < n_iter ? place(it + ctas) : -1;      // arrives while the scores are formed
         if (a.kv_planes == 2) mma16::cp_async_wait<1>(); else mma16::cp_async_wait<0>();
@@ -324,7 +332,7 @@ __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAtt
         if (tid < AR_BK) off_s[side(it + ctas)][tid] = next;
         __syncthreads();                                 // the scores are here; keys are free
         if (a.kv_planes == 2 && more) load(k_s, it + ctas, 0);
-        if constexpr (SPLIT) {
+        if (SPLIT && shared) {
             float* p = p_s + (tid >> 2) * (AR_BK + 4) + (tid & 3) * 4;
             if (tid < 4 * R) {
                 float m = -INFINITY;
@@ -428,7 +436,7 @@ __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAtt
             if constexpr (R == 8) weigh(mixed);
             else if (mixed) weigh(std::true_type{});
             else weigh(std::false_type{});
-            if constexpr (SPLIT) {
+            if (SPLIT && shared) {
 #pragma unroll
                 for (int j = 0; j < JJ; ++j)
                     if (tx * 4 + 64 * j < d)
@@ -462,7 +470,7 @@ __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAtt
             if (a.kv_planes == 2) load(v_s, it + ctas, plane); else load(k_s, it + ctas, 0);
         }
     }
-    if constexpr (SPLIT) cluster_sync();                 // nobody reads this CTA's shared memory any more
+    if (SPLIT && shared) cluster_sync();                 // nobody reads this CTA's shared memory any more
     else __syncthreads();
     if (tid < 4 * R && (tid & 3) == 0) {
         float shrink = 1.0f;
@@ -479,7 +487,7 @@ __global__ void __launch_bounds__(AR_THREADS) attention_rows_f32_kernel(PagedAtt
         corr_s[r] = shrink / l_run;
     }
     __syncthreads();
-    if constexpr (SPLIT) {
+    if (SPLIT && shared) {
         if (unit_r < n_rows) {
             const float f = corr_s[unit_r];
             float* out = (float*)a.out + ((size_t)(t + unit_r / heads_here) * a.nq + head0 + unit_r % heads_here) * d;
@@ -548,7 +556,7 @@ static int launch_rows_f32(const PagedAttnArgs& a, int B, cudaStream_t stream) {
     const int per_sm = a.d <= 64 ? 6 : a.d <= 128 ? 3 : 1;
     if (ctas(8) > 148 * per_sm && 2 * ctas(8) > 5 * ctas(32)) return launch_rows_f32<32>(a, 1, stream);
     // CTAs of 8 rows that leave SMs empty share their tiles in clusters, as long as those fit two thirds of the places at once.  us,
-    // without / with clusters, 8 heads on 2, head size 128: one row at 30 keys 11.6 / 13.8, at 100 20.8 / 14.6; 16 rows at 400 65 / 18;
+    // without / with clusters, 8 heads on 2, head size 128: one row at 30 keys 11.6 / 11.6, at 100 20.8 / 13.0; 16 rows at 400 65 / 18;
     // 60 rows behind 300 57 / 30; 32 heads on 8, 16 rows at 2000 287 / 205; four portions of 40 rows behind 250 (pairs, three quarters
     // of the places) 65 / 67.
     const long long grid = (long long)a.T * a.nkv * ((G + 7) / 8);
