@@ -354,14 +354,14 @@ __global__ void __launch_bounds__(DEC_THREADS, 3) attn_decode_split_kernel(const
         for (int w = 0; w < DEC_WARPS; ++w) {
             const float mw = base_o[w * warp_stride + 16 * D + g * 2];
             const float f = (mw == -INFINITY) ? 0.0f : exp2f(mw - M);
-            acc += f * base_o[w * warp_stride + g * D + dd];
-            L += f * base_o[w * warp_stride + 16 * D + g * 2 + 1];
+            acc = __fmaf_rn(f, base_o[w * warp_stride + g * D + dd], acc);
+            L = __fmaf_rn(f, base_o[w * warp_stride + 16 * D + g * 2 + 1], L);
         }
-        if constexpr (ONE) {                 // as the merge forms it: the split's weight is 1, or next to a larger sink less
+        if constexpr (ONE) {                 // the merge's operations, each rounded as there: the split's weight is 1, or next to a larger sink less
             const float sink = a.sinks ? a.sinks[head0 + g] * 1.4426950408889634f : -INFINITY;
             const float top = fmaxf(M, sink), w = exp2f(M - top);
-            const float inv = 1.0f / (w * L + (a.sinks ? exp2f(sink - top) : 0.0f));
-            a.out[((size_t)r * a.nq + head0 + g) * D + dd] = __float2bfloat16_rn(w * acc * inv);
+            const float inv = 1.0f / __fadd_rn(__fmaf_rn(w, L, 0.0f), a.sinks ? exp2f(sink - top) : 0.0f);
+            a.out[((size_t)r * a.nq + head0 + g) * D + dd] = __float2bfloat16_rn(__fmul_rn(__fmaf_rn(w, acc, 0.0f), inv));
             continue;
         }
         const size_t slot = ((size_t)ri * a.nq + head0 + g) * a.max_splits + split_in_row;
@@ -430,8 +430,9 @@ __global__ void __launch_bounds__(PARTS / PER_WARP * 32) attn_decode_merge_kerne
 #pragma unroll
             for (int u = 0; u < MERGE_UNROLL; ++u) {
                 const float w = exp2f(st[q][u].x - M);       // 0 for the splits past the end
-                l[q] += w * st[q][u].y;
-                acc[q].x += w * v[q][u].x; acc[q].y += w * v[q][u].y; acc[q].z += w * v[q][u].z; acc[q].w += w * v[q][u].w;
+                l[q] = __fmaf_rn(w, st[q][u].y, l[q]);
+                acc[q].x = __fmaf_rn(w, v[q][u].x, acc[q].x); acc[q].y = __fmaf_rn(w, v[q][u].y, acc[q].y);
+                acc[q].z = __fmaf_rn(w, v[q][u].z, acc[q].z); acc[q].w = __fmaf_rn(w, v[q][u].w, acc[q].w);
             }
         s0 += parts * MERGE_UNROLL;
         if (s0 < n_s) load(s0);
@@ -445,7 +446,7 @@ __global__ void __launch_bounds__(PARTS / PER_WARP * 32) attn_decode_merge_kerne
     __syncthreads();
     if (threadIdx.x < D / 4) {
         float4 o = acc_s[0][threadIdx.x];
-        float L = l_s[0] + (a.sinks ? exp2f(sink - M) : 0.0f);
+        float L = __fadd_rn(l_s[0], a.sinks ? exp2f(sink - M) : 0.0f);
         for (int w = 1; w < parts; ++w) {
             const float4 t = acc_s[w][threadIdx.x];
             o.x += t.x; o.y += t.y; o.z += t.z; o.w += t.w;

@@ -129,6 +129,26 @@ def test_decode_rows_of_one_split_need_no_merge(ops, sinks):
             assert torch.allclose(full[r].view(nq, d)[h].double(), want, rtol=2e-2, atol=2e-2)
 
 
+# (two million outputs: a denominator that is rounded otherwise moves about one bfloat16 in 60000)
+@pytest.mark.parametrize("d,level", [(128, 6.0), (64, 2.0), (128, None)])
+def test_decode_rows_of_one_split_are_the_bits_of_the_merge(ops, d, level):
+    """Rows of up to 256 keys, most of them with sinks above their scores: alone, and in one launch with a longer row."""
+    nq, nkv, ps, n = 8, 2, 64, 2000 * 128 // d
+    kv, q = rnd(16, 2, nkv, ps, d, seed=1).bfloat16(), rnd(n + 1, nq, d, seed=2).bfloat16()
+    table = torch.arange(16, dtype=torch.int32, device=DEV).view(1, -1)
+    pos = torch.randint(0, 256, (n + 1,), generator=torch.Generator().manual_seed(3)).to(torch.int32).to(DEV)
+    pos[n] = 700
+    sink = None if level is None else rnd(nq, seed=4) + level
+
+    def run(rows, context):
+        out = torch.zeros(rows, nq * d, dtype=torch.bfloat16, device=DEV)
+        ops.attention_decode(q[:rows].contiguous(), kv, table, torch.zeros(rows, dtype=torch.int32, device=DEV), pos[:rows].contiguous(), out,
+                             rows=None, num_rows=rows, nq=nq, nkv=nkv, d=d, page_size=ps, mask_kind=0, mask_span=1, scale=d ** -0.5,
+                             max_context=context, sinks=sink)
+        return out
+    assert torch.equal(run(n, 256), run(n + 1, 701)[:n])
+
+
 # rows that fill a tile of activations and that do not, one and two weight tiles a CTA, output rows wider than the product, one head
 @pytest.mark.parametrize("E,T,N,K,ld", [(3, 6, 40, 64, 48), (2, 130, 256, 128, 320), (8, 257, 300, 72, 300), (1, 33, 128, 256, 128)])
 def test_product_a_head_with_the_heads_minor(ops, E, T, N, K, ld):
