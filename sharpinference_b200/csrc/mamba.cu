@@ -592,16 +592,22 @@ struct ScanRing {
     }
 };
 
-// softplus(v) = max(v, 0) + log(1 + w), w = exp(-|v|) in [0, 1]; log(1 + w) / w as the polynomial through its Chebyshev points of
-// degree 9 (5e-9 of the value; one unit in the last place with the roundings).  Two at a time.
+// softplus(v) = max(v, 0) + log(1 + w), w = exp(-|v|) in [0, 1]; log(1 + w) = w + w q, q = w Q(w), Q of degree 8 fitted by reweighted
+// least squares (Lawson's method), its coefficients rounded one after the other: 5e-9 of the value.  The large term joins in the last,
+// rounded once operation: w where v < 0, v where not.  Two at a time.  Error against 64 bits, here / log1pf(expf(v)) as the walk has
+// it: v in [-30, 0] 1.9e-7 / 1.8e-7 at most and the same root mean square (4e-8 to 5e-8 by range), v in [0, 1] 1.4e-7 / 1.3e-7 and 3.5e-8 /
+// 3.7e-8, above less than there.  2048 rows of 4096 channels: the chunks 111 us so, 116 with log1pf(expf(v)), 110 with ex2.approx of
+// v log2(e), whose argument is rounded once: 9e-7 off near v = -10.
 __device__ __forceinline__ f32x2 softplus2(float v0, float v1) {
-    constexpr float P[10] = {1.0f, -0.49999892711639404f, 0.33329710364341736f, -0.24951615929603577f, 0.1966327428817749f,
-                             -0.1526966691017151f, 0.10543623566627502f, -0.05637361481785774f, 0.019542528316378593f, -0.0031760570127516985f};
-    const f32x2 w = pair2(ex2_approx(fabsf(v0) * -1.4426950408889634f), ex2_approx(fabsf(v1) * -1.4426950408889634f));
-    f32x2 p = pair2(P[9], P[9]);
+    constexpr float Q[9] = {-0.4999993145465851f, 0.333304762840271f, -0.24958248436450958f, 0.19693760573863983f, -0.15350909531116486f,
+                            0.10673291236162186f, -0.057595446705818176f, 0.020169047638773918f, -0.0033108105417340994f};
+    const f32x2 w = pair2(expf(-fabsf(v0)), expf(-fabsf(v1)));
+    f32x2 q = pair2(Q[8], Q[8]);
 #pragma unroll
-    for (int i = 8; i >= 0; --i) p = fma2(p, w, pair2(P[i], P[i]));
-    return fma2(p, w, pair2(fmaxf(v0, 0.0f), fmaxf(v1, 0.0f)));
+    for (int i = 7; i >= 0; --i) q = fma2(q, w, pair2(Q[i], Q[i]));
+    q = mul2(q, w);
+    const float q0 = low2(q), q1 = high2(q);
+    return fma2(w, pair2(v0 < 0.0f ? q0 : 1.0f + q0, v1 < 0.0f ? q1 : 1.0f + q1), pair2(v0 < 0.0f ? low2(w) : v0, v1 < 0.0f ? high2(w) : v1));
 }
 
 // Columns col .. col + N - 1 of the chunk's rows of B or C, zeros behind N

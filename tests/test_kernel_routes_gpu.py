@@ -248,3 +248,22 @@ def test_matrix_memory_step_is_the_walk(ops, d, dv):
     alone = before.clone()
     want = run(proj[:2], off[:2].contiguous(), slots[:1].contiguous(), alone)
     assert torch.equal(got[0][:2], want[0]) and torch.equal(dealt[3], alone[3]) and torch.equal(dealt[0], before[0])
+
+
+@pytest.mark.parametrize("split", [False, True])
+def test_step_sizes_of_the_selective_scan(ops, split):
+    """softplus of raw step sizes in [-30, 30], walked and in chunks, against 64 bits.  Rates so large that nothing is carried and ones
+    elsewhere: an output is the step size times the gate, silu(64) = 64.  The bound is two units in the last place (2^-23 each at
+    worst): what an exponential and a logarithm of float32 may be off, or the exponential and the roundings behind it in chunks."""
+    T, C, N = 2048, 256, 16
+    v = (torch.rand(T, C, generator=torch.Generator().manual_seed(1)) * 60 - 30).to(DEV)
+    v[:1024] *= 0.25                                     # half of them in [-7.5, 7.5]
+    v[0, 0] = 0.0
+    bc = torch.zeros(T, 2 * N, device=DEV)
+    bc[:, 0] = bc[:, N] = 1.0
+    ones, off = torch.ones(T, C, device=DEV), torch.tensor([0, T], dtype=torch.int32, device=DEV)
+    y = ops.selective_scan(ones, v, bc, 0, N, torch.full((C, N), 80.0, device=DEV), torch.zeros(C, device=DEV), 64.0 * ones, 0,
+                           row_offsets=off, state_slots=off[:1], state=torch.zeros(1, C * N, device=DEV), out_dtype=torch.float32,
+                           dt_bias=torch.zeros(C, device=DEV), max_rows=T, split=split)
+    want = torch.clamp(v.double(), min=0) + torch.log1p(torch.exp(-v.double().abs()))
+    assert float(((y.double() / 64 - want) / want).abs().max()) < 2 * 2.0 ** -23
