@@ -110,7 +110,8 @@ __global__ void __launch_bounds__(32) mlstm_gates_kernel(MlstmArgs a) {
 // reads finished gates (two rows a load, in registers before the chain needs them) and stores the maxima four rows at a time,
 // while the others, a row a thread, store the coefficients of the rows before, form the gates of the rows after (tanh and
 // logsigmoid) and have the projections behind those on their way.  8 heads, 2048 rows / three requests of at most 1118: 42 / 22 us when the
-// walking warp did the rest too (the gates in a kernel of their own), 16 / 10 us so.
+// walking warp did the rest too (the gates in a kernel of their own), 16 / 10 us so.  A warp alone (above) where no request brings that
+// many rows, or where many requests make many blocks of one row each (see the launch).
 constexpr int GATE_ROWS = 128;
 
 __global__ void __launch_bounds__(GATE_ROWS + 32) mlstm_gates_long_kernel(MlstmArgs a) {
@@ -162,6 +163,7 @@ __global__ void __launch_bounds__(GATE_ROWS + 32) mlstm_gates_long_kernel(MlstmA
             for (int j = 0; j < STEP; ++j) now[j] = g[j];
 #pragma unroll
             for (int q = 0; q < GATE_ROWS / 2; q += STEP) {
+                if (r0 + k * GATE_ROWS + 2 * q >= r1) break;
 #pragma unroll
                 for (int j = 0; j < STEP; ++j) next[j] = g[(q + STEP + j) % (GATE_ROWS / 2)];
 #pragma unroll
@@ -469,14 +471,15 @@ struct MlstmChunks {
 };
 
 // `sums` (nullable; `chunks` * heads * (d * dv + d + 1) floats): requests of at least `least` rows run in chunks, `chunks` of
-// them at most, on the tensor cores; the others, and without it all, are walked (`walk` = 0: there are no others).
+// them at most, on the tensor cores; the others, and without it all, are walked (`walk` = 0: there are no others).  `longest`: the
+// rows of the longest request, 0 where it is not known (a choice of kernels, no result depends on it).
 // The recurrence over the step's rows: leaves the numerators o_raw [T, heads * dv], n . q in nq [T, heads], the
 // running maximum of every row in coef[.., 2] (coef: T * heads * 4 floats) and the new state.
 SHARPI_API int sharpi_mlstm_recurrence(const float* proj, int ld, int col_q, int col_k, int col_v, int col_i, int col_f,
                                        const float* bias_i, const float* bias_f, const int* row_offsets,
                                        const int* state_slots, float* state, long long state_stride, int head_stride,
                                        int B, int T, int heads, int d, int dv, float cap, float q_scale, float* coef,
-                                       float* o_raw, float* nq, float* sums, int chunks, int least,
+                                       float* o_raw, float* nq, int longest, float* sums, int chunks, int least,
                                        int walk, cudaStream_t stream) {
     if (B <= 0 || T <= 0) return SHARPI_OK;
     if (heads <= 0 || d <= 0 || dv <= 0 || d > MLSTM_MAX_D || !(cap > 0.0f)) return SHARPI_BAD_ARGUMENT;
@@ -487,7 +490,11 @@ SHARPI_API int sharpi_mlstm_recurrence(const float* proj, int ld, int col_q, int
     a.state = state; a.state_stride = state_stride; a.head_stride = head_stride; a.heads = heads; a.d = d; a.dv = dv;
     a.slices = (dv + 31) / 32; a.cap = cap; a.q_scale = q_scale; a.coef = coef; a.o_raw = o_raw; a.nq = nq; a.skip = 0x7fffffff;
     if ((long long)head_stride < (long long)a.slices * d * 32 + d + 1) return SHARPI_BAD_ARGUMENT;
-    if (T - B + 1 > 32) SHARPI_LAUNCH_PDL(mlstm_gates_long_kernel, dim3(B, heads), GATE_ROWS + 32, 0, stream, a);
+    // The long kernel's blocks are five warps, and what they gain is the longest request's.  us of the whole recurrence, one warp / five,
+    // 8 heads of 128 x 256: one request of 40 rows 11.2 / 10.9, of 120 24.2 / 22.7; 100 rows beside 63 single ones 56.7 / 54.6, 40 beside 63
+    // 36.3 / 36.0; 33, 40 and 100 beside 199 97.1 / 99.3, 98.2 / 100.3 and 114.1 / 115.2.
+    const int rows = longest > 0 ? longest : T - B + 1;
+    if (rows > 32 + (long long)B * heads / 13) SHARPI_LAUNCH_PDL(mlstm_gates_long_kernel, dim3(B, heads), GATE_ROWS + 32, 0, stream, a);
     else SHARPI_LAUNCH_PDL(mlstm_gates_kernel, dim3(B, heads), 32, 0, stream, a);
     SHARPI_CHECK_LAUNCH();
     if (sums) {

@@ -975,7 +975,7 @@ def mlstm_recurrence(proj: torch.Tensor, *, col_q: int, col_k: int, col_v: int, 
     check(kernel("sharpi_mlstm_recurrence")(proj.data_ptr(), ld, col_q, col_k, col_v, col_i, col_f, bias_i.data_ptr(),
                                             bias_f.data_ptr(), row_offsets.data_ptr(), state_slots.data_ptr(),
                                             state.data_ptr(), state.stride(0), per_head, B, T, heads, d, dv,
-                                            float(cap), float(q_scale), coef.data_ptr(), o_raw.data_ptr(), nq.data_ptr(),
+                                            float(cap), float(q_scale), coef.data_ptr(), o_raw.data_ptr(), nq.data_ptr(), int(max_rows or 0),
                                             _ptr(sums), chunks, *(_chunk_border("mlstm", T, B, max_rows, min_rows, heads) if chunks else (0, 1)), _stream()),
           "sharpi_mlstm_recurrence")
     return o_raw, nq, coef

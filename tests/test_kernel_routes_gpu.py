@@ -267,3 +267,24 @@ def test_step_sizes_of_the_selective_scan(ops, split):
                            dt_bias=torch.zeros(C, device=DEV), max_rows=T, split=split)
     want = torch.clamp(v.double(), min=0) + torch.log1p(torch.exp(-v.double().abs()))
     assert float(((y.double() / 64 - want) / want).abs().max()) < 2 * 2.0 ** -23
+
+
+def test_matrix_memory_gates_of_a_request_do_not_depend_on_its_company(ops):
+    """A request of 60 rows: its gates are walked by a warp with helpers where it is alone, by one warp beside 100 single rows."""
+    heads, d, dv, lens = 8, 32, 32, [60] + [1] * 100
+    T, ld = sum(lens), 8 * 96 + 16
+    proj, bias = rnd(T, ld, seed=1), rnd(heads, seed=2)
+    floats = ops.mlstm_state_floats(heads, d, dv)[1]
+
+    def run(n):
+        rows, state = sum(lens[:n]), torch.zeros(n, floats, device=DEV)
+        off = torch.tensor([sum(lens[:i]) for i in range(n + 1)], dtype=torch.int32, device=DEV)
+        out = ops.mlstm_recurrence(proj[:rows].contiguous(), col_q=0, col_k=heads * d, col_v=2 * heads * d, col_i=ld - 16, col_f=ld - 8,
+                                   bias_i=bias, bias_f=bias + 1.0, row_offsets=off, state_slots=torch.arange(n, dtype=torch.int32, device=DEV),
+                                   state=state, heads=heads, d=d, dv=dv, cap=15.0, q_scale=d ** -0.5, max_rows=60)
+        return (*out, state)
+    alone, beside = run(1), run(len(lens))
+    for a, b in zip(alone[:3], beside[:3]):
+        n = 3 if a is alone[2] else None                     # (a row's and head's coefficients: the fourth place is empty)
+        assert torch.equal(a[..., :n], b[:60, ..., :n])
+    assert torch.equal(alone[3][0], beside[3][0])
