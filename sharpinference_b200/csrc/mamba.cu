@@ -476,12 +476,11 @@ __global__ void __launch_bounds__(SPLIT ? 64 * (1 + SCAN_HELPERS) : 128) selecti
 }
 
 template <typename TO, int NPT, int G, bool SPLIT = false>
-static int launch_scan(ScanArgs a, int B, int T, cudaStream_t stream) {
+static int launch_scan(ScanArgs a, int B, int most, cudaStream_t stream) {
     // two walking warps a block spread a single prompt's channels evenly over the SMs; otherwise four
     const int warps = SPLIT ? 2 : 4;
     const int cpb = warps * (32 / G);
     const dim3 grid((a.C + cpb - 1) / cpb, B);
-    const int most = T - B + 1 < 1 ? 1 : T - B + 1;                  // no request brings more rows
     a.ch = most < SCAN_CH ? most : SCAN_CH;
     a.alone = most > SCAN_CH;
     const size_t smem = (size_t)(SPLIT ? 4 : 3) * a.ch * (5 * cpb + 2 * G * NPT) * sizeof(float);
@@ -502,8 +501,9 @@ static int launch_scan(ScanArgs a, int B, int T, cudaStream_t stream) {
     return SHARPI_OK;
 }
 
+// `T`: the rows to walk; `most`: a request's at most
 template <typename TO>
-static int launch_scan(const ScanArgs& a, int B, int T, int longest, cudaStream_t stream) {
+static int launch_scan(const ScanArgs& a, int B, int T, int longest, int most, cudaStream_t stream) {
     const int NP = a.N <= 4 ? 4 : a.N <= 8 ? 8 : a.N <= 16 ? 16 : a.N <= 32 ? 32 : a.N <= 64 ? 64 : a.N <= 128 ? 128 : 256;
     // Rows to walk and fewer warps (of eight states a lane) than schedulers: two states a lane.  us, two split / four / eight
     // states a lane, 4096 channels of 16 states: one prompt of 2048 rows 152 / 296 / 455; two of 1024 133 / 165 / 230; three of
@@ -515,18 +515,18 @@ static int launch_scan(const ScanArgs& a, int B, int T, int longest, cudaStream_
     // with their set-up, 1.2 us with two states a lane and 0.25 with four at 4096 channels, and a row of the longest 0.08 us less
     // with two: hence the last condition.  One prompt beside 63 single rows, two / four states a lane: 1985 rows 174 / 332,
     // 300 rows 94 / 56, 60 rows 83 / 27; 1800 rows beside 200 337 / 311; of 2048 channels 1985 rows 137 / 300, 300 rows 48 / 50.
-    const bool walk = (longest ? longest : T - B + 1) > SCAN_CH;
+    const bool walk = (longest ? longest : most) > SCAN_CH;
     const double walks = longest ? (double)T / longest : B;
     const bool few = walk && NP <= 16 && walks * a.C * NP / (8 * 32) < 4 * 148 &&
-                     (long long)(longest ? longest : T - B + 1) * 340 > (long long)a.C * B;
+                     (long long)(longest ? longest : most) * 340 > (long long)a.C * B;
     switch (NP) {
-        case 4: return few ? launch_scan<TO, 2, 2, true>(a, B, T, stream) : launch_scan<TO, 4, 1>(a, B, T, stream);
-        case 8: return few ? launch_scan<TO, 2, 4, true>(a, B, T, stream) : launch_scan<TO, 8, 1>(a, B, T, stream);
-        case 16: return few ? launch_scan<TO, 2, 8, true>(a, B, T, stream) : walk ? launch_scan<TO, 4, 4>(a, B, T, stream) : launch_scan<TO, 8, 2>(a, B, T, stream);
-        case 32: return launch_scan<TO, 8, 4>(a, B, T, stream);
-        case 64: return launch_scan<TO, 8, 8>(a, B, T, stream);
-        case 128: return launch_scan<TO, 8, 16>(a, B, T, stream);
-        default: return launch_scan<TO, 8, 32>(a, B, T, stream);
+        case 4: return few ? launch_scan<TO, 2, 2, true>(a, B, most, stream) : launch_scan<TO, 4, 1>(a, B, most, stream);
+        case 8: return few ? launch_scan<TO, 2, 4, true>(a, B, most, stream) : launch_scan<TO, 8, 1>(a, B, most, stream);
+        case 16: return few ? launch_scan<TO, 2, 8, true>(a, B, most, stream) : walk ? launch_scan<TO, 4, 4>(a, B, most, stream) : launch_scan<TO, 8, 2>(a, B, most, stream);
+        case 32: return launch_scan<TO, 8, 4>(a, B, most, stream);
+        case 64: return launch_scan<TO, 8, 8>(a, B, most, stream);
+        case 128: return launch_scan<TO, 8, 16>(a, B, most, stream);
+        default: return launch_scan<TO, 8, 32>(a, B, most, stream);
     }
 }
 
@@ -879,18 +879,21 @@ static int launch_scan_step(const ScanArgs& a, int B, cudaStream_t stream) {
 
 // `longest`: the rows of the longest request, 0 where it is not known (a choice of kernels, no result depends on it).  `work`
 // (nullable; T * C + `chunks` * C * (N + 1) floats): requests of at least `least` rows run in chunks, `chunks` of them at most; the
-// others, and without it all, are walked (`walk` = 0: there are no others).
+// others, and without it all, are walked (`walk` = 0: there are no others; `walked` rows, `longest_walked` of one request, 0 where
+// that is not known).
 SHARPI_API int sharpi_selective_scan(const float* x, const float* dtraw, const float* dt_bias, const float* bc,
                                      int ld_bc, int col_b, int col_c, const float* a_log, const float* dskip,
                                      const float* z, int ld_z, const int* row_offsets, const int* state_slots,
                                      float* state, long long state_stride, void* out, int out_dtype, int T, int B,
-                                     int C, int N, int longest, float* work, int chunks, int least, int walk, cudaStream_t stream) {
+                                     int C, int N, int longest, float* work, int chunks, int least, int walk, int walked, int longest_walked,
+                                     cudaStream_t stream) {
     if (B <= 0) return SHARPI_OK;
     if (C <= 0 || N <= 0 || N > 256) return SHARPI_BAD_ARGUMENT;
     ScanArgs a;
     a.x = x; a.dtraw = dtraw; a.dt_bias = dt_bias; a.bc = bc; a.ld_bc = ld_bc; a.col_b = col_b; a.col_c = col_c;
     a.a_log = a_log; a.dskip = dskip; a.z = z; a.ld_z = ld_z; a.row_offsets = row_offsets; a.state_slots = state_slots;
     a.state = state; a.state_stride = state_stride; a.out = out; a.C = C; a.N = N; a.skip = 0x7fffffff;
+    int most = T - B + 1 < 1 ? 1 : T - B + 1;              // no request brings more rows
     if (work) {
         if (N > 16 || chunks < 1 || chunks > 65535 || B > 65535 || least < 1) return SHARPI_BAD_ARGUMENT;
         ScanChunks q;
@@ -900,14 +903,17 @@ SHARPI_API int sharpi_selective_scan(const float* x, const float* dtraw, const f
         if (out_dtype == SHARPI_BF16) rc = launch_scan_chunks<bf16>(q, chunks, stream);
         if (rc != SHARPI_OK || !walk) return rc;
         a.skip = least;
-        if (longest >= least) longest = least - 1;
+        // The kernel for the others goes by their rows, not by the step's.  us, all walked / chunks with a walk chosen by the prompt's
+        // rows / so: 60 single rows beside a prompt of 1286, 2048 channels 94 / 98 / 73, 4096 channels 139 / 175 / 106.
+        if (walked > 0) { T = walked; longest = most = longest_walked; }
+        else if (longest >= least) longest = least - 1;
     }
     const uintptr_t bases = (uintptr_t)state | (uintptr_t)bc | (uintptr_t)a_log;
     if (T <= B && longest <= SCAN_CH && N == 16 && state_stride % 4 == 0 && ld_bc % 4 == 0 && col_b % 4 == 0 && col_c % 4 == 0 && (bases & 15) == 0) {
         if (out_dtype == SHARPI_F32) return launch_scan_step<float>(a, B, stream);
         if (out_dtype == SHARPI_BF16) return launch_scan_step<bf16>(a, B, stream);
     }
-    if (out_dtype == SHARPI_F32) return launch_scan<float>(a, B, T, longest, stream);
-    if (out_dtype == SHARPI_BF16) return launch_scan<bf16>(a, B, T, longest, stream);
+    if (out_dtype == SHARPI_F32) return launch_scan<float>(a, B, T, longest, most, stream);
+    if (out_dtype == SHARPI_BF16) return launch_scan<bf16>(a, B, T, longest, most, stream);
     return SHARPI_BAD_ARGUMENT;
 }

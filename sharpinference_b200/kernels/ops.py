@@ -7,7 +7,7 @@ is no CPU path: a tensor that is not on a CUDA device is an error.
 from __future__ import annotations
 
 import math
-from typing import Optional
+from typing import Optional, Sequence
 
 import torch
 
@@ -932,25 +932,31 @@ def _chunks(kind: str, T: int, B: int, max_rows: Optional[int], heads: int, d: i
     return chunks if max(chunks, B, heads) <= 65535 and d * dv <= 1 << 24 else 0
 
 
-def _chunk_border(kind: str, T: int, B: int, max_rows: Optional[int], min_rows: Optional[int], heads: int) -> tuple:
-    """For a step with chunks: the rows from which on a request runs so, and whether others may have rows to walk: not where the one
-    request is known to have all of the step's rows (the row count alone does not say so: rows may lie behind the last request's), nor
-    where the shortest request is known to run in chunks."""
+def _chunk_border(kind: str, T: int, B: int, max_rows: Optional[int], lengths: Optional[Sequence[int]], heads: int) -> tuple:
+    """For a step with chunks: the rows from which on a request runs so, whether others may have rows to walk, and of those the rows
+    together and the longest one's (0, 0: not known).  Without the requests' ``lengths`` the one request of a step is known to leave
+    nothing where it has all of the step's rows (the row count alone does not say so: rows may lie behind the last request's)."""
     least = chunked_least(kind, heads)
-    return least, int(not (B == 1 and max_rows == T or (min_rows or 0) >= least))
+    if not lengths:
+        return least, int(not (B == 1 and max_rows == T)), 0, 0
+    if len(lengths) != B or sum(lengths) > T:
+        raise KernelError(f"{len(lengths)} lengths of {sum(lengths)} rows together for {B} requests and {T} rows")
+    walked = [n for n in lengths if n < least]
+    return least, int(sum(walked) > 0), sum(walked), max(walked, default=0)
 
 
 def mlstm_recurrence(proj: torch.Tensor, *, col_q: int, col_k: int, col_v: int, col_i: int, col_f: int,
                      bias_i: torch.Tensor, bias_f: torch.Tensor, row_offsets: torch.Tensor, state_slots: torch.Tensor,
                      state: torch.Tensor, heads: int, d: int, dv: int, cap: float, q_scale: float, split: bool = False,
-                     max_rows: Optional[int] = None, min_rows: Optional[int] = None):
+                     max_rows: Optional[int] = None, lengths: Optional[Sequence[int]] = None):
     """The matrix-memory recurrence over the step's rows (``mlstm.cu``): reads q, k, v and the raw gates from the
     fused float32 projection ``proj [T, ld]`` at the given first columns and advances ``state [slots, floats]`` of
     the step's requests (``state_slots [B]``, rows ``row_offsets [B + 1]``).  Returns ``(num, nq, coef)``: the
     numerators ``S^T q`` float32 ``[T, heads * dv]``, ``n . q`` ``[T, heads]`` and per row and head ``(log a, log b,
     m, -)``, which :func:`mlstm_out` turns into the mixer's output.  ``split``: requests of many rows may run in chunks
     whose products are formed on the tensor cores, every float32 operand in bfloat16 pieces of 24 bits together;
-    ``max_rows``, ``min_rows``: the rows of the longest and of the shortest request, if known (no result depends on them)."""
+    ``max_rows``, ``lengths``: the rows of the longest request and of every request, on the host, if known (they choose kernels and
+    have to be true; no result depends on whether they are given)."""
     _need(proj, "proj", torch.float32)
     _need(bias_i, "bias_i", torch.float32)
     _need(bias_f, "bias_f", torch.float32)
@@ -976,7 +982,7 @@ def mlstm_recurrence(proj: torch.Tensor, *, col_q: int, col_k: int, col_v: int, 
                                             bias_f.data_ptr(), row_offsets.data_ptr(), state_slots.data_ptr(),
                                             state.data_ptr(), state.stride(0), per_head, B, T, heads, d, dv,
                                             float(cap), float(q_scale), coef.data_ptr(), o_raw.data_ptr(), nq.data_ptr(), int(max_rows or 0),
-                                            _ptr(sums), chunks, *(_chunk_border("mlstm", T, B, max_rows, min_rows, heads) if chunks else (0, 1)), _stream()),
+                                            _ptr(sums), chunks, *(_chunk_border("mlstm", T, B, max_rows, lengths, heads)[:2] if chunks else (0, 1)), _stream()),
           "sharpi_mlstm_recurrence")
     return o_raw, nq, coef
 
@@ -1191,10 +1197,10 @@ WKV_MAX_HEAD_SIZE = 256
 def wkv_recurrence(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, wraw: torch.Tensor, w0: torch.Tensor,
                    u: torch.Tensor, *, row_offsets: torch.Tensor, state_slots: torch.Tensor, state: torch.Tensor,
                    heads: int, d: int, split: bool = False, max_rows: Optional[int] = None,
-                   min_rows: Optional[int] = None) -> torch.Tensor:
+                   lengths: Optional[Sequence[int]] = None) -> torch.Tensor:
     """``o_t = (S + diag(u) k_t v_t^T)^T r_t``, ``S <- diag(exp(-exp(wraw_t + w0))) S + k_t v_t^T`` per head over
     the rows of every request, from and into ``state [slots, heads * d * d]``; float32 ``[T, heads * d]``.
-    ``wraw`` is overwritten.  ``split``, ``max_rows``, ``min_rows``: as in :func:`mlstm_recurrence` (heads of up to 64 elements)."""
+    ``wraw`` is overwritten.  ``split``, ``max_rows``, ``lengths``: as in :func:`mlstm_recurrence` (heads of up to 64 elements)."""
     for name, t in (("r", r), ("k", k), ("v", v), ("wraw", wraw), ("w0", w0), ("u", u), ("state", state)):
         _need(t, name, torch.float32)
     T = r.shape[0]
@@ -1212,7 +1218,7 @@ def wkv_recurrence(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, wraw: torc
                                           u.data_ptr(), row_offsets.data_ptr(), state_slots.data_ptr(),
                                           state.data_ptr(), state.stride(0), o.data_ptr(), bonus.data_ptr(), T,
                                           B, heads, d, _ptr(sums), chunks,
-                                          *(_chunk_border("wkv", T, B, max_rows, min_rows, heads) if chunks else (0, 1)), _stream()),
+                                          *(_chunk_border("wkv", T, B, max_rows, lengths, heads)[:2] if chunks else (0, 1)), _stream()),
           "sharpi_wkv_recurrence")
     return o
 
@@ -1277,13 +1283,13 @@ def selective_scan(x: torch.Tensor, dt: torch.Tensor, bc: torch.Tensor, col_b: i
                    col_c: int, a_log: torch.Tensor, dskip: torch.Tensor, xz: torch.Tensor, col_z: int, *,
                    row_offsets: torch.Tensor, state_slots: torch.Tensor, state: torch.Tensor,
                    out_dtype: torch.dtype, dt_bias: Optional[torch.Tensor] = None,
-                   max_rows: Optional[int] = None, split: bool = False, min_rows: Optional[int] = None) -> torch.Tensor:
+                   max_rows: Optional[int] = None, split: bool = False, lengths: Optional[Sequence[int]] = None) -> torch.Tensor:
     """The selective scan over the rows of every request from and into ``state [slots, channels * states]``:
     ``(S C + D x) * g`` in ``out_dtype``, with ``dt`` the step sizes themselves (after their softplus) and ``g`` the
     gate (already ``silu(z)``) in the columns of ``xz`` from ``col_z``, for programs that have them so.  With ``dt_bias
     [channels]``, as in the mixer, both come raw: the step sizes are ``softplus(dt + dt_bias)`` and the gate ``silu`` of
-    those columns.  ``max_rows``, ``min_rows``: the rows of the longest and of the shortest request, if known (a choice of kernels, no result depends
-    on them).  ``split``: requests of many rows may run in chunks that work side by side, from a number of rows on that the sizes fix (the
+    those columns.  ``max_rows``, ``lengths``: the rows of the longest request and of every request, on the host, if known (as in
+    :func:`mlstm_recurrence`).  ``split``: requests of many rows may run in chunks that work side by side, from a number of rows on that the sizes fix (the
     sums are then rounded in another order than the walk's)."""
     if dt_bias is not None:
         _need(dt_bias, "dt_bias", torch.float32)
@@ -1307,7 +1313,7 @@ def selective_scan(x: torch.Tensor, dt: torch.Tensor, bc: torch.Tensor, col_b: i
                                           bc.shape[1], col_b, col_c, a_log.data_ptr(), dskip.data_ptr(), z.data_ptr(),
                                           xz.shape[1], row_offsets.data_ptr(), state_slots.data_ptr(), state.data_ptr(),
                                           state.stride(0), out.data_ptr(), dtype_code(out_dtype), T, B, C, N, int(max_rows or 0),
-                                          _ptr(work), chunks, *(_chunk_border("scan", T, B, max_rows, min_rows, C) if chunks else (0, 1)),
+                                          _ptr(work), chunks, *(_chunk_border("scan", T, B, max_rows, lengths, C) if chunks else (0, 1, 0, 0)),
                                           _stream()), "sharpi_selective_scan")
     return out
 
@@ -1513,11 +1519,11 @@ SSD_MAX_STATES = 256
 def ssd_scan(xbc: torch.Tensor, proj: torch.Tensor, *, col_x: int, col_b: int, col_c: int, col_dt: int,
              dt_bias: torch.Tensor, a_log: torch.Tensor, dskip: torch.Tensor, row_offsets: torch.Tensor,
              state_slots: torch.Tensor, state: torch.Tensor, heads: int, groups: int, states: int, vdim: int,
-             split: bool = False, max_rows: Optional[int] = None, min_rows: Optional[int] = None) -> torch.Tensor:
+             split: bool = False, max_rows: Optional[int] = None, lengths: Optional[Sequence[int]] = None) -> torch.Tensor:
     """The state-space-duality recurrence over the rows of every request, from and into ``state [slots, heads *
     states * vdim]``: ``y`` float32 ``[T, heads * vdim]``.  ``xbc`` float32 holds x, B and C at the given columns,
     ``proj`` float32 the raw step sizes at ``col_dt``; ``dt = softplus(raw + dt_bias)``, decay ``exp(-exp(A_log) dt)``.
-    ``split``, ``max_rows``, ``min_rows``: as in :func:`mlstm_recurrence`."""
+    ``split``, ``max_rows``, ``lengths``: as in :func:`mlstm_recurrence`."""
     for name, t in (("xbc", xbc), ("proj", proj), ("dt_bias", dt_bias), ("a_log", a_log), ("dskip", dskip), ("state", state)):
         _need(t, name, torch.float32)
     T = xbc.shape[0]
@@ -1532,7 +1538,7 @@ def ssd_scan(xbc: torch.Tensor, proj: torch.Tensor, *, col_x: int, col_b: int, c
                                     dt_bias.data_ptr(), a_log.data_ptr(), dskip.data_ptr(), row_offsets.data_ptr(),
                                     state_slots.data_ptr(), state.data_ptr(), state.stride(0), y.data_ptr(), T,
                                     B, heads, groups, states, vdim, _ptr(sums), chunks,
-                                    *(_chunk_border("ssd", T, B, max_rows, min_rows, heads) if chunks else (0, 1)), _stream()),
+                                    *(_chunk_border("ssd", T, B, max_rows, lengths, heads)[:2] if chunks else (0, 1)), _stream()),
           "sharpi_ssd_scan")
     return y
 

@@ -72,7 +72,7 @@ class SelectiveScanMixer(Mixer):
         y = ops.selective_scan(x32, dt, dbc, self.dt_rank, self.dt_rank + self.states, self.a_log,
                                self.d_skip, xz, self.inner, row_offsets=ctx.row_offsets, state_slots=ctx.state_slots,
                                state=slot.states["S"], out_dtype=self.act_dtype, dt_bias=self.dt_bias,
-                               max_rows=ctx.max_rows_per_request, min_rows=min(ctx.host_lengths, default=0), split=self.act_dtype == torch.bfloat16)
+                               max_rows=ctx.max_rows_per_request, lengths=ctx.host_lengths, split=self.act_dtype == torch.bfloat16)
         return self.out(y)
 
 
@@ -118,7 +118,7 @@ class StateSpaceDualityMixer(Mixer):
                          col_dt=self.channels + self.inner, dt_bias=self.dt_bias, a_log=self.a_log, dskip=self.d_skip,
                          row_offsets=ctx.row_offsets, state_slots=ctx.state_slots, state=slot.states["S"],
                          heads=self.heads, groups=self.groups, states=self.states, vdim=self.value_dim,
-                         split=self.act_dtype == torch.bfloat16, max_rows=ctx.max_rows_per_request, min_rows=min(ctx.host_lengths, default=0))
+                         split=self.act_dtype == torch.bfloat16, max_rows=ctx.max_rows_per_request, lengths=ctx.host_lengths)
         u = ops.gated_group_norm(y, proj, self.channels, self.norm_weight, self.eps, self.norm_groups, self.act_dtype)
         return self.out(u)
 

@@ -81,7 +81,7 @@ class MLSTMMixer(Mixer):
             p, col_q=self.col_q, col_k=self.col_k, col_v=self.col_v, col_i=self.col_i, col_f=self.col_f,
             bias_i=self.bias_i, bias_f=self.bias_f, row_offsets=ctx.row_offsets, state_slots=ctx.state_slots,
             state=slot.state, heads=self.heads, d=self.key_dim, dv=self.value_dim, cap=self.gate_cap,
-            q_scale=self.q_scale, split=self.act_dtype == torch.bfloat16, max_rows=ctx.max_rows_per_request, min_rows=min(ctx.host_lengths, default=0))
+            q_scale=self.q_scale, split=self.act_dtype == torch.bfloat16, max_rows=ctx.max_rows_per_request, lengths=ctx.host_lengths)
         o = ops.mlstm_out(num, nq, coef, p, self.col_g, self.head_norm_weight, self.eps, self.heads, self.value_dim,
                           self.act_dtype)
         return self.out(o)

@@ -92,5 +92,5 @@ class WKVMixer(Mixer):
         wraw = self.w2(ops.tanh(self.w1(mixes[4]), self.act_dtype))
         o = ops.wkv_recurrence(r, k, v, wraw, self.w0, self.u, row_offsets=ctx.row_offsets,
                                state_slots=ctx.state_slots, state=slot.states["S"], heads=self.heads, d=self.head_dim,
-                               split=self.act_dtype == torch.bfloat16, max_rows=ctx.max_rows_per_request, min_rows=min(ctx.host_lengths, default=0))
+                               split=self.act_dtype == torch.bfloat16, max_rows=ctx.max_rows_per_request, lengths=ctx.host_lengths)
         return self.out(ops.wkv_out(o, g, self.head_norm_weight, self.eps, self.heads, self.head_dim, self.act_dtype))

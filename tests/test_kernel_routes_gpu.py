@@ -288,3 +288,40 @@ def test_matrix_memory_gates_of_a_request_do_not_depend_on_its_company(ops):
         n = 3 if a is alone[2] else None                     # (a row's and head's coefficients: the fourth place is empty)
         assert torch.equal(a[..., :n], b[:60, ..., :n])
     assert torch.equal(alone[3][0], beside[3][0])
+
+
+# requests with a row less than the border between walk and chunks, that many and one more, beside single rows and short prompts
+@pytest.mark.parametrize("kind", ["mlstm", "ssd", "wkv", "scan"])
+@pytest.mark.parametrize("over", [[0, 0], [1, 0, None], [-1, 0], [-1, 1, None, None], [5, -1000]])
+def test_recurrences_with_the_lengths_known(ops, monkeypatch, kind, over):
+    """What the host knows of the requests' rows chooses kernels (none behind the chunks, the single rows' one, a walk) and no bit."""
+    from sharpinference_b200.parts.mlstm import fused_mlstm_columns
+    monkeypatch.setattr(ops, "_WALK_OR_CHUNKS", dict.fromkeys(ops._WALK_OR_CHUNKS, (1.0, 150, 0.0)))
+    heads, d, dv, C, N = 2, 32, 32, 64, 16
+    least = ops.chunked_least(kind, heads)
+    lens = [1 if o is None else max(least + o, 3) for o in over]
+    B, T, hd = len(lens), sum(lens), heads * d
+    ins, vec = [rnd(T, hd, seed=i) for i in range(4)], [rnd(hd, scale=0.3, seed=9 + i) for i in range(3)]
+    xbc, dt = rnd(T, heads * dv + 2 * d, scale=0.5, seed=7), rnd(T, C, seed=8)
+    cols = fused_mlstm_columns(heads, d, dv)
+    proj, bc, a_log = rnd(T, cols[-1], seed=6), rnd(T, 2 * N, seed=5), rnd(C, N, seed=4)
+    floats = {"mlstm": ops.mlstm_state_floats(heads, d, dv)[1], "scan": C * N}.get(kind, heads * d * dv)
+
+    def run(lengths):
+        state = torch.zeros(B, floats, device=DEV)
+        kw = dict(row_offsets=torch.tensor([sum(lens[:i]) for i in range(B + 1)], dtype=torch.int32, device=DEV), state=state,
+                  state_slots=torch.arange(B, dtype=torch.int32, device=DEV), split=True, max_rows=max(lens), lengths=lengths)
+        if kind == "scan":
+            return ops.selective_scan(ins[0], dt, bc, 0, N, a_log, vec[0], ins[1], 0, out_dtype=torch.float32, dt_bias=vec[1], **kw), state
+        kw["heads"] = heads
+        if kind == "wkv":
+            r, k, v, w = (x.clone() for x in ins)
+            return ops.wkv_recurrence(r, k, v, w, vec[0], vec[1], d=d, **kw), state
+        if kind == "ssd":
+            return ops.ssd_scan(xbc, dt, col_x=0, col_b=heads * dv, col_c=heads * dv + d, col_dt=0, dt_bias=vec[0], a_log=vec[1],
+                                dskip=vec[2], groups=1, states=d, vdim=dv, **kw), state
+        return ops.mlstm_recurrence(proj, col_q=cols[0], col_k=cols[1], col_v=cols[2], col_i=cols[4], col_f=cols[5], bias_i=vec[0],
+                                    bias_f=vec[1], d=d, dv=dv, cap=15.0, q_scale=d ** -0.5, **kw)[0], state
+    assert max(lens) >= least
+    for got, want in zip(run(lens), run(None)):
+        assert torch.equal(got, want) and bool(torch.isfinite(got).all())

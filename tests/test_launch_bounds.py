@@ -1,6 +1,8 @@
 """Host-side bounds that size kernel launches: they must never be below what the kernels will need (no GPU)."""
 import random
 
+import pytest
+
 from sharpinference_b200.kernels import ops
 
 
@@ -91,6 +93,27 @@ def test_chunk_bounds_hold_for_drawn_steps():
             got = ops._chunks(kind, sum(lens), len(lens), known, heads, 64, 64)
             assert got >= need, (kind, heads, lens)
             assert known is None or (got > 0) == (max(lens) >= least)
+
+
+def test_what_is_walked_behind_the_chunks():
+    """Whether a step with chunks leaves requests to walk, their rows and the longest one's: from the lengths, and without them safely."""
+    r = random.Random(2)
+    for _ in range(2000):
+        kind, heads = r.choice(["mlstm", "ssd", "wkv", "scan"]), r.choice([1, 8, 64, 1000, 4096, 20000])
+        least = ops.chunked_least(kind, heads)
+        assert least >= ops.CHUNKED_LEAST
+        lens = [r.choice([1, r.randint(1, 300), least - 1, least, least + 1]) for _ in range(r.randint(1, 8))]
+        T = sum(lens) + r.choice([0, 0, 5])                   # rows may lie behind the last request's
+        if max(lens) < least:
+            continue                                          # no chunks
+        rest = [n for n in lens if n < least]
+        assert ops._chunk_border(kind, T, len(lens), max(lens), lens, heads) == (least, int(bool(rest)), sum(rest), max(rest, default=0))
+        for known in (None, max(lens)):
+            unknown = ops._chunk_border(kind, T, len(lens), known, None, heads)
+            assert unknown[0] == least and unknown[1] >= int(bool(rest)) and unknown[2:] == (0, 0)
+    for wrong in ([2000], [2000, 2000], [1, 1, 1]):
+        with pytest.raises(ops.KernelError):
+            ops._chunk_border("ssd", 3000, 2, 2000, wrong, 8)
 
 
 def test_chunk_kernels_are_left_alone_beyond_their_sizes():
