@@ -907,16 +907,25 @@ CHUNKED_LEAST = 128
 #   wkv   32 heads of 64        33 / 27, 63 / 28, 390 / 120;  40 / 70, 77 / 138, 134 / 135
 #         16 heads of 64        33 / 27, 61 / 27, 367 / 62;   36 / 39, 68 / 68, 124 / 67
 #         64 heads of 64        35 / 28, 64 / 31, 488 / 209;  80 / 144, 163 / 257, 160 / 252
-#   scan  4096 channels of 16   250 rows 24 / 30, 400 35 / 41, 2048 155 / 111; 2048 channels 19 / 29, -, 121 / 70; 1117, 558 and 372 rows of
-#         4096 in a step 120 / 120, 576, 288, 192 and 144 rows 73 / 107: the walk takes several requests side by side, and one that
-#         runs in chunks has what is left walked behind it, so s is such that the request's gain pays for a walk of half its rows
-_WALK_OR_CHUNKS = {"mlstm": (0.16, 30, 0.0), "ssd": (0.32, 30, 0.0), "wkv": (0.21, 15, 0.8), "scan": (0.028, 36, 0.0)}
+# The scan's walk takes requests side by side, and what runs in chunks has the others walked behind it: its border, given as such (w = 1;
+# heads: the channels, up to 8192 of which were measured), is where a step of 2048 rows with a second prompt in the rows that are left
+# loses next to nothing (6144 channels lose 31 us of 180 with 1400 and 648 rows), not where a request alone gains.
+# us, walked / in chunks, 16 states a channel; one request of 1286, 1500, 2048 rows; 1286 and 762, 1500 and 548, 1700 and 348 in a step:
+#   scan   512 channels         71 / 42, 82 / 55, 109 / 62;  71 / 86, 82 / 82, 92 / 79
+#         1024                  71 / 65, 82 / 66, 110 / 75;  76 / 109, 85 / 98, 94 / 87
+#         2048                  78 / 79, 90 / 75, 120 / 79;  91 / 120, 101 / 108, 112 / 101
+#         4096                  99 / 84, 116 / 88, 154 / 112;  131 / 144, 146 / 134, 158 / 131
+#         6144                  138 / 111, 159 / 124, 212 / 161;  227 / 218, 191 / 204, 206 / 191
+#         1286 beside 60 single rows 82 / 44, 95 / 73, 139 / 106 with 1024, 2048, 4096 channels; four, eight, sixteen of 2048, 4096
+#         channels 438 / 377, 793 / 719, 1357 / 1408; 2048 and 1024 in a step 115 / 125, 138 / 150, 199 / 192 with 1024, 2048, 4096 channels
+_WALK_OR_CHUNKS = {"mlstm": (0.16, 30, 0.0), "ssd": (0.32, 30, 0.0), "wkv": (0.21, 15, 0.8), "scan": (1.0, 1650, -0.06)}
 
 
 def chunked_least(kind: str, heads: int) -> int:
-    """The rows from which on a request's recurrence (``mlstm``, ``ssd``, ``wkv``) runs in chunks where a caller allows it."""
+    """The rows from which on a request's recurrence (``mlstm``, ``ssd``, ``wkv``; ``scan``, with its channels as ``heads``) runs in chunks
+    where a caller allows it."""
     w, s, c = _WALK_OR_CHUNKS[kind]
-    return max(CHUNKED_LEAST, math.ceil((s + c * heads) / w))
+    return max(CHUNKED_LEAST, math.ceil((s + c * min(heads, 8192)) / w))
 
 
 def _chunks(kind: str, T: int, B: int, max_rows: Optional[int], heads: int, d: int, dv: int, *aligned: int, size: int = 64) -> int:

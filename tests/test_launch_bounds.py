@@ -95,6 +95,14 @@ def test_chunk_bounds_hold_for_drawn_steps():
             assert known is None or (got > 0) == (max(lens) >= least)
 
 
+@pytest.mark.parametrize("channels,alone,shared", [(512, 1700, 1500), (1024, 1700, 1500), (2048, 1700, 1500), (4096, 1500, 1300),
+                                                    (8192, 1286, 1000)])
+def test_the_scans_border_follows_the_channels(channels, alone, shared):
+    """A request that gains in chunks beside what a step of 2048 rows has left for another one, and one that loses there."""
+    assert shared < ops.chunked_least("scan", channels) <= alone
+    assert ops.chunked_least("scan", 1 << 16) == ops.chunked_least("scan", 8192) > ops.CHUNKED_LEAST
+
+
 def test_what_is_walked_behind_the_chunks():
     """Whether a step with chunks leaves requests to walk, their rows and the longest one's: from the lengths, and without them safely."""
     r = random.Random(2)
