@@ -45,8 +45,8 @@ class WKVMixer(Mixer):
                  head_dim: int, eps: float, act_dtype: torch.dtype = torch.bfloat16,
                  rkvg_weight: torch.Tensor = None):
         """``mu [5, H]``: the mixing vectors of r, k, v, g, w in this order.  ``rkvg_weight [4, heads * head_dim, H]``:
-        the weights of r, k, v, g stacked (the four ``Linear`` may be views of it), for the grouped product of
-        small steps; None: four products at every size."""
+        the weights of r, k, v, g stacked, for the grouped product of small steps and, while the four ``Linear`` are views of
+        it, for the batched product of larger ones; None: four products at every size."""
         hd = heads * head_dim
         H = r.in_features
         if head_dim > ops.WKV_MAX_HEAD_SIZE:
@@ -68,10 +68,18 @@ class WKVMixer(Mixer):
         if (rkvg_weight is not None and rkvg_weight.dtype == torch.bfloat16 and act_dtype == torch.bfloat16
                 and H % 8 == 0 and tuple(rkvg_weight.shape) == (4, hd, H)):
             self.rkvg_weight = rkvg_weight
-        self._batched = self.rkvg_weight is not None and all(lin.bias is None for lin in (r, k, v, g))
         self._group_offsets = {}
         self.state_specs = {"prev": StateSpec((H,), torch.float32),
                             "S": StateSpec((heads * head_dim * head_dim,), torch.float32)}
+
+    def _stacked(self) -> bool:
+        """Whether r, k, v and g are, now, nothing but products with their parts of the stacked weight (a program may have put
+        others in their places since)."""
+        w = self.rkvg_weight
+        return w is not None and all(
+            type(lin) is Linear and lin.bias is None and lin.weight.dtype == w.dtype and lin.weight.shape == w.shape[1:]
+            and lin.weight.stride() == w.stride()[1:] and lin.weight.data_ptr() == w.data_ptr() + i * w.stride(0) * w.element_size()
+            for i, lin in enumerate((self.r, self.k, self.v, self.g)))
 
     def forward(self, ctx: StepContext, slot: LayerSlot, h: torch.Tensor) -> torch.Tensor:
         mixes = ops.token_shift(h, self.mu, slot.states["prev"], row_request=ctx.row_request,
@@ -85,7 +93,7 @@ class WKVMixer(Mixer):
                 offsets = self._group_offsets[T] = torch.arange(5, dtype=torch.int32, device=h.device) * T
             r, k, v, g = ops.tc_grouped_gemm(mixes[:4].view(4 * T, -1), self.rkvg_weight, offsets,
                                              mode=ops.TC_MODE_STORE).view(4, T, -1).unbind(0)
-        elif self._batched:                              # the library's batched product: one grid for the four (2048 rows 74 -> 58 us)
+        elif self._stacked():                           # the library's batched product: one grid for the four (2048 rows 74 -> 58 us)
             r, k, v, g = torch.bmm(mixes[:4], self.rkvg_weight.transpose(1, 2), out_dtype=torch.float32).unbind(0)
         else:
             r, k, v, g = self.r(mixes[0]), self.k(mixes[1]), self.v(mixes[2]), self.g(mixes[3])

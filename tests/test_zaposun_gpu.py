@@ -160,6 +160,32 @@ def test_small_and_large_steps_give_the_same_bits():
     assert torch.equal(st_a[0], h[-1]) and torch.equal(st_b[0], h[19])
 
 
+@pytest.mark.parametrize("rows", [129, 300])
+def test_projections_that_were_replaced_are_the_ones_in_use(rows):
+    """r, k, v and g of a mixer with stacked weights, one of them replaced, given a bias or a weight elsewhere after construction: larger
+    steps multiply with what is there now."""
+    from types import SimpleNamespace
+    from sharpinference_b200.parts import Linear, WKVMixer
+    g = torch.Generator().manual_seed(3)
+    H, heads, d = 64, 2, 32
+    mat = lambda *shape: (torch.randn(*shape, generator=g) * 0.2).bfloat16().to(DEV)
+    vec = lambda *shape: torch.randn(*shape, generator=g).to(DEV)
+    stacked, other, bias = mat(4, heads * d, H), mat(heads * d, H), vec(heads * d)
+    shared = dict(mu=torch.rand(5, H, generator=g).to(DEV), w1=Linear(mat(16, H)), w2=Linear(mat(heads * d, 16)), w0=vec(heads * d),
+                  u=vec(heads * d), head_norm_weight=vec(heads * d), out=Linear(mat(H, heads * d)), heads=heads, head_dim=d, eps=1e-5)
+    h = torch.randn(rows, H, generator=g).to(DEV)
+    rr, off, sl = _step_meta([rows], [0])
+    ctx = SimpleNamespace(row_request=rr, row_offsets=off, state_slots=sl, max_rows_per_request=rows, host_lengths=[rows])
+
+    def run(stack, name, lin):
+        m = WKVMixer(**dict(zip("rkvg", (Linear(w) for w in stacked))), rkvg_weight=stacked if stack else None, **shared)
+        setattr(m, name, lin)
+        state = {"prev": torch.zeros(1, H, device=DEV), "S": torch.zeros(1, heads * d * d, device=DEV)}
+        return m.forward(ctx, SimpleNamespace(states=state), h)
+    for name, lin in (("r", Linear(other)), ("g", Linear(stacked[3], bias=bias)), ("v", Linear(stacked[1])), ("k", Linear(stacked[1].clone()))):
+        assert torch.equal(run(True, name, lin), run(False, name, lin)), name
+
+
 @pytest.mark.parametrize("T,heads,d", [(1, 1, 64), (37, 3, 64), (5, 2, 128), (600, 1, 64), (5, 2, 60)])
 def test_wkv_out_sixteen_bytes_a_lane(T, heads, d):
     """Heads of 64 and 128 elements have a kernel of their own, whose last block may be part empty; 60 keeps the general one."""
