@@ -100,10 +100,10 @@ __device__ __forceinline__ int chunks_before(const int* row_offsets, int b, int 
 }
 
 // R x C floats (C a power of two; those with r < rows and c < cols, zeros elsewhere) as three planes of bfloat16 pieces,
-// rows C + 8 apart (neighbouring rows start in other banks); row r times f[r] where `f` is given.  All of a thread's loads
-// are under way before the first is split.  Returns whether all that this thread loaded is finite.
+// rows C + 8 apart (neighbouring rows start in other banks).  All of a thread's loads are under way before the first is
+// split.  Returns whether all that this thread loaded is finite.
 template <int R, int C>
-__device__ __forceinline__ bool load_split(bf16* dst, const float* src, size_t ld, int rows, int cols, const float* f) {
+__device__ __forceinline__ bool load_split(bf16* dst, const float* src, size_t ld, int rows, int cols) {
     constexpr int LD = C + 8, PLANE = R * LD, N = R * C / 4 / THREADS;
     float4 x[N];
 #pragma unroll
@@ -116,10 +116,6 @@ __device__ __forceinline__ bool load_split(bf16* dst, const float* src, size_t l
     for (int p = 0; p < N; ++p) {
         const int i = threadIdx.x + p * THREADS, r = i / (C / 4), e = (i % (C / 4)) * 4;
         zero = fmaf(x[p].x, 0.0f, fmaf(x[p].y, 0.0f, fmaf(x[p].z, 0.0f, fmaf(x[p].w, 0.0f, zero))));
-        if (f) {
-            const float s = f[r];
-            x[p].x *= s; x[p].y *= s; x[p].z *= s; x[p].w *= s;
-        }
         const mma16::Pieces lo = mma16::split3(x[p].x, x[p].y), hi = mma16::split3(x[p].z, x[p].w);
 #pragma unroll
         for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(dst + q * PLANE + r * LD + e) = make_uint2(lo.v[q], hi.v[q]);
@@ -236,7 +232,8 @@ __device__ __forceinline__ void load_decays(const F& f, const Place& p, int h, f
 
 // In the first two warps, a row a thread: b of the row times the decays behind it in its block of 16 rows, and every block's decay.
 // With them D_ij of rows in different blocks is three factors: the decays up to i in its block, those of the blocks between, and
-// this.  (All factors are at most 1, so none is zero where their product is not.)
+// this.  (The decays are at most 1, so a product of some is not zero where that of all is not; b may be larger than 1 and joins the
+// decays behind it in one product, which is zero where it falls below float32's least number.)
 __device__ __forceinline__ void block_tails(float al, float be, float* tail_s, float* block_s) {
     const int l = threadIdx.x % BLOCK;
     float z = al;
@@ -274,7 +271,7 @@ __global__ void __launch_bounds__(THREADS, 2) sums_kernel(Args a, F f) {
     float al = 1.0f, be = 0.0f;
     fetch(first);
     if (warp < 2) load_decays(f, p, kh * per + first / tiles, al, be);
-    load_split<ROWS, DP>(k_s, keys, a.ld_k, p.rows, a.d, nullptr);
+    load_split<ROWS, DP>(k_s, keys, a.ld_k, p.rows, a.d);
     __syncthreads();
     uint32_t x[MT][4][3][4];
 #pragma unroll
@@ -420,7 +417,7 @@ __global__ void __launch_bounds__(THREADS, 2) outs_kernel(Args a, F f) {
     float al = 1.0f, be = 0.0f;
     fetch_values(first);
     if (warp < 2) load_decays(f, p, kh * per + first / tiles, al, be);
-    load_split<ROWS, DP>(k_s, a.k + (size_t)p.row0 * a.ld_k + (size_t)kh * a.d, a.ld_k, p.rows, a.d, nullptr);
+    load_split<ROWS, DP>(k_s, a.k + (size_t)p.row0 * a.ld_k + (size_t)kh * a.d, a.ld_k, p.rows, a.d);
     uint32_t x[KT][3][4];
 #pragma unroll
     for (int kk = 0; kk < KT; ++kk)
@@ -467,7 +464,7 @@ __global__ void __launch_bounds__(THREADS, 2) outs_kernel(Args a, F f) {
         const float* values = a.v + (size_t)p.row0 * a.ld_v + (size_t)h * a.dv + c0;
         mma16::cp_async_wait_all();
         __syncthreads();                                       // the keys, or the tile before: done with
-        load_split<DP, COLS>(k_s, a.sums + head * a.d * a.dv + c0, a.dv, a.d, a.dv - c0, nullptr);
+        load_split<DP, COLS>(k_s, a.sums + head * a.d * a.dv + c0, a.dv, a.d, a.dv - c0);
         const bool odd = __syncthreads_or(!split_raw<ROWS, COLS>(v_s, raw, [](int, int) { return 1.0f; }));
         if (h != have && warp < 2) {
             const int l = lane % BLOCK;

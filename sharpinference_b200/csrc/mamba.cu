@@ -14,8 +14,10 @@
 //                        all in float32 (exp(dt A) as exp2 of dt A log2(e)); or with dt before bias and softplus and z
 //                        before its silu, which the walk's warps then apply to every element once.  A group of lanes owns
 //                        one channel, a lane two states in registers; the sum over the states is a fixed tree of exchanges,
-//                        and the walk over a request's rows is sequential, so a row's result does not depend on how
-//                        the prompt was cut or batched.
+//                        and the walk over a request's rows is sequential, so a walked row's result does not depend on how
+//                        the prompt was cut or batched.  A portion of many rows may run in chunks instead (further down), whose
+//                        sums are rounded in another order: its rows do not depend on the rest of the step either, but they are
+//                        not the bits of the same prompt in shorter portions.
 #include "common.cuh"
 #include "chunk_mma.cuh"
 
@@ -814,7 +816,7 @@ static int launch_scan_chunks(const ScanChunks& q, int chunks, cudaStream_t stre
 // channel needs once a row (step size, gate, output) is formed by one of the four.  The operations of a channel and their order
 // are the walk's.  4096 channels: 200 requests 48 us with the walk (its blocks stage, prepare and meet for one row), 21 us so
 // (31 where every lane formed all of its channels' step sizes); 20 requests 8.4 and 4.1.  Two or four requests a warp, for one
-// set of decay rates: 22 us.
+// set of decay rates: 22 us.  Four lanes of four states make 16, the usual count; others stay with the walk.
 constexpr int SS_THREADS = 128;
 
 template <typename TO, bool RAW>

@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(WC_THREADS, 3) wkv_sums_kernel(WkvChunkArgs a)
     if (!chunked::find_chunk(a.row_offsets, a.B, a.least, blockIdx.y, p)) return;
     const int head = blockIdx.x, d = a.d, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const size_t hd = (size_t)a.heads * d, at0 = (size_t)p.row0 * hd + (size_t)head * d;
-    chunked::load_split<chunked::ROWS, WC_D>(v_s, a.v + at0, hd, p.rows, d, nullptr);
+    chunked::load_split<chunked::ROWS, WC_D>(v_s, a.v + at0, hd, p.rows, d);
     {
         constexpr int HALF = chunked::ROWS / 2;
         const int c = threadIdx.x % WC_D, half = threadIdx.x / WC_D;
@@ -479,7 +479,7 @@ __global__ void __launch_bounds__(WC_THREADS, 2) wkv_outs_kernel(WkvChunkArgs a)
                 k[i][e] = ok ? a.k[at] : 0.0f;
                 w[i][e] = ok ? a.w[at] : 1.0f;
             }
-        finite = chunked::load_split<chunked::ROWS, WC_D>(v_s, a.v + at0, hd, p.rows, d, nullptr);
+        finite = chunked::load_split<chunked::ROWS, WC_D>(v_s, a.v + at0, hd, p.rows, d);
         // columns s and s + 1 of the block's A: a lane's channels down the rows, then lane 16 e + t has A of row t, column s + e
 #pragma unroll
         for (int s = 0; s < 16; s += 2) {
@@ -576,7 +576,7 @@ __global__ void __launch_bounds__(WC_THREADS, 2) wkv_outs_kernel(WkvChunkArgs a)
         chunked::add_small(score[J], few);
     }
     __syncthreads();                                           // the keys are free
-    chunked::load_split<WC_D, WC_D>(k_s, a.sums + ((size_t)blockIdx.y * a.heads + head) * d * d, d, d, d, nullptr);
+    chunked::load_split<WC_D, WC_D>(k_s, a.sums + ((size_t)blockIdx.y * a.heads + head) * d * d, d, d, d);
     __syncthreads();
     float acc[8][4], small[8][4];
     chunked::clear(acc);

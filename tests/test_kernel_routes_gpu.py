@@ -238,8 +238,8 @@ def test_matrix_memory_step_is_the_walk(ops, d, dv):
     want = run(proj, first * rows, slots, whole)
     for r in range(rows):
         at = torch.arange(B, device=DEV) * rows + r
-        for g, w in zip(run(proj[at], first, slots, single), want):
-            assert torch.equal(g[..., :3], w[at][..., :3]), r
+        (num, nq, coef), (num_w, nq_w, coef_w) = run(proj[at], first, slots, single), want
+        assert torch.equal(num, num_w[at]) and torch.equal(nq, nq_w[at]) and torch.equal(coef[..., :3], coef_w[at][..., :3]), r
     assert torch.equal(single, whole)
     # as many rows as requests, dealt otherwise: one request has two, another none
     off = torch.tensor([0, 2, 2, 3, 4, 5], dtype=torch.int32, device=DEV)
