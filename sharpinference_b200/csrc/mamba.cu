@@ -541,7 +541,7 @@ static int launch_scan(const ScanArgs& a, int B, int T, int longest, int most, c
 // A lane is a channel with all its states, two of them an instruction (f32x2); nothing is exchanged between lanes, a row's B and C are
 // read by all lanes of a warp at once, and a lane's own numbers of the next rows are on their way into shared memory, where it alone
 // reads them.  The exponentials are formed twice, and still the walk, whose rows follow one another, is the slower form for one long
-// prompt (us, walked / in chunks, 16 states: 2048 rows of 4096 channels 155 / 111, of 2048 channels 121 / 70; 400 rows of 4096
+// prompt (us, walked / in chunks, 16 states: 2048 rows of 4096 channels 154 / 112, of 2048 channels 120 / 79; 400 rows of 4096
 // channels 35 / 41).  Bound by the special-function unit (two thirds busy: 36 operations a row and channel) and the last wave;
 // an eighth to a half of the exponentials as polynomials on the multiply-add pipe instead were slower (115 to 135 us).
 // -------------------------------------------------------------------------------------------------------------

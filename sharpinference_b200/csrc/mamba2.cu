@@ -191,8 +191,7 @@ static int ssd_launch(const SsdArgs& a, dim3 grid, cudaStream_t stream) {
 // Steps that bring about a row a request: the state's bytes, read and written once.  A thread has four neighbouring value columns
 // of the states that a lane of the walk has (a row of 64 columns is 256 contiguous bytes of sixteen threads, where the walk's lanes
 // take 16 bytes of eight rows each), all of them on their way at once.  The operations of a column and their order are the walk's.
-// 64 heads of 128 x 64, the mixer's step: 200 requests
-// 333 us walked, 180 us so; 40 requests 88 and 58; 8 requests 36 and 29.
+// 64 heads of 128 x 64: 200 requests 287 us walked, 141 us so (the mixer's step 333 and 180); 40 requests 56 and 25; 8 requests 14 and 6.
 constexpr int STEP_LANES = SSD_LANES, STEP_COLS = 64, STEP_THREADS = STEP_LANES * STEP_COLS / 4;
 
 template <int NPL>
